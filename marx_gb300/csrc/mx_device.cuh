@@ -305,7 +305,7 @@ MXD double rcp_fast(double d) {
 // last ones are summed in single precision where their size keeps the
 // rounding below 2^-48.  The result is within 2^-44 of the true sine or
 // cosine of the double argument.
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
 struct F2 { float h, l; };
 __device__ __forceinline__ F2 quick_sum(float a, float b) {   // |a| >= |b|
   const float s = __fadd_rn(a, b);
