@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
   const size_t n = io.stride;   // component stride of the 3-vector columns
   const uint32_t lane = threadIdx.x & 31;
 
-  // Phase A: generation, dither, aperture, paraboloid intersection.
+  // Phase A: generation, dither, aperture.
   for (;;) {
     const uint32_t base = claim(&b.ctr[2], b.tile);
     if (base >= io.n) break;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
     for (uint32_t j = base; j < end; j += 32) {
       const uint32_t i = j + lane;
       bool keep = false;
-      MxRec rec;
+      MxRecA rec;
       if (i < end) {
         const int s = source_of(i, sstart, b.nsrc);
         Ph q;
@@ -250,18 +250,18 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
         if (T.dither) dither_stage(T, q, r);
         if (io.dith) for (int k = 0; k < 3; k++) io.dith[k * n + i] = q.dith[k];
         MirrorState m;
-        if (mirror_front(T, sh, optc, slope, q, r, m)) {
+        if (mirror_front(T, sh, q, r, m)) {
           keep = true;
-          to_rec(rec, q, m, r, i);
+          to_rec_a(rec, q, m, r, i);
         } else
           store_core(io, i, q, r.overrun);
       }
-      append(keep, rec, b.q1, &b.ctr[0]);
+      append(keep, rec, (MxRecA *) b.q1, &b.ctr[0]);
     }
   }
   grid.sync();
 
-  // Phase T: the paraboloid's normal blur and reflectivity test.
+  // Phase T: the paraboloid's intersection, normal blur and reflectivity test.
   const uint32_t nt = __ldcg(&b.ctr[0]);
   for (;;) {
     const uint32_t base = claim(&b.ctr[6], b.tile);
@@ -272,14 +272,14 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
       bool keep = false;
       MxRec rec;
       if (k < end) {
-        rec = b.q1[k];
         Ph q; MirrorState m; Rng r;
-        from_rec(rec, q, m, r, io);
-        if (mirror_ptest(T, sh, q, r, m)) {
+        const MxRecA rec_in = ((const MxRecA *) b.q1)[k];
+        from_rec_a(rec_in, q, m, r, io);
+        if (mirror_ptest(T, sh, optc, slope, q, r, m)) {
           keep = true;
-          to_rec(rec, q, m, r, rec.i);
+          to_rec(rec, q, m, r, r.i);
         } else
-          store_core(io, rec.i, q, r.overrun);
+          store_core(io, r.i, q, r.overrun);
       }
       append(keep, rec, b.q2, &b.ctr[1]);
     }

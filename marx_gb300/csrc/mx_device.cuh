@@ -1032,8 +1032,9 @@ MXD bool cap_struts_block(const MxTables &T, const MxShellDev &h, D3 x, D3 p) {
   return struts_block_exact(T, 1, x, p);
 }
 
-// Mirror state carried between the three parts of the HRMA trace: the
-// photon at a conic intersection (OSAC frame of that optic) that passed
+// Mirror state carried between the parts of the HRMA trace: after part 1 the
+// photon at the front plane and its direction (the paraboloid's frame), then
+// the photon at a conic intersection (OSAC frame of that optic) that passed
 // that optic's reflectivity test, its incoming direction, the blurred
 // normal there and p.n, and the optical constants at the photon's energy.
 struct MirrorState {
@@ -1042,12 +1043,41 @@ struct MirrorState {
   float beta, delta;
 };
 
+// Whether a ray (x, p in the paraboloid's frame) certainly misses the
+// paraboloid, in single precision.  Along the ray, as a function of x, the
+// difference G of the squared radii of the ray and of the conic is a
+// quadratic, and the intersections are its roots; on [xmin, xmax] it lies
+// within |curvature| L^2 / 4 of the chord between its end values, so that
+// end values of one sign further than that from zero leave no root inside.
+// The float evaluation of G is good to about 0.2 mm^2 (positions of 700 mm)
+// or 1e-6 of the squares; the margin is ten times that.  Rays it does not
+// rule out, NaN among them, take the double-precision intersection, which
+// alone decides a hit.
+MXD bool paraboloid_missed(const MxShellDev &h, D3 x, D3 p) {
+#ifdef __CUDA_ARCH__
+  const float x0 = d2f_trunc(x.x), y0 = d2f_trunc(x.y), z0 = d2f_trunc(x.z);
+  const float inv = 1.0f / d2f_trunc(p.x), my = d2f_trunc(p.y) * inv, mz = d2f_trunc(p.z) * inv;
+  const float xa = h.xlimf[0], xb = h.xlimf[1];
+  const float ya = fmaf(xa - x0, my, y0), za = fmaf(xa - x0, mz, z0);
+  const float yb = fmaf(xb - x0, my, y0), zb = fmaf(xb - x0, mz, z0);
+  const float ra = fmaf(ya, ya, za * za), rb = fmaf(yb, yb, zb * zb);
+  const float ga = ra - h.r2limf[0], gb = rb - h.r2limf[1];
+  const float bow = fabsf(fmaf(my, my, mz * mz) - h.am1f) * h.quarter_l2f;
+  const float margin = 2.0f + 1e-5f * (ra + rb) + bow;
+  return (ga > margin && gb > margin) || (ga < -margin && gb < -margin);
+#else
+  (void) h; (void) x; (void) p;
+  return false;
+#endif
+}
+
 // _marx_hrma_mirror_reflect per photon (hrma.c:1183-1339), part 1:
 // vignetting, project_photon_to_hrma (hrma.c:984-1050), transform into the
-// paraboloid's frame, optical constants, paraboloid intersection.  Returns
-// true if the photon reached the paraboloid.
-MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
-                      Rng &rng, MirrorState &m) {
+// paraboloid's frame.  Returns false when the photon's trace ends here, the
+// rays that certainly miss the paraboloid (half of all photons: the aperture
+// annuli are wider than the mirrors' shadows) among them, so that the
+// wavefront intersects the others on full warps.
+MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m) {
   rng.window(MX_U_MIRROR, 12, MX_N_MIRROR, 2);
   if (!T.ideal) {
     // a uniform in [0, 1) never exceeds a vignetting factor of 1
@@ -1094,6 +1124,17 @@ MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, const float *
            fma(f[8], z, fma(f[7], y, h.front_fwd[2])));
   }
   p = mat_mul(h.fwd[0], p);
+  if (paraboloid_missed(h, x, p)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false; }
+  m.x = x; m.p = p;
+  return true;
+}
+
+// Part 2: optical constants, paraboloid intersection, normal blur and
+// reflectivity test there.  Returns false if the photon misses the
+// paraboloid or is absorbed.
+MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
+                      Rng &rng, MirrorState &m) {
+  const MxShellDev &h = shells[ph.shell];
   m.beta = 0.0f; m.delta = 1.0f; m.corr = 1.0;
   if (T.opt_n) {
     float fe = d2f_rn(ph.e);
@@ -1103,16 +1144,8 @@ MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, const float *
       m.corr = sqrt_of_float(interp_f(fe, ce, ce + h.corr_n, slope + h.corr_slope_off, h.corr_n));
     }
   }
-  D3 n;
-  if (-1 == conic_intersection(h, 0, x, p, n)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false; }
-  m.x = x; m.p = p; m.n = n;
-  return true;
-}
-
-// Part 2: normal blur and reflectivity test at the paraboloid.  Returns
-// false if the photon is absorbed there.
-MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m) {
-  if (!reflect_test(T, shells[ph.shell], 0, m.p, m.n, m.pdn, m.beta, m.delta, m.corr, rng)) {
+  if (-1 == conic_intersection(h, 0, m.x, m.p, m.n) ||
+      !reflect_test(T, h, 0, m.p, m.n, m.pdn, m.beta, m.delta, m.corr, rng)) {
     ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = m.x; ph.p = m.p; return false;
   }
   return true;
@@ -1168,7 +1201,7 @@ MXD void mirror_back(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &r
 MXD void mirror_stage(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
                       Rng &rng) {
   MirrorState m;
-  if (mirror_front(T, shells, optc, slope, ph, rng, m) && mirror_ptest(T, shells, ph, rng, m) &&
+  if (mirror_front(T, shells, ph, rng, m) && mirror_ptest(T, shells, optc, slope, ph, rng, m) &&
       mirror_middle(T, shells, ph, rng, m))
     mirror_back(T, shells, ph, rng, m);
 }

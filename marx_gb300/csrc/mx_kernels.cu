@@ -188,16 +188,21 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 // ------------------------------------------------------------ wavefront --
 // The same trace as mx_trace_kernel split where photons are lost, so that
 // lost photons stop occupying SIMT lanes: phase A runs every photon up to
-// the paraboloid intersection (the photons between the shells are lost
-// there) and appends the rest to queue 1; phase T draws the paraboloid's
-// normal blur and reflectivity test and moves the photons it reflects to
-// queue 2; phase B finishes that reflection, intersects the hyperboloid and
+// the front plane in its shell's frame, where single precision rules out the
+// photons that pass between the mirrors (half of them), and appends the rest
+// to queue 1; phase T intersects the paraboloid, draws its normal blur and
+// reflectivity test and moves the photons it reflects to queue 2; phase B finishes that reflection, intersects the hyperboloid and
 // applies its reflectivity test, appending survivors to queue 1 again;
 // phase C finishes the hyperboloid reflection and runs the detector, or,
 // with a grating, the grating up to its order choice, appending the photons
 // given an order to queue 2 for phase D (diffraction and detector).
 // Appends are warp-aggregated (one atomic per warp); the order of records
 // in a queue does not affect any photon's result.
+// Bound by the FP64 pipe (62-74 % busy per phase).  With the intersection in
+// phase A its 56 FP64 operations ran for every photon, and half of them miss:
+// per 1e6 plain_scatter photons phase A + T took 326 + 66 us and 5.2e6 FP64
+// instructions, with it in phase T 199 + 165 us and 4.0e6 (1e7 photons 5.76
+// -> 5.37 ms, 1e6 on axis 416 -> 368 us, the 256-source batch 17.4 -> 15.3 ms).
 
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_a(MxTables T, TraceIO io, WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
@@ -208,7 +213,7 @@ __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_a(M
   for (uint32_t base = warp * 32; base < io.n; base += nwarps * 32) {
     const uint32_t i = base + lane;
     bool keep = false;
-    MxRec rec;
+    MxRecA rec;
     if (i < io.n) {
       Ph q;
       q.e = io.energy[i];
@@ -238,20 +243,26 @@ __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_a(M
       if (io.dith) for (int k = 0; k < 3; k++) io.dith[k * n + i] = q.dith[k];
       store_det_dither(T, io, n, i, q.t, q.flags);
       MirrorState m;
-      if (!(q.flags & MX_BAD_PHOTON_MASK) && mirror_front(T, sh, optc, slope, q, r, m)) {
+      if (!(q.flags & MX_BAD_PHOTON_MASK) && mirror_front(T, sh, q, r, m)) {
         keep = true;
-        to_rec(rec, q, m, r, i);
+        to_rec_a(rec, q, m, r, i);
       } else
         store_core(io, i, q, r.overrun);
     }
-    append(keep, rec, w.q1, &w.counts[0]);
+    append(keep, rec, (MxRecA *) w.q1, &w.counts[0]);
   }
 }
 
 // One queue-to-queue phase: records of `in` (count at *in_count) through
 // `step`; survivors are appended to `out`, the rest stored.
-template <typename Step>
-__device__ __forceinline__ void wave_pass(const TraceIO &io, const MxRec *in, const unsigned int *in_count, MxRec *out,
+__device__ __forceinline__ void load_rec(const MxRecA &r, Ph &q, MirrorState &m, Rng &rng, const TraceIO &io) {
+  from_rec_a(r, q, m, rng, io);
+}
+__device__ __forceinline__ void load_rec(const MxRec &r, Ph &q, MirrorState &m, Rng &rng, const TraceIO &io) {
+  from_rec(r, q, m, rng, io);
+}
+template <typename Rec, typename Step>
+__device__ __forceinline__ void wave_pass(const TraceIO &io, const Rec *in, const unsigned int *in_count, MxRec *out,
                                           unsigned int *out_count, Step step) {
   const uint32_t count = *(volatile const unsigned int *) in_count;
   const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -261,14 +272,14 @@ __device__ __forceinline__ void wave_pass(const TraceIO &io, const MxRec *in, co
     bool keep = false;
     MxRec rec;
     if (k < count) {
-      rec = in[k];
       Ph q; MirrorState m; Rng r;
-      from_rec(rec, q, m, r, io);
+      const Rec rec_in = in[k];
+      load_rec(rec_in, q, m, r, io);
       if (step(q, r, m)) {
         keep = true;
-        to_rec(rec, q, m, r, rec.i);
+        to_rec(rec, q, m, r, r.i);
       } else
-        store_core(io, rec.i, q, r.overrun);
+        store_core(io, r.i, q, r.overrun);
     }
     append(keep, rec, out, out_count);
   }
@@ -277,8 +288,8 @@ __device__ __forceinline__ void wave_pass(const TraceIO &io, const MxRec *in, co
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_t(MxTables T, TraceIO io, WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
-  wave_pass(io, w.q1, &w.counts[0], w.q2, &w.counts[1],
-            [&](Ph &q, Rng &r, MirrorState &m) { return mirror_ptest(T, sh, q, r, m); });
+  wave_pass(io, (const MxRecA *) w.q1, &w.counts[0], w.q2, &w.counts[1],
+            [&](Ph &q, Rng &r, MirrorState &m) { return mirror_ptest(T, sh, optc, slope, q, r, m); });
 }
 
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_b(MxTables T, TraceIO io, WaveBufs w) {

@@ -44,8 +44,17 @@ struct __align__(16) MxRec {
   double pdn;                   // p.n with the blurred normal (reflectivity test passed)
 };
 
+// One photon between phases A and T (80 bytes): at the front plane in the
+// paraboloid's frame.
+struct __align__(16) MxRecA {
+  double x[3], p[3], e, t;
+  uint32_t i, tag, flags;
+  uint8_t shell, upos, npos, overrun;
+};
+static_assert(sizeof(MxRecA) <= sizeof(MxRec), "phase A's records share a queue's memory");
+
 // Wavefront scratch: two record queues of n entries and their fill counts.
-// Phase A appends to q1, the paraboloid test moves survivors to q2, phase B
+// Phase A appends to q1 (as MxRecA), the paraboloid test moves survivors to q2, phase B
 // appends to q1 again (its first use is over), phase C reads it and, with a
 // grating, appends the photons given an order to q2 for phase D.
 struct WaveBufs {

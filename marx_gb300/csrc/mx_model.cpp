@@ -834,6 +834,13 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
       for (int k = 0; k < 9; k++) h.bwd0f[k] = (float) h.bwd[0][k];
       for (int r = 0; r < 3; r++) h.osac0f[r] = (float) h.to_osac[0][r];
     }
+    for (int k = 0; k < 2; k++) {
+      const double x = k ? h.xmax[0] : h.xmin[0];
+      h.xlimf[k] = (float) x;
+      h.r2limf[k] = (float) (h.c[0] + x * (h.b[0] + x * h.am1[0]));
+    }
+    h.am1f = (float) h.am1[0];
+    h.quarter_l2f = (float) (0.25 * (h.xmax[0] - h.xmin[0]) * (h.xmax[0] - h.xmin[0]));
     const double *qp = rdb + i * 9;
     h.front_position = cap_pos - qp[2] + h.xmax[0];
     for (int r = 0; r < 3; r++) h.front_fwd[r] = h.fwd[0][3 * r] * (h.front_position + h.to_osac[0][0]);

@@ -33,7 +33,9 @@ struct MxShellDev {
   // memory start on banks 0, 24, 16 and 8, so lanes of a warp that load
   // one field of different shells do not conflict (at 704 bytes shells 0
   // and 2, and 1 and 3, shared their banks).
-  double bank_pad[4];
+  float xlimf[2], r2limf[2];                   // the paraboloid's x-limits and its squared radii there,
+  float am1f, quarter_l2f;                     // a - 1 and a quarter of its squared length (its miss screen)
+  double bank_pad;
 };
 static_assert(sizeof(MxShellDev) % 128 == 96, "shell records of 736 + 128 k bytes: four distinct bank offsets");
 

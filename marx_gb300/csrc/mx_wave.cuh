@@ -40,7 +40,8 @@ __device__ __forceinline__ void stage_tables(const MxTables &T, MxShellDev *&sh,
   __syncthreads();
 }
 
-__device__ __forceinline__ void append(bool keep, const MxRec &r, MxRec *q, unsigned int *cnt) {
+template <class Rec>
+__device__ __forceinline__ void append(bool keep, const Rec &r, Rec *q, unsigned int *cnt) {
   const unsigned lane = threadIdx.x & 31;
   unsigned mask = __ballot_sync(0xffffffffu, keep);
   if (mask == 0) return;
@@ -49,6 +50,23 @@ __device__ __forceinline__ void append(bool keep, const MxRec &r, MxRec *q, unsi
   if ((int) lane == leader) base = atomicAdd(cnt, (unsigned) __popc(mask));
   base = __shfl_sync(0xffffffffu, base, leader);
   if (keep) q[base + __popc(mask & ((1u << lane) - 1u))] = r;
+}
+
+__device__ __forceinline__ void to_rec_a(MxRecA &r, const Ph &q, const MirrorState &m, const Rng &rng, uint32_t i) {
+  r.x[0] = m.x.x; r.x[1] = m.x.y; r.x[2] = m.x.z;
+  r.p[0] = m.p.x; r.p[1] = m.p.y; r.p[2] = m.p.z;
+  r.e = q.e; r.t = q.t;
+  r.i = i; r.tag = rng.tag; r.flags = q.flags;
+  r.shell = (uint8_t) q.shell; r.upos = (uint8_t) rng.upos; r.npos = (uint8_t) rng.npos;
+  r.overrun = rng.overrun ? 1 : 0;
+}
+
+__device__ __forceinline__ void from_rec_a(const MxRecA &r, Ph &q, MirrorState &m, Rng &rng, const TraceIO &io) {
+  m.x = mk(r.x[0], r.x[1], r.x[2]); m.p = mk(r.p[0], r.p[1], r.p[2]);
+  q.e = r.e; q.t = r.t; q.flags = r.flags; q.shell = r.shell; q.set = 0;
+  rng.U = io.U; rng.N = io.N; rng.seed = io.seed; rng.n = io.n; rng.i = r.i; rng.tag = r.tag;
+  rng.upos = r.upos; rng.uend = MX_U_MIRROR + 12; rng.npos = r.npos; rng.nend = MX_N_MIRROR + 2;
+  rng.overrun = r.overrun != 0;
 }
 
 __device__ __forceinline__ void to_rec(MxRec &r, const Ph &q, const MirrorState &m, const Rng &rng, uint32_t i) {
