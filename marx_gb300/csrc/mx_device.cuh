@@ -340,6 +340,42 @@ __device__ __forceinline__ F2 df_from(double d) {
 }
 __device__ __forceinline__ double df_to(F2 a) { return f2d(a.h) + f2d(a.l); }
 
+// d as hi + lo without an FP64 operation: hi the truncation of d to float,
+// lo the 29 bits below it.  |d| outside 2^-60 .. 2^60 gives lo = 0.
+__device__ __forceinline__ F2 split(double d) {
+  const unsigned long long b = dbits(d);
+  const uint32_t hi = (uint32_t) (b >> 32), lo = (uint32_t) b & 0x1FFFFFFFu, e = (hi >> 20) & 0x7ffu;
+  const float l = (float) (int) lo;                                    // below 2^29, rounded to 24 bits
+  const float scale = __uint_as_float((hi & 0x80000000u) | ((e - (1023u + 52u - 127u)) << 23));   // +-2^(e - 1023 - 52)
+  return {d2f_trunc(d), e - 963u < 120u ? l * scale : 0.0f};
+}
+// a normalised hi + lo (|lo| at most half an ulp of hi) as the double nearest
+// it, on the integer pipe: lo in units of the double ulp of hi, a whole
+// number below 2^29, is added to hi's bits.  Sizes outside 2^-63 .. 2^65,
+// and zero, take the FP64 sum.
+__device__ __forceinline__ double df_join(F2 a) {
+  const uint32_t u = __float_as_uint(a.h), e = (u >> 23) & 0xffu;
+  if (e - 64u < 128u) {
+    int l = __float2int_rn(a.l * __uint_as_float((306u - e) << 23));   // lo 2^(52 - exponent)
+    if (u & 0x80000000u) l = -l;
+    if ((u & 0x7fffffu) == 0u && l < 0) l += l;                        // below a power of two the ulp halves
+    const unsigned long long m = ((unsigned long long) (((u & 0x7fffffffu) >> 3) + (896u << 20)) << 32) | (u << 29);
+    return __longlong_as_double((long long) ((m + (long long) l) | ((unsigned long long) (u & 0x80000000u) << 32)));
+  }
+  return f2d(a.h) + f2d(a.l);
+}
+// f 2^-64 for a signed 64-bit f, in units of a quarter turn, as radians
+// (|f| 2^-64 <= 1/2): the top 23 bits of f as a float (a whole number within
+// 2^22 of 1.5 2^23), the next 24 as another, both exact, and the last 17
+// added to the low part, times pi/2.
+__device__ __forceinline__ F2 quarter_turns(long long f) {
+  const float a = __uint_as_float(0x4B400000u + (uint32_t) (int) (f >> 41)) - 12582912.0f;
+  const float b = (float) (int) ((uint32_t) (f >> 17) & 0xffffffu), c = (float) (int) ((uint32_t) f & 0x1ffffu);
+  F2 q = quick_sum(a * 0x1p-23f, b * 0x1p-47f);
+  q.l = __fmaf_rn(c, 0x1p-64f, q.l);
+  return df_mul(F2{0x1.921fb6p+0f, -0x1.777a5cp-25f}, q);
+}
+
 // sin and cos of r (|r| <= pi/4 + a little) in double-float.
 __device__ __forceinline__ void df_sincos(F2 r, F2 &sr, F2 &cr) {
   const F2 z = df_mul(r, r);
@@ -363,6 +399,23 @@ __device__ __forceinline__ void df_sincos(F2 r, F2 &sr, F2 &cr) {
   Q = df_add(F2{0x1.555556p-5f, -0x1.555556p-30f}, df_mul(z, Q));
   Q = df_add(F2{-0.5f, 0.0f}, df_mul(z, Q));
   cr = df_add(F2{1.0f, 0.0f}, df_mul(z, Q));
+}
+
+// sin or cos of r alone: the two series above with their coefficients
+// selected, sin r = r + r W and cos r = (1 - z/2) + z W with W = z times the
+// next four terms' series, at the cost of one.
+__device__ __forceinline__ F2 df_sin_or_cos(F2 r, bool cosine) {
+  const F2 z = df_mul(r, r);
+  const float zf = z.h;
+  float g = __fmaf_rn(zf, cosine ? 0x1.ae7f3ep-45f : -0x1.ae7f3ep-41f, cosine ? -0x1.93974ap-37f : 0x1.612462p-33f);
+  g = __fmaf_rn(zf, g, cosine ? 0x1.1eed8ep-29f : -0x1.ae6456p-26f);
+  F2 w = df_add(cosine ? F2{-0x1.27e4fcp-22f, 0x1.10ec14p-47f} : F2{0x1.71de3ap-19f, 0x1.55b1ccp-45f}, df_mul_f(z, g));
+  w = df_add(cosine ? F2{0x1.a01a02p-16f, -0x1.7f97fap-42f} : F2{-0x1.a01a02p-13f, 0x1.7f97fap-39f}, df_mul(z, w));
+  w = df_add(cosine ? F2{-0x1.6c16c2p-10f, 0x1.27d27ep-35f} : F2{0x1.111112p-7f, -0x1.dddddep-32f}, df_mul(z, w));
+  w = df_add(cosine ? F2{0x1.555556p-5f, -0x1.555556p-30f} : F2{-0x1.555556p-3f, 0x1.555556p-28f}, df_mul(z, w));
+  w = df_mul(z, w);
+  const F2 a = cosine ? df_add(F2{1.0f, 0.0f}, F2{-0.5f * z.h, -0.5f * z.l}) : r, b = cosine ? z : r;
+  return df_add(a, df_mul(b, w));
 }
 
 __device__ __forceinline__ F2 df_neg(F2 a) { return {-a.h, -a.l}; }
@@ -497,6 +550,32 @@ MXD float sine_to_float(double amp, int amp_exp, double arg) {
   return (float) (amp * std::sin(arg));
 #endif
 }
+
+// u 2^64, truncated, for 0 <= u < 1.
+MXD unsigned long long unit_to_fixed(double u) {
+  const unsigned long long b = dbits(u);
+  const int e = (int) ((b >> 52) & 0x7ff);                        // u = 1.m 2^(e - 1023)
+  if (e < 1023 - 64) return 0ull;
+  return ((b << 11) | 0x8000000000000000ull) >> (1022 - e);
+}
+#ifdef __CUDACC__
+// sin and cos of 2 pi u - pi/4 for u = f 2^-64 (the aperture's azimuth; its
+// quarter turns are the top two bits of f, and the eighth taken off centres
+// the rest) and of 2 pi u, in double-float: the reduction is exact on the
+// integer pipe.
+__device__ __forceinline__ void df_turn_sincos(unsigned long long f, bool less_eighth, F2 &s, F2 &c) {
+  unsigned n = (unsigned) (f >> 62);
+  long long r = (long long) (f << 2);                             // the fraction of a quarter turn, 2^64 of one
+  if (less_eighth) r ^= (long long) 0x8000000000000000ull;        // less a half
+  else n += (unsigned) ((unsigned long long) r >> 63);            // to the nearest quarter turn
+  F2 sr, cr;
+  df_sincos(quarter_turns(r), sr, cr);
+  s = (n & 1) ? cr : sr;
+  c = (n & 1) ? sr : cr;
+  if (n & 2) s = F2{-s.h, -s.l};
+  if ((n + 1) & 2) c = F2{-c.h, -c.l};
+}
+#endif
 
 // sqrt of a float: in double-float on the FP32 pipe (within 2^-46 of the
 // double root; it scales the reflectivity, whose test leaves values within
@@ -646,11 +725,14 @@ MXD double unit_from_bits(uint64_t m) {
   return (double) m * (1.0 / 9007199254740992.0);
 #endif
 }
-MXD double philox_uniform(uint64_t seed, uint32_t tag, uint32_t k) {
+// The 53 bits of uniform slot k as the top bits of a 64-bit fraction.
+MXD uint64_t philox_fixed(uint64_t seed, uint32_t tag, uint32_t k) {
   uint32_t c[4] = {tag, k, 0x5A5A0001u, 0u};
   philox(c, (uint32_t) seed, (uint32_t) (seed >> 32));
-  uint64_t b = ((uint64_t) c[0] << 32) | c[1];
-  return unit_from_bits(b >> 11);
+  return (((uint64_t) c[0] << 32) | c[1]) & ~(uint64_t) 0x7ff;
+}
+MXD double philox_uniform(uint64_t seed, uint32_t tag, uint32_t k) {
+  return unit_from_bits(philox_fixed(seed, tag, k) >> 11);
 }
 // Single-precision natural log and cos(2 pi u) for the normal variates,
 // from their series (ln m = 2 atanh((m-1)/(m+1)); Taylor series of sin and
@@ -698,14 +780,15 @@ MXD float series_cos2pi(float u) {   // cos(2 pi u), u in [0, 1)
             FMUL(t2, 1.60590438e-10f)))))))))))));
   return q == 0 ? c : (q == 1 ? -s : (q == 2 ? -c : s));
 }
-MXD double philox_normal(uint64_t seed, uint32_t tag, uint32_t k) {
+MXD float philox_normal_f(uint64_t seed, uint32_t tag, uint32_t k) {
   uint32_t c[4] = {tag, k, 0x5A5A0002u, 0u};
   philox(c, (uint32_t) seed, (uint32_t) (seed >> 32));
   float u1 = (float) ((c[0] >> 8) + 1u) * (1.0f / 16777216.0f);
   float u2 = (float) (c[1] >> 8) * (1.0f / 16777216.0f);
   float r = FSQRT(FMUL(-2.0f, series_logf(u1)));
-  return f2d(FMUL(r, series_cos2pi(u2)));
+  return FMUL(r, series_cos2pi(u2));
 }
+MXD double philox_normal(uint64_t seed, uint32_t tag, uint32_t k) { return f2d(philox_normal_f(seed, tag, k)); }
 
 // Source-level draws (photon generation) use their own Philox domain, so
 // they never coincide with a stage's slots: draw k of photon `tag`.
@@ -729,6 +812,12 @@ struct Rng {
     int k = upos++;
     return U ? MX_LDG(U + (size_t) k * n + i) : philox_uniform(seed, tag, (uint32_t) k);
   }
+  // The same draw times 2^64, truncated to a whole number.
+  MXD unsigned long long uniform_fixed() {
+    if (upos >= uend) { overrun = true; return 0x8000000000000000ull; }
+    int k = upos++;
+    return U ? unit_to_fixed(MX_LDG(U + (size_t) k * n + i)) : philox_fixed(seed, tag, (uint32_t) k);
+  }
   // Pass over the next uniform slot without drawing it (a test whose
   // outcome is known: a probability of 1).
   MXD void skip_uniform() {
@@ -746,6 +835,15 @@ struct Rng {
     int k = npos++;
     return N ? MX_LDG(N + (size_t) k * n + i) : philox_normal(seed, tag, (uint32_t) k);
   }
+#ifdef __CUDACC__
+  // The same draw in double-float (exact for Philox's single-precision normals).
+  __device__ __forceinline__ F2 normal_df() {
+    if (npos >= nend) { overrun = true; return {0.0f, 0.0f}; }
+    int k = npos++;
+    if (N) return split(MX_LDG(N + (size_t) k * n + i));
+    return {philox_normal_f(seed, tag, (uint32_t) k), 0.0f};
+  }
+#endif
 };
 
 // Photon state held in registers through the fused trace.
@@ -1053,22 +1151,16 @@ struct MirrorState {
 // or 1e-6 of the squares; the margin is ten times that.  Rays it does not
 // rule out, NaN among them, take the double-precision intersection, which
 // alone decides a hit.
-MXD bool paraboloid_missed(const MxShellDev &h, D3 x, D3 p) {
-#ifdef __CUDA_ARCH__
-  const float x0 = d2f_trunc(x.x), y0 = d2f_trunc(x.y), z0 = d2f_trunc(x.z);
-  const float inv = 1.0f / d2f_trunc(p.x), my = d2f_trunc(p.y) * inv, mz = d2f_trunc(p.z) * inv;
+MXD bool paraboloid_missed(const MxShellDev &h, float x0, float y0, float z0, float px, float py, float pz) {
+  const float inv = 1.0f / px, my = py * inv, mz = pz * inv;
   const float xa = h.xlimf[0], xb = h.xlimf[1];
-  const float ya = fmaf(xa - x0, my, y0), za = fmaf(xa - x0, mz, z0);
-  const float yb = fmaf(xb - x0, my, y0), zb = fmaf(xb - x0, mz, z0);
-  const float ra = fmaf(ya, ya, za * za), rb = fmaf(yb, yb, zb * zb);
+  const float ya = (xa - x0) * my + y0, za = (xa - x0) * mz + z0;
+  const float yb = (xb - x0) * my + y0, zb = (xb - x0) * mz + z0;
+  const float ra = ya * ya + za * za, rb = yb * yb + zb * zb;
   const float ga = ra - h.r2limf[0], gb = rb - h.r2limf[1];
-  const float bow = fabsf(fmaf(my, my, mz * mz) - h.am1f) * h.quarter_l2f;
+  const float bow = fabsf(my * my + mz * mz - h.am1f) * h.quarter_l2f;
   const float margin = 2.0f + 1e-5f * (ra + rb) + bow;
   return (ga > margin && gb > margin) || (ga < -margin && gb < -margin);
-#else
-  (void) h; (void) x; (void) p;
-  return false;
-#endif
 }
 
 // _marx_hrma_mirror_reflect per photon (hrma.c:1183-1339), part 1:
@@ -1102,29 +1194,62 @@ MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &
     radius = sqrt_fast(r0 * r0 + (r1 * r1 - r0 * r0) * rng.uniform());
   } else
     radius = h.min_radius + h.dr * rng.uniform();
-  double theta;
+  unsigned long long theta;
   for (int guard = 0;; guard++) {
-    theta = rng.uniform();
-    unsigned quad = quarter_of(theta);
+    theta = rng.uniform_fixed();
     if (rng.overrun || guard >= 64) { rng.overrun = true; return false; }
-    if (h.shutter & (1u << quad)) break;
+    if (h.shutter & (1u << (unsigned) (theta >> 62))) break;
   }
-  double st, ct;
-  sincospi_fast(fma(theta, 2.0, -0.25), &st, &ct);   // angle 2 pi (u - 1/8)
-  x = mk(h.front_position, radius * st - h.to_osac[0][1], radius * ct - h.to_osac[0][2]);
-  if (dkey(T.source_distance) > 0) p = normalized(x + T.source_distance * p);
-  if (T.use_struts && struts_block(T, 0, x, p)) ph.flags |= MX_PHOTON_MIRROR_VBLOCKED;
-
-  // fwd (x + to_osac): (r sin - t1) + t1 is r sin to within an ulp of t1,
-  // and the first column's product with the front plane is a constant
+  double st, ct;   // of the angle 2 pi (u - 1/8)
+#ifdef __CUDA_ARCH__
   {
-    const double y = radius * st, z = radius * ct;
+    F2 s2, c2;
+    df_turn_sincos(theta, true, s2, c2);
+    st = df_join(s2);
+    ct = df_join(c2);
+  }
+#else
+  sincospi_fast(std::ldexp((double) theta, -63) - 0.25, &st, &ct);
+#endif
+  // the point on the front plane, turned with the paraboloid (r sin, r cos
+  // less and plus its offsets) and, for a source at a distance and the
+  // struts, in the MARX frame
+  const double y = radius * st, z = radius * ct;
+  if (dkey(T.source_distance) > 0)
+    p = normalized(mk(h.front_position, y - h.to_osac[0][1], z - h.to_osac[0][2]) + T.source_distance * p);
+  const float yf = d2f_trunc(y), zf = d2f_trunc(z);
+  float pxf = d2f_trunc(p.x), pyf = d2f_trunc(p.y), pzf = d2f_trunc(p.z);
+  if (T.use_struts) {
+    int blocked = -1;
+#ifdef __CUDA_ARCH__
+    blocked = struts_screen(T, 0, h.frontf, yf - h.osac0f[1], zf - h.osac0f[2], pxf, pyf, pzf);
+#endif
+    if (blocked < 0)
+      blocked = struts_block_exact(T, 0, mk(h.front_position, y - h.to_osac[0][1], z - h.to_osac[0][2]), p) ? 1 : 0;
+    if (blocked) ph.flags |= MX_PHOTON_MIRROR_VBLOCKED;
+  }
+  // into the paraboloid's frame, fwd (x + to_osac): (r sin - t1) + t1 is
+  // r sin to within an ulp of t1, and the first column's product with the
+  // front plane is a constant.  The calibration's paraboloids are not
+  // turned (fwd is the identity): nothing to multiply then.
+  float xf = h.front_fwdf, ypf = yf, zpf = zf;
+  if (T.p_unturned)
+    x = mk(h.front_fwd[0], y, z);
+  else {
     const double *f = h.fwd[0];
     x = mk(fma(f[2], z, fma(f[1], y, h.front_fwd[0])), fma(f[5], z, fma(f[4], y, h.front_fwd[1])),
            fma(f[8], z, fma(f[7], y, h.front_fwd[2])));
+    p = mat_mul(h.fwd[0], p);
+    xf = d2f_trunc(x.x); ypf = d2f_trunc(x.y); zpf = d2f_trunc(x.z);
+    pxf = d2f_trunc(p.x); pyf = d2f_trunc(p.y); pzf = d2f_trunc(p.z);
   }
-  p = mat_mul(h.fwd[0], p);
-  if (paraboloid_missed(h, x, p)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false; }
+#ifdef __CUDA_ARCH__
+  if (paraboloid_missed(h, xf, ypf, zpf, pxf, pyf, pzf)) {
+    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false;
+  }
+#else
+  (void) xf; (void) ypf; (void) zpf;
+#endif
   m.x = x; m.p = p;
   return true;
 }
@@ -1234,7 +1359,7 @@ MXD bool aspsol_state(const MxTables &T, double t, float s[6]) {
   return true;
 }
 
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
 // apply_dither's rotation (below) for offsets ra, dec under 1e-4 rad, as the
 // change it makes: p' = p + D with
 //   D = -d p + k n + n x p,  n = (0, sin dec, -cos dec sin ra),
@@ -1243,26 +1368,56 @@ MXD bool aspsol_state(const MxTables &T, double t, float s[6]) {
 // with p in double.  sin and cos go to x^3 and x^2 (the next terms are
 // below 1e-18 relative) as in sincos_small, and d is formed as
 // (ra^2 + dec^2)/2 - ra^2 dec^2/4, without the cancellation that costs the
-// double evaluation seven digits of d.  Eleven FP64 operations (the
-// splits, the sums back to double and the additions to p) instead of about
-// thirty-five; the result is within an ulp or two of the double evaluation.
-__device__ __forceinline__ D3 dither_rotate_df(D3 p, double ra, double dec) {
+// double evaluation seven digits of d.  Three FP64 operations (the
+// additions to p; the splits and joins run on the integer pipe) instead of
+// about thirty-five; the result is within an ulp or two of the double
+// evaluation.
+__device__ __forceinline__ D3 dither_rotate_df(D3 p, F2 r, F2 e) {
   const F2 sixth = {0x1.555556p-3f, -0x1.555556p-28f};   // 1/6
-  const F2 r = df_from(ra), e = df_from(dec);
   const F2 r2 = df_sqr(r), e2 = df_sqr(e);
   const F2 sr = df_sub(r, df_mul(df_mul(r, r2), sixth)), sd = df_sub(e, df_mul(df_mul(e, e2), sixth));
   const F2 cd = df_add(F2{1.0f, 0.0f}, F2{-0.5f * e2.h, -0.5f * e2.l});
   const F2 ny = sd, nz = df_neg(df_mul(cd, sr));
   const F2 h = df_add(r2, e2), q = df_mul(r2, e2);
   const F2 d = df_sub(F2{0.5f * h.h, 0.5f * h.l}, F2{0.25f * q.h, 0.25f * q.l});
-  const F2 px = df_from(p.x), py = df_from(p.y), pz = df_from(p.z);
+  const F2 px = split(p.x), py = split(p.y), pz = split(p.z);
   const F2 pn = df_add(df_mul(py, ny), df_mul(pz, nz));
   const F2 k = df_mul(pn, df_add(F2{0.5f, 0.0f}, df_mul(d, df_add(F2{0.25f, 0.0f}, df_mul_f(d, 0.125f)))));
   const F2 md = df_neg(d);
   const F2 dx = df_add(df_mul(md, px), df_sub(df_mul(ny, pz), df_mul(nz, py)));
   const F2 dy = df_add(df_add(df_mul(md, py), df_mul(k, ny)), df_mul(nz, px));
   const F2 dz = df_sub(df_add(df_mul(md, pz), df_mul(k, nz)), df_mul(ny, px));
-  return mk(p.x + df_to(dx), p.y + df_to(dy), p.z + df_to(dz));
+  return mk(p.x + df_join(dx), p.y + df_join(dy), p.z + df_join(dz));
+}
+
+// (float) (amp[k] sin(2 pi t / period[k])) as the double-precision
+// expression rounds it, without an FP64 operation; ok is cleared where that
+// is not certain.  t 4 / period, in quarter turns, is a 64 x 64-bit product
+// (4 / period to 2^-64), whose integer part picks the quadrant and whose
+// fraction is the angle, exact to 2^-50 of a quarter turn for up to 2^12 of
+// them; sine and amplitude in double-float.  The value is within
+// amp (2^-44 + q 2^-51) of the double expression's (q quarter turns, whose
+// two roundings of the argument are the second term): when no float rounding
+// boundary lies within eight and four times that, both round to the same
+// float.  About one value in 10^4 is left to the library sine.
+__device__ __forceinline__ float dither_sine(const MxTables &T, int k, double t, bool &ok) {
+  const unsigned long long b = dbits(t);
+  const int e = (int) ((b >> 52) & 0x7ff), frac = 1022 - e - T.dith_qexp[k];   // fraction bits of the product's high word
+  if (!T.dith_q[k] || e == 0x7ff || frac < 52) { ok = false; return 0.0f; }
+  if ((b << 1) == 0ull) return 0.0f * T.dith_ampf[k][0];
+  const unsigned long long hi = __umul64hi((b << 11) | 0x8000000000000000ull, T.dith_q[k]);
+  unsigned n = frac < 64 ? (unsigned) (hi >> frac) : 0u;
+  const float turns = (float) n;
+  long long f = (long long) (frac < 64 ? hi << (64 - frac) : (frac < 128 ? hi >> (frac - 64) : 0ull));
+  n += (unsigned) ((unsigned long long) f >> 63);                 // to the nearest quarter turn
+  const F2 w = df_sin_or_cos(quarter_turns(f), (n & 1) != 0);
+  const F2 v = df_mul(F2{T.dith_ampf[k][0], T.dith_ampf[k][1]}, w);
+  const uint32_t ve = __float_as_uint(v.h) & 0x7f800000u;
+  const float half = __uint_as_float(ve) * 0x1p-24f;              // half an ulp of v.h; a power of two's lower side is half that
+  const float away = ((__float_as_uint(v.h) & 0x7fffffu) ? half : 0.5f * half) - fabsf(v.l);
+  const float margin = fabsf(T.dith_ampf[k][0]) * (0x1p-41f + turns * 0x1p-49f);
+  if (!(away > margin)) ok = false;
+  return ((n & 2) != 0) != neg_bit(t) ? -v.h : v.h;
 }
 #endif
 
@@ -1283,26 +1438,27 @@ MXD void dither_stage(const MxTables &T, Ph &ph, Rng &rng) {
     froll = T.asp_record_only ? 0.0f : s[2];
   } else {
     // (a zero start time or phase is added exactly: skipped)
-    double t = (2.0 * PI) * (is_zero(T.start_time) ? ph.t : T.start_time + ph.t);
+    const double t = is_zero(T.start_time) ? ph.t : T.start_time + ph.t;
     // amp * sin(2 pi t / period + phase) rounded to float as the reference
     // stores it; a zero amplitude makes it zero whatever the sine
     float f[2];
-    for (int k = 0; k < 2; k++)
-      f[k] = !is_zero(T.dith_amp[k])
-                 ? sine_to_float(T.dith_amp[k], T.dith_amp_exp[k],
-                                 is_zero(T.dith_phase[k]) ? div_by(t, T.dith_period[k], T.dith_inv_period[k])
-                                                          : div_by(t, T.dith_period[k], T.dith_inv_period[k]) +
-                                                                T.dith_phase[k])
-                 : 0.0f;
+    for (int k = 0; k < 2; k++) {
+      if (is_zero(T.dith_amp[k])) { f[k] = 0.0f; continue; }
+#ifdef __CUDA_ARCH__
+      bool ok = true;
+      f[k] = dither_sine(T, k, t, ok);
+      if (ok) continue;
+#endif
+      const double turn = div_by((2.0 * PI) * t, T.dith_period[k], T.dith_inv_period[k]);
+      f[k] = sine_to_float(T.dith_amp[k], T.dith_amp_exp[k], is_zero(T.dith_phase[k]) ? turn : turn + T.dith_phase[k]);
+    }
     fra = f[0];
     fdec = f[1];
     if (T.roll_fixed) froll = T.roll_f;
-    else froll = (float) (T.nominal_roll + T.dith_amp[2] * sin(div_by(t, T.dith_period[2], T.dith_inv_period[2]) +
-                                                                T.dith_phase[2]));
+    else froll = (float) (T.nominal_roll + T.dith_amp[2] * sin(div_by((2.0 * PI) * t, T.dith_period[2],
+                                                                      T.dith_inv_period[2]) + T.dith_phase[2]));
     ph.dith[0] = fra; ph.dith[1] = fdec; ph.dith[2] = froll;
   }
-  double ra = f2d(fra) + T.aspect_blur * rng.normal();
-  double dec = f2d(fdec) + T.aspect_blur * rng.normal();
   // roll about the x axis (JDMv_rotate_unit_vector with n = x); a fixed
   // roll of zero leaves p as it is
   D3 p = ph.p;
@@ -1314,11 +1470,16 @@ MXD void dither_stage(const MxTables &T, Ph &ph, Rng &rng) {
     p = rotate_x(p, T.roll_cos, T.roll_sin);
 #ifdef __CUDA_ARCH__
   // arcsecond offsets (the usual case): the same rotation in double-float
-  const double ara = fabs(ra), adec = fabs(dec);
-  if (lt_pos(ara, 1e-4) && lt_pos(adec, 1e-4) && (lt_pos(1e-19, ara) || lt_pos(1e-19, adec))) {
-    ph.p = dither_rotate_df(p, ra, dec);
+  const F2 blur = {T.aspect_blurf[0], T.aspect_blurf[1]}, n0 = rng.normal_df(), n1 = rng.normal_df();
+  const F2 ra2 = df_add(F2{fra, 0.0f}, df_mul(blur, n0)), dec2 = df_add(F2{fdec, 0.0f}, df_mul(blur, n1));
+  const float ara = fabsf(ra2.h), adec = fabsf(dec2.h);
+  if (ara < 1e-4f && adec < 1e-4f && (ara > 1e-19f || adec > 1e-19f)) {
+    ph.p = dither_rotate_df(p, ra2, dec2);
     return;
   }
+  const double ra = f2d(fra) + T.aspect_blur * (f2d(n0.h) + f2d(n0.l)), dec = f2d(fdec) + T.aspect_blur * (f2d(n1.h) + f2d(n1.l));
+#else
+  const double ra = f2d(fra) + T.aspect_blur * rng.normal(), dec = f2d(fdec) + T.aspect_blur * rng.normal();
 #endif
   double sr, cr, sd, cd;
   sincos_small(ra, &sr, &cr);

@@ -122,15 +122,6 @@ __device__ __forceinline__ bool mid_range(double x) {
   const unsigned e = (unsigned) (dbits(x) >> 52) & 0x7ffu;
   return e - 623u < 800u || is_zero(x);
 }
-// d as hi + lo without an FP64 operation: hi the truncation of d to float,
-// lo the 29 bits below it.  |d| outside 2^-60 .. 2^60 gives lo = 0.
-__device__ __forceinline__ F2 split(double d) {
-  const unsigned long long b = dbits(d);
-  const uint32_t hi = (uint32_t) (b >> 32), lo = (uint32_t) b & 0x1FFFFFFFu, e = (hi >> 20) & 0x7ffu;
-  const float l = (float) (int) lo;                                    // below 2^29, rounded to 24 bits
-  const float scale = u2f((hi & 0x80000000u) | ((e - (1023u + 52u - 127u)) << 23));   // +-2^(e - 1023 - 52)
-  return {d2f_trunc(d), e - 963u < 120u ? l * scale : 0.0f};
-}
 // 1 / d, 2^-40 < |d| < 2^40: the float reciprocal and one Newton step on the
 // FP32 pipe give it to 2^-45, a second step in double leaves half an ulp and
 // 2^-37 of one: three FP64 operations where the correctly rounded

@@ -521,7 +521,9 @@ cudaError_t launch_compact(const uint32_t *flags, uint32_t n, uint32_t *idx_out,
 // (y = the float nearest x), 3 sine_to_float with amp 1, amp_exp 0
 // (y = (float) sin x), 4 f2d of d2f_trunc (y = x truncated to float),
 // 5 the Fresnel numerator and denominator in double-float and in double,
-// 6 (double) (unsigned) x on the integer pipe, 7 sqrt_fast, 8 quarter_of.
+// 6 (double) (unsigned) x on the integer pipe, 7 sqrt_fast, 8 quarter_of,
+// 9 df_join of split, 10 df_turn_sincos less an eighth (y[2i], y[2i+1] = sin,
+// cos of 2 pi x - pi/4, 0 <= x < 1).
 __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, double *y, size_t n) {
   const size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -538,6 +540,13 @@ __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, d
   else if (fn == 6) y[i] = mx::u2d(mx::trunc_to_unsigned(v));
   else if (fn == 7) y[i] = mx::sqrt_fast(v);
   else if (fn == 8) y[i] = mx::quarter_of(v);
+  else if (fn == 9) y[i] = mx::df_join(mx::split(v));
+  else if (fn == 10) {
+    mx::F2 sn, cs;
+    mx::df_turn_sincos(mx::unit_to_fixed(v), true, sn, cs);
+    y[2 * i] = mx::df_join(sn);
+    y[2 * i + 1] = mx::df_join(cs);
+  }
   else {
     // x: n triples (cos, beta, delta); y: n quadruples, the double-float
     // numerator and denominator, then the double-precision ones

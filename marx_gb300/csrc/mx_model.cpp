@@ -797,6 +797,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
   append_slopes(M.optc_slope, opt, opt + optn, optn);          // beta
   append_slopes(M.optc_slope, opt, opt + 2 * optn, optn);      // delta
   double total_area = 0.0;
+  T.p_unturned = 1;
   M.shells.resize(4);
   for (int i = 0; i < 4; i++) {
     MxShellDev &h = M.shells[i];
@@ -844,6 +845,10 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
     const double *qp = rdb + i * 9;
     h.front_position = cap_pos - qp[2] + h.xmax[0];
     for (int r = 0; r < 3; r++) h.front_fwd[r] = h.fwd[0][3 * r] * (h.front_position + h.to_osac[0][0]);
+    h.frontf = (float) h.front_position;
+    h.front_fwdf = (float) h.front_fwd[0];
+    for (int k = 0; k < 9; k++)
+      if (h.fwd[0][k] != (k % 4 == 0 ? 1.0 : 0.0)) T.p_unturned = 0;
     auto radius = [](double a, double b, double c, double x) { return sqrt(c + x * (b + x * (a - 1))); };
     h.min_radius = radius(h.a[0], h.b[0], h.c[0], h.xmin[0]);
     h.max_radius = radius(h.a[0], h.b[0], h.c[0], h.xmax[0]);
@@ -1095,7 +1100,28 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
     int e = 0;
     frexp(T.dith_amp[k], &e);   // |amp| = m 2^e, 1/2 <= m < 1
     T.dith_amp_exp[k] = e;
+    if (k == 2) break;
+    T.dith_ampf[k][0] = (float) T.dith_amp[k];
+    T.dith_ampf[k][1] = (float) (T.dith_amp[k] - (double) T.dith_ampf[k][0]);
+    // 4 / period = q 2^qexp with 64 bits of q: period = m 2^e with a 53-bit
+    // whole m, and 2^115 / m is divided in two steps (2^62 <= 2^115 / m < 2^64)
+    T.dith_q[k] = 0;
+    if (cfg.dither_phase[k] == 0.0 && cfg.dither_period[k] > 1e-3 && cfg.dither_period[k] < 1e30) {
+      const uint64_t m = (uint64_t) ldexp(frexp(cfg.dither_period[k], &e), 53);   // period = m 2^(e - 53)
+      uint64_t q = 0, r = 1ull << 52;                                             // the remainder ahead of each bit
+      for (int b = 0; b < 64; b++) {                                              // q = 2^116 / m or 2^115 / m
+        r <<= 1;
+        q = (q << 1) | (r >= m);
+        if (r >= m) r -= m;
+      }
+      // 2^52 2^64 / m = 2^116 / m lies in [2^63, 2^64]: 4 / period = q 2^(2 + 53 - e - 116)
+      if (m == 1ull << 52) q = 1ull << 63, T.dith_qexp[k] = 2 + 53 - e - 115;
+      else T.dith_qexp[k] = 2 + 53 - e - 116;
+      T.dith_q[k] = q;
+    }
   }
+  T.aspect_blurf[0] = (float) T.aspect_blur;
+  T.aspect_blurf[1] = (float) (T.aspect_blur - (double) T.aspect_blurf[0]);
   double roll = cfg.roll_nom * (PI_ / 180.0);
   double xr = fmod(roll, 2 * PI_);
   if (xr >= PI_) xr -= (2 * PI_);

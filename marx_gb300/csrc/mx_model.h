@@ -35,7 +35,7 @@ struct MxShellDev {
   // and 2, and 1 and 3, shared their banks).
   float xlimf[2], r2limf[2];                   // the paraboloid's x-limits and its squared radii there,
   float am1f, quarter_l2f;                     // a - 1 and a quarter of its squared length (its miss screen)
-  double bank_pad;
+  float frontf, front_fwdf;                    // front_position and front_fwd[0] in float
 };
 static_assert(sizeof(MxShellDev) % 128 == 96, "shell records of 736 + 128 k bytes: four distinct bank offsets");
 
@@ -164,6 +164,9 @@ struct MxTables {
   double dith_amp[3], dith_period[3], dith_phase[3], nominal_roll, aspect_blur, start_time;
   double dith_inv_period[3];    // correctly rounded 1 / dith_period
   int32_t dith_amp_exp[3];      // dith_amp <= 2^dith_amp_exp (sine_to_float)
+  int32_t dith_qexp[2], p_unturned;   // 4 / dith_period = dith_q 2^dith_qexp; no paraboloid is turned (fwd[0] the identity)
+  uint64_t dith_q[2];           // 2^63 <= dith_q < 2^64, truncated; 0: the phase is not zero (dither_sine does not apply)
+  float dith_ampf[2][2], aspect_blurf[2];   // dith_amp and aspect_blur as hi + lo
   float roll_f;                 // (float) nominal_roll, the roll of every photon when roll_fixed
   int32_t roll_fixed, roll_zero;// roll amplitude 0: the roll angle is the same for every photon (zero: no roll)
   double roll_cos, roll_sin;    // cos and sin of -(float) nominal_roll, when roll_fixed
