@@ -41,7 +41,7 @@ static int upload_model(mx_context *c) {
          o_fe = put(blob, M.fold_ealpha), o_ft = put(blob, M.fold_theta), o_gr = put(blob, M.gratings),
          o_sl = put(blob, M.optc_slope), o_fi = put(blob, M.fold_inv_de),
          o_ge = put(blob, M.geff_energy), o_gc = put(blob, M.geff_cum), o_ok = put(blob, M.order_k),
-         o_se = put(blob, M.sectors), o_ch = put(blob, M.chips);
+         o_se = put(blob, M.sectors), o_ch = put(blob, M.chips), o_fq = put(blob, M.fold_q), o_ee = put(blob, M.fold_e);
   if (M.support_energy.empty()) { M.support_energy.push_back(0.f); M.support_cum.push_back(0.f); M.support_k.push_back(0.0); }
   size_t o_pe = put(blob, M.support_energy), o_pc = put(blob, M.support_cum), o_pk = put(blob, M.support_k);
   size_t o_ht = put(blob, M.hrc_tab), o_hs = put(blob, M.hrc_slope);
@@ -58,6 +58,8 @@ static int upload_model(mx_context *c) {
   c->T.fold_hdr = (const double *) (b + o_fh);
   c->T.fold_ealpha = (const double *) (b + o_fe);
   c->T.fold_theta = (const float *) (b + o_ft);
+  c->T.fold_q = (const uint64_t *) (b + o_fq);
+  c->T.fold_e = (const float *) (b + o_ee);
   c->T.optc_slope = (const double *) (b + o_sl);
   c->T.fold_inv_de = (const double *) (b + o_fi);
   c->T.gratings = (const MxGratingDev *) (b + o_gr);
@@ -97,9 +99,10 @@ static int configure(mx_context *c, const mx_config *cfg) {
     if (e != cudaSuccess) return cuda_fail(c, e, "querying occupancy");
     if (c->trace_blocks[s] < 1) return fail(c, MX_ERANGE, "trace kernel cannot be resident");
   }
-  cudaError_t e = wave_occupancy((int) c->shared_bytes, &c->wave_blocks);
+  cudaError_t e = wave_occupancy((int) c->shared_bytes, c->wave_blocks);
   if (e != cudaSuccess) return cuda_fail(c, e, "querying occupancy");
-  if (c->wave_blocks < 1) return fail(c, MX_ERANGE, "wavefront kernels cannot be resident");
+  for (int b : c->wave_blocks)
+    if (b < 1) return fail(c, MX_ERANGE, "wavefront kernels cannot be resident");
   return MX_OK;
 }
 
@@ -391,7 +394,7 @@ int mx_trace_queues(mx_context *c, const MxTables &T, const mx_photons *ph, uint
     w.q1 = (MxRec *) queues.ptr;
     w.q2 = (MxRec *) ((char *) queues.ptr + qbytes);
     w.counts = (unsigned int *) ((char *) queues.ptr + 2 * qbytes);
-    e = launch_wavefront(T, io, w, c->num_sms * c->wave_blocks, (int) c->shared_bytes, st);
+    e = launch_wavefront(T, io, w, c->num_sms, c->wave_blocks, (int) c->shared_bytes, st);
     c->launches += wave_kernels(T, stages);
   } else {
     e = launch_trace(T, io, c->num_sms * c->trace_blocks[slots ? 0 : 1], (int) c->shared_bytes, slots != 0, st);

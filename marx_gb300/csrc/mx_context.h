@@ -45,7 +45,7 @@ struct mx_context {
   DevBuf scan;             // compaction block counts
   DevBuf wave;             // wavefront record queues
   DevBuf spec;             // FILE spectrum of the last mx_generate_source call
-  int wave_blocks = 0;     // resident blocks per SM for the wavefront kernels
+  int wave_blocks[5] = {};     // resident blocks per SM of the wavefront kernels a, t, b, c, d
   int mode = MX_MODE_AUTO;
   unsigned long long *d_overrun = nullptr;
   unsigned long long launches = 0;

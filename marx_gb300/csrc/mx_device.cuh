@@ -17,8 +17,10 @@
 #include <cstring>
 #ifdef __CUDACC__
 #define MXD __host__ __device__ __forceinline__
+#define MXD_COLD static __host__ __device__ __noinline__   // steps few photons take, out of the hot path's registers
 #else
 #define MXD inline
+#define MXD_COLD static inline
 #endif
 
 namespace mx {
@@ -215,24 +217,27 @@ MXD D3 mat_mul(const double *m, D3 v) {  // JDM3m_vector_mul (rotate.c:121), row
 
 // Conversions between float and double on the integer pipe.  On GB300 a
 // F2F conversion issues on the FP64 pipe, the one this trace is bound by.
-// f2d is exact (as the cast is); zeros, subnormals, infinities and NaN
-// take the cast.
+// They are inlined many times over, and kernels of this size wait for
+// instructions when they grow, so each is a few integer operations without a
+// branch.  f2d is exact, as the cast is.
 MXD double f2d(float f) {
 #ifdef __CUDA_ARCH__
+  const uint32_t a0 = __float_as_uint(f) & 0x7fffffffu;
+  const bool sub = a0 < 0x00800000u;                                  // zero or subnormal: 2^64 f is a normal number
+  const uint32_t u = sub ? __float_as_uint(f * 0x1p64f) : __float_as_uint(f), a = u & 0x7fffffffu;
+  // the exponent rebiased by 1023 - 127, less the 64; infinity's and NaN's to 2047
+  uint32_t hi = (a >> 3) + (sub ? 832u << 20 : (a0 >= 0x7f800000u ? 1792u << 20 : 896u << 20));
+  hi = a != 0u ? hi : 0u;
+  return __hiloint2double((int) ((u & 0x80000000u) | hi), (int) (u << 29));
+#else
+  return (double) f;
+#endif
+}
+// The same for a normal number or zero; others come out as some number.
+MXD double f2d_normal(float f) {
+#ifdef __CUDA_ARCH__
   const uint32_t u = __float_as_uint(f), a = u & 0x7fffffffu;
-  uint32_t hi, lo;
-  if (a >= 0x00800000u) {               // normal: rebias the exponent by 1023 - 127
-    hi = (a >> 3) + (896u << 20);
-    lo = a << 29;
-    if (a >= 0x7f800000u) hi = 0x7ff00000u | ((a & 0x7fffffu) >> 3);   // infinity, NaN
-  } else if (a != 0u) {                 // subnormal: a 2^-149 with a normalised
-    const uint32_t lz = (uint32_t) __clz((int) a);
-    const uint32_t m = (a << (lz - 8u)) & 0x7fffffu;
-    hi = ((905u - lz) << 20) | (m >> 3);
-    lo = m << 29;
-  } else
-    hi = lo = 0u;
-  return __hiloint2double((int) ((u & 0x80000000u) | hi), (int) lo);
+  return __hiloint2double((int) ((u & 0x80000000u) | (a != 0u ? (a >> 3) + (896u << 20) : 0u)), (int) (u << 29));
 #else
   return (double) f;
 #endif
@@ -242,12 +247,12 @@ MXD double f2d(float f) {
 // single-precision screens only, never for a stored result.
 MXD float d2f_trunc(double d) {
 #ifdef __CUDA_ARCH__
-  const unsigned long long b = (unsigned long long) __double_as_longlong(d);
-  const uint32_t hi = (uint32_t) (b >> 32), lo = (uint32_t) b, e = (hi >> 20) & 0x7ffu;
-  uint32_t r = hi & 0x80000000u;
-  if (e - 897u < 254u) r |= ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
-  else if (e >= 1151u) r |= 0x7f800000u | ((e == 2047u && ((hi & 0xfffffu) | lo)) ? 0x400000u : 0u);
-  return __uint_as_float(r);
+  const uint32_t hi = (uint32_t) __double2hiint(d), lo = (uint32_t) __double2loint(d), e = (hi >> 20) & 0x7ffu;
+  // the 8 low exponent bits rebiased and the 23 high mantissa bits
+  uint32_t r = __funnelshift_l(lo, hi, 3) - 0xC0000000u;
+  if (e >= 1151u) r = 0x7f800000u | (e == 2047u ? (hi & 0xfffffu) << 3 : 0u);
+  if (e < 897u) r = 0u;
+  return __uint_as_float((hi & 0x80000000u) | r);
 #else
   return (float) d;
 #endif
@@ -305,8 +310,9 @@ MXD double rcp_fast(double d) {
 // last ones are summed in single precision where their size keeps the
 // rounding below 2^-48.  The result is within 2^-44 of the true sine or
 // cosine of the double argument.
+struct F2 { float h, l; };   // hi + lo
+MXD double f2_double(F2 a);
 #ifdef __CUDACC__
-struct F2 { float h, l; };
 __device__ __forceinline__ F2 quick_sum(float a, float b) {   // |a| >= |b|
   const float s = __fadd_rn(a, b);
   return {s, __fsub_rn(b, __fsub_rn(s, a))};
@@ -340,29 +346,39 @@ __device__ __forceinline__ F2 df_from(double d) {
 }
 __device__ __forceinline__ double df_to(F2 a) { return f2d(a.h) + f2d(a.l); }
 
+// Product and sum without the last renormalisation (the low part may reach an
+// ulp or two of the high one): for terms that a further step adds to
+// something larger.
+__device__ __forceinline__ F2 df_prod(F2 a, F2 b) {
+  const float p = __fmul_rn(a.h, b.h);
+  float e = __fmaf_rn(a.h, b.h, -p);
+  e = __fmaf_rn(a.h, b.l, e);
+  return {p, __fmaf_rn(a.l, b.h, e)};
+}
+__device__ __forceinline__ F2 df_sum(F2 a, F2 b) {
+  const F2 s = two_sum(a.h, b.h);
+  return {s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l))};
+}
 // d as hi + lo without an FP64 operation: hi the truncation of d to float,
 // lo the 29 bits below it.  |d| outside 2^-60 .. 2^60 gives lo = 0.
 __device__ __forceinline__ F2 split(double d) {
-  const unsigned long long b = dbits(d);
-  const uint32_t hi = (uint32_t) (b >> 32), lo = (uint32_t) b & 0x1FFFFFFFu, e = (hi >> 20) & 0x7ffu;
-  const float l = (float) (int) lo;                                    // below 2^29, rounded to 24 bits
+  const uint32_t hi = (uint32_t) __double2hiint(d), lo = (uint32_t) __double2loint(d), e = (hi >> 20) & 0x7ffu;
+  const float l = (float) (int) (lo & 0x1FFFFFFFu);                  // below 2^29, rounded to 24 bits
   const float scale = __uint_as_float((hi & 0x80000000u) | ((e - (1023u + 52u - 127u)) << 23));   // +-2^(e - 1023 - 52)
   return {d2f_trunc(d), e - 963u < 120u ? l * scale : 0.0f};
 }
 // a normalised hi + lo (|lo| at most half an ulp of hi) as the double nearest
 // it, on the integer pipe: lo in units of the double ulp of hi, a whole
-// number below 2^29, is added to hi's bits.  Sizes outside 2^-63 .. 2^65,
-// and zero, take the FP64 sum.
+// number below 2^29, is added to hi's bits.  For sizes outside 2^-63 .. 2^65
+// lo is left out; hi is finite.
 __device__ __forceinline__ double df_join(F2 a) {
-  const uint32_t u = __float_as_uint(a.h), e = (u >> 23) & 0xffu;
-  if (e - 64u < 128u) {
-    int l = __float2int_rn(a.l * __uint_as_float((306u - e) << 23));   // lo 2^(52 - exponent)
-    if (u & 0x80000000u) l = -l;
-    if ((u & 0x7fffffu) == 0u && l < 0) l += l;                        // below a power of two the ulp halves
-    const unsigned long long m = ((unsigned long long) (((u & 0x7fffffffu) >> 3) + (896u << 20)) << 32) | (u << 29);
-    return __longlong_as_double((long long) ((m + (long long) l) | ((unsigned long long) (u & 0x80000000u) << 32)));
-  }
-  return f2d(a.h) + f2d(a.l);
+  const uint32_t u = __float_as_uint(a.h), e = (u >> 23) & 0xffu, sign = u & 0x80000000u;
+  const float units = a.l * __uint_as_float((306u - e) << 23);       // lo 2^(52 - exponent)
+  int l = __float2int_rn(__uint_as_float(__float_as_uint(units) ^ sign));
+  if ((u & 0x7fffffu) == 0u && l < 0) l += l;                        // below a power of two the ulp halves
+  if (e - 64u >= 128u) l = 0;
+  const long long m = __double_as_longlong(f2d_normal(__uint_as_float(u ^ sign)));
+  return __longlong_as_double((m + (long long) l) | ((long long) (unsigned long long) sign << 32));
 }
 // f 2^-64 for a signed 64-bit f, in units of a quarter turn, as radians
 // (|f| 2^-64 <= 1/2): the top 23 bits of f as a float (a whole number within
@@ -453,8 +469,7 @@ __device__ __forceinline__ F2 df_div(F2 a, F2 b) {
 // 0.05-3 degrees and beta, delta of 1e-9..1e-2, typically 2^-42; the worst
 // case is the numerator of a reflectivity near 1e-7, which cancels in
 // cos - root as the double evaluation does.
-__device__ __forceinline__ void reflectivity_df(double cos_t, float beta, float delta, F2 &num, F2 &den) {
-  const F2 c = df_from(cos_t);
+__device__ __forceinline__ void reflectivity_df(F2 c, float beta, float delta, F2 &num, F2 &den) {
   const F2 nr = two_sum(1.0f, -delta);
   const float b2 = __fmul_rn(beta, beta);
   const F2 bsq = {b2, __fmaf_rn(beta, beta, -b2)};
@@ -581,11 +596,14 @@ __device__ __forceinline__ void df_turn_sincos(unsigned long long f, bool less_e
 // double root; it scales the reflectivity, whose test leaves values within
 // 2^-24 of the threshold to a double comparison that a last-bit difference
 // of the root cannot reach but with a probability near 1e-16).
-MXD double sqrt_of_float(float f) {
+MXD double f2_double(F2 a) { return f2d(a.h) + f2d(a.l); }
+MXD F2 sqrt_of_float(float f) {
 #ifdef __CUDA_ARCH__
-  if (f > 0.0f && f < 3.0e38f) return df_to(df_sqrt(F2{f, 0.0f}));
+  if (f > 0.0f && f < 3.0e38f) return df_sqrt(F2{f, 0.0f});
 #endif
-  return sqrt((double) f);
+  const double r = sqrt((double) f);
+  const float h = (float) r;
+  return F2{h, (float) (r - (double) h)};
 }
 
 // a / b from the correctly rounded reciprocal rb = 1/b by one Markstein
@@ -886,7 +904,7 @@ MXD int quadratic_root(double a, double b, double c, double &rp, double &rm) {
 }
 
 // compute_conic_intersection (hrma.c:411-478) for x^2+y^2+z^2 = a x^2+b x+c.
-MXD int conic_intersection(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal) {
+MXD_COLD int conic_intersection_double(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal) {
   double a = h.a[o], b = h.b[o];
   double t_plus = -x0.x * rcp_fast(p.x), t_minus;
   double x_y = x0.y + t_plus * p.y, x_z = x0.z + t_plus * p.z;
@@ -909,6 +927,75 @@ MXD int conic_intersection(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal)
   return 0;
 }
 
+#ifdef __CUDACC__
+// 1 / sqrt(d), 2^-40 < d < 2^40: the float estimate refined to 2^-44 on the
+// FP32 pipe, then one Newton step in double: three FP64 operations and half
+// an ulp, where the library's takes six.
+__device__ __forceinline__ double rsqrt_seeded(double d) {
+  const double y = df_join(df_rsqrt(split(d)));
+  const double half = __longlong_as_double(__double_as_longlong(y) - (1ll << 52));
+  return fma(half, fma(-(d * y), y, 1.0), y);
+}
+
+// The same intersection for the usual ray, one that crosses the conic once
+// between its ends and not along its surface.  As a function of x the
+// difference G of the squared radii of ray and conic is a quadratic: its
+// values at the ends, in float, show that it changes sign between them (each
+// ten times the float error or more from zero: there is one root inside, and
+// it is the one the reference takes), and give the root to about 0.01 mm.
+// Two Newton steps on the exact equation c + b x + (a - 1) x^2 - y^2 - z^2,
+// its value in double, its derivative and the step in float, square that
+// error away (the first with the quadratic term, 1e-6 mm left at worst, the
+// second times the derivative's 1e-6); what remains is the rounding of the
+// equation's own terms, as in the closed form.  27 FP64 operations with the
+// normal instead of 56.  1: hit; -1: a certain miss (end values of one sign
+// further from zero than the quadratic can bow between them, see
+// paraboloid_missed); 0, for other rays: not known.  Nothing is written but
+// for a hit.
+__device__ __forceinline__ int conic_newton(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal) {
+  const float fx = d2f_trunc(x0.x), fy = d2f_trunc(x0.y), fz = d2f_trunc(x0.z);
+  const float px = d2f_trunc(p.x), py = d2f_trunc(p.y), pz = d2f_trunc(p.z);
+  const float inv = 1.0f / px, my = py * inv, mz = pz * inv;
+  const float xa = h.xlimf[o][0], len = h.xlimf[o][1] - xa, am1 = h.am1f[o];
+  const float ya = fmaf(xa - fx, my, fy), za = fmaf(xa - fx, mz, fz);
+  const float yb = fmaf(len, my, ya), zb = fmaf(len, mz, za);
+  const float ra = fmaf(ya, ya, za * za), rb = fmaf(yb, yb, zb * zb);
+  const float ga = ra - h.r2limf[o][0], gb = rb - h.r2limf[o][1], rise = gb - ga;
+  const float margin = fmaf(1e-5f, ra + rb, 2.0f);
+  const float A = fmaf(my, my, fmaf(mz, mz, -am1)) * len * len, B = rise - A;
+  if (!(fabsf(ga) > margin && fabsf(gb) > margin && (ga < 0.0f) != (gb < 0.0f) && fabsf(rise) > 1000.0f &&
+        fabsf(A) < 0.25f * fabsf(rise))) {
+    const float far = fmaf(0.25f, fabsf(A), margin);
+    return (ga > far && gb > far) || (ga < -far && gb < -far) ? -1 : 0;
+  }
+  // the root of A s^2 + B s + ga in (0, 1), the smaller one (|A| < |rise| / 4)
+  const float q = -0.5f * (B + copysignf(sqrtf(fmaf(B, B, -4.0f * A * ga)), B));
+  const float x = fmaf(ga / q, len, xa), t = (x - fx) * inv;
+  const float slope = fmaf(px, fmaf(2.0f * am1, x, h.bf[o]), -2.0f * fmaf(fmaf(t, py, fy), py, fmaf(t, pz, fz) * pz));
+  const float down = -1.0f / slope, bend = fmaf(px * px, am1, -fmaf(py, py, pz * pz)) * down;
+  const double am = h.am1[o], b = h.b[o], c = h.c[o];
+  double td = f2d_normal(t);
+  D3 r = mk(fma(td, p.x, x0.x), fma(td, p.y, x0.y), fma(td, p.z, x0.z));
+  float d = d2f_trunc(fma(-r.z, r.z, fma(-r.y, r.y, fma(fma(r.x, am, b), r.x, c)))) * down;
+  d = fmaf(d * d, bend, d);
+  td = f2d_normal(d);
+  r = mk(fma(td, p.x, r.x), fma(td, p.y, r.y), fma(td, p.z, r.z));
+  td = f2d_normal(d2f_trunc(fma(-r.z, r.z, fma(-r.y, r.y, fma(fma(r.x, am, b), r.x, c)))) * down);
+  r = mk(fma(td, p.x, r.x), fma(td, p.y, r.y), fma(td, p.z, r.z));
+  x0 = r;
+  const double nx = fma(am, r.x, h.hb[o]);   // ((a - 1) x + b/2, -y, -z)
+  const double s = rsqrt_seeded(fma(nx, nx, fma(r.y, r.y, r.z * r.z)));
+  normal = mk(nx * s, -s * r.y, -s * r.z);
+  return 1;
+}
+#endif
+MXD int conic_intersection(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal) {
+#ifdef __CUDA_ARCH__
+  if (const int r = conic_newton(h, o, x0, p, normal)) return r < 0 ? -1 : 0;
+#endif
+  return conic_intersection_double(h, o, x0, p, normal);
+}
+
 // blur_normal (hrma.c:1054-1093): rotate n by a normal-distributed angle
 // about a random axis perpendicular to it.
 // With e1 = (0, n.z, -n.y) / len the first perpendicular, e2 = n x e1 and
@@ -917,11 +1004,10 @@ MXD int conic_intersection(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal)
 // perp x n = sin(phi) e1 - cos(phi) e2, where
 // e2 = (-len, n.x n.y / len, n.x n.z / len): the two Rodrigues rotations
 // of the reference in closed form, one normalisation.
-MXD void blur_normal(D3 &n, double blur_rad, Rng &rng) {
+MXD void blur_normal_double(D3 &n, double phi_pi, double ang) {
   const double l2 = n.y * n.y + n.z * n.z, inv = mx_rsqrt(l2), len = l2 * inv;
   double s, c;
-  sincospi_fast(2.0 * rng.uniform(), &s, &c);   // phi = 2 pi u
-  double ang = blur_rad * rng.normal();
+  sincospi_fast(phi_pi, &s, &c);   // phi = 2 pi u
   double sa, ca;
   sincos_small(ang, &sa, &ca);
   const double nxy = n.x * n.y, nxz = n.x * n.z;
@@ -930,12 +1016,41 @@ MXD void blur_normal(D3 &n, double blur_rad, Rng &rng) {
   // reference's renormalisation, which moves it by less than 1e-15
   n = ca * n + sa * w;
 }
+// For the calibration's arcsecond angles the change of n, sin(ang) w less
+// (1 - cos(ang)) n, is formed in double-float (to 2^-42 of its 1e-6) and
+// added to n: three FP64 operations instead of about thirty-five.
+MXD void blur_normal(D3 &n, const MxShellDev &h, int o, Rng &rng) {
+#ifdef __CUDA_ARCH__
+  const unsigned long long u = rng.uniform_fixed();
+  const F2 ang = df_prod(F2{h.blurf[o][0], h.blurf[o][1]}, rng.normal_df());
+  if (fabsf(ang.h) < 2e-5f) {
+    F2 s, c;
+    df_turn_sincos(u, false, s, c);
+    const F2 nx = split(n.x), ny = split(n.y), nz = split(n.z);
+    const F2 l2 = df_sum(df_prod(ny, ny), df_prod(nz, nz)), inv = df_rsqrt(l2);
+    const float a2 = ang.h * ang.h;
+    const F2 sa = df_sum(ang, F2{ang.h * a2 * (-1.0f / 6.0f), 0.0f}), si = df_prod(sa, inv), cx = df_prod(c, nx);
+    const float v = -0.5f * a2;   // cos(ang) - 1, below 2e-10
+    const F2 dx = df_prod(sa, df_prod(c, df_prod(l2, inv)));
+    const F2 dy = df_prod(si, df_sum(df_prod(s, nz), df_neg(df_prod(cx, ny))));
+    const F2 dz = df_prod(df_neg(si), df_sum(df_prod(s, ny), df_prod(cx, nz)));
+    n.x = n.x + df_join(quick_sum(dx.h, fmaf(v, nx.h, dx.l)));
+    n.y = n.y + df_join(df_add(dy, F2{v * ny.h, v * ny.l}));
+    n.z = n.z + df_join(df_add(dz, F2{v * nz.h, v * nz.l}));
+    return;
+  }
+  blur_normal_double(n, 2.0 * unit_from_bits(u >> 11), f2d(ang.h) + f2d(ang.l));
+#else
+  const double phi = 2.0 * rng.uniform();
+  blur_normal_double(n, phi, h.blur[o] * rng.normal());
+#endif
+}
 
 // marx_reflectivity (reflect.c:39-77): polarisation-averaged Fresnel
 // |r|^2 for n = 1 - delta + i beta (Jackson 7.39, 7.41), with
 // |num/den|^2 = |num|^2 / |den|^2, returned as num / den (den > 0) so that
 // the reflectivity test can decide u * den < num without the division.
-MXD void reflectivity_parts(double cos_t, double beta, double delta, double &num, double &den) {
+MXD_COLD void reflectivity_parts(double cos_t, double beta, double delta, double &num, double &den) {
   double nr = 1.0 - delta, ni = beta;
   double sin2 = 1.0 - cos_t * cos_t;                     // sin_theta^2
   double sr = nr * nr - ni * ni, si = 2.0 * nr * ni;     // n^2
@@ -1006,9 +1121,9 @@ MXD double wfold_interp(const MxTables &T, int table, double energy, double sin_
 // the reflection.  reflect_test: normal blur and the reflectivity test;
 // false if the photon is absorbed (p is left as the reference leaves it).
 // pdn receives p.n with the blurred normal n.
-MXD bool reflect_test(const MxTables &T, const MxShellDev &h, int o, D3 p, D3 &n, double &pdn, double beta,
-                      double delta, double corr, Rng &rng) {
-  if (T.use_blur) blur_normal(n, h.blur[o], rng);
+MXD bool reflect_test(const MxTables &T, const MxShellDev &h, int o, D3 p, D3 &n, double &pdn, float beta,
+                      float delta, F2 corr, Rng &rng) {
+  if (T.use_blur) blur_normal(n, h, o, rng);
   pdn = dot(p, n);
   if (!T.ideal) {
     double r = rng.uniform();
@@ -1018,36 +1133,123 @@ MXD bool reflect_test(const MxTables &T, const MxShellDev &h, int o, D3 p, D3 &n
     // then the double-precision values decide, as below
     {
       F2 fn, fd;
-      reflectivity_df(fabs(pdn), d2f_trunc(beta), d2f_trunc(delta), fn, fd);
-      const double x = r * df_to(fd), y = df_to(fn) * corr, gap = x - y, ag = fabs(gap);
-      if (lt_pos(0x1p-100, y) && lt_pos(0x1p-24 * y, ag) && lt_pos(ag, 0x1p+100)) return neg_bit(gap);
+      reflectivity_df(split(fabs(pdn)), beta, delta, fn, fd);
+      const F2 y = df_mul(fn, corr), gap = df_sub(df_mul(split(r), fd), y);
+      const float ag = fabsf(gap.h);
+      if (y.h > 0x1p-40f && ag > 0x1p-24f * y.h && ag < 0x1p+40f) return gap.h < 0.0f;
     }
 #endif
     double num, den;
-    reflectivity_parts(fabs(pdn), beta, delta, num, den);
+    reflectivity_parts(fabs(pdn), f2d(beta), f2d(delta), num, den);
     // r >= rfl * corr with rfl = num / den, den > 0, decided without the
     // division (the two differ only for r within an ulp of the threshold)
-    if (dkey(r * den) >= dkey(num * corr)) return false;
+    if (dkey(r * den) >= dkey(num * f2_double(corr))) return false;
   }
   return true;
 }
 // reflect_finish: specular reflection and WFold scattering.  Returns -1 if
 // the scattering angle exceeds pi/4 (p then holds the specular direction,
 // as in the reference), 0 otherwise.
-MXD int reflect_finish(const MxTables &T, const MxShellDev &h, int o, int table, D3 &p, D3 n, double pdn,
-                       double energy, Rng &rng) {
-  p = p + (-2.0 * pdn) * n;
-  if (!T.use_wfold) return 0;
-  double r = rng.uniform();
-  double dg = wfold_interp(T, table, energy, -pdn, r) * h.scat[o];
-  if (dkey(dg) > dkey(PI / 4)) return -1;
-  if (lt_pos(rng.uniform(), 0.5)) dg = -dg;
-  // JDMv_rotate_unit_vector(p, p x n, dg): with a = p x n, p.a = 0 and
-  // a x p = n - (p.n) p for unit p, so p becomes cos(dg) p + sin(dg) (n - (p.n) p)
+MXD_COLD double wfold_angle(const MxTables &T, int table, double energy, double sin_alpha, double r) {
+  return wfold_interp(T, table, energy, sin_alpha, r);
+}
+// JDMv_rotate_unit_vector(p, p x n, dg): with a = p x n, p.a = 0 and
+// a x p = n - (p.n) p for unit p, p becomes cos(dg) p + sin(dg) (n - (p.n) p).
+MXD_COLD D3 scatter_double(D3 p, D3 n, double dg) {
   double sg, cg;
   sincos_small(dg, &sg, &cg);
   const double pn = dot(p, n);
-  p = normalized_unit(cg * p + sg * (n + (-pn) * p));
+  return normalized_unit(cg * p + sg * (n + (-pn) * p));
+}
+#ifdef __CUDACC__
+// fold_theta in double-float for a probability p 2^-64 inside the table; tail
+// is set for those in the power law beyond it (1 %), which the double form
+// evaluates.  The cell and the position in it come from a 64 x 64-bit
+// product of p - p_min and 1 / delta_p, exact to 2^-50 of a cell: the angle
+// steepens toward the tail until it would show the 2^-47 of a double-float.
+__device__ __forceinline__ F2 fold_theta_df(const MxTables &T, int table, unsigned a, unsigned long long p, bool &tail) {
+  const ulonglong2 *row = (const ulonglong2 *) T.fold_q + ((size_t) table * MX_FOLD_MAX + a) * 2;
+  const ulonglong2 lim = __ldg(row), step = __ldg(row + 1);   // p_min, p_max; mantissa of 1 / delta_p; num, left and right shifts
+  if (p < lim.x) return {0.0f, 0.0f};
+  if (p >= lim.y) tail = true;
+  // (p - p_min) / delta_p with 55 fraction bits
+  const unsigned long long di = (__umul64hi(p - lim.x, step.x) >> (step.y & 0xffu)) << ((step.y >> 8) & 0xffu);
+  const int num = (int) (step.y >> 32), i = min((int) (di >> 55), num - 1);
+  const float *t = T.fold_theta + ((size_t) table * MX_FOLD_MAX + a) * MX_FOLD_THETA;
+  const float t0 = __ldg(t + i);
+  if (i + 1 >= num) return {t0, 0.0f};
+  const F2 f = quick_sum((float) (int) ((uint32_t) (di >> 31) & 0xffffffu) * 0x1p-24f,
+                         (float) (int) ((uint32_t) (di >> 7) & 0xffffffu) * 0x1p-48f);
+  return df_add(F2{t0, 0.0f}, df_prod(f, two_sum(__ldg(t + i + 1), -t0)));
+}
+// The WFold angle (marx_wfold_table_interp, wfold.c:334-363) in double-float,
+// relative error below 2^-40.  The row is found from the first row's
+// energy and the mean step of the table (the calibration's rows are evenly
+// spaced) and moved if need be.
+__device__ __forceinline__ F2 wfold_df(const MxTables &T, int table, F2 energy, F2 sin_alpha, unsigned long long r,
+                                      bool &tail) {
+  const int num = (int) T.fold_num[table];
+  if (num < 2) { tail = true; return {0.0f, 0.0f}; }
+  const F2 ea = df_mul(energy, sin_alpha);
+  const float4 *row = (const float4 *) T.fold_e + (size_t) table * MX_FOLD_MAX;   // e_alpha, 1 / (next - this)
+  int k = (int) ((ea.h - T.fold_e0[table]) * T.fold_per_e[table]);
+  k = min(max(k, 0), num - 2);
+  const auto below = [&](const float4 &r) { return ea.h < r.x || (ea.h == r.x && ea.l < r.y); };
+  float4 e = __ldg(row + k), next = __ldg(row + k + 1);
+  while (k > 0 && below(e)) { next = e; e = __ldg(row + --k); }
+  while (k < num - 2 && !below(next)) { e = next; next = __ldg(row + ++k + 1); }
+  const F2 t0 = fold_theta_df(T, table, (unsigned) k, r, tail), t1 = fold_theta_df(T, table, (unsigned) k + 1, r, tail);
+  const F2 w = df_prod(df_add(ea, F2{-e.x, -e.y}), F2{e.z, e.w});
+  return df_add(t0, df_prod(df_add(t1, df_neg(t0)), w));
+}
+#endif
+// late: whether a photon scattered into the far tail may be left for later
+// (2 is returned then, with p and the draws as they were): the wavefront
+// gathers these few and turns them on full warps.
+MXD int reflect_finish(const MxTables &T, const MxShellDev &h, int o, int table, D3 &p, D3 n, double pdn,
+                       double energy, Rng &rng, bool late = false) {
+  const D3 q = p + (-2.0 * pdn) * n;
+  if (!T.use_wfold) { p = q; return 0; }
+  const int upos = rng.upos;
+#ifdef __CUDA_ARCH__
+  // Angles below 2^-10 (all but the far tail): the turn as the change it
+  // makes to p, -(1 - cos dg) p + sin dg (n - (p.n) p) with p.n = -pdn, in
+  // double-float, and added to p: three FP64 operations instead of 25, and
+  // none in the tables instead of 20.
+  bool tail = false;
+  const F2 pd = split(pdn);
+  const F2 a = df_mul(wfold_df(T, table, split(energy), df_neg(pd), rng.uniform_fixed(), tail),
+                      F2{h.scatf[o][0], h.scatf[o][1]});
+  if (!tail && fabsf(a.h) < 0x1p-10f) {
+    p = q;
+    const F2 dg = (rng.uniform_fixed() >> 63) ? a : df_neg(a);   // a uniform below 1/2 turns the other way
+    const F2 z = df_sqr(dg);
+    F2 sg = df_sum(dg, F2{-dg.h * (z.h * fmaf(z.h, -1.0f / 120.0f, 1.0f / 6.0f)), 0.0f});
+    F2 v = {0.5f * z.h, fmaf(z.h * z.h, -1.0f / 24.0f, 0.5f * z.l)};   // 1 - cos dg
+    // p x n is sqrt(1 - pdn^2) long, and the turned vector is made unit
+    // again: both coefficients times 1 + (pdn sin dg)^2 / 2 (the next term
+    // is below 1e-18)
+    const float eps = 0.5f * (sg.h * sg.h) * (pd.h * pd.h);
+    sg.l = fmaf(sg.h, eps, sg.l);
+    v.l = v.l + fmaf(v.h, eps, -eps);
+    const F2 px = split(p.x), py = split(p.y), pz = split(p.z);
+    const F2 dx = df_prod(sg, df_sum(split(n.x), df_prod(pd, px))), dy = df_prod(sg, df_sum(split(n.y), df_prod(pd, py))),
+             dz = df_prod(sg, df_sum(split(n.z), df_prod(pd, pz)));
+    p.x = p.x + df_join(df_sub(dx, df_prod(v, px)));
+    p.y = p.y + df_join(df_sub(dy, df_prod(v, py)));
+    p.z = p.z + df_join(df_sub(dz, df_prod(v, pz)));
+    return 0;
+  }
+  rng.upos = upos;
+  if (late) return 2;
+#else
+  (void) upos; (void) late;
+#endif
+  p = q;
+  double dg = wfold_angle(T, table, energy, -pdn, rng.uniform()) * h.scat[o];
+  if (dkey(dg) > dkey(PI / 4)) return -1;
+  if (lt_pos(rng.uniform(), 0.5)) dg = -dg;
+  p = scatter_double(p, n, dg);
   return 0;
 }
 
@@ -1137,7 +1339,8 @@ MXD bool cap_struts_block(const MxTables &T, const MxShellDev &h, D3 x, D3 p) {
 // normal there and p.n, and the optical constants at the photon's energy.
 struct MirrorState {
   D3 x, p, n;
-  double corr, pdn;
+  double pdn;
+  F2 corr;
   float beta, delta;
 };
 
@@ -1153,12 +1356,12 @@ struct MirrorState {
 // alone decides a hit.
 MXD bool paraboloid_missed(const MxShellDev &h, float x0, float y0, float z0, float px, float py, float pz) {
   const float inv = 1.0f / px, my = py * inv, mz = pz * inv;
-  const float xa = h.xlimf[0], xb = h.xlimf[1];
+  const float xa = h.xlimf[0][0], xb = h.xlimf[0][1];
   const float ya = (xa - x0) * my + y0, za = (xa - x0) * mz + z0;
   const float yb = (xb - x0) * my + y0, zb = (xb - x0) * mz + z0;
   const float ra = ya * ya + za * za, rb = yb * yb + zb * zb;
-  const float ga = ra - h.r2limf[0], gb = rb - h.r2limf[1];
-  const float bow = fabsf(my * my + mz * mz - h.am1f) * h.quarter_l2f;
+  const float ga = ra - h.r2limf[0][0], gb = rb - h.r2limf[0][1];
+  const float bow = fabsf(my * my + mz * mz - h.am1f[0]) * h.quarter_l2f;
   const float margin = 2.0f + 1e-5f * (ra + rb) + bow;
   return (ga > margin && gb > margin) || (ga < -margin && gb < -margin);
 }
@@ -1260,7 +1463,7 @@ MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &
 MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
                       Rng &rng, MirrorState &m) {
   const MxShellDev &h = shells[ph.shell];
-  m.beta = 0.0f; m.delta = 1.0f; m.corr = 1.0;
+  m.beta = 0.0f; m.delta = 1.0f; m.corr = F2{1.0f, 0.0f};
   if (T.opt_n) {
     float fe = d2f_rn(ph.e);
     interp2_f(fe, optc, optc + T.opt_n, optc + 2 * T.opt_n, slope, slope + (T.opt_n - 1), T.opt_n, m.beta, m.delta);
@@ -1279,15 +1482,17 @@ MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *
 // Part 3: the rest of the reflection from the paraboloid, back to the MARX
 // frame, cap struts, into the hyperboloid's frame, its intersection, normal
 // blur and reflectivity test.
-MXD bool mirror_middle(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m) {
+// 1: the photon goes on, 0: it ends here, 2: left for later (late), as it was.
+MXD int mirror_middle(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m, bool late = false) {
   const MxShellDev &h = shells[ph.shell];
   D3 x = m.x, p = m.p;
-  if (0 != reflect_finish(T, h, 0, 2 * ph.shell, p, m.n, m.pdn, ph.e, rng)) {
-    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false;
+  if (const int r = reflect_finish(T, h, 0, 2 * ph.shell, p, m.n, m.pdn, ph.e, rng, late)) {
+    if (r == 2) return 2;
+    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0;
   }
   if (T.use_struts && cap_struts_block(T, h, x, p)) {
     paraboloid_to_marx(h, x, p);   // a blocked photon stays in the MARX frame
-    ph.flags |= MX_PHOTON_MIRROR_VBLOCKED; ph.x = x; ph.p = p; return false;
+    ph.flags |= MX_PHOTON_MIRROR_VBLOCKED; ph.x = x; ph.p = p; return 0;
   }
   // into the hyperboloid's frame: bwd[0], less to_osac[0], plus to_osac[1],
   // fwd[1] as one matrix and offset (18 operations instead of 42; within a
@@ -1300,27 +1505,30 @@ MXD bool mirror_middle(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng 
            fma(M[6], x.x, fma(M[7], x.y, fma(M[8], x.z, c[2]))));
   }
   D3 n;
-  if (-1 == conic_intersection(h, 1, x, p, n)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false; }
+  if (-1 == conic_intersection(h, 1, x, p, n)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0; }
   if (!reflect_test(T, h, 1, p, n, m.pdn, m.beta, m.delta, m.corr, rng)) {
-    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return false;
+    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0;
   }
   m.x = x; m.p = p; m.n = n;
-  return true;
+  return 1;
 }
 
 // Part 4: the rest of the reflection from the hyperboloid, back to the
 // MARX frame, post-collimator struts.  Leaves the photon in ph.
-MXD void mirror_back(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m) {
+// False when the photon is left for later (late), as it was.
+MXD bool mirror_back(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m, bool late = false) {
   const MxShellDev &h = shells[ph.shell];
   D3 x = m.x, p = m.p;
-  if (0 != reflect_finish(T, h, 1, 2 * ph.shell + 1, p, m.n, m.pdn, ph.e, rng)) {
-    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return;
+  if (const int r = reflect_finish(T, h, 1, 2 * ph.shell + 1, p, m.n, m.pdn, ph.e, rng, late)) {
+    if (r == 2) return false;
+    ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return true;
   }
   p = mat_mul(h.bwd[1], p);
   x = mat_mul(h.bwd[1], x);
   x = x - mk(h.to_osac[1][0], h.to_osac[1][1], h.to_osac[1][2]);
   if (T.use_struts && struts_block(T, 2, x, p)) ph.flags |= MX_PHOTON_MIRROR_VBLOCKED;
   ph.x = x; ph.p = p;
+  return true;
 }
 
 MXD void mirror_stage(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
@@ -2154,7 +2362,7 @@ MXD void drake_reflect(const MxTables &T, const MxHrcDev &h, Ph &ph, Rng &rng) {
       // the double-float reflectivity decides unless u den and num lie
       // within 2^-24 of each other, as in reflect_test
       F2 fn, fd;
-      reflectivity_df(fabs(pdn), beta, delta, fn, fd);
+      reflectivity_df(split(fabs(pdn)), beta, delta, fn, fd);
       const double y = df_to(fn), gap = y - u * df_to(fd), ag = fabs(gap);
       if (lt_pos(0x1p-100, y) && lt_pos(0x1p-24 * y, ag) && lt_pos(ag, 0x1p+100)) blocked = neg_bit(gap) ? 1 : 0;
     }

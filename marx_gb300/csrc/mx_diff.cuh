@@ -238,7 +238,7 @@ template <class S> MXG S fresnel(const S &cos_t, double beta, double delta) {
     // the value alone: in double-float on the FP32 pipe (mx::reflectivity_df,
     // beta and delta are floats), within about 2^-40 of the expression below
     mx::F2 num, den;
-    mx::reflectivity_df(cos_t, mx::d2f_trunc(beta), mx::d2f_trunc(delta), num, den);
+    mx::reflectivity_df(mx::split(cos_t), mx::d2f_trunc(beta), mx::d2f_trunc(delta), num, den);
     return mx::df_to(mx::df_div(num, den));
   }
 #endif

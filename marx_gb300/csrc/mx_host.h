@@ -24,7 +24,8 @@ struct HostModel {
   std::vector<float> optc;
   std::vector<double> optc_slope;
   std::vector<double> fold_hdr, fold_ealpha, fold_inv_de;
-  std::vector<float> fold_theta;
+  std::vector<float> fold_theta, fold_e;
+  std::vector<uint64_t> fold_q;
   std::vector<MxGratingDev> gratings;
   std::vector<float> geff_energy, geff_cum;
   std::vector<double> order_k, sectors;

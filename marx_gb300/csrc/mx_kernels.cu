@@ -1,6 +1,8 @@
 // Trace, compaction and probe kernels.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "mx_device.cuh"
 #include "mx_kernels.cuh"
 #include "mx_wave.cuh"
@@ -26,7 +28,8 @@ __device__ __forceinline__ void store_det_dither(const MxTables &T, const TraceI
 
 // Fused dither -> mirror -> grating -> detector trace, one photon per
 // thread, grid-stride over the photon list with a resident grid.
-__global__ void __launch_bounds__(MX_TRACE_BLOCK) mx_trace_kernel(MxTables T, TraceIO io) {
+__global__ void __launch_bounds__(MX_TRACE_BLOCK) mx_trace_kernel(const __grid_constant__ MxTables T,
+                                                                  const __grid_constant__ TraceIO io) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
 
@@ -198,13 +201,30 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 // given an order to queue 2 for phase D (diffraction and detector).
 // Appends are warp-aggregated (one atomic per warp); the order of records
 // in a queue does not affect any photon's result.
-// Bound by the FP64 pipe (62-74 % busy per phase).  With the intersection in
-// phase A its 56 FP64 operations ran for every photon, and half of them miss:
-// per 1e6 plain_scatter photons phase A + T took 326 + 66 us and 5.2e6 FP64
-// instructions, with it in phase T 199 + 165 us and 4.0e6 (1e7 photons 5.76
-// -> 5.37 ms, 1e6 on axis 416 -> 368 us, the 256-source batch 17.4 -> 15.3 ms).
+//
+// GB300 issues an FP64 instruction every 16 cycles per SM, an FP32 one four
+// times a cycle, so the phases keep in double only what a double must hold:
+// positions, directions and their sums.  Angles are reduced on the integer
+// pipe; what a reflection changes (blur, scattering, dither: 1e-4 or less of
+// a unit vector) is formed in double-float on the FP32 pipe and added; roots
+// and reciprocals start from FP32 seeds; conversions run on the integer pipe.
+// FP64 instructions per warp and time per 1e6 plain_scatter photons, when
+// everything was in double / with the intersection behind the miss screen /
+// with phase A's angles off the pipe / with blur, scattering and the Newton
+// intersection:
+//   A 140  69  12  14     326 199 126 110 us
+//   T  52 128 128  57      66 165 167 108
+//   B 222 222 222 113     180 188 181 147
+//   C 116 116 116  81      89  89  88  79
+// 1e7 photons 5.76 5.37 4.70 3.83 ms; 1e6 on axis 416 368 340 284 us.  A is
+// bound by the issue of FP32 and integer instructions now (61 %), C by the
+// FP64 pipe (60 %), T and B by latency (FP64 46 and 51 %, issue 43 and 31 %;
+// B also waits for instructions), which is why A, T and B are compiled for
+// three resident blocks (80 registers, 100 bytes of spills in B) and gain
+// 8-11 % over two, while C loses 6 % and D is not bound by either.
 
-__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_a(MxTables T, TraceIO io, WaveBufs w) {
+__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_A_BLOCKS)
+mx_wave_a(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   const size_t n = io.stride;   // component stride of the 3-vector columns
@@ -285,18 +305,20 @@ __device__ __forceinline__ void wave_pass(const TraceIO &io, const Rec *in, cons
   }
 }
 
-__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_t(MxTables T, TraceIO io, WaveBufs w) {
+__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_T_BLOCKS)
+mx_wave_t(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   wave_pass(io, (const MxRecA *) w.q1, &w.counts[0], w.q2, &w.counts[1],
             [&](Ph &q, Rng &r, MirrorState &m) { return mirror_ptest(T, sh, optc, slope, q, r, m); });
 }
 
-__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_b(MxTables T, TraceIO io, WaveBufs w) {
+__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_B_BLOCKS)
+mx_wave_b(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   wave_pass(io, w.q2, &w.counts[1], w.q1, &w.counts[2],
-            [&](Ph &q, Rng &r, MirrorState &m) { return mirror_middle(T, sh, q, r, m); });
+            [&](Ph &q, Rng &r, MirrorState &m) { return mirror_middle(T, sh, q, r, m) != 0; });
 }
 
 // The end of a photon's trace in phases C and D: the detector (when the
@@ -327,7 +349,8 @@ __device__ __forceinline__ void load_supports(const MxTables &T, const TraceIO &
 // with a grating its vignetting, Rowland torus and order choice, sending the
 // photons given an order to phase D; every other photon runs the detector
 // (without a grating) and is stored here.
-__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_c(MxTables T, TraceIO io, WaveBufs w) {
+__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_C_BLOCKS)
+mx_wave_c(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   const uint32_t count = *(volatile unsigned int *) &w.counts[2];
@@ -363,7 +386,8 @@ __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_c(M
 
 // Phase D (with a grating): the diffraction into the chosen order (and the
 // LETG's supports), the detector and the output columns.
-__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_d(MxTables T, TraceIO io, WaveBufs w) {
+__global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_D_BLOCKS)
+mx_wave_d(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   const uint32_t count = *(volatile unsigned int *) &w.counts[3];
@@ -388,34 +412,29 @@ __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_MIN_BLOCKS) mx_wave_d(M
   }
 }
 
-cudaError_t wave_occupancy(int shared_bytes, int *blocks_per_sm) {
+cudaError_t wave_occupancy(int shared_bytes, int blocks_per_sm[5]) {
   const void *f[5] = {(const void *) mx_wave_a, (const void *) mx_wave_t, (const void *) mx_wave_b,
                       (const void *) mx_wave_c, (const void *) mx_wave_d};
-  int best = 1 << 30;
   for (int k = 0; k < 5; k++) {
-    int b = 0;
     cudaError_t e = cudaFuncSetAttribute(f[k], cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm[k], f[k], MX_WAVE_BLOCK, shared_bytes);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f[k], MX_WAVE_BLOCK, shared_bytes);
-    if (e != cudaSuccess) return e;
-    if (b < best) best = b;
   }
-  *blocks_per_sm = best;
   return cudaSuccess;
 }
 
-cudaError_t launch_wavefront(const MxTables &T, const TraceIO &io, const WaveBufs &w, int grid, int shared_bytes,
-                             cudaStream_t st) {
-  uint32_t need = (io.n + MX_WAVE_BLOCK - 1) / MX_WAVE_BLOCK;
-  int ga = (uint32_t) grid > need ? (int) need : grid;
-  if (ga < 1) ga = 1;
+cudaError_t launch_wavefront(const MxTables &T, const TraceIO &io, const WaveBufs &w, int num_sms,
+                             const int blocks_per_sm[5], int shared_bytes, cudaStream_t st) {
+  const uint32_t need = (io.n + MX_WAVE_BLOCK - 1) / MX_WAVE_BLOCK;
+  auto grid = [&](int k) { return std::max(1u, std::min((uint32_t) (num_sms * blocks_per_sm[k]), need)); };
   cudaError_t e = cudaMemsetAsync(w.counts, 0, 4 * sizeof(unsigned int), st);
   if (e != cudaSuccess) return e;
-  mx_wave_a<<<ga, MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
-  mx_wave_t<<<ga, MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
-  mx_wave_b<<<ga, MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
-  mx_wave_c<<<ga, MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
-  if (wave_kernels(T, io.stages) == 5) mx_wave_d<<<ga, MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
+  mx_wave_a<<<grid(0), MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
+  mx_wave_t<<<grid(1), MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
+  mx_wave_b<<<grid(2), MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
+  mx_wave_c<<<grid(3), MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
+  if (wave_kernels(T, io.stages) == 5) mx_wave_d<<<grid(4), MX_WAVE_BLOCK, shared_bytes, st>>>(T, io, w);
   return cudaGetLastError();
 }
 
@@ -553,7 +572,7 @@ __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, d
 #ifdef __CUDA_ARCH__
     const double c = x[3 * i], b = x[3 * i + 1], d = x[3 * i + 2];
     mx::F2 fn, fd;
-    mx::reflectivity_df(c, mx::d2f_trunc(b), mx::d2f_trunc(d), fn, fd);
+    mx::reflectivity_df(mx::split(c), mx::d2f_trunc(b), mx::d2f_trunc(d), fn, fd);
     double num, den;
     mx::reflectivity_parts(c, b, d, num, den);
     y[4 * i] = mx::df_to(fn); y[4 * i + 1] = mx::df_to(fd);

@@ -7,8 +7,14 @@
 #include "mx_model.h"
 
 #define MX_TRACE_BLOCK 256
-#define MX_WAVE_BLOCK 256         // threads per block of the wavefront kernels
-#define MX_WAVE_MIN_BLOCKS 2     // resident blocks per SM they are compiled for: up to 128 registers, no spills (256 x 3 with 80 registers and 256 x 4, 128 x 5 and 128 x 7 measured no faster)
+// Threads per block of the wavefront kernels, and the resident blocks per SM
+// each is compiled for.
+#define MX_WAVE_BLOCK 256
+#define MX_WAVE_A_BLOCKS 3
+#define MX_WAVE_T_BLOCKS 3
+#define MX_WAVE_B_BLOCKS 3
+#define MX_WAVE_C_BLOCKS 2
+#define MX_WAVE_D_BLOCKS 2
 #define MX_WAVE_KERNELS 4        // kernels of one wavefront trace without a grating (5 with one)
 #define MX_COMPACT_THREADS 256
 #define MX_COMPACT_ITEMS 16
@@ -37,8 +43,8 @@ struct TraceIO {
 // One photon between wavefront phases (128 bytes, written and read whole).
 struct __align__(16) MxRec {
   double x[3], p[3], n[3];      // state at the last conic intersection: incoming direction, blurred normal
-  double e, t, corr;
-  float beta, delta;
+  double e, t;
+  float corr[2], beta, delta;   // corr: hi + lo
   uint32_t i, tag, flags;       // photon index in the list, generator counter, flags
  uint8_t shell, upos, npos, overrun;   // overrun: a stage already ran past its variate slots
   double pdn;                   // p.n with the blurred normal (reflectivity test passed)
@@ -67,9 +73,9 @@ __host__ __device__ inline int wave_kernels(const MxTables &T, uint32_t stages) 
 }
 
 size_t trace_shared_bytes(const MxTables &T);
-cudaError_t wave_occupancy(int shared_bytes, int *blocks_per_sm);
-cudaError_t launch_wavefront(const MxTables &T, const TraceIO &io, const WaveBufs &w, int grid, int shared_bytes,
-                             cudaStream_t st);
+cudaError_t wave_occupancy(int shared_bytes, int blocks_per_sm[5]);   // of kernels a, t, b, c, d
+cudaError_t launch_wavefront(const MxTables &T, const TraceIO &io, const WaveBufs &w, int num_sms,
+                             const int blocks_per_sm[5], int shared_bytes, cudaStream_t st);
 cudaError_t trace_occupancy(bool philox, int shared_bytes, int *blocks_per_sm);
 // The ACIS FEF pass over the photons the trace put on a chip (a no-op
 // without the chip and pixel columns); seed_dev: the Philox seed in device

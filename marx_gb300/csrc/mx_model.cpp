@@ -109,6 +109,12 @@ static void append_slopes(std::vector<double> &out, const float *x, const float 
   }
 }
 
+// d as the unevaluated sum of two floats.
+static void hi_lo(double d, float f[2]) {
+  f[0] = (float) d;
+  f[1] = (float) (d - (double) f[0]);
+}
+
 // True if every energy row of a cumulative table [energy][order] is
 // non-decreasing in the order index (the trace may then bisect it).
 static bool rows_monotone(const float *cum, size_t nenergy, int norders) {
@@ -835,12 +841,15 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
       for (int k = 0; k < 9; k++) h.bwd0f[k] = (float) h.bwd[0][k];
       for (int r = 0; r < 3; r++) h.osac0f[r] = (float) h.to_osac[0][r];
     }
-    for (int k = 0; k < 2; k++) {
-      const double x = k ? h.xmax[0] : h.xmin[0];
-      h.xlimf[k] = (float) x;
-      h.r2limf[k] = (float) (h.c[0] + x * (h.b[0] + x * h.am1[0]));
+    for (int o = 0; o < 2; o++) {
+      for (int k = 0; k < 2; k++) {
+        const double x = k ? h.xmax[o] : h.xmin[o];
+        h.xlimf[o][k] = (float) x;
+        h.r2limf[o][k] = (float) (h.c[o] + x * (h.b[o] + x * h.am1[o]));
+      }
+      h.am1f[o] = (float) h.am1[o];
+      h.bf[o] = (float) h.b[o];
     }
-    h.am1f = (float) h.am1[0];
     h.quarter_l2f = (float) (0.25 * (h.xmax[0] - h.xmin[0]) * (h.xmax[0] - h.xmin[0]));
     const double *qp = rdb + i * 9;
     h.front_position = cap_pos - qp[2] + h.xmax[0];
@@ -861,6 +870,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
     h.blur[0] = cfg.blur_p[i] * (1.0 / 3600.0 * PI_ / 180.0);
     h.blur[1] = cfg.blur_h[i] * (1.0 / 3600.0 * PI_ / 180.0);
     h.scat[0] = cfg.scat_p[i]; h.scat[1] = cfg.scat_h[i];
+    for (int o = 0; o < 2; o++) { hi_lo(h.blur[o], h.blurf[o]); hi_lo(h.scat[o], h.scatf[o]); }
     const float *corr = pk.get<float>("hrma/corr" + std::to_string(ids[i]), &cnt, err);
     if (!corr) return false;
     h.corr_off = (int32_t) (M.optc.size() - 3 * optn);
@@ -881,6 +891,8 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
   M.fold_ealpha.assign((size_t) 8 * MX_FOLD_MAX, 0.0);
   M.fold_inv_de.assign((size_t) 8 * MX_FOLD_MAX, 0.0);
   M.fold_theta.assign((size_t) 8 * MX_FOLD_MAX * MX_FOLD_THETA, 0.0f);
+  M.fold_q.assign((size_t) 8 * MX_FOLD_MAX * 4, 0);
+  M.fold_e.assign((size_t) 8 * MX_FOLD_MAX * 4, 0.0f);
   for (int i = 0; i < 4; i++)
     for (int o = 0; o < 2; o++) {
       std::string base = std::string("wfold/") + (o ? "h" : "p") + std::to_string(ids[i]);
@@ -900,7 +912,29 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
         dst[7] = 1.0 / hd[7 * a + 2];
         if (a + 1 < narr) M.fold_inv_de[(size_t) t * MX_FOLD_MAX + a] = 1.0 / (hd[7 * (a + 1)] - hd[7 * a]);
         memcpy(&M.fold_theta[((size_t) t * MX_FOLD_MAX + a) * MX_FOLD_THETA], th + a * nmax, nmax * sizeof(float));
+        // p < p_min exactly when p 2^64 < ceil(p_min 2^64), and likewise
+        // above p_max; 1 / delta_p = inv 2^(ex - 64) with 2^63 <= inv < 2^64,
+        // so the high word of (p - p_min) 2^64 times inv is (p - p_min) / delta_p
+        // times 2^(64 - ex): shifted right by 9 - ex (left, if that is
+        // negative) it has 55 fraction bits
+        uint64_t *q = &M.fold_q[((size_t) t * MX_FOLD_MAX + a) * 4];
+        int ex = 0;
+        const double inv = frexp(dst[7], &ex);
+        const double lo = ceil(ldexp(hd[7 * a + 1], 64)), hi = floor(ldexp(hd[7 * a + 3], 64));
+        if (!(dst[7] > 0.0 && ex > -50 && ex < 60 && lo >= 0.0 && hi >= lo && hi < 0x1p64)) {   // never inside: the double form decides
+          q[0] = q[1] = 0;
+          q[3] = (uint64_t) 1 << 32;
+        } else {
+          q[0] = (uint64_t) lo; q[1] = (uint64_t) hi; q[2] = (uint64_t) ldexp(inv, 64);
+          const uint32_t right = ex < 9 ? 9 - ex : 0, left = ex > 9 ? ex - 9 : 0;
+          q[3] = ((uint64_t) (int32_t) hd[7 * a + 6] << 32) | (left << 8) | right;
+        }
+        float *e = &M.fold_e[((size_t) t * MX_FOLD_MAX + a) * 4];
+        hi_lo(hd[7 * a], e); hi_lo(M.fold_inv_de[(size_t) t * MX_FOLD_MAX + a], e + 2);
       }
+      const double span = hd[7 * (narr - 1)] - hd[0];
+      T.fold_e0[t] = (float) hd[0];
+      T.fold_per_e[t] = span > 0 ? (float) ((narr - 1) / span) : 0.0f;
     }
 
   // ---- HETG
@@ -1101,8 +1135,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
     frexp(T.dith_amp[k], &e);   // |amp| = m 2^e, 1/2 <= m < 1
     T.dith_amp_exp[k] = e;
     if (k == 2) break;
-    T.dith_ampf[k][0] = (float) T.dith_amp[k];
-    T.dith_ampf[k][1] = (float) (T.dith_amp[k] - (double) T.dith_ampf[k][0]);
+    hi_lo(T.dith_amp[k], T.dith_ampf[k]);
     // 4 / period = q 2^qexp with 64 bits of q: period = m 2^e with a 53-bit
     // whole m, and 2^115 / m is divided in two steps (2^62 <= 2^115 / m < 2^64)
     T.dith_q[k] = 0;
@@ -1120,8 +1153,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
       T.dith_q[k] = q;
     }
   }
-  T.aspect_blurf[0] = (float) T.aspect_blur;
-  T.aspect_blurf[1] = (float) (T.aspect_blur - (double) T.aspect_blurf[0]);
+  hi_lo(T.aspect_blur, T.aspect_blurf);
   double roll = cfg.roll_nom * (PI_ / 180.0);
   double xr = fmod(roll, 2 * PI_);
   if (xr >= PI_) xr -= (2 * PI_);

@@ -29,13 +29,16 @@ struct MxShellDev {
   // fwd[1] (to_osac[1] - to_osac[0]))
   double mid[9], mid_off[3];
   float bwd0f[9], osac0f[3];                   // bwd[0] and to_osac[0] in float (the cap struts' screen)
-  // Padding to 736 bytes (184 words): the four shells' copies in shared
-  // memory start on banks 0, 24, 16 and 8, so lanes of a warp that load
-  // one field of different shells do not conflict (at 704 bytes shells 0
-  // and 2, and 1 and 3, shared their banks).
-  float xlimf[2], r2limf[2];                   // the paraboloid's x-limits and its squared radii there,
-  float am1f, quarter_l2f;                     // a - 1 and a quarter of its squared length (its miss screen)
-  float frontf, front_fwdf;                    // front_position and front_fwd[0] in float
+  // Padded to 736 + 128 k bytes: the four shells' copies in shared memory
+  // start on banks 0, 24, 16 and 8, so lanes of a warp that load one field of
+  // different shells do not conflict.
+  // in float: x-limits, squared radii there, a - 1 and b of both conics (the
+  // start of the Newton intersection), a quarter of the paraboloid's squared
+  // length (its miss screen), front_position and front_fwd[0]; blur and scat
+  // as hi + lo
+  float xlimf[2][2], r2limf[2][2], am1f[2], bf[2], quarter_l2f, frontf, front_fwdf;
+  float blurf[2][2], scatf[2][2];
+  float bank_pad[17];
 };
 static_assert(sizeof(MxShellDev) % 128 == 96, "shell records of 736 + 128 k bytes: four distinct bank offsets");
 
@@ -141,6 +144,9 @@ struct MxTables {
   const double *fold_inv_de;    // [8][MX_FOLD_MAX]: 1 / (e_alpha[k+1] - e_alpha[k])
   const double *fold_ealpha;    // [8][MX_FOLD_MAX]
   const float *fold_theta;      // [8][MX_FOLD_MAX][MX_FOLD_THETA]
+  const uint64_t *fold_q;       // [8][MX_FOLD_MAX][4]: p_min and p_max in 2^-64; 1/delta_p's mantissa; num << 32 | left shift << 8 | right shift
+  const float *fold_e;          // [8][MX_FOLD_MAX][4]: e_alpha, 1 / (e_alpha[k+1] - e_alpha[k]) as hi + lo
+  float fold_e0[8], fold_per_e[8];   // first e_alpha and rows per unit of it, a guess at a row
   uint32_t fold_num[8];         // table index = 2 * shell + optic
   const MxGratingDev *gratings;
   const float *geff_energy;

@@ -73,7 +73,7 @@ __device__ __forceinline__ void to_rec(MxRec &r, const Ph &q, const MirrorState 
   r.x[0] = m.x.x; r.x[1] = m.x.y; r.x[2] = m.x.z;
   r.p[0] = m.p.x; r.p[1] = m.p.y; r.p[2] = m.p.z;
   r.n[0] = m.n.x; r.n[1] = m.n.y; r.n[2] = m.n.z;
-  r.e = q.e; r.t = q.t; r.corr = m.corr; r.beta = m.beta; r.delta = m.delta;
+  r.e = q.e; r.t = q.t; r.corr[0] = m.corr.h; r.corr[1] = m.corr.l; r.beta = m.beta; r.delta = m.delta;
   r.i = i; r.tag = rng.tag; r.flags = q.flags;
   r.shell = (uint8_t) q.shell; r.upos = (uint8_t) rng.upos; r.npos = (uint8_t) rng.npos;
   r.overrun = rng.overrun ? 1 : 0;
@@ -82,7 +82,7 @@ __device__ __forceinline__ void to_rec(MxRec &r, const Ph &q, const MirrorState 
 
 __device__ __forceinline__ void from_rec(const MxRec &r, Ph &q, MirrorState &m, Rng &rng, const TraceIO &io) {
   m.x = mk(r.x[0], r.x[1], r.x[2]); m.p = mk(r.p[0], r.p[1], r.p[2]); m.n = mk(r.n[0], r.n[1], r.n[2]);
-  m.corr = r.corr; m.beta = r.beta; m.delta = r.delta; m.pdn = r.pdn;
+  m.corr = F2{r.corr[0], r.corr[1]}; m.beta = r.beta; m.delta = r.delta; m.pdn = r.pdn;
   q.e = r.e; q.t = r.t; q.flags = r.flags; q.shell = r.shell; q.set = 0;
   q.x = m.x; q.p = m.p;
   rng.U = io.U; rng.N = io.N; rng.seed = io.seed; rng.n = io.n; rng.i = r.i; rng.tag = r.tag;

@@ -115,3 +115,31 @@ def test_turned_paraboloids(cuda, tmp_path):
     write_pack(pack, S)
     w = W.plain_scatter()
     _against_oracle(w.cfg, w.photons(70_000, seed=8), pack=pack)
+
+
+@pytest.mark.parametrize("blur,scat,emin,emax", [(30.0, 1.0, 0.3, 8.0),      # blur angles past the series' 2e-5 rad
+                                                 (0.3, 40.0, 0.3, 8.0),      # scattering past its 2^-10 rad
+                                                 (0.0, 1.0, 0.02, 12.0),     # energies outside the tables' rows
+                                                 (0.3, 0.0, 0.3, 8.0)])      # no scattering angle at all
+def test_reflections_at_the_edges_of_their_series(cuda, blur, scat, emin, emax):
+    """Blur and scattering on both sides of the angles their double-float
+    forms take: every photon's fate, and where the survivors arrive."""
+    from marx_gb300._native import Engine
+    from oracle.bindings import Oracle
+    w = W.plain_scatter()
+    for k in range(4):
+        w.cfg.blur_p[k] = w.cfg.blur_h[k] = blur
+        w.cfg.scat_p[k] *= scat
+        w.cfg.scat_h[k] *= scat
+    n, r = 70_000, np.random.default_rng(10)
+    ph = w.photons(n, seed=10)
+    ph.energy[:] = np.exp(r.uniform(np.log(emin), np.log(emax), n))
+    q, o = ph.copy(), ph.copy()
+    Engine(w.cfg).trace_host(q, seed=11)
+    Oracle(w.cfg).trace(o, seed=11, threads=os.cpu_count() or 1)
+    for c in ("flags", "mirror_shell", "ccd_num"):
+        np.testing.assert_array_equal(getattr(q, c), getattr(o, c), err_msg=c)
+    good = q.good()
+    assert good.sum() > 1000
+    assert np.max(np.abs(q.x - o.x)[:, good]) < 1e-9
+    assert np.max(np.abs(q.p - o.p)[:, good]) < 1e-12
