@@ -273,8 +273,60 @@ mx_wave_a(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io
   }
 }
 
+// The order in which a warp takes the records of a queue: grid-stride groups
+// of 32, then, when records may be left for later, the block's list of those
+// (a group of 32 to each warp in turn).  Scattering into the far tail takes
+// a logarithm, two exponentials and a rotation in double, 135 FP64
+// operations, for one photon in a hundred: in line, a quarter of the warps
+// would run them for a lane or two.  Gathering pays when a block has many
+// groups (MX_LATE_ROUNDS per warp; with 1, 2, 3, 4 and 6 rounds 2e6
+// plain_scatter photons take 787, 789, 787, 803 and 809 us, 806 without);
+// a shorter queue would only wait for the extra round.  1e7 photons
+// 3.86 -> 3.58 ms, HETG 2e7 8.99 -> 8.43 ms.
+#define MX_LATE_CAP 1024
+#define MX_LATE_ROUNDS 3
+struct LateList {
+  uint32_t rec[MX_LATE_CAP];
+  int n;
+};
+struct Rounds {
+  LateList &list;
+  uint32_t count, base, step;
+  bool late, second;
+  __device__ __forceinline__ Rounds(LateList &l, uint32_t n) : list(l), count(n), second(false) {
+    base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+    step = gridDim.x * blockDim.x;
+    late = count >= MX_LATE_ROUNDS * step;
+  }
+  // The next group: whether there is one, and this lane's record in it (>=
+  // the bound returned in n: none).
+  __device__ __forceinline__ bool next(uint32_t &k, bool &have) {
+    if (!second && base >= count) {
+      if (!late) return false;
+      __syncthreads();   // every warp of the block comes here once
+      second = true;
+      base = threadIdx.x & ~31u;
+      step = blockDim.x;
+      count = (uint32_t) list.n;
+    }
+    if (base >= count) return false;
+    k = base + (threadIdx.x & 31u);
+    have = k < count;
+    if (second && have) k = list.rec[k];
+    base += step;
+    return true;
+  }
+  // Whether a record may be left for later: not in the second pass, and not
+  // when the list could fill up (every thread may add one after it looks).
+  __device__ __forceinline__ bool may_defer() const {
+    return late && !second && *(volatile int *) &list.n < MX_LATE_CAP - MX_WAVE_BLOCK;
+  }
+  __device__ __forceinline__ void defer(uint32_t k) { list.rec[atomicAdd(&list.n, 1)] = k; }
+};
+
 // One queue-to-queue phase: records of `in` (count at *in_count) through
-// `step`; survivors are appended to `out`, the rest stored.
+// `step` (1: goes on, 0: ends, 2: left for later); survivors are appended to
+// `out`, the rest stored.
 __device__ __forceinline__ void load_rec(const MxRecA &r, Ph &q, MirrorState &m, Rng &rng, const TraceIO &io) {
   from_rec_a(r, q, m, rng, io);
 }
@@ -282,23 +334,24 @@ __device__ __forceinline__ void load_rec(const MxRec &r, Ph &q, MirrorState &m, 
   from_rec(r, q, m, rng, io);
 }
 template <typename Rec, typename Step>
-__device__ __forceinline__ void wave_pass(const TraceIO &io, const Rec *in, const unsigned int *in_count, MxRec *out,
+__device__ __forceinline__ void wave_pass(const TraceIO &io, const Rec *in, Rounds rounds, MxRec *out,
                                           unsigned int *out_count, Step step) {
-  const uint32_t count = *(volatile const unsigned int *) in_count;
-  const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = warp * 32; base < count; base += nwarps * 32) {
-    const uint32_t k = base + lane;
+  uint32_t k;
+  bool have;
+  while (rounds.next(k, have)) {
     bool keep = false;
     MxRec rec;
-    if (k < count) {
+    if (have) {
       Ph q; MirrorState m; Rng r;
       const Rec rec_in = in[k];
       load_rec(rec_in, q, m, r, io);
-      if (step(q, r, m)) {
+      const int s = step(q, r, m, rounds.may_defer());
+      if (s == 1) {
         keep = true;
         to_rec(rec, q, m, r, r.i);
-      } else
+      } else if (s == 2)
+        rounds.defer(k);
+      else
         store_core(io, r.i, q, r.overrun);
     }
     append(keep, rec, out, out_count);
@@ -307,18 +360,23 @@ __device__ __forceinline__ void wave_pass(const TraceIO &io, const Rec *in, cons
 
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_T_BLOCKS)
 mx_wave_t(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
+  __shared__ LateList late;
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
-  wave_pass(io, (const MxRecA *) w.q1, &w.counts[0], w.q2, &w.counts[1],
-            [&](Ph &q, Rng &r, MirrorState &m) { return mirror_ptest(T, sh, optc, slope, q, r, m); });
+  Rounds rounds(late, *(volatile const unsigned int *) &w.counts[0]);
+  rounds.late = false;
+  wave_pass(io, (const MxRecA *) w.q1, rounds, w.q2, &w.counts[1],
+            [&](Ph &q, Rng &r, MirrorState &m, bool) { return (int) mirror_ptest(T, sh, optc, slope, q, r, m); });
 }
 
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_B_BLOCKS)
 mx_wave_b(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
+  __shared__ LateList late;
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
-  stage_tables(T, sh, gr, ch, optc, slope);
-  wave_pass(io, w.q2, &w.counts[1], w.q1, &w.counts[2],
-            [&](Ph &q, Rng &r, MirrorState &m) { return mirror_middle(T, sh, q, r, m) != 0; });
+  if (threadIdx.x == 0) late.n = 0;
+  stage_tables(T, sh, gr, ch, optc, slope);   // ends with a barrier
+  wave_pass(io, w.q2, Rounds(late, *(volatile const unsigned int *) &w.counts[1]), w.q1, &w.counts[2],
+            [&](Ph &q, Rng &r, MirrorState &m, bool defer) { return mirror_middle(T, sh, q, r, m, defer); });
 }
 
 // The end of a photon's trace in phases C and D: the detector (when the
@@ -351,17 +409,18 @@ __device__ __forceinline__ void load_supports(const MxTables &T, const TraceIO &
 // (without a grating) and is stored here.
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_C_BLOCKS)
 mx_wave_c(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
+  __shared__ LateList late;
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
-  stage_tables(T, sh, gr, ch, optc, slope);
-  const uint32_t count = *(volatile unsigned int *) &w.counts[2];
+  if (threadIdx.x == 0) late.n = 0;
+  stage_tables(T, sh, gr, ch, optc, slope);   // ends with a barrier
+  Rounds rounds(late, *(volatile const unsigned int *) &w.counts[2]);
   const bool grating = (io.stages & MX_STAGE_GRATING) && T.grating;
-  const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = warp * 32; base < count; base += nwarps * 32) {
-    const uint32_t k = base + lane;
+  uint32_t k;
+  bool have;
+  while (rounds.next(k, have)) {
     bool to_d = false;
     MxRec rec;
-    if (k < count) {
+    if (have) {
       rec = w.q1[k];
       const uint32_t i = rec.i;
       Ph q; MirrorState m; Rng r;
@@ -369,8 +428,9 @@ mx_wave_c(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io
       const int unset = 0x7fff;
       q.order = unset; q.ccd = unset;
       load_supports(T, io, i, q);
-      mirror_back(T, sh, q, r, m);
-      if (!r.overrun && grating && !(q.flags & MX_BAD_PHOTON_MASK)) {
+      const bool done = mirror_back(T, sh, q, r, m, rounds.may_defer());
+      if (!done) rounds.defer(k);
+      else if (!r.overrun && grating && !(q.flags & MX_BAD_PHOTON_MASK)) {
         D3 gx, gp;
         const int chosen = grating_front(T, gr, T.grating, q, r, gx, gp);
         if (chosen >= 0) {
@@ -378,7 +438,7 @@ mx_wave_c(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io
           to_rec_d(rec, gx, gp, q, r, i, chosen);
         }
       }
-      if (!to_d) finish_photon(T, ch, io, i, q, r);
+      if (done && !to_d) finish_photon(T, ch, io, i, q, r);
     }
     if (grating) append(to_d, rec, w.q2, &w.counts[3]);
   }

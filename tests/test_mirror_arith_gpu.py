@@ -143,3 +143,24 @@ def test_reflections_at_the_edges_of_their_series(cuda, blur, scat, emin, emax):
     assert good.sum() > 1000
     assert np.max(np.abs(q.x - o.x)[:, good]) < 1e-9
     assert np.max(np.abs(q.p - o.p)[:, good]) < 1e-12
+
+
+@pytest.mark.parametrize("scat", [1.0, 30.0])
+def test_photons_left_for_later_equal_the_fused_trace(cuda, scat):
+    """A list long enough for phases B and C to gather the far-scattered
+    photons, with few of them and with so many that their lists fill up."""
+    import torch
+    from marx_gb300._native import DevicePhotons, Engine, MODE_FUSED, MODE_WAVEFRONT
+    w = W.plain_scatter()
+    for k in range(4):
+        w.cfg.scat_p[k] *= scat
+        w.cfg.scat_h[k] *= scat
+    eng, out = Engine(w.cfg), []
+    ph = w.photons(3_000_001, seed=12)
+    for mode in (MODE_FUSED, MODE_WAVEFRONT):
+        d = DevicePhotons.from_host(ph)
+        eng.set_mode(mode)
+        eng.trace(d, seed=13)
+        out.append(d)
+    for c in ("x", "p", "flags", "mirror_shell", "ccd_num", "y_pixel", "z_pixel"):
+        assert torch.equal(getattr(out[0], c), getattr(out[1], c)), c
