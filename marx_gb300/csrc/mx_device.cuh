@@ -338,14 +338,6 @@ __device__ __forceinline__ F2 df_mul_f(F2 a, float b) {
   e = __fmaf_rn(a.l, b, e);
   return quick_sum(p, e);
 }
-// d as hi + lo: hi the truncation of d to float, lo that of the remainder
-// (exact in double); |d - hi - lo| < 2^-46 |d|.  One FP64 subtraction.
-__device__ __forceinline__ F2 df_from(double d) {
-  const float h = d2f_trunc(d);
-  return {h, d2f_trunc(d - f2d(h))};
-}
-__device__ __forceinline__ double df_to(F2 a) { return f2d(a.h) + f2d(a.l); }
-
 // Product and sum without the last renormalisation (the low part may reach an
 // ulp or two of the high one): for terms that a further step adds to
 // something larger.
@@ -359,6 +351,19 @@ __device__ __forceinline__ F2 df_sum(F2 a, F2 b) {
   const F2 s = two_sum(a.h, b.h);
   return {s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l))};
 }
+// The sum again for |a| >= |b| (a series' coefficient and the rest of the series).
+__device__ __forceinline__ F2 df_add_less(F2 a, F2 b) {
+  const float s = __fadd_rn(a.h, b.h);
+  return {s, __fadd_rn(__fsub_rn(b.h, __fsub_rn(s, a.h)), __fadd_rn(a.l, b.l))};
+}
+// d as hi + lo: hi the truncation of d to float, lo that of the remainder
+// (exact in double); |d - hi - lo| < 2^-46 |d|.  One FP64 subtraction.
+__device__ __forceinline__ F2 df_from(double d) {
+  const float h = d2f_trunc(d);
+  return {h, d2f_trunc(d - f2d(h))};
+}
+__device__ __forceinline__ double df_to(F2 a) { return f2d(a.h) + f2d(a.l); }
+
 // d as hi + lo without an FP64 operation: hi the truncation of d to float,
 // lo the 29 bits below it.  |d| outside 2^-60 .. 2^60 gives lo = 0.
 __device__ __forceinline__ F2 split(double d) {
@@ -400,23 +405,27 @@ __device__ __forceinline__ void df_sincos(F2 r, F2 &sr, F2 &cr) {
   // from z^4/11! on in single precision
   float g = __fmaf_rn(zf, -0x1.ae7f3ep-41f, 0x1.612462p-33f);
   g = __fmaf_rn(zf, g, -0x1.ae6456p-26f);
-  F2 P = df_add(F2{0x1.71de3ap-19f, 0x1.55b1ccp-45f}, df_mul_f(z, g));
-  P = df_add(F2{-0x1.a01a02p-13f, 0x1.7f97fap-39f}, df_mul(z, P));
-  P = df_add(F2{0x1.111112p-7f, -0x1.dddddep-32f}, df_mul(z, P));
-  P = df_add(F2{-0x1.555556p-3f, 0x1.555556p-28f}, df_mul(z, P));
-  sr = df_add(r, df_mul(r, df_mul(z, P)));
+  F2 P = df_add_less(F2{0x1.71de3ap-19f, 0x1.55b1ccp-45f}, df_prod(z, F2{g, 0.0f}));
+  P = df_add_less(F2{-0x1.a01a02p-13f, 0x1.7f97fap-39f}, df_prod(z, P));
+  P = df_add_less(F2{0x1.111112p-7f, -0x1.dddddep-32f}, df_prod(z, P));
+  P = df_add_less(F2{-0x1.555556p-3f, 0x1.555556p-28f}, df_prod(z, P));
+  sr = df_add(r, df_mul(r, df_prod(z, P)));
   // C(z) = (cos r - 1) / z = -1/2! + z/4! - z^2/6! + ...: from z^5/12! on
   // in single precision
   float gc = __fmaf_rn(zf, 0x1.ae7f3ep-45f, -0x1.93974ap-37f);
   gc = __fmaf_rn(zf, gc, 0x1.1eed8ep-29f);
-  F2 Q = df_add(F2{-0x1.27e4fcp-22f, 0x1.10ec14p-47f}, df_mul_f(z, gc));
-  Q = df_add(F2{0x1.a01a02p-16f, -0x1.7f97fap-42f}, df_mul(z, Q));
-  Q = df_add(F2{-0x1.6c16c2p-10f, 0x1.27d27ep-35f}, df_mul(z, Q));
-  Q = df_add(F2{0x1.555556p-5f, -0x1.555556p-30f}, df_mul(z, Q));
-  Q = df_add(F2{-0.5f, 0.0f}, df_mul(z, Q));
+  F2 Q = df_add_less(F2{-0x1.27e4fcp-22f, 0x1.10ec14p-47f}, df_prod(z, F2{gc, 0.0f}));
+  Q = df_add_less(F2{0x1.a01a02p-16f, -0x1.7f97fap-42f}, df_prod(z, Q));
+  Q = df_add_less(F2{-0x1.6c16c2p-10f, 0x1.27d27ep-35f}, df_prod(z, Q));
+  Q = df_add_less(F2{0x1.555556p-5f, -0x1.555556p-30f}, df_prod(z, Q));
+  Q = df_add_less(F2{-0.5f, 0.0f}, df_prod(z, Q));
   cr = df_add(F2{1.0f, 0.0f}, df_mul(z, Q));
 }
 
+__device__ __forceinline__ F2 df_neg(F2 a) { return {-a.h, -a.l}; }
+__device__ __forceinline__ F2 df_sub(F2 a, F2 b) { return df_add(a, df_neg(b)); }
+__device__ __forceinline__ F2 df_less(F2 a, F2 b) { return df_sum(a, df_neg(b)); }
+__device__ __forceinline__ F2 df_sqr(F2 a) { return df_mul(a, a); }
 // sin or cos of r alone: the two series above with their coefficients
 // selected, sin r = r + r W and cos r = (1 - z/2) + z W with W = z times the
 // next four terms' series, at the cost of one.
@@ -425,32 +434,29 @@ __device__ __forceinline__ F2 df_sin_or_cos(F2 r, bool cosine) {
   const float zf = z.h;
   float g = __fmaf_rn(zf, cosine ? 0x1.ae7f3ep-45f : -0x1.ae7f3ep-41f, cosine ? -0x1.93974ap-37f : 0x1.612462p-33f);
   g = __fmaf_rn(zf, g, cosine ? 0x1.1eed8ep-29f : -0x1.ae6456p-26f);
-  F2 w = df_add(cosine ? F2{-0x1.27e4fcp-22f, 0x1.10ec14p-47f} : F2{0x1.71de3ap-19f, 0x1.55b1ccp-45f}, df_mul_f(z, g));
-  w = df_add(cosine ? F2{0x1.a01a02p-16f, -0x1.7f97fap-42f} : F2{-0x1.a01a02p-13f, 0x1.7f97fap-39f}, df_mul(z, w));
-  w = df_add(cosine ? F2{-0x1.6c16c2p-10f, 0x1.27d27ep-35f} : F2{0x1.111112p-7f, -0x1.dddddep-32f}, df_mul(z, w));
-  w = df_add(cosine ? F2{0x1.555556p-5f, -0x1.555556p-30f} : F2{-0x1.555556p-3f, 0x1.555556p-28f}, df_mul(z, w));
-  w = df_mul(z, w);
+  F2 w = df_add_less(cosine ? F2{-0x1.27e4fcp-22f, 0x1.10ec14p-47f} : F2{0x1.71de3ap-19f, 0x1.55b1ccp-45f}, df_prod(z, F2{g, 0.0f}));
+  w = df_add_less(cosine ? F2{0x1.a01a02p-16f, -0x1.7f97fap-42f} : F2{-0x1.a01a02p-13f, 0x1.7f97fap-39f}, df_prod(z, w));
+  w = df_add_less(cosine ? F2{-0x1.6c16c2p-10f, 0x1.27d27ep-35f} : F2{0x1.111112p-7f, -0x1.dddddep-32f}, df_prod(z, w));
+  w = df_add_less(cosine ? F2{0x1.555556p-5f, -0x1.555556p-30f} : F2{-0x1.555556p-3f, 0x1.555556p-28f}, df_prod(z, w));
+  w = df_prod(z, w);
   const F2 a = cosine ? df_add(F2{1.0f, 0.0f}, F2{-0.5f * z.h, -0.5f * z.l}) : r, b = cosine ? z : r;
   return df_add(a, df_mul(b, w));
 }
 
-__device__ __forceinline__ F2 df_neg(F2 a) { return {-a.h, -a.l}; }
-__device__ __forceinline__ F2 df_sub(F2 a, F2 b) { return df_add(a, df_neg(b)); }
-__device__ __forceinline__ F2 df_sqr(F2 a) { return df_mul(a, a); }
-// sqrt(a), a > 0: the float root s corrected by (a - s^2) / (2 s), the
-// residual from a fused multiply-add (one Newton step; Karp and Markstein
-// 1997).
+// sqrt(a), a > 0: the float root s = a y, y = 1 / sqrt(a) to 2^-22, corrected
+// by (a - s^2) y / 2 with the residual from a fused multiply-add (one Newton
+// step; Karp and Markstein 1997).
 __device__ __forceinline__ F2 df_sqrt(F2 a) {
-  const float s = __fsqrt_rn(a.h);
+  const float y = rsqrtf(a.h), s = __fmul_rn(a.h, y);
   const float e = __fadd_rn(__fmaf_rn(-s, s, a.h), a.l);
-  return quick_sum(s, __fmul_rn(e, __fdiv_rn(0.5f, s)));
+  return quick_sum(s, __fmul_rn(e, __fmul_rn(0.5f, y)));
 }
 // 1 / sqrt(a), a > 0: the float estimate y and one Newton step
 // y (1 + (1 - a y^2) / 2), with 1 - a y^2 formed in double-float.
 __device__ __forceinline__ F2 df_rsqrt(F2 a) {
-  const float y = __frsqrt_rn(a.h);
+  const float y = rsqrtf(a.h);
   const float p = __fmul_rn(y, y);
-  const F2 q = df_mul(a, F2{p, __fmaf_rn(y, y, -p)});
+  const F2 q = df_prod(a, F2{p, __fmaf_rn(y, y, -p)});
   const float e = __fsub_rn(__fsub_rn(1.0f, q.h), q.l);
   return quick_sum(y, __fmul_rn(__fmul_rn(0.5f, y), e));
 }
@@ -470,35 +476,32 @@ __device__ __forceinline__ F2 df_div(F2 a, F2 b) {
 // case is the numerator of a reflectivity near 1e-7, which cancels in
 // cos - root as the double evaluation does.
 __device__ __forceinline__ void reflectivity_df(F2 c, float beta, float delta, F2 &num, F2 &den) {
-  const F2 nr = two_sum(1.0f, -delta);
+  const F2 nr = quick_sum(1.0f, -delta);
   const float b2 = __fmul_rn(beta, beta);
   const F2 bsq = {b2, __fmaf_rn(beta, beta, -b2)};
-  const F2 sr = df_sub(df_sqr(nr), bsq);
-  const F2 si = df_mul_f(nr, 2.0f * beta);
+  const F2 sr = df_less(df_prod(nr, nr), bsq);
+  const F2 si = df_prod(nr, F2{2.0f * beta, 0.0f});
   // wr = sr - (1 - c^2) as c^2 - (delta (2 - delta) + beta^2): the same
   // value without the cancellation of two numbers near 1
-  const F2 k = df_add(df_mul_f(two_sum(2.0f, -delta), delta), bsq);
-  const F2 wr = df_sub(df_sqr(c), k), wi = si;
-  const F2 r = df_sqrt(df_add(df_sqr(wr), df_sqr(wi)));
-  F2 rr, ri;
-  const F2 half_wi = {0.5f * wi.h, 0.5f * wi.l};
-  if (wr.h >= 0.0f) {
-    const F2 h = df_add(r, wr);
-    const F2 hh = {0.5f * h.h, 0.5f * h.l}, inv = df_rsqrt(hh);
-    rr = df_mul(hh, inv); ri = df_mul(half_wi, inv);
-  } else {
-    const F2 h = df_sub(r, wr);
-    const F2 hh = {0.5f * h.h, 0.5f * h.l}, inv = df_rsqrt(hh);
-    rr = df_mul(half_wi, inv); ri = df_mul(hh, inv);
-    if (rr.h < 0.0f) { rr = df_neg(rr); ri = df_neg(ri); }
-  }
-  const F2 ri2 = df_sqr(ri);
-  const F2 a1 = df_add(df_sqr(df_sub(c, rr)), ri2), bb1 = df_add(df_sqr(df_add(c, rr)), ri2);
-  const F2 pr = df_mul(c, sr), pi_ = df_mul(c, si);
-  const F2 a2 = df_add(df_sqr(df_sub(pr, rr)), df_sqr(df_sub(pi_, ri)));
-  const F2 bb2 = df_add(df_sqr(df_add(pr, rr)), df_sqr(df_add(pi_, ri)));
-  const F2 t = df_add(df_mul(a1, bb2), df_mul(a2, bb1));
-  num = {0.5f * t.h, 0.5f * t.l};
+  const F2 k = df_sum(df_prod(quick_sum(2.0f, -delta), F2{delta, 0.0f}), bsq);
+  const F2 wr = df_sub(df_prod(c, c), k), wi = si;
+  const F2 r = df_sqrt(df_sum(df_prod(wr, wr), df_prod(wi, wi)));
+  // h = (r + |wr|) / 2, q = sqrt(h) and wi / (2 q): the root's larger and
+  // smaller part
+  const bool right = wr.h >= 0.0f;
+  const F2 h = df_sum(r, right ? wr : df_neg(wr));
+  const F2 hh = quick_sum(0.5f * h.h, 0.5f * h.l), inv = df_rsqrt(hh);
+  const F2 big = df_prod(hh, inv), small = df_prod(F2{0.5f * wi.h, 0.5f * wi.l}, inv);
+  F2 rr = right ? big : small, ri = right ? small : big;
+  if (!right && rr.h < 0.0f) { rr = df_neg(rr); ri = df_neg(ri); }
+  const F2 ri2 = df_prod(ri, ri);
+  const F2 cm = df_sub(c, rr), cp = df_sum(c, rr);
+  const F2 a1 = df_sum(df_prod(cm, cm), ri2), bb1 = df_sum(df_prod(cp, cp), ri2);
+  const F2 pr = df_prod(c, sr), pi_ = df_prod(c, si);
+  const F2 pm = df_sub(pr, rr), pp = df_sum(pr, rr), im = df_less(pi_, ri), ip = df_sum(pi_, ri);
+  const F2 a2 = df_sum(df_prod(pm, pm), df_prod(im, im)), bb2 = df_sum(df_prod(pp, pp), df_prod(ip, ip));
+  const F2 t = df_sum(df_prod(a1, bb2), df_prod(a2, bb1));
+  num = quick_sum(0.5f * t.h, 0.5f * t.l);
   den = df_mul(bb1, bb2);
 }
 #endif
@@ -1572,30 +1575,28 @@ MXD bool aspsol_state(const MxTables &T, double t, float s[6]) {
 // change it makes: p' = p + D with
 //   D = -d p + k n + n x p,  n = (0, sin dec, -cos dec sin ra),
 //   d = 1 - cos dec cos ra,  k = (p.n) (1/2 + d/4 + d^2/8),
-// the terms of D (below 1e-4) in double-float on the FP32 pipe and the sum
-// with p in double.  sin and cos go to x^3 and x^2 (the next terms are
-// below 1e-18 relative) as in sincos_small, and d is formed as
+// the terms of D (below 1e-4) in double-float on the FP32 pipe (in single
+// precision where they are below 1e-9 of those) and the sum with p in
+// double.  sin and cos go to x^3 and x^2 (the next terms are below 1e-18
+// relative) as in sincos_small, and d is formed as
 // (ra^2 + dec^2)/2 - ra^2 dec^2/4, without the cancellation that costs the
 // double evaluation seven digits of d.  Three FP64 operations (the
 // additions to p; the splits and joins run on the integer pipe) instead of
 // about thirty-five; the result is within an ulp or two of the double
 // evaluation.
 __device__ __forceinline__ D3 dither_rotate_df(D3 p, F2 r, F2 e) {
-  const F2 sixth = {0x1.555556p-3f, -0x1.555556p-28f};   // 1/6
-  const F2 r2 = df_sqr(r), e2 = df_sqr(e);
-  const F2 sr = df_sub(r, df_mul(df_mul(r, r2), sixth)), sd = df_sub(e, df_mul(df_mul(e, e2), sixth));
-  const F2 cd = df_add(F2{1.0f, 0.0f}, F2{-0.5f * e2.h, -0.5f * e2.l});
-  const F2 ny = sd, nz = df_neg(df_mul(cd, sr));
-  const F2 h = df_add(r2, e2), q = df_mul(r2, e2);
-  const F2 d = df_sub(F2{0.5f * h.h, 0.5f * h.l}, F2{0.25f * q.h, 0.25f * q.l});
   const F2 px = split(p.x), py = split(p.y), pz = split(p.z);
-  const F2 pn = df_add(df_mul(py, ny), df_mul(pz, nz));
-  const F2 k = df_mul(pn, df_add(F2{0.5f, 0.0f}, df_mul(d, df_add(F2{0.25f, 0.0f}, df_mul_f(d, 0.125f)))));
-  const F2 md = df_neg(d);
-  const F2 dx = df_add(df_mul(md, px), df_sub(df_mul(ny, pz), df_mul(nz, py)));
-  const F2 dy = df_add(df_add(df_mul(md, py), df_mul(k, ny)), df_mul(nz, px));
-  const F2 dz = df_sub(df_add(df_mul(md, pz), df_mul(k, nz)), df_mul(ny, px));
-  return mk(p.x + df_join(dx), p.y + df_join(dy), p.z + df_join(dz));
+  const F2 r2 = df_prod(r, r), e2 = df_prod(e, e), h = df_sum(r2, e2);
+  const F2 d = {0.5f * h.h, __fmaf_rn(-0.25f * r2.h, e2.h, 0.5f * h.l)};
+  // sin dec and -cos dec sin ra: their cubes, 1e-9 of them, in single precision
+  const F2 ny = {e.h, __fmaf_rn(-0x1.555556p-3f * e.h, e2.h, e.l)};
+  const F2 nz = {-r.h, __fmaf_rn(r.h, __fmaf_rn(0x1.555556p-3f, r2.h, 0.5f * e2.h), -r.l)};
+  // in y and z the terms d p and k n are below 1e-9 of n x p: single precision
+  const float k = 0.5f * __fmaf_rn(py.h, ny.h, __fmul_rn(pz.h, nz.h));
+  const float ty = __fmaf_rn(k, ny.h, -__fmul_rn(d.h, py.h)), tz = __fmaf_rn(k, nz.h, -__fmul_rn(d.h, pz.h));
+  const F2 dx = df_sub(df_less(df_prod(ny, pz), df_prod(nz, py)), df_prod(d, px));
+  const F2 dy = df_prod(nz, px), dz = df_prod(df_neg(ny), px);
+  return mk(p.x + df_join(dx), p.y + df_join(quick_sum(dy.h, dy.l + ty)), p.z + df_join(quick_sum(dz.h, dz.l + tz)));
 }
 
 // (float) (amp[k] sin(2 pi t / period[k])) as the double-precision
