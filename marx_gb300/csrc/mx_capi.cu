@@ -314,6 +314,22 @@ static int pipe_streams(mx_context *c) {
   return e == cudaSuccess ? MX_OK : cuda_fail(c, e, "creating the trace streams");
 }
 
+// Whether a list of n photons takes the wavefront kernels.  In AUTO mode those
+// of MX_WAVEFRONT_MIN_PHOTONS or more do, but without a grating only where
+// the fused kernel could not hold them all at once, a photon to a thread
+// (97 280 on 152 SMs): its single round then saves four launches and the
+// queues (66 000 plain_scatter photons 78 against 116 us, on axis 56 against
+// 75; 100 000 120 against 122; with the HETG 66 000 109 against 145 us but
+// 100 000 173 against 153, with the LETG 66 000 198 against 209 and 100 000
+// 338 against 217).  Both give the same results bit for bit.
+static bool takes_wavefront(const mx_context *c, const MxTables &T, uint32_t n, uint32_t stages) {
+  if (!(stages & MX_STAGE_MIRROR) || c->mode == MX_MODE_FUSED) return false;
+  if (c->mode == MX_MODE_WAVEFRONT) return true;
+  const uint32_t resident = (uint32_t) (c->num_sms * c->trace_blocks[1]) * MX_TRACE_BLOCK;
+  const bool grating = (stages & MX_STAGE_GRATING) && T.grating;
+  return n >= (grating ? MX_WAVEFRONT_MIN_PHOTONS : std::max((uint32_t) MX_WAVEFRONT_MIN_PHOTONS, resident + 1));
+}
+
 // A device trace that takes the wavefront kernels with Philox draws, from
 // MX_SPLIT_MIN_PHOTONS photons, runs as MX_PIPE_STREAMS consecutive parts
 // traced at once on the context's pipeline streams (each with its own
@@ -323,9 +339,7 @@ static int pipe_streams(mx_context *c) {
 // its first photon's index), so the results equal the one-pass trace's.
 int mx_trace_tables(mx_context *c, const MxTables &T, const mx_photons *ph, uint32_t stages, const double *U,
                     const double *N, uint64_t seed, cudaStream_t st, bool fresh) {
-  const bool wave = ph && (stages & MX_STAGE_MIRROR) &&
-                    (c->mode == MX_MODE_WAVEFRONT || (c->mode == MX_MODE_AUTO && ph->n >= MX_WAVEFRONT_MIN_PHOTONS));
-  if (!wave || U || N || ph->n < MX_SPLIT_MIN_PHOTONS)
+  if (!ph || !takes_wavefront(c, T, ph->n, stages) || U || N || ph->n < MX_SPLIT_MIN_PHOTONS)
     return mx_trace_queues(c, T, ph, stages, U, N, seed, st, fresh, c->wave);
   TraceIO io;   // the argument checks, before anything is queued
   int r = mx_trace_io(c, T, ph, stages, U, N, seed, fresh, io, "mx_trace");
@@ -383,10 +397,8 @@ int mx_trace_queues(mx_context *c, const MxTables &T, const mx_photons *ph, uint
   if (r) return r;
   io.tag0 = tag0;
   int slots = U != nullptr;
-  bool wave = (stages & MX_STAGE_MIRROR) &&
-              (c->mode == MX_MODE_WAVEFRONT || (c->mode == MX_MODE_AUTO && (force_wave || ph->n >= MX_WAVEFRONT_MIN_PHOTONS)));
   cudaError_t e;
-  if (wave) {
+  if ((stages & MX_STAGE_MIRROR) && c->mode != MX_MODE_FUSED && (force_wave || takes_wavefront(c, T, ph->n, stages))) {
     size_t qbytes = (size_t) ph->n * sizeof(MxRec);
     e = queues.ensure(2 * qbytes + 256);
     if (e != cudaSuccess) return cuda_fail(c, e, "allocating wavefront queues");

@@ -6,7 +6,10 @@
 
 #include "mx_model.h"
 
-#define MX_TRACE_BLOCK 256
+// Threads per block of the fused kernel: its lists are short, and small blocks
+// spread them evenly over the SMs (48611 HETG photons 107 us at 256 threads,
+// 97 at 128, 94 at 64, 95 at 32; a thousand photons 58, 55, 56, 56 us).
+#define MX_TRACE_BLOCK 64
 // Threads per block of the wavefront kernels, and the resident blocks per SM
 // each is compiled for.
 #define MX_WAVE_BLOCK 256

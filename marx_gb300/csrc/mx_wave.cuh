@@ -22,6 +22,11 @@ __device__ __forceinline__ void copy_words(uint32_t *dst, const uint32_t *src, s
   for (size_t k = threadIdx.x; k < words; k += blockDim.x) dst[k] = __ldg(src + k);
 }
 
+__device__ __forceinline__ void copy_quads(void *dst, const void *src, uint32_t quads) {   // both 16-byte aligned
+#pragma unroll 4
+  for (uint32_t k = threadIdx.x; k < quads; k += blockDim.x) ((uint4 *) dst)[k] = __ldg((const uint4 *) src + k);
+}
+
 // Shared-memory layout: shells | gratings | chips | optical-constant and
 // correction tables (float) | their interval slopes (double).
 __device__ __forceinline__ void stage_tables(const MxTables &T, MxShellDev *&sh, MxGratingDev *&gr, MxChipDev *&ch,
@@ -34,9 +39,11 @@ __device__ __forceinline__ void stage_tables(const MxTables &T, MxShellDev *&sh,
   ch = (MxChipDev *) (smem + o_ch);
   optc = (float *) T.optc;
   slope = (double *) T.optc_slope;
-  copy_words((uint32_t *) sh, (const uint32_t *) T.shells, 4 * sizeof(MxShellDev) / 4);
-  copy_words((uint32_t *) gr, (const uint32_t *) T.gratings, MX_MAX_GRATINGS * sizeof(MxGratingDev) / 4);
-  copy_words((uint32_t *) ch, (const uint32_t *) T.chips, MX_MAX_CHIPS * sizeof(MxChipDev) / 4);
+  static_assert(4 * sizeof(MxShellDev) % 16 == 0 && MX_MAX_GRATINGS * sizeof(MxGratingDev) % 16 == 0 &&
+                MX_MAX_CHIPS * sizeof(MxChipDev) % 16 == 0, "tables copied 16 bytes at a time");
+  copy_quads(sh, T.shells, 4 * sizeof(MxShellDev) / 16);
+  copy_quads(gr, T.gratings, MX_MAX_GRATINGS * sizeof(MxGratingDev) / 16);
+  copy_quads(ch, T.chips, MX_MAX_CHIPS * sizeof(MxChipDev) / 16);
   __syncthreads();
 }
 
