@@ -1721,40 +1721,95 @@ MXD D3 comb3(double a, D3 l, double b, D3 d, double c, D3 n) {
   return mk(fma(a, l.x, fma(b, d.x, MX_DMUL(c, n.x))), fma(a, l.y, fma(b, d.y, MX_DMUL(c, n.y))),
             fma(a, l.z, fma(b, d.z, MX_DMUL(c, n.z))));
 }
-// intersect + newtons_quartic (diffract.c:622-687): Rowland torus.
-MXD int rowland_intersect(D3 &x0, D3 p, double rowland) {
-  double t = -x0.x * rcp_fast(p.x);
-  x0 = mk(0.0, x0.y + p.y * t, x0.z + p.z * t);
-  double pxpz = p.x * p.x + p.z * p.z;
-  double x2 = x0.z * x0.z + x0.y * x0.y;
-  double r2 = rowland * rowland;
-  double pdotx = p.y * x0.y + p.z * x0.z;
-  double a = 4.0 * pdotx;
-  double b = 2.0 * x2 + a * pdotx - r2 * pxpz;
-  double c = a * x2 - 2.0 * r2 * p.z * x0.z;
-  double d = x2 * x2 - r2 * x0.z * x0.z;
-  double t0 = -rowland * sqrt_fast(pxpz);
+// intersect + newtons_quartic (diffract.c:622-687): Rowland torus, the root
+// of t^4 + a t^3 + b t^2 + c t + d near -R sqrt(px^2 + pz^2).
+MXD_COLD int newtons_quartic(double a, double b, double c, double d, double t0, double &root) {
   double a2 = 2.0 * a, a3 = 3.0 * a, b2 = 2.0 * b;
   for (int it = 0; it < 10; it++) {
     double tt = t0 * t0;
     double num = tt * (3.0 * tt + a2 * t0 + b) - d;
     double den = tt * (4.0 * t0 + a3) + b2 * t0 + c;
-    t = num * rcp_fast(den);
-    if (lt_pos(fabs(t - t0), 1.0e-4)) { x0 = x0 + t * p; return 0; }
+    double t = num * rcp_fast(den);
+    if (lt_pos(fabs(t - t0), 1.0e-4)) { root = t; return 0; }
     t0 = t;
   }
   return -1;
 }
+// The Newton iteration runs in single precision until its step falls below
+// 0.1 mm (a root to about 0.01 mm); two more steps with the quartic's value
+// in double and its derivative in float leave 1e-13 mm: ten FP64 operations
+// where two or three iterations in double take 20 each.
+MXD int rowland_intersect(D3 &x0, D3 p, double rowland) {
+  double t = -x0.x * rcp_fast(p.x);
+  x0 = mk(0.0, fma(p.y, t, x0.y), fma(p.z, t, x0.z));
+  const double pxpz = fma(p.x, p.x, MX_DMUL(p.z, p.z)), z2 = MX_DMUL(x0.z, x0.z);
+  const double x2 = fma(x0.y, x0.y, z2), r2 = MX_DMUL(rowland, rowland);
+  const double pdotx = fma(p.y, x0.y, MX_DMUL(p.z, x0.z));
+  const double a = 4.0 * pdotx;
+  const double b = fma(-r2, pxpz, fma(a, pdotx, 2.0 * x2));
+  const double c = fma(MX_DMUL(-2.0 * r2, p.z), x0.z, MX_DMUL(a, x2));
+  const double d = fma(x2, x2, MX_DMUL(-r2, z2));
+#ifdef __CUDA_ARCH__
+  {
+    const float fa = d2f_trunc(a), fb = d2f_trunc(b), fc = d2f_trunc(c), fd = d2f_trunc(d);
+    float f = -d2f_trunc(rowland) * sqrtf(d2f_trunc(pxpz)), down = 0.0f;
+    bool found = false;
+    for (int it = 0; it < 8 && !found; it++) {
+      const float tt = f * f;
+      down = 1.0f / fmaf(tt, fmaf(4.0f, f, 3.0f * fa), fmaf(2.0f * fb, f, fc));
+      const float next = fmaf(tt, fmaf(3.0f, tt, fmaf(2.0f * fa, f, fb)), -fd) * down;
+      found = fabsf(next - f) < 0.1f;
+      f = next;
+    }
+    if (found) {
+      double r = f2d_normal(f);
+      for (int k = 0; k < 2; k++)
+        r = r - f2d_normal(d2f_trunc(fma(fma(fma(r + a, r, b), r, c), r, d)) * down);
+      x0 = mk(MX_DMUL(r, p.x), fma(r, p.y, x0.y), fma(r, p.z, x0.z));
+      return 0;
+    }
+  }
+#endif
+  if (newtons_quartic(a, b, c, d, -rowland * sqrt_fast(pxpz), t)) return -1;
+  x0 = mk(MX_DMUL(t, p.x), fma(t, p.y, x0.y), fma(t, p.z, x0.z));
+  return 0;
+}
+
+// The facet basis at a point x of the torus: n toward its centre, l and d
+// along and across the lines (l.y = 0).
+struct MxFacet { D3 n, l, d; };
+MXD double unit_scale(double xx) {   // 1 / sqrt(xx), or 1 for 0 (a vector of no length stays as it is)
+  if (is_zero(xx)) return 1.0;
+#ifdef __CUDA_ARCH__
+  if (lt_pos(0x1p-39, xx) && lt_pos(xx, 0x1p+39)) return rsqrt_seeded(xx);
+#endif
+  return mx_rsqrt(xx);
+}
+MXD MxFacet facet_basis(D3 x) {
+  MxFacet f;
+  f.n = -unit_scale(fma(x.x, x.x, fma(x.y, x.y, MX_DMUL(x.z, x.z)))) * x;
+  const double s = unit_scale(fma(f.n.x, f.n.x, MX_DMUL(f.n.z, f.n.z)));
+  f.l = mk(MX_DMUL(s, f.n.z), 0.0, -MX_DMUL(s, f.n.x));
+  f.d = mk(MX_DMUL(f.n.y, f.l.z), fma(f.n.z, f.l.x, -MX_DMUL(f.n.x, f.l.z)), -MX_DMUL(f.n.y, f.l.x));   // n x l
+  return f;
+}
+MXD D3 facet_vector(const MxFacet &f, D3 c) {   // c.x l + c.y d + c.z n
+  return mk(fma(c.x, f.l.x, fma(c.y, f.d.x, MX_DMUL(c.z, f.n.x))), fma(c.y, f.d.y, MX_DMUL(c.z, f.n.y)),
+            fma(c.x, f.l.z, fma(c.y, f.d.z, MX_DMUL(c.z, f.n.z))));
+}
+// The components of a photon's direction along l and d.
+MXD void facet_components(const MxFacet &f, D3 p, double &pl, double &pd) {
+  pl = fma(p.x, f.l.x, MX_DMUL(p.z, f.l.z));
+  pd = fma(p.x, f.d.x, fma(p.y, f.d.y, MX_DMUL(p.z, f.d.z)));
+}
 
 // diffract_photon (diffract.c:706-823) for a primary grating (theta = 0)
-// with facet sectors when the grating has them.
-MXD int diffract_photon(const MxTables &T, const MxGratingDev &g, int order_idx, double energy,
-                        D3 x, D3 &P, Rng &rng) {
-  double nlod = MX_LDG(T.order_k + g.order_off + order_idx) * rcp_fast(energy);
-  const double xx = dot(x, x);
-  const D3 n = is_zero(xx) ? -1.0 * x : (-mx_rsqrt(xx)) * x;   // -x / |x|
-  D3 l = normalized(mk(n.z, 0.0, -n.x));
-  D3 d = cross(n, l);
+// with facet sectors when the grating has them, at the torus point x: the
+// components (l, d, n) of the new direction from pl, pd, those of the old
+// one.  Returns -1, with c untouched, for a photon that is not diffracted.
+MXD int diffract_photon(const MxTables &T, const MxGratingDev &g, int order_idx, double inv_energy,
+                        D3 x, double pl0, double pd0, Rng &rng, D3 &c) {
+  double nlod = MX_LDG(T.order_k + g.order_off + order_idx) * inv_energy;
   double dtheta, dpp;
   if (g.nsec > 0) {
     const double *smin = T.sectors + g.sec_off;          // [6][nsec]: min max dth dthb dpp dppb
@@ -1768,10 +1823,10 @@ MXD int diffract_photon(const MxTables &T, const MxGratingDev &g, int order_idx,
       // in double precision too.  Others take the double-precision search.
       float af = atan2f(d2f_trunc(x.y), d2f_trunc(x.z));
       if (af < 0.0f) af += 6.28318531f;
-      const double a = f2d(af);
+      const double a = f2d(af), lo = f2d(fmaxf(af - 1e-5f, 0.0f)), hi = f2d(af + 1e-5f);
       const unsigned k = bsearch_d(a, smin, ns);
-      if (k > 0 && lt_pos(MX_LDG(smin + k - 1) + 1e-5, a) && lt_pos(a + 1e-5, MX_LDG(smin + ns + k - 1)) &&
-          (k == ns || lt_pos(a + 1e-5, MX_LDG(smin + k))))
+      if (k > 0 && lt_pos(MX_LDG(smin + k - 1), lo) && lt_pos(hi, MX_LDG(smin + ns + k - 1)) &&
+          (k == ns || lt_pos(hi, MX_LDG(smin + k))))
         sn = k - 1;
     }
 #endif
@@ -1796,20 +1851,19 @@ MXD int diffract_photon(const MxTables &T, const MxGratingDev &g, int order_idx,
   // coefficients of l, d and n
   double sn = 0.0, cs = 1.0;
   if (!is_zero(theta)) sincos_small(theta, &sn, &cs);
-  const double pl0 = dot(P, l), pd0 = dot(P, d);
   const double p_l = fma(cs, pl0, MX_DMUL(sn, pd0)), p_d = nlod + fma(cs, pd0, -MX_DMUL(sn, pl0));
   const double pn2 = fma(-p_d, p_d, fma(-p_l, p_l, 1.0));
   if (neg_bit(pn2) && !is_zero(pn2)) return -1;
   double p_n, inv_pn;
   sqrt_rsqrt(pn2, p_n, inv_pn);
   double cl = fma(p_l, cs, -MX_DMUL(p_d, sn)), cd = fma(p_l, sn, MX_DMUL(p_d, cs)), cn = p_n;
-  if (is_zero(dpp)) {
-    P = comb3(cl, l, cd, d, cn, n);
-    return 0;
+  if (!is_zero(dpp)) {
+    const double f = MX_DMUL(nlod, dpp);
+    cl = fma(f, sn, cl); cd = fma(-f, cs, cd); cn = fma(f, MX_DMUL(p_d, inv_pn), cn);
+    const double s = unit_scale(fma(cl, cl, fma(cd, cd, MX_DMUL(cn, cn))));   // made unit again
+    cl = MX_DMUL(s, cl); cd = MX_DMUL(s, cd); cn = MX_DMUL(s, cn);
   }
-  const double f = MX_DMUL(nlod, dpp);
-  cl = fma(f, sn, cl); cd = fma(-f, cs, cd); cn = fma(f, MX_DMUL(p_d, inv_pn), cn);
-  P = normalized(comb3(cl, l, cd, d, cn, n));
+  c = mk(cl, cd, cn);
   return 0;
 }
 
@@ -1830,13 +1884,8 @@ MXD bool order_reaches(const float *c0, int norders, int k, bool flat, double w,
   }
   return !lt_pos(f2d(c), r);
 }
-MXD int choose_order(const float *ge, unsigned n, const float *cum, int norders, bool monotone, float fe, double r) {
-  unsigned lo = 1, hi = n - 1;
-  while (lo < hi) {
-    unsigned mid = (lo + hi) >> 1;
-    if (fe > MX_LDG(ge + mid)) lo = mid + 1; else hi = mid;   // floats compare as their doubles do
-  }
-  unsigned idx = lo;
+MXD_COLD int choose_order_double(const float *ge, unsigned idx, const float *cum, int norders, bool monotone, float fe,
+                                 double r) {
   double x0 = f2d(MX_LDG(ge + idx - 1)), x1 = f2d(MX_LDG(ge + idx)), dx = MX_DADD(x1, -x0);
   double w = MX_DADD(f2d(fe), -x0);
   const float *c0 = cum + (size_t) (idx - 1) * norders;
@@ -1859,29 +1908,53 @@ MXD int choose_order(const float *ge, unsigned n, const float *cum, int norders,
     if (order_reaches(c0, norders, k, flat, w, dx, rdx, r)) return k;
   return -1;
 }
+// The same choice by the same probes in single precision: an interpolated
+// cumulative efficiency (at most 1) is good to 3e-7 there, so that a draw
+// more than 1e-6 from every probe falls on the same side of each in double.
+// Other draws (one in 10^5 or so) take the double form, 10 FP64 operations
+// and 6 for each of 3 to 7 probes.
+MXD int choose_order(const float *ge, unsigned n, const float *cum, int norders, bool monotone, float fe, double r) {
+  unsigned lo = 1, hi = n - 1;
+  while (lo < hi) {
+    unsigned mid = (lo + hi) >> 1;
+    if (fe > MX_LDG(ge + mid)) lo = mid + 1; else hi = mid;   // floats compare as their doubles do
+  }
+  const unsigned idx = lo;
+#ifdef __CUDA_ARCH__
+  const float x0 = MX_LDG(ge + idx - 1), x1 = MX_LDG(ge + idx);
+  if (monotone && fe >= x0 && fe <= x1 && x1 > x0) {
+    const float w = (fe - x0) / (x1 - x0), rf = d2f_trunc(r);
+    const float *c0 = cum + (size_t) (idx - 1) * norders, *c1 = c0 + norders;
+    bool sure = true;
+    int a = 0, b = norders;
+    while (a < b) {
+      const int m = (a + b) >> 1;
+      const float y0 = MX_LDG(c0 + m), gap = fmaf(MX_LDG(c1 + m) - y0, w, y0) - rf;
+      if (!(fabsf(gap) > 1e-6f)) sure = false;
+      if (gap > 0.0f) b = m; else a = m + 1;
+    }
+    if (sure) return a < norders ? a : -1;
+  }
+#endif
+  return choose_order_double(ge, idx, cum, norders, monotone, fe, r);
+}
 
 // diffract_photon for an LETG support grating (diffract_from_support_grating,
-// diffract.c:917-970): no facet sectors, no alignment blur and no dP/P
-// (both zero for the support gratings, though their normals are still
-// drawn), the facet basis rotated about n by the support's fixed angle.
-MXD int diffract_support(const MxTables &T, const MxSupportDev &g, int order_idx, double energy, D3 x, D3 &P,
-                         Rng &rng) {
-  double nlod = MX_LDG(T.support_k + g.order_off + order_idx) * rcp_fast(energy);
-  const double xx = dot(x, x);
-  const D3 n = is_zero(xx) ? -1.0 * x : (-mx_rsqrt(xx)) * x;   // -x / |x|
-  D3 l = normalized(mk(n.z, 0.0, -n.x));
-  D3 d = cross(n, l);
+// diffract.c:917-970) on the direction's components c (l, d, n): no facet
+// sectors, no alignment blur and no dP/P (both zero for the support
+// gratings, though their normals are still drawn), the facet basis rotated
+// about n by the support's fixed angle.
+MXD int diffract_support(const MxTables &T, const MxSupportDev &g, int order_idx, double inv_energy, D3 &c, Rng &rng) {
+  const double nlod = MX_LDG(T.support_k + g.order_off + order_idx) * inv_energy;
   rng.skip_normal();   // dtheta = 0 x N
   rng.skip_normal();   // dP/P = 0 x N
   // the basis turned by the support's angle enters through its components,
   // as in diffract_photon
   const double cs = g.rotate ? g.cos_t : 1.0, sn = g.rotate ? g.sin_t : 0.0;
-  const double pl0 = dot(P, l), pd0 = dot(P, d);
-  const double p_l = fma(cs, pl0, MX_DMUL(sn, pd0)), p_d = nlod + fma(cs, pd0, -MX_DMUL(sn, pl0));
+  const double p_l = fma(cs, c.x, MX_DMUL(sn, c.y)), p_d = nlod + fma(cs, c.y, -MX_DMUL(sn, c.x));
   const double pn2 = fma(-p_d, p_d, fma(-p_l, p_l, 1.0));
   if (neg_bit(pn2) && !is_zero(pn2)) return -1;
-  const double p_n = sqrt_fast(pn2);
-  P = comb3(fma(p_l, cs, -MX_DMUL(p_d, sn)), l, fma(p_l, sn, MX_DMUL(p_d, cs)), d, p_n, n);
+  c = mk(fma(p_l, cs, -MX_DMUL(p_d, sn)), fma(p_l, sn, MX_DMUL(p_d, cs)), sqrt_fast(pn2));
   return 0;
 }
 
@@ -1923,21 +1996,31 @@ MXD int grating_front(const MxTables &T, const MxGratingDev *grs, int kind, Ph &
 MXD void grating_back(const MxTables &T, const MxGratingDev *grs, int kind, Ph &ph, Rng &rng, D3 x, D3 p, int chosen) {
   const bool letg = kind == MX_GRATING_LETG;
   const MxGratingDev &g = grs[(letg ? 4 : 0) + ph.shell];
-  if (-1 == diffract_photon(T, g, chosen, ph.e, x, p, rng)) ph.flags |= MX_PHOTON_UNDIFFRACTED;
-  if (letg) {
-    const float fe = d2f_rn(ph.e);
-    for (int s = 0; s < 4; s++) {
-      const MxSupportDev &sg = T.supports[s];
-      if (!sg.norders) continue;
-      if (ph.flags & MX_BAD_PHOTON_MASK) continue;
-      int k = choose_order(T.support_energy, (unsigned) T.support_nenergy, T.support_cum + sg.cum_off, sg.norders,
-                           sg.monotone != 0, fe, rng.uniform());
-      if (k < 0) { ph.flags |= MX_PHOTON_UNDIFFRACTED; continue; }
-      // order list 0, +1, -1, +2, -2, ... (init_one_grating, diffract.c:392-405)
-      ph.sup[s] = (int8_t) ((k & 1) ? (k + 1) / 2 : -(k / 2));
-      ph.set |= MX_SET_SUPPORT;
-      if (-1 == diffract_support(T, sg, k, ph.e, x, p, rng)) ph.flags |= MX_PHOTON_UNDIFFRACTED;
+  // the primary and the supports diffract at one point: one facet basis, and
+  // the direction kept in its components from one to the next
+  const MxFacet f = facet_basis(x);
+  const double inv_energy = rcp_fast(ph.e);
+  double pl, pd;
+  facet_components(f, p, pl, pd);
+  D3 c;
+  if (-1 == diffract_photon(T, g, chosen, inv_energy, x, pl, pd, rng, c)) ph.flags |= MX_PHOTON_UNDIFFRACTED;
+  else {
+    if (letg) {
+      const float fe = d2f_rn(ph.e);
+      for (int s = 0; s < 4; s++) {
+        const MxSupportDev &sg = T.supports[s];
+        if (!sg.norders) continue;
+        if (ph.flags & MX_BAD_PHOTON_MASK) continue;
+        int k = choose_order(T.support_energy, (unsigned) T.support_nenergy, T.support_cum + sg.cum_off, sg.norders,
+                             sg.monotone != 0, fe, rng.uniform());
+        if (k < 0) { ph.flags |= MX_PHOTON_UNDIFFRACTED; continue; }
+        // order list 0, +1, -1, +2, -2, ... (init_one_grating, diffract.c:392-405)
+        ph.sup[s] = (int8_t) ((k & 1) ? (k + 1) / 2 : -(k / 2));
+        ph.set |= MX_SET_SUPPORT;
+        if (-1 == diffract_support(T, sg, k, inv_energy, c, rng)) ph.flags |= MX_PHOTON_UNDIFFRACTED;
+      }
     }
+    p = facet_vector(f, c);
   }
   ph.x = rot_x(x, g.cos_p, g.sin_p);
   ph.p = rot_x(p, g.cos_p, g.sin_p);

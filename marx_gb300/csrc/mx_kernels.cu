@@ -28,7 +28,7 @@ __device__ __forceinline__ void store_det_dither(const MxTables &T, const TraceI
 
 // Fused dither -> mirror -> grating -> detector trace, one photon per
 // thread, grid-stride over the photon list with a resident grid.
-__global__ void __launch_bounds__(MX_TRACE_BLOCK) mx_trace_kernel(const __grid_constant__ MxTables T,
+__global__ void __launch_bounds__(MX_TRACE_BLOCK, 10) mx_trace_kernel(const __grid_constant__ MxTables T,
                                                                   const __grid_constant__ TraceIO io) {
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
@@ -222,6 +222,13 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 // B also waits for instructions), which is why A, T and B are compiled for
 // three resident blocks (80 registers, 100 bytes of spills in B) and gain
 // 8-11 % over two, while C loses 6 % and D is not bound by either.
+// With a grating: the Rowland torus from a float iteration and two steps on
+// the quartic's double value, the order choice decided in float away from
+// its thresholds, and one facet basis for the LETG's primary and four
+// supports, whose direction stays in its components: per 2e6 photons C
+// 114 -> 95 us and D 45 -> 51 (HETG) and 219 -> 190 us (LETG, 3.4e6 -> 2.0e6
+// FP64 instructions); HETG 2e7 7.73 -> 7.08 ms, LETG + HRC-S 4e6 2.35 ->
+// 1.88 ms.
 
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_A_BLOCKS)
 mx_wave_a(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io, const __grid_constant__ WaveBufs w) {
