@@ -33,11 +33,18 @@ struct MxSourceDev {
 };
 static_assert(sizeof(MxSourceDev) % 16 == 0, "source record size");
 
+// The directions and sizes of a GAUSS or DISK source as hi + lo floats: p, its
+// normal pn, pn x p, and a, b, c.
+struct MxSourceFine {
+  float p[3][2], pn[3][2], w[3][2], a[2], b[2], c[2];
+};
+
 #define MX_BATCH_MAX_SOURCES 4096
 
 struct BatchIO {
   TraceIO io;                   // the batch's photon list (n = all photons), fresh outputs
   const MxSourceDev *src;
+  const MxSourceFine *fine;
   const uint32_t *start;        // nsrc + 1 offsets
   int32_t nsrc, tile;
   MxRec *q1, *q2;
@@ -89,8 +96,42 @@ __device__ __forceinline__ unsigned bsearch_cdf(float x, const double *xp, unsig
 // normal by each photon's own azimuth (the reference carries the rotated
 // normal from one photon to the next; each photon's azimuth is uniform
 // either way).
-__device__ __forceinline__ void generate_photon(const MxSourceDev &S, const double *spec, uint64_t seed, uint32_t tag,
-                                                Ph &q) {
+//
+// GAUSS and DISK photons leave p by angles of arcseconds: with the azimuth's
+// sine and cosine and the angle in double-float, the change
+// sin(ang) (cos(phi) pn x p + sin(phi) pn) - (1 - cos(ang)) p is formed on
+// the FP32 pipe and added to p, three FP64 operations where the logarithm,
+// roots, sines and two rotations in double take about 165 (BETA keeps its
+// power law in double).  Angles of 2^-10 rad (200 arcsec) and more take
+// those, and so do all photons of a GAUSS or BETA source of size over 80
+// arcsec, where a warp would run both.  1e6 photons: GAUSS 277 -> 31 us (of
+// 300 arcsec 227), DISK 219 -> 29 us, BETA 391 -> 305 us.
+__device__ __forceinline__ F2 fine(const float f[2]) { return F2{f[0], f[1]}; }
+__device__ __forceinline__ uint64_t source_fixed(uint64_t seed, uint32_t tag, uint32_t k) {
+  uint32_t c[4] = {tag, k, 0x5A5A0003u, 0u};
+  philox(c, (uint32_t) seed, (uint32_t) (seed >> 32));
+  return (((uint64_t) c[0] << 32) | c[1]) & ~(uint64_t) 0x7ff;
+}
+// The angle of a GAUSS, BETA or DISK photon from its source, and the
+// direction at an angle and azimuth 2 pi phi, in double.
+__device__ __forceinline__ double source_angle(const MxSourceDev &S, uint64_t seed, uint32_t tag) {
+  double rnd = source_uniform(seed, tag, 2);
+  if (S.kind == MX_SOURCE_DISK) return S.a * sqrt(S.b + S.c * rnd);
+  for (uint32_t k = 3; rnd == 0.0 && k < 8; k++) rnd = source_uniform(seed, tag, k);
+  return S.kind == MX_SOURCE_GAUSS ? S.a * sqrt(-log(rnd)) : S.a * sqrt(pow(rnd, S.b) - 1.0);
+}
+__device__ __forceinline__ D3 source_direction(const MxSourceDev &S, double ang, double phi) {
+  const D3 p = mk(S.p[0], S.p[1], S.p[2]);
+  double sphi, cphi, sa, ca;
+  sincospi(2.0 * phi, &sphi, &cphi);
+  sincos(ang, &sa, &ca);
+  // p turned by ang about pn turned by the azimuth about p, both
+  // perpendicular to p: along pn x p and pn
+  const D3 pn = mk(S.pn[0], S.pn[1], S.pn[2]);
+  return normalized_unit(ca * p + (sa * cphi) * cross(pn, p) + (sa * sphi) * pn);
+}
+__device__ __forceinline__ void generate_photon(const MxSourceDev &S, const MxSourceFine &F, const double *spec,
+                                                uint64_t seed, uint32_t tag, Ph &q) {
   if (S.spec_n > 0) {
     const double *e = spec + S.spec_off, *cum = e + S.spec_n;
     q.e = interp_d(source_uniform(seed, tag, 0), cum, e, (unsigned) S.spec_n);
@@ -122,20 +163,33 @@ __device__ __forceinline__ void generate_photon(const MxSourceDev &S, const doub
     D3 p0 = mk(-ct, sin_theta * S.b, sin_theta * S.c);
     q.p = rotate_unit(p0, mk(S.axis[0], S.axis[1], S.axis[2]), S.cos_al, S.sin_al);
   } else {
-    double sphi, cphi;
-    sincos(2.0 * PI * source_uniform(seed, tag, 1), &sphi, &cphi);
-    D3 normal = rotate_unit(mk(S.pn[0], S.pn[1], S.pn[2]), p, cphi, sphi);
-    double ang;
-    if (S.kind == MX_SOURCE_DISK)
-      ang = S.a * sqrt(S.b + S.c * source_uniform(seed, tag, 2));
+    // the angle: in double-float for a GAUSS or DISK source small enough
+    // (a draw of exactly 0 is drawn again, in double), else in double
+    const bool small = F.a[0] < (S.kind == MX_SOURCE_DISK ? 1.0f : 0.4f) * 0x1p-10f;
+    const uint64_t u = source_fixed(seed, tag, 2);
+    F2 ang = {1.0f, 0.0f};
+    double angle = 0.0;
+    if (small && S.kind == MX_SOURCE_DISK)
+      ang = df_mul(fine(F.a), df_sqrt(df_add(fine(F.b), df_mul(fine(F.c), split(unit_from_bits(u >> 11))))));
+    else if (small && S.kind == MX_SOURCE_GAUSS && u)
+      ang = df_mul(fine(F.a), df_sqrt(df_neg_log(u)));
     else {
-      double rnd = source_uniform(seed, tag, 2);
-      for (uint32_t k = 3; rnd == 0.0 && k < 8; k++) rnd = source_uniform(seed, tag, k);
-      ang = S.kind == MX_SOURCE_GAUSS ? S.a * sqrt(-log(rnd)) : S.a * sqrt(pow(rnd, S.b) - 1.0);
+      angle = source_angle(S, seed, tag);
+      if (small) ang = split(angle);
     }
-    double sa, ca;
-    sincos(ang, &sa, &ca);
-    q.p = rotate_unit(p, normal, ca, sa);
+    if (fabsf(ang.h) < 0x1p-10f) {
+      F2 sp, cp, sa, v;
+      df_turn_sincos(source_fixed(seed, tag, 1), false, sp, cp);
+      df_small_turn(ang, sa, v);
+      double d[3];
+      for (int k = 0; k < 3; k++)
+        d[k] = S.p[k] + df_join(df_sub(df_prod(sa, df_sum(df_prod(cp, fine(F.w[k])), df_prod(sp, fine(F.pn[k])))),
+                                       df_prod(v, fine(F.p[k]))));
+      q.p = mk(d[0], d[1], d[2]);
+    } else {
+      if (angle == 0.0) angle = source_angle(S, seed, tag);
+      q.p = source_direction(S, angle, source_uniform(seed, tag, 1));
+    }
   }
   q.t = 0.0;
   q.x = mk(0.0, 0.0, 0.0);
@@ -146,13 +200,14 @@ __device__ __forceinline__ void generate_photon(const MxSourceDev &S, const doub
   for (int k = 0; k < 4; k++) q.sup[k] = 0;
 }
 
-__global__ void __launch_bounds__(256) mx_generate_kernel(MxSourceDev S, const double *spec, uint32_t first_tag,
-                                                           uint64_t seed, double *energy, double *p, double *t,
+__global__ void __launch_bounds__(256) mx_generate_kernel(const __grid_constant__ MxSourceDev S,
+                                                           const __grid_constant__ MxSourceFine F, const double *spec,
+                                                           uint32_t first_tag, uint64_t seed, double *energy, double *p, double *t,
                                                            uint32_t *flags, uint32_t *tag, uint32_t n, uint32_t stride) {
   const size_t nn = stride;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     Ph q;
-    generate_photon(S, spec, seed, first_tag + k, q);
+    generate_photon(S, F, spec, seed, first_tag + k, q);
     energy[k] = q.e;
     p[k] = q.p.x; p[nn + k] = q.p.y; p[2 * nn + k] = q.p.z;
     if (t) t[k] = 0.0;
@@ -234,7 +289,7 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
       if (i < end) {
         const int s = source_of(i, sstart, b.nsrc);
         Ph q;
-        generate_photon(ssrc[s], b.spec, seed, i, q);
+        generate_photon(ssrc[s], b.fine[s], b.spec, seed, i, q);
         clear_extra(io, i);
         io.energy[i] = q.e;
         if (io.t) io.t[i] = 0.0;
@@ -380,11 +435,12 @@ struct mx_batch {
   mx_context *ctx = nullptr;
   std::vector<mx_source> src;
   std::vector<MxSourceDev> dsrc;
+  std::vector<MxSourceFine> fine;
   std::vector<double> spec;     // FILE spectra of the sources (host copy)
   DevBuf d_spec;
   std::vector<uint32_t> start;
   uint64_t total = 0;
-  DevBuf d_src;                 // sources then starts
+  DevBuf d_src;                 // sources, their MxSourceFine, then starts
   DevBuf cols[12];              // photon list columns
   DevBuf queues;                // two record queues
   DevBuf ctr;                   // 9 counters, the seed at byte 64
@@ -443,7 +499,8 @@ static int build_graph(mx_batch *b) {
   io.io.U = nullptr; io.io.N = nullptr; io.io.n = d.n; io.io.stride = d.n; io.io.stages = MX_STAGE_ALL; io.io.fresh = 1;
   io.io.overrun = c->d_overrun;
   io.src = (const MxSourceDev *) b->d_src.ptr;
-  io.start = (const uint32_t *) ((const char *) b->d_src.ptr + b->dsrc.size() * sizeof(MxSourceDev));
+  io.fine = (const MxSourceFine *) ((const char *) b->d_src.ptr + b->dsrc.size() * sizeof(MxSourceDev));
+  io.start = (const uint32_t *) (io.fine + b->dsrc.size());
   io.nsrc = (int32_t) b->dsrc.size();
   io.tile = b->params.tile;
   size_t qbytes = (size_t) b->total * sizeof(MxRec);
@@ -628,6 +685,16 @@ static bool source_dev(const mx_source &q, MxSourceDev &S, std::vector<double> &
   return true;
 }
 
+static MxSourceFine source_fine(const MxSourceDev &S) {
+  MxSourceFine F;
+  auto hi_lo = [](double d, float f[2]) { f[0] = (float) d; f[1] = (float) (d - (double) f[0]); };
+  const double w[3] = {S.pn[1] * S.p[2] - S.pn[2] * S.p[1], S.pn[2] * S.p[0] - S.pn[0] * S.p[2],
+                       S.pn[0] * S.p[1] - S.pn[1] * S.p[0]};
+  for (int k = 0; k < 3; k++) { hi_lo(S.p[k], F.p[k]); hi_lo(S.pn[k], F.pn[k]); hi_lo(w[k], F.w[k]); }
+  hi_lo(S.a, F.a); hi_lo(S.b, F.b); hi_lo(S.c, F.c);
+  return F;
+}
+
 static std::mutex g_tune_mu;
 static std::map<std::string, mx_batch_params> g_tune_cache;
 
@@ -652,7 +719,7 @@ int mx_generate_source(mx_context *c, const mx_source *s, uint32_t first_tag, ui
   int grid = std::max(1, std::min((int) ((d->n + 255) / 256), c->num_sms * 8));
   uint32_t stride = d->stride ? d->stride : d->n;
   if (stride < d->n) return mx_fail(c, MX_EINVAL, "mx_generate_source: stride below n");
-  mx_generate_kernel<<<grid, 256, 0, (cudaStream_t) stream>>>(S, dspec, first_tag, seed, d->energy, d->p,
+  mx_generate_kernel<<<grid, 256, 0, (cudaStream_t) stream>>>(S, source_fine(S), dspec, first_tag, seed, d->energy, d->p,
                                                               d->arrival_time, d->flags, d->tag, d->n, stride);
   c->launches++;
   cudaError_t e = cudaGetLastError();
@@ -681,6 +748,7 @@ mx_batch *mx_batch_create(mx_context *c, const mx_source *sources, int nsrc) {
     S.chip_off = q.detector == MX_DETECTOR_ACIS_S ? 4 : 0;
     S.nchips = q.detector == MX_DETECTOR_ACIS_S ? 6 : 4;
     b->dsrc.push_back(S);
+    b->fine.push_back(source_fine(S));
     tot += q.num_photons;
     b->start.push_back((uint32_t) tot);
   }
@@ -689,7 +757,7 @@ mx_batch *mx_batch_create(mx_context *c, const mx_source *sources, int nsrc) {
   b->total = tot;
   b->shared_bytes = tables_shared_bytes(c->T) + align16((size_t) nsrc * sizeof(MxSourceDev)) + align16((size_t) (nsrc + 1) * 4);
   const size_t elem[12] = {8, 24, 24, 8, 4, 4, 1, 1, 1, 4, 4, 12};
-  cudaError_t e = b->d_src.ensure(b->dsrc.size() * sizeof(MxSourceDev) + b->start.size() * 4);
+  cudaError_t e = b->d_src.ensure(b->dsrc.size() * (sizeof(MxSourceDev) + sizeof(MxSourceFine)) + b->start.size() * 4);
   for (int k = 0; k < 12 && e == cudaSuccess; k++) e = b->cols[k].ensure(std::max<size_t>(16, tot * elem[k]));
   if (e == cudaSuccess) e = b->queues.ensure(std::max<size_t>(256, 2 * tot * sizeof(MxRec)));
   if (e == cudaSuccess) e = b->ctr.ensure(128);
@@ -699,8 +767,10 @@ mx_batch *mx_batch_create(mx_context *c, const mx_source *sources, int nsrc) {
   if (e == cudaSuccess) e = cudaMallocHost((void **) &b->h_seed, sizeof(uint64_t));
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_src.ptr, b->dsrc.data(), b->dsrc.size() * sizeof(MxSourceDev), cudaMemcpyHostToDevice);
+  char *after = (char *) b->d_src.ptr + b->dsrc.size() * sizeof(MxSourceDev);
+  if (e == cudaSuccess) e = cudaMemcpy(after, b->fine.data(), b->fine.size() * sizeof(MxSourceFine), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
-    e = cudaMemcpy((char *) b->d_src.ptr + b->dsrc.size() * sizeof(MxSourceDev), b->start.data(), b->start.size() * 4,
+    e = cudaMemcpy(after + b->fine.size() * sizeof(MxSourceFine), b->start.data(), b->start.size() * 4,
                    cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     g_create_err = std::string("mx_batch_create: ") + cudaGetErrorString(e);

@@ -385,16 +385,19 @@ __device__ __forceinline__ double df_join(F2 a) {
   const long long m = __double_as_longlong(f2d_normal(__uint_as_float(u ^ sign)));
   return __longlong_as_double((m + (long long) l) | ((long long) (unsigned long long) sign << 32));
 }
-// f 2^-64 for a signed 64-bit f, in units of a quarter turn, as radians
-// (|f| 2^-64 <= 1/2): the top 23 bits of f as a float (a whole number within
-// 2^22 of 1.5 2^23), the next 24 as another, both exact, and the last 17
-// added to the low part, times pi/2.
-__device__ __forceinline__ F2 quarter_turns(long long f) {
+// f 2^-64 for a signed 64-bit f: the top 23 bits as a float (a whole number
+// within 2^22 of 1.5 2^23), the next 24 as another, both exact, and the last
+// 17 added to the low part.
+__device__ __forceinline__ F2 fixed_to_df(long long f) {
   const float a = __uint_as_float(0x4B400000u + (uint32_t) (int) (f >> 41)) - 12582912.0f;
   const float b = (float) (int) ((uint32_t) (f >> 17) & 0xffffffu), c = (float) (int) ((uint32_t) f & 0x1ffffu);
   F2 q = quick_sum(a * 0x1p-23f, b * 0x1p-47f);
   q.l = __fmaf_rn(c, 0x1p-64f, q.l);
-  return df_mul(F2{0x1.921fb6p+0f, -0x1.777a5cp-25f}, q);
+  return q;
+}
+// The same in units of a quarter turn (|f| 2^-64 <= 1/2), as radians.
+__device__ __forceinline__ F2 quarter_turns(long long f) {
+  return df_mul(F2{0x1.921fb6p+0f, -0x1.777a5cp-25f}, fixed_to_df(f));
 }
 
 // sin and cos of r (|r| <= pi/4 + a little) in double-float.
@@ -465,6 +468,30 @@ __device__ __forceinline__ F2 df_div(F2 a, F2 b) {
   const float q = __fdiv_rn(a.h, b.h);
   const F2 r = df_sub(a, df_mul_f(b, q));
   return quick_sum(q, __fdiv_rn(r.h, b.h));
+}
+
+// -ln(f 2^-64), f > 0: with u = m 2^e, 1/sqrt(2) < m <= sqrt(2), and
+// s = (m - 1) / (m + 1), ln m = 2 atanh s = 2 s (1 + z/3 + z^2/5 + ...),
+// z = s^2 < 0.0295; the terms from z^4/9 on in single precision.  Relative
+// error below 2^-43 (m - 1 is exact, and e = 0 next to u = 1).
+__device__ __forceinline__ F2 df_neg_log(unsigned long long f) {
+  const int lz = __clzll((long long) f);
+  const unsigned long long m = f << lz;                           // u = m 2^-64 2^-lz, the top bit set
+  const bool upper = m > 0xB504F333F9DE6485ull;                   // sqrt(2) / 2: m - 1 as it is, else twice it
+  const F2 t = fixed_to_df((long long) (upper ? m : m << 1));
+  const float e = (float) (upper ? lz : lz + 1);
+  const F2 den = df_add_less(F2{2.0f, 0.0f}, t);
+  const float inv = __frcp_rn(den.h), s0 = __fmul_rn(t.h, inv);
+  const F2 rem = df_sub(t, df_mul_f(den, s0));
+  const F2 s = quick_sum(s0, __fmul_rn(rem.h, inv)), z = df_mul(s, s);
+  float g = __fmaf_rn(z.h, 0x1.111112p-4f, 0x1.3b13b2p-4f);       // 1/13 + z/15
+  g = __fmaf_rn(z.h, g, 0x1.745d18p-4f);                          // 1/11
+  g = __fmaf_rn(z.h, g, 0x1.c71c72p-4f);                          // 1/9
+  F2 w = df_add_less(F2{0x1.24924ap-3f, -0x1.b6db6ep-28f}, df_prod(z, F2{g, 0.0f}));
+  w = df_add_less(F2{0x1.99999ap-3f, -0x1.99999ap-29f}, df_prod(z, w));
+  w = df_add_less(F2{0x1.555556p-2f, -0x1.555556p-27f}, df_prod(z, w));
+  const F2 h = df_add(s, df_mul(s, df_prod(z, w)));                // ln(m) / 2
+  return df_add(df_mul_f(F2{0x1.62e430p-1f, -0x1.05c610p-29f}, e), F2{-2.0f * h.h, -2.0f * h.l});
 }
 
 // The Fresnel numerator and denominator of reflectivity_parts in
@@ -1206,6 +1233,14 @@ __device__ __forceinline__ F2 wfold_df(const MxTables &T, int table, F2 energy, 
   return df_add(t0, df_prod(df_add(t1, df_neg(t0)), w));
 }
 #endif
+#ifdef __CUDACC__
+// sin a and 1 - cos a for |a| < 2^-10, in double-float.
+__device__ __forceinline__ void df_small_turn(F2 a, F2 &s, F2 &v) {
+  const F2 z = df_sqr(a);
+  s = df_sum(a, F2{-a.h * (z.h * fmaf(z.h, -1.0f / 120.0f, 1.0f / 6.0f)), 0.0f});
+  v = F2{0.5f * z.h, fmaf(z.h * z.h, -1.0f / 24.0f, 0.5f * z.l)};
+}
+#endif
 // late: whether a photon scattered into the far tail may be left for later
 // (2 is returned then, with p and the draws as they were): the wavefront
 // gathers these few and turns them on full warps.
@@ -1226,9 +1261,8 @@ MXD int reflect_finish(const MxTables &T, const MxShellDev &h, int o, int table,
   if (!tail && fabsf(a.h) < 0x1p-10f) {
     p = q;
     const F2 dg = (rng.uniform_fixed() >> 63) ? a : df_neg(a);   // a uniform below 1/2 turns the other way
-    const F2 z = df_sqr(dg);
-    F2 sg = df_sum(dg, F2{-dg.h * (z.h * fmaf(z.h, -1.0f / 120.0f, 1.0f / 6.0f)), 0.0f});
-    F2 v = {0.5f * z.h, fmaf(z.h * z.h, -1.0f / 24.0f, 0.5f * z.l)};   // 1 - cos dg
+    F2 sg, v;
+    df_small_turn(dg, sg, v);
     // p x n is sqrt(1 - pdn^2) long, and the turned vector is made unit
     // again: both coefficients times 1 + (pdn sin dg)^2 / 2 (the next term
     // is below 1e-18)

@@ -225,8 +225,8 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 // With a grating: the Rowland torus from a float iteration and two steps on
 // the quartic's double value, the order choice decided in float away from
 // its thresholds, and one facet basis for the LETG's primary and four
-// supports, whose direction stays in its components: per 2e6 photons C
-// 114 -> 95 us and D 45 -> 51 (HETG) and 219 -> 190 us (LETG, 3.4e6 -> 2.0e6
+// supports, whose direction stays in its components: per 1e6 photons C
+// 114 -> 95 us (HETG) and D 219 -> 190 us (LETG and HRC-S, 3.4e6 -> 2.0e6
 // FP64 instructions); HETG 2e7 7.73 -> 7.08 ms, LETG + HRC-S 4e6 2.35 ->
 // 1.88 ms.
 
