@@ -2,8 +2,9 @@
 // images, and the adjoint of the image with respect to the 18 geometry and
 // pointing parameters.
 //
-// Forward: one persistent kernel traces each ray in FP64 (mxd::weighted_ray
-// over double) and splats it with an 11 x 11 Gaussian.  The splat is
+// Forward: one persistent kernel traces each ray in FP64 (ray_front and
+// ray_image, on the trace's own shell records) and splats it with an 11 x 11
+// Gaussian.  The splat is
 // accumulated in 64-bit fixed point -- exact integer sums, so the image does
 // not depend on the order of the atomics and repeats bit for bit -- first in
 // a 64 x 64 shared-memory window about the image centre, which takes nearly
@@ -22,6 +23,7 @@
 // traces only those, so that its lanes do not idle through the rays that
 // were lost.  Sums are deterministic: fixed tiles per block, fixed warp
 // order, fixed block order, one final reduction.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -32,6 +34,7 @@
 #include "mx_diff.cuh"
 
 using mxd::Dual6;
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -54,6 +57,7 @@ struct ImageGeom {
   float inv_s2;                  // 1 / sigma^2
   float knorm;                   // 1 / (sqrt(2 pi) sigma)
   float pad2;
+  long long top_u, top_v;        // mx::dkey of nx + HALF and ny + HALF
 };
 
 // What the aperture sampling needs of each shell (project_photon_to_hrma).
@@ -63,13 +67,23 @@ struct Aperture {
   int32_t ideal, area_uniform;
 };
 
+// One shell at theta: its geometry in the trace's own record (so that the
+// rays take the trace's conics, screens and struts), the source direction in
+// the paraboloid's frame, and the reflection's constants.
+struct DiffShell {
+  MxShellDev h;
+  double p1[3];                  // fwd[0] p0
+  double wscale;                 // vignetting times the square of the effective-area correction
+  float p1f[3], beta, delta;     // p1 and the optical constants at the ray energy
+  float pad[19];                 // 992 bytes: the four shells start on distinct banks
+};
+static_assert(sizeof(DiffShell) % 128 == 96, "four shells on distinct bank offsets");
+
 struct FwdArgs {
-  mxd::Optic<double> opt[4][2];
-  mxd::Between<double> mid[4];
-  mxd::RayConst rc[4];
-  Aperture ap;
+  DiffShell sh[4];
   double p0[3];
   double vig;
+  int32_t ideal, area_uniform, weighted, pad;
   ImageGeom g;
 };
 
@@ -151,19 +165,28 @@ __device__ __forceinline__ bool aperture(const Aperture &ap, uint64_t seed, uint
   return true;
 }
 
+// The pixel nearest to coordinate u, floor(u + 1/2), and the offset u - pixel
+// rounded to float; false unless -(HALF + 1) < u < n + HALF (the ray's 11 x 11
+// window misses the image).  Two FP64 additions; floor, comparisons and
+// conversions on the integer and FP32 pipes.
+__device__ __forceinline__ bool nearest_pixel(double u, long long top, int &ic, float &f) {
+  const long long k = mx::dkey(u);
+  if (!(k > mx::dkey(-(mxd::HALF + 1.0)) && k < top)) return false;
+  const double s = MX_DADD(u, 0.5);
+  const float t = mx::d2f_trunc(s);
+  float c = floorf(t);                          // of s >= 0: truncation does not cross an integer
+  if (s < 0.0 && c == t && mx::f2d_normal(t) != s) c -= 1.0f;
+  ic = (int) c;
+  f = mx::d2f_rn(MX_DADD(u, -mx::f2d_normal(c)));
+  return true;
+}
+
 // Nearest pixel and the ray's offset from it on both axes; false when the
 // ray's 11 x 11 window misses the image.
 __device__ __forceinline__ bool splat_origin(const ImageGeom &g, double y, double z, int &ic, int &jc, float &fu,
                                              float &fv) {
-  const double u = mxd::pixel_coord(y, g.cy, g.inv_pitch, g.cx_pix);
-  const double v = mxd::pixel_coord(z, g.cz, g.inv_pitch, g.cz_pix);
-  if (!(u > -(mxd::HALF + 1.0) && u < g.nx + (double) mxd::HALF && v > -(mxd::HALF + 1.0) &&
-        v < g.ny + (double) mxd::HALF))
-    return false;
-  const double uc = floor(u + 0.5), vc = floor(v + 0.5);
-  ic = (int) uc; jc = (int) vc;
-  fu = (float) (u - uc); fv = (float) (v - vc);
-  return true;
+  return nearest_pixel(mxd::pixel_coord(y, g.cy, g.inv_pitch, g.cx_pix), g.top_u, ic, fu) &&
+         nearest_pixel(mxd::pixel_coord(z, g.cz, g.inv_pitch, g.cz_pix), g.top_v, jc, fv);
 }
 
 __device__ __forceinline__ float tap(const ImageGeom &g, int k, float f) {
@@ -176,118 +199,330 @@ __device__ __forceinline__ float tap(const ImageGeom &g, int k, float f) {
 // ------------------------------------------------------------ forward --
 namespace {
 
+constexpr int FWD_BLOCKS = 3;
+constexpr int LIST = 64;                            // a warp's rays waiting: up to 31 left over and 32 new
+constexpr int WSTRIDE = WIN + mxd::TAPS;            // window row stride, 11 mod 32 words: tap t of 121 falls on bank t
+
+// A warp's list of rays that passed the aperture: index, shell, radius and
+// the azimuth's sine and cosine.
+struct RayList {
+  double r[LIST];
+  mx::F2 s[LIST], c[LIST];
+  uint32_t i[LIST], shell[LIST];
+};
+
+// w 2^31 rounded to the nearest integer (ties to even), at most 2^32 - 1, on
+// the integer pipe; 0 < w.
+__device__ __forceinline__ uint32_t weight_fixed(double w) {
+  const unsigned long long b = mx::dbits(w);
+  const int sh = 1044 - (int) (b >> 52);              // w 2^31 = m 2^-sh
+  if (sh < 21) return 0xffffffffu;                    // w >= 2
+  if (sh > 54) return 0u;
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  const unsigned long long q = (m + ((1ull << (sh - 1)) - 1ull) + ((m >> sh) & 1ull)) >> sh;
+  return q > 0xffffffffull ? 0xffffffffu : (uint32_t) q;
+}
+
+// The 121 taps as the lanes of a warp take them: tap t = lane + 32 j is
+// (t % 11, t / 11).
+struct TapLane {
+  int ky[4], kz[4], at[4];
+  __device__ __forceinline__ explicit TapLane(int lane) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      kz[j] = (lane + 32 * j) / mxd::TAPS;
+      ky[j] = lane + 32 * j - mxd::TAPS * kz[j];
+      at[j] = kz[j] * WSTRIDE + ky[j];
+    }
+  }
+};
+
+// The shared window as the splat tests it, in registers: its origin, the
+// last origin of an 11 x 11 patch inside it (images
+// are 16 pixels or more on a side) and the fixed-point shift, below 32 for every n_rays and sigma.
+struct SplatWindow {
+  int x0, y0;
+  unsigned last_x, last_y, shift;
+};
+
 // Splat the warp's rays: lane L's ray is valid when valid is set, with its
 // window origin and taps computed by that lane into its stage row; then
-// the warp adds the 121 taps of each valid ray together.
-__device__ __forceinline__ void splat_warp(const ImageGeom &g, bool valid, double y, double z, double w,
-                                           uint32_t *stage, unsigned long long *win, unsigned long long *acc,
+// the warp adds the 121 taps of each valid ray together.  The window's 64-bit
+// sums are kept as two planes of 32-bit words, the carry added to the upper
+// one: 9.5 cycles of the SM for a warp's update where a 64-bit shared atomic
+// takes 13.6.
+// A lane writes its taps for half a warp's rays at a time (16 rows of the
+// stage).
+__device__ __forceinline__ void splat_warp(const ImageGeom &g, const SplatWindow &W, bool valid, double y, double z, double w, uint32_t *stage,
+                                           uint32_t *lo, uint32_t *hi, unsigned long long *acc, const TapLane &tl,
                                            int lane) {
   int ic = 0, jc = 0;
   float fu = 0.f, fv = 0.f;
-  if (valid) valid = w > 0.0 && splat_origin(g, y, z, ic, jc, fu, fv);
+  if (valid) valid = mx::dkey(w) > 0 && splat_origin(g, y, z, ic, jc, fu, fv);
+  uint32_t ty[mxd::TAPS], tz[mxd::TAPS];
   if (valid) {
-    uint32_t *row = stage + lane * STAGE_STRIDE;
-    const uint32_t wq = __double2uint_rn(fmin(MX_DMUL(w, 2147483648.0), 4294967295.0));   // w 2^31
-    row[0] = (uint32_t) ic;
-    row[1] = (uint32_t) jc;
+    const uint32_t wq = weight_fixed(w);
 #pragma unroll
     for (int k = 0; k < mxd::TAPS; k++) {
       const uint32_t gy = __float2uint_rn(FMUL(tap(g, k, fu), 2147483648.0f));   // K 2^31
-      row[2 + k] = (uint32_t) (((unsigned long long) wq * gy) >> 32);             // w K 2^30
-      row[2 + mxd::TAPS + k] = __float2uint_rn(FMUL(tap(g, k, fv), 2147483648.0f));
+      ty[k] = __umulhi(wq, gy);                                                  // w K 2^30
+      tz[k] = __float2uint_rn(FMUL(tap(g, k, fv), 2147483648.0f));
     }
   }
+  const unsigned vm = __ballot_sync(0xffffffffu, valid);
+#pragma unroll 1
+  for (int half = 0; half < 32; half += 16) {
+  if (valid && (lane & 16) == half) {
+    uint32_t *row = stage + (lane & 15) * STAGE_STRIDE;
+    row[0] = (uint32_t) ic;
+    row[1] = (uint32_t) jc;
+#pragma unroll
+    for (int k = 0; k < mxd::TAPS; k++) { row[2 + k] = ty[k]; row[2 + mxd::TAPS + k] = tz[k]; }
+  }
   __syncwarp();
-  unsigned vm = __ballot_sync(0xffffffffu, valid);
-  while (vm) {
-    const int r = __ffs(vm) - 1;
-    vm &= vm - 1;
-    const uint32_t *row = stage + r * STAGE_STRIDE;
-    const int ric = (int) row[0], rjc = (int) row[1];
-    for (int t = lane; t < mxd::TAPS * mxd::TAPS; t += 32) {
-      const int kz = t / mxd::TAPS, ky = t - mxd::TAPS * kz;
-      const int col = ric - mxd::HALF + ky, rr = rjc - mxd::HALF + kz;
-      if ((unsigned) col < (unsigned) g.nx && (unsigned) rr < (unsigned) g.ny) {
-        const unsigned long long c = ((unsigned long long) row[2 + ky] * row[2 + mxd::TAPS + kz]) >> g.shift;
-        if (c) {
-          const unsigned wc = (unsigned) (col - g.wx0), wr = (unsigned) (rr - g.wy0);
-          if (wc < (unsigned) g.wnx && wr < (unsigned) g.wny) atomicAdd(win + wr * g.wnx + wc, c);
-          else atomicAdd(acc + (size_t) rr * g.nx + col, c);
+  for (unsigned hm = (vm >> half) & 0xffffu; hm; hm &= hm - 1) {
+    const uint32_t *row = stage + (__ffs(hm) - 1) * STAGE_STRIDE;
+    const int c0 = (int) row[0] - mxd::HALF, r0 = (int) row[1] - mxd::HALF;
+    const int wc0 = c0 - W.x0, wr0 = r0 - W.y0;
+    if ((unsigned) wc0 <= W.last_x && (unsigned) wr0 <= W.last_y) {   // all 121 in the window
+      const int at = wr0 * WSTRIDE + wc0;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (j < 3 || lane < mxd::TAPS * mxd::TAPS - 96) {
+          const unsigned long long c = (unsigned long long) row[2 + tl.ky[j]] * row[2 + mxd::TAPS + tl.kz[j]];
+          const int k = at + tl.at[j];
+          const uint32_t cl = __funnelshift_r((uint32_t) c, (uint32_t) (c >> 32), W.shift), old = atomicAdd(lo + k, cl);
+          atomicAdd(hi + k, ((uint32_t) (c >> 32) >> W.shift) + (old + cl < cl ? 1u : 0u));
         }
+      }
+    } else {
+#pragma unroll 1
+      for (int t = lane; t < mxd::TAPS * mxd::TAPS; t += 32) {
+        const int kz = t / mxd::TAPS, ky = t - mxd::TAPS * kz;
+        const int col = c0 + ky, rr = r0 + kz;
+        if ((unsigned) col >= (unsigned) g.nx || (unsigned) rr >= (unsigned) g.ny) continue;
+        const unsigned long long c = ((unsigned long long) row[2 + ky] * row[2 + mxd::TAPS + kz]) >> g.shift;
+        const unsigned wc = (unsigned) (col - g.wx0), wr = (unsigned) (rr - g.wy0);
+        if (wc < (unsigned) g.wnx && wr < (unsigned) g.wny) {
+          const int k = (int) wr * WSTRIDE + (int) wc;
+          const uint32_t cl = (uint32_t) c, old = atomicAdd(lo + k, cl);
+          atomicAdd(hi + k, (uint32_t) (c >> 32) + (old + cl < cl ? 1u : 0u));
+        } else if (c)
+          atomicAdd(acc + (size_t) rr * g.nx + col, c);
       }
     }
   }
   __syncwarp();
+  }
+}
+
+// Part 1 of a ray: its point on the aperture (the shell pick, radius and
+// azimuth the mirror stage draws for the photon of that tag, mirror_front,
+// with the vignetting draw consumed but turned into a weight), and unless it
+// is replayed the pre-collimator struts and the float screen for rays that
+// certainly miss the paraboloid.  False for a ray that ends here.
+__device__ __forceinline__ bool ray_front(const FwdArgs &A, const MxTables &T, uint64_t seed, uint32_t tag, bool replay,
+                                          int &si, double &radius, mx::F2 &s, mx::F2 &c) {
+  mx::Rng rng;
+  rng.U = nullptr; rng.N = nullptr; rng.seed = seed; rng.n = 0; rng.i = 0; rng.tag = tag; rng.overrun = false;
+  rng.window(MX_U_MIRROR, 12, MX_N_MIRROR, 2);
+  if (!A.ideal) rng.skip_uniform();
+  si = -1;
+  for (int guard = 0; guard < 64 && si < 0; guard++) {
+    const double r = rng.uniform();
+    if (rng.overrun) return false;
+    for (int i = 0; i < 4; i++)
+      if (mx::lt_pos(r, A.sh[i].h.area_fraction)) { si = i; break; }
+  }
+  if (si < 0) return false;
+  const MxShellDev &h = A.sh[si].h;
+  if (A.area_uniform) {
+    const double r0 = h.min_radius, r1 = h.max_radius;
+    radius = mx::sqrt_fast(r0 * r0 + (r1 * r1 - r0 * r0) * rng.uniform());
+  } else
+    radius = fma(h.dr, rng.uniform(), h.min_radius);
+  unsigned long long theta;
+  for (int guard = 0;; guard++) {
+    theta = rng.uniform_fixed();
+    if (rng.overrun || guard >= 64) return false;
+    if (h.shutter & (1u << (unsigned) (theta >> 62))) break;
+  }
+  mx::df_turn_sincos(theta, true, s, c);   // of the angle 2 pi (u - 1/8)
+  if (replay) return true;
+  const float rf = mx::d2f_trunc(radius), yf = rf * s.h, zf = rf * c.h;
+  if (T.use_struts) {
+    const float pxf = mx::d2f_trunc(A.p0[0]), pyf = mx::d2f_trunc(A.p0[1]), pzf = mx::d2f_trunc(A.p0[2]);
+    int blocked = mx::struts_screen(T, 0, h.frontf, yf - h.osac0f[1], zf - h.osac0f[2], pxf, pyf, pzf);
+    if (blocked < 0)
+      blocked = mx::struts_block_exact(T, 0, mx::mk(h.front_position, radius * mx::df_join(s) - h.to_osac[0][1],
+                                                    radius * mx::df_join(c) - h.to_osac[0][2]),
+                                       mx::mk(A.p0[0], A.p0[1], A.p0[2])) ? 1 : 0;
+    if (blocked) return false;
+  }
+  const double *f = h.fwd[0];
+  const float f1 = mx::d2f_trunc(f[1]), f2 = mx::d2f_trunc(f[2]), f4 = mx::d2f_trunc(f[4]), f5 = mx::d2f_trunc(f[5]);
+  const float f7 = mx::d2f_trunc(f[7]), f8 = mx::d2f_trunc(f[8]);
+  return !mx::paraboloid_missed(h, fmaf(f2, zf, fmaf(f1, yf, h.front_fwdf)),
+                                fmaf(f5, zf, fmaf(f4, yf, mx::d2f_trunc(h.front_fwd[1]))),
+                                fmaf(f8, zf, fmaf(f7, yf, mx::d2f_trunc(h.front_fwd[2]))), A.sh[si].p1f[0], A.sh[si].p1f[1],
+                                A.sh[si].p1f[2]);
+}
+
+// Part 2: through both mirrors to the focal plane x = 0.  root holds the
+// recorded conic roots (RAY_ROOT_* bits) of a replayed ray, and receives
+// those taken otherwise.
+__device__ __forceinline__ bool ray_image(const FwdArgs &A, const MxTables &T, int si, double ry, double rz, bool replay,
+                                          int &root, double &y, double &z, double &w) {
+  const DiffShell &S = A.sh[si];
+  const MxShellDev &h = S.h;
+  // fwd (x + to) with x + to = (front + to[0], ry, rz): (ry - to[1]) + to[1]
+  // is ry to within an ulp of to[1]
+  const double *f = h.fwd[0];
+  mx::D3 x = mx::mk(fma(f[2], rz, fma(f[1], ry, h.front_fwd[0])), fma(f[5], rz, fma(f[4], ry, h.front_fwd[1])),
+                    fma(f[8], rz, fma(f[7], ry, h.front_fwd[2])));
+  mx::D3 p = mx::mk(S.p1[0], S.p1[1], S.p1[2]), n;
+  const int rp = mxd::conic_root(h, 0, x, p, n, replay ? ((root & mxd::RAY_ROOT_P) ? 1 : 0) : -1);
+  if (rp < 0) return false;
+  mx::F2 num{1.0f, 0.0f}, den{1.0f, 0.0f};
+  double pdn = mx::dot(p, n);
+  if (A.weighted) mx::reflectivity_df(mx::split(fabs(pdn)), S.beta, S.delta, num, den);
+  p = mxd::reflected(p, n, pdn);
+  if (!replay && T.use_struts && mx::cap_struts_block(T, h, x, p)) return false;
+  {
+    const double *M = h.mid, *c = h.mid_off;
+    p = mx::mat_mul(M, p);
+    x = mx::mk(fma(M[0], x.x, fma(M[1], x.y, fma(M[2], x.z, c[0]))), fma(M[3], x.x, fma(M[4], x.y, fma(M[5], x.z, c[1]))),
+               fma(M[6], x.x, fma(M[7], x.y, fma(M[8], x.z, c[2]))));
+  }
+  const int rh = mxd::conic_root(h, 1, x, p, n, replay ? ((root & mxd::RAY_ROOT_H) ? 1 : 0) : -1);
+  if (rh < 0) return false;
+  pdn = mx::dot(p, n);
+  if (A.weighted) {
+    mx::F2 n2, d2;
+    mx::reflectivity_df(mx::split(fabs(pdn)), S.beta, S.delta, n2, d2);
+    w = mx::df_join(mx::df_div(mx::df_mul(num, n2), mx::df_mul(den, d2))) * S.wscale;
+  } else
+    w = A.vig;
+  p = mxd::reflected(p, n, pdn);
+  p = mx::mat_mul(h.bwd[1], p);
+  x = mx::mat_mul(h.bwd[1], x);
+  x = x - mx::mk(h.to_osac[1][0], h.to_osac[1][1], h.to_osac[1][2]);
+  if (!replay && T.use_struts && mx::struts_block(T, 2, x, p)) return false;
+  const double t = -x.x * mx::rcp_fast(p.x);
+  y = fma(t, p.y, x.y);
+  z = fma(t, p.z, x.z);
+  root = (rp ? mxd::RAY_ROOT_P : 0) | (rh ? mxd::RAY_ROOT_H : 0);
+  return true;
 }
 
 // SPLAT: accumulate the image; otherwise write each ray's y, z, w.
-// part[block][4]: the block's sum w, sum w y, sum w z and hits.
-template <bool SPLAT>
-__global__ void __launch_bounds__(DBLOCK) diff_forward_kernel(const __grid_constant__ FwdArgs args, const __grid_constant__ MxTables T,
+// MOMENTS: part[block][4], the block's sum w, sum w y, sum w z and hits.
+//
+// A warp takes 32 rays at a time through the aperture, keeps those that go on
+// in a list of its own and traces 32 of the list together: half the rays miss
+// the paraboloid, and traced where they stood they left 24 lanes of a warp
+// busy on average and the FP64 work of a whole ray to every warp.  With the
+// Newton intersections the FP64 instructions fall from 8.3 to 2.6 million per
+// 1e6 rays (48 % of the pipe; the splat's atomics and the aperture's and
+// weights' FP32 steps are the rest): 697 -> 315 us per 1e6 rays.  Three
+// blocks per SM (80 registers, 190 bytes spilled) rather than two of 110
+// without spills: a gradient step over 4e6 rays takes 3.05 instead of 3.38 ms.
+template <bool SPLAT, bool MOMENTS>
+__global__ void __launch_bounds__(DBLOCK, FWD_BLOCKS) diff_forward_kernel(const __grid_constant__ FwdArgs args, const __grid_constant__ MxTables T,
                                                                uint64_t n, uint64_t seed, uint8_t *codes, int mode,
                                                                unsigned long long *acc, double *part, double *yzw) {
   extern __shared__ __align__(16) unsigned char smem[];
   FwdArgs &A = *reinterpret_cast<FwdArgs *>(smem);
-  unsigned long long *win = reinterpret_cast<unsigned long long *>(smem + align_up(sizeof(FwdArgs)));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *stage = reinterpret_cast<uint32_t *>(win + (SPLAT ? WIN * WIN : 0)) + warp * 32 * STAGE_STRIDE;
+  RayList &list = reinterpret_cast<RayList *>(smem + align_up(sizeof(FwdArgs)))[warp];
+  uint32_t *lo = reinterpret_cast<uint32_t *>(smem + align_up(sizeof(FwdArgs)) + DWARPS * sizeof(RayList));
+  uint32_t *hi = lo + WIN * WSTRIDE;
+  uint32_t *stage = hi + WIN * WSTRIDE + warp * 16 * STAGE_STRIDE;   // SPLAT only, as lo and hi
   {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(&args);
     uint32_t *dst = reinterpret_cast<uint32_t *>(smem);
     for (int k = threadIdx.x; k < (int) (sizeof(FwdArgs) / 4); k += DBLOCK) dst[k] = src[k];
     if (SPLAT)
-      for (int k = threadIdx.x; k < WIN * WIN; k += DBLOCK) win[k] = 0ull;
+      for (int k = threadIdx.x; k < 2 * WIN * WSTRIDE; k += DBLOCK) lo[k] = 0u;
   }
   __syncthreads();
   const bool replay = mode == MX_DIFF_REPLAY;
-  const StrutTest struts{&T};
-  mxd::V3<double> p0 = mxd::v3<double>(A.p0[0], A.p0[1], A.p0[2]);
-  double sw = 0.0, swy = 0.0, swz = 0.0, hits = 0.0;
+  const TapLane tl(lane);
+  const SplatWindow W{args.g.wx0, args.g.wy0, (unsigned) (args.g.wnx - mxd::TAPS), (unsigned) (args.g.wny - mxd::TAPS),
+                      (unsigned) args.g.shift};
+  double sw = 0.0, swy = 0.0, swz = 0.0;
+  uint32_t hits = 0;
   const uint64_t step = (uint64_t) gridDim.x * DWARPS * 32;
-  for (uint64_t base = ((uint64_t) blockIdx.x * DWARPS + warp) * 32; base < n; base += step) {
-    const uint64_t i = base + lane;
+  uint64_t base = ((uint64_t) blockIdx.x * DWARPS + warp) * 32;
+  int have = 0;
+  while (base < n || have > 0) {
+    if (base < n) {
+      const uint64_t i = base + lane;
+      base += step;
+      int si = 0;
+      double radius = 0.0;
+      mx::F2 s{0.f, 0.f}, c{0.f, 0.f};
+      bool on = i < n;
+      if (on && replay) on = (codes[i] & mxd::RAY_HIT) != 0;
+      if (on) on = ray_front(A, T, seed, (uint32_t) i, replay, si, radius, s, c);
+      if (i < n && !on) {
+        if (mode == MX_DIFF_RECORD) codes[i] = 0;
+        if (!SPLAT) {
+          yzw[i] = yzw[n + i] = __longlong_as_double(0x7ff8000000000000ll);
+          yzw[2 * n + i] = 0.0;
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      if (on) {
+        const int k = have + __popc(m & ((1u << lane) - 1u));
+        list.r[k] = radius; list.s[k] = s; list.c[k] = c;
+        list.i[k] = (uint32_t) i; list.shell[k] = (uint32_t) si;
+      }
+      have += __popc(m);
+      __syncwarp();
+      if (have < 32 && base < n) continue;
+    }
+    const int take = have < 32 ? have : 32;
+    have -= take;
     bool hit = false;
     double y = 0.0, z = 0.0, w = 0.0;
-    if (i < n) {
-      uint8_t code = replay ? codes[i] : 0;
-      int si;
-      double ry, rz;
-      if (aperture(A.ap, seed, (uint32_t) i, si, ry, rz))
-        hit = mxd::weighted_ray<double>(A.opt[si][0], A.opt[si][1], A.mid[si], A.rc[si], ry, rz, p0, replay, code, struts,
-                                        y, z, w);
-      else
-        code = 0;
-      if (mode == MX_DIFF_RECORD) codes[i] = code;
-      if (hit) {
-        w = w * A.vig;
-        sw += w; swy += w * y; swz += w * z; hits += 1.0;
-      }
+    if (lane < take) {
+      const int k = have + lane, si = (int) list.shell[k];
+      const uint64_t i = list.i[k];
+      const double radius = list.r[k], ry = radius * mx::df_join(list.s[k]), rz = radius * mx::df_join(list.c[k]);
+      int root = replay ? codes[i] : 0;
+      hit = ray_image(A, T, si, ry, rz, replay, root, y, z, w);
+      if (mode == MX_DIFF_RECORD) codes[i] = hit ? (uint8_t) (mxd::RAY_HIT | root) : (uint8_t) 0;
+      if (MOMENTS && hit) { sw += w; swy += w * y; swz += w * z; hits++; }
       if (!SPLAT) {
         yzw[i] = hit ? y : __longlong_as_double(0x7ff8000000000000ll);
         yzw[n + i] = hit ? z : __longlong_as_double(0x7ff8000000000000ll);
         yzw[2 * n + i] = hit ? w : 0.0;
       }
     }
-    if (SPLAT) splat_warp(A.g, hit, y, z, w, stage, win, acc, lane);
+    __syncwarp();   // the list's entries are read before they are written again
+    if (SPLAT) splat_warp(A.g, W, hit, y, z, w, stage, lo, hi, acc, tl, lane);
   }
-  // block partial moments, fixed order
-  for (int o = 16; o > 0; o >>= 1) {
-    sw += __shfl_down_sync(0xffffffffu, sw, o);
-    swy += __shfl_down_sync(0xffffffffu, swy, o);
-    swz += __shfl_down_sync(0xffffffffu, swz, o);
-    hits += __shfl_down_sync(0xffffffffu, hits, o);
+  __shared__ double red[4 * DWARPS];
+  if (MOMENTS) {   // block partial moments, fixed order
+    double nh = (double) hits;
+    for (int o = 16; o > 0; o >>= 1) {
+      sw += __shfl_down_sync(0xffffffffu, sw, o);
+      swy += __shfl_down_sync(0xffffffffu, swy, o);
+      swz += __shfl_down_sync(0xffffffffu, swz, o);
+      nh += __shfl_down_sync(0xffffffffu, nh, o);
+    }
+    if (lane == 0) { red[4 * warp] = sw; red[4 * warp + 1] = swy; red[4 * warp + 2] = swz; red[4 * warp + 3] = nh; }
   }
   __syncthreads();
-  double *red = reinterpret_cast<double *>(win + (SPLAT ? WIN * WIN : 0));   // reuses the stage
-  if (lane == 0) { red[4 * warp] = sw; red[4 * warp + 1] = swy; red[4 * warp + 2] = swz; red[4 * warp + 3] = hits; }
   if (SPLAT) {
     for (int k = threadIdx.x; k < A.g.wnx * A.g.wny; k += DBLOCK) {
-      const unsigned long long v = win[k];
-      if (v) atomicAdd(acc + (size_t) (A.g.wy0 + k / A.g.wnx) * A.g.nx + A.g.wx0 + k % A.g.wnx, v);
+      const int r = k / A.g.wnx, c = k - r * A.g.wnx;
+      const unsigned long long v = ((unsigned long long) hi[r * WSTRIDE + c] << 32) | lo[r * WSTRIDE + c];
+      if (v) atomicAdd(acc + (size_t) (A.g.wy0 + r) * A.g.nx + A.g.wx0 + c, v);
     }
   }
-  __syncthreads();
-  if (threadIdx.x < 4) {
+  if (MOMENTS && threadIdx.x < 4) {
     double s = 0.0;
     for (int k = 0; k < DWARPS; k++) s += red[4 * k + threadIdx.x];
     part[4 * blockIdx.x + threadIdx.x] = s;
@@ -300,35 +535,53 @@ __global__ void diff_image_kernel(const unsigned long long *acc, size_t npix, do
     image[k] = (double) acc[k] * scale;
 }
 
-// out[v] = scale * sum over b of part[b * nv + v], in block order.
-__global__ void diff_sum_kernel(const double *part, int nblocks, int nv, double scale, double *out) {
-  const int v = threadIdx.x;
+// out[v] = scale * sum over b of part[b * nv + v]: warp v, its lanes' strided
+// sums added in a tree (a fixed order).  7 us for the 18 sums of a gradient; one
+// thread a value waited for one load after the other, 39 us.
+__global__ void __launch_bounds__(32 * NP) diff_sum_kernel(const double *part, int nblocks, int nv, double scale,
+                                                           double *out) {
+  const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (v >= nv) return;
   double s = 0.0;
-  for (int b = 0; b < nblocks; b++) s += part[(size_t) b * nv + v];
-  out[v] = s * scale;
+#pragma unroll 4
+  for (int b = lane; b < nblocks; b += 32) s += part[(size_t) b * nv + v];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) out[v] = s * scale;
 }
 
-// loss = mean (image - target)^2 and, optionally, its gradient; one block,
-// fixed reduction order.
-__global__ void __launch_bounds__(1024) diff_mse_kernel(const double *image, const double *target, size_t npix,
-                                                        double *dl, double *loss) {
-  __shared__ double red[32];
+// loss = mean (image - target)^2 and, optionally, its gradient.  One cluster
+// of blocks: each sums its part in a fixed order, and the first adds theirs
+// from distributed shared memory, in the order of their ranks.  256 x 256
+// pixels: 14 us; one block alone took 81 us, waiting for its loads.
+constexpr int MSE_BLOCKS = 8, MSE_THREADS = 1024;
+__global__ void __cluster_dims__(MSE_BLOCKS, 1, 1) __launch_bounds__(MSE_THREADS)
+    diff_mse_kernel(const double *image, const double *target, size_t npix, double inv, double *dl, double *loss) {
+  __shared__ double red[MSE_THREADS / 32];
+  __shared__ double total;
   double s = 0.0;
-  const double inv = 1.0 / (double) npix;
-  for (size_t k = threadIdx.x; k < npix; k += blockDim.x) {
+  const double inv2 = 2.0 * inv;
+#pragma unroll 4
+  for (size_t k = (size_t) blockIdx.x * MSE_THREADS + threadIdx.x; k < npix; k += (size_t) MSE_BLOCKS * MSE_THREADS) {
     const double r = image[k] - target[k];
     s += r * r;
-    if (dl) dl[k] = 2.0 * r * inv;
+    if (dl) dl[k] = r * inv2;
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) total = s;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     double t = 0.0;
-    for (int k = 0; k < (int) (blockDim.x >> 5); k++) t += red[k];
+    for (int b = 0; b < MSE_BLOCKS; b++) t += *cluster.map_shared_rank(&total, b);
     *loss = t * inv;
   }
+  cluster.sync();   // every block's shared memory stays until it is read
 }
 
 }  // namespace
@@ -498,7 +751,7 @@ struct mx_diff {
   DevBuf codes, acc, part, out;   // out: 4 moments, then NP gradient values
   double *h_out = nullptr;        // pinned: moments and gradient read back
   bool recorded = false;
-  int fwd_blocks = 0, rays_blocks = 0, adj_blocks = 0;
+  int fwd_blocks = 0, mom_blocks = 0, rays_blocks = 0, adj_blocks = 0;
   size_t fwd_smem = 0, rays_smem = 0, adj_smem = 0;
 };
 
@@ -574,24 +827,30 @@ int fill_fwd(mx_diff *d, const double *theta, FwdArgs &F) {
   if (r) return r;
   memset(&F, 0, sizeof(F));
   for (int s = 0; s < 4; s++) {
-    for (int k = 0; k < 9; k++) F.mid[s].m[k] = mid[s].m[k].v;
-    for (int k = 0; k < 3; k++) F.mid[s].c[k] = mid[s].c[k].v;
-    for (int k = 0; k < 9; k++) F.mid[s].bwdf[k] = mid[s].bwdf[k];
-    for (int k = 0; k < 3; k++) F.mid[s].tof[k] = mid[s].tof[k];
-  }
-  for (int s = 0; s < 4; s++)
+    DiffShell &S = F.sh[s];
+    MxShellDev &h = S.h;
+    h = d->ctx->hm.shells[s];
     for (int o = 0; o < 2; o++) {
-      const mxd::Optic<Dual6> &a = opt[s][o];
-      mxd::Optic<double> &b = F.opt[s][o];
-      b.a = a.a; b.b = a.b; b.c = a.c; b.xmin = a.xmin; b.xmax = a.xmax;
-      for (int k = 0; k < 3; k++) b.to[k] = a.to[k].v;
-      for (int k = 0; k < 9; k++) { b.fwd[k] = a.fwd[k].v; b.bwd[k] = a.bwd[k].v; }
-      for (int k = 0; k < 3; k++) b.ff[k] = a.ff[k].v;
+      for (int k = 0; k < 3; k++) h.to_osac[o][k] = opt[s][o].to[k].v;
+      for (int k = 0; k < 9; k++) { h.fwd[o][k] = opt[s][o].fwd[k].v; h.bwd[o][k] = opt[s][o].bwd[k].v; }
     }
-  for (int s = 0; s < 4; s++) F.rc[s] = d->rc[s];
-  F.ap = d->ap;
+    for (int k = 0; k < 3; k++) { h.front_fwd[k] = opt[s][0].ff[k].v; h.osac0f[k] = mid[s].tof[k]; }
+    h.front_fwdf = (float) h.front_fwd[0];
+    for (int k = 0; k < 9; k++) { h.mid[k] = mid[s].m[k].v; h.bwd0f[k] = mid[s].bwdf[k]; }
+    for (int k = 0; k < 3; k++) h.mid_off[k] = mid[s].c[k].v;
+    for (int k = 0; k < 3; k++) {
+      S.p1[k] = h.fwd[0][3 * k] * p0[0].v + h.fwd[0][3 * k + 1] * p0[1].v + h.fwd[0][3 * k + 2] * p0[2].v;
+      S.p1f[k] = (float) S.p1[k];
+    }
+    S.beta = (float) d->rc[s].beta;
+    S.delta = (float) d->rc[s].delta;
+    S.wscale = d->rc[s].corr * d->rc[s].corr * d->vig;
+  }
   for (int k = 0; k < 3; k++) F.p0[k] = p0[k].v;
   F.vig = d->vig;
+  F.ideal = d->ap.ideal;
+  F.area_uniform = d->ap.area_uniform;
+  F.weighted = d->rc[0].weighted;
   F.g = d->g;
   return MX_OK;
 }
@@ -654,6 +913,8 @@ mx_diff *mx_diff_create(mx_context *c, const mx_diff_config *cfg) {
   g.knorm = (float) (1.0 / (std::sqrt(2.0 * PI_D) * k.sigma));
   // Each tap product is below w K^2 2^61 with w < 2; a pixel sums at most
   // n_rays of them, so shifting by log2(n K^2 / 4) + 1 keeps it in 64 bits.
+  g.top_u = mx::dkey(g.nx + (double) mxd::HALF);
+  g.top_v = mx::dkey(g.ny + (double) mxd::HALF);
   const double kmax = g.knorm;
   int shift = (int) std::ceil(std::log2((double) k.n_rays * kmax * kmax / 4.0)) + 1;
   g.shift = shift < 0 ? 0 : shift;
@@ -690,15 +951,16 @@ mx_diff *mx_diff_create(mx_context *c, const mx_diff_config *cfg) {
 
   cudaError_t e = cudaSetDevice(c->device);
   if (e == cudaSuccess) {
-    d->fwd_smem = align_up(sizeof(FwdArgs)) + sizeof(unsigned long long) * WIN * WIN + 4 * DWARPS * 32 * STAGE_STRIDE;
-    d->rays_smem = align_up(sizeof(FwdArgs)) + 4 * DWARPS * 32 * STAGE_STRIDE;
+    d->rays_smem = align_up(sizeof(FwdArgs)) + DWARPS * sizeof(RayList);
+    d->fwd_smem = d->rays_smem + 4 * (2 * WIN * WSTRIDE + DWARPS * 16 * STAGE_STRIDE);
     d->adj_smem = align_up(sizeof(AdjArgs)) + 4 * WIN * (WIN + 1) + 4 * DWARPS * 32 * ADJ_STAGE + 4 * ADJ_TILE +
                   4 * DWARPS;
-    e = occupancy(diff_forward_kernel<true>, d->fwd_smem, c->num_sms, &d->fwd_blocks);
+    e = occupancy(diff_forward_kernel<true, false>, d->fwd_smem, c->num_sms, &d->fwd_blocks);
   }
-  if (e == cudaSuccess) e = occupancy(diff_forward_kernel<false>, d->rays_smem, c->num_sms, &d->rays_blocks);
+  if (e == cudaSuccess) e = occupancy(diff_forward_kernel<true, true>, d->fwd_smem, c->num_sms, &d->mom_blocks);
+  if (e == cudaSuccess) e = occupancy(diff_forward_kernel<false, false>, d->rays_smem, c->num_sms, &d->rays_blocks);
   if (e == cudaSuccess) e = occupancy(diff_adjoint_kernel, d->adj_smem, c->num_sms, &d->adj_blocks);
-  const int maxb = std::max(d->fwd_blocks, std::max(d->rays_blocks, d->adj_blocks));
+  const int maxb = std::max(d->mom_blocks, d->adj_blocks);
   if (e == cudaSuccess) e = d->codes.ensure(k.n_rays);
   if (e == cudaSuccess) e = d->acc.ensure(sizeof(unsigned long long) * k.nx * k.ny);
   if (e == cudaSuccess) e = d->part.ensure(sizeof(double) * (size_t) maxb * NP);
@@ -736,13 +998,18 @@ int mx_diff_forward(mx_diff *d, const double *theta, int mode, double *image, do
   const size_t npix = (size_t) d->cfg.nx * d->cfg.ny;
   cudaError_t e = cudaMemsetAsync(d->acc.ptr, 0, npix * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return mx_cuda_fail(c, e, "mx_diff_forward");
-  diff_forward_kernel<true><<<d->fwd_blocks, DBLOCK, d->fwd_smem, st>>>(
-      F, c->T, d->cfg.n_rays, d->cfg.seed, (uint8_t *) d->codes.ptr, mode, (unsigned long long *) d->acc.ptr,
-      (double *) d->part.ptr, nullptr);
+  unsigned long long *acc = (unsigned long long *) d->acc.ptr;
+  if (moments)
+    diff_forward_kernel<true, true><<<d->mom_blocks, DBLOCK, d->fwd_smem, st>>>(
+        F, c->T, d->cfg.n_rays, d->cfg.seed, (uint8_t *) d->codes.ptr, mode, acc, (double *) d->part.ptr, nullptr);
+  else
+    diff_forward_kernel<true, false><<<d->fwd_blocks, DBLOCK, d->fwd_smem, st>>>(
+        F, c->T, d->cfg.n_rays, d->cfg.seed, (uint8_t *) d->codes.ptr, mode, acc, nullptr, nullptr);
   const double scale = std::ldexp(1.0, d->g.shift - 61) / (double) d->cfg.n_rays;
-  diff_image_kernel<<<2 * c->num_sms, 256, 0, st>>>((const unsigned long long *) d->acc.ptr, npix, scale, image);
-  diff_sum_kernel<<<1, 32, 0, st>>>((const double *) d->part.ptr, d->fwd_blocks, 4, 1.0, (double *) d->out.ptr);
-  c->launches += 3;
+  diff_image_kernel<<<2 * c->num_sms, 256, 0, st>>>(acc, npix, scale, image);
+  if (moments)
+    diff_sum_kernel<<<1, 32 * 4, 0, st>>>((const double *) d->part.ptr, d->mom_blocks, 4, 1.0, (double *) d->out.ptr);
+  c->launches += moments ? 3 : 2;
   if ((e = cudaGetLastError()) != cudaSuccess) return mx_cuda_fail(c, e, "mx_diff_forward: launch");
   if (mode == MX_DIFF_RECORD) d->recorded = true;
   if (moments) {
@@ -767,8 +1034,8 @@ int mx_diff_rays(mx_diff *d, const double *theta, int mode, double *yzw, void *s
   if ((r = fill_fwd(d, theta, F))) return r;
   mx_context *c = d->ctx;
   cudaStream_t st = (cudaStream_t) stream;
-  diff_forward_kernel<false><<<d->rays_blocks, DBLOCK, d->rays_smem, st>>>(
-      F, c->T, d->cfg.n_rays, d->cfg.seed, (uint8_t *) d->codes.ptr, mode, nullptr, (double *) d->part.ptr, yzw);
+  diff_forward_kernel<false, false><<<d->rays_blocks, DBLOCK, d->rays_smem, st>>>(
+      F, c->T, d->cfg.n_rays, d->cfg.seed, (uint8_t *) d->codes.ptr, mode, nullptr, nullptr, yzw);
   c->launches += 1;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return mx_cuda_fail(c, e, "mx_diff_rays: launch");
@@ -780,7 +1047,9 @@ int mx_diff_mse(mx_diff *d, const double *image, const double *target, double *d
                 void *stream) {
   if (!d) return mx_fail(nullptr, MX_EINVAL, "mx_diff_mse: null handle");
   if (!image || !target || !loss) return diff_fail(d, MX_EINVAL, "mx_diff_mse: image, target and loss are required");
-  diff_mse_kernel<<<1, 1024, 0, (cudaStream_t) stream>>>(image, target, (size_t) d->cfg.nx * d->cfg.ny, dl_dimage, loss);
+  const size_t npix = (size_t) d->cfg.nx * d->cfg.ny;
+  diff_mse_kernel<<<MSE_BLOCKS, MSE_THREADS, 0, (cudaStream_t) stream>>>(
+      image, target, npix, 1.0 / (double) npix, dl_dimage, loss);
   d->ctx->launches += 1;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MX_OK : mx_cuda_fail(d->ctx, e, "mx_diff_mse: launch");
@@ -799,7 +1068,7 @@ int mx_diff_adjoint_async(mx_diff *d, const double *theta, const double *dl_dima
   diff_adjoint_kernel<<<d->adj_blocks, DBLOCK, d->adj_smem, st>>>(A, d->cfg.n_rays, d->cfg.seed,
                                                                    (const uint8_t *) d->codes.ptr, dl_dimage,
                                                                    (double *) d->part.ptr);
-  diff_sum_kernel<<<1, 32, 0, st>>>((const double *) d->part.ptr, d->adj_blocks, NP, 1.0 / (double) d->cfg.n_rays,
+  diff_sum_kernel<<<1, 32 * NP, 0, st>>>((const double *) d->part.ptr, d->adj_blocks, NP, 1.0 / (double) d->cfg.n_rays,
                                     grad_dev);
   c->launches += 2;
   cudaError_t e = cudaGetLastError();

@@ -307,6 +307,50 @@ MXG bool conic_hit(const Optic<S> &o, V3<S> &x0, const V3<S> &p, V3<S> &n, int r
 // afresh.  Replaying it keeps the traced function smooth in the parameters.
 enum : uint8_t { RAY_HIT = 1, RAY_ROOT_P = 2, RAY_ROOT_H = 4 };
 
+#ifdef __CUDACC__
+// conic_hit in double for the few rays conic_root leaves to it: the root
+// taken (0 or 1), -1 for a miss.
+static __device__ __noinline__ int conic_root_double(const MxShellDev &h, int o, mx::D3 &x, const mx::D3 &p, mx::D3 &n,
+                                                     int root) {
+  Optic<double> op;
+  op.a = h.a[o]; op.b = h.b[o]; op.c = h.c[o]; op.xmin = h.xmin[o]; op.xmax = h.xmax[o];
+  V3<double> r = v3<double>(x.x, x.y, x.z), m;
+  int chosen = root;
+  if (!conic_hit<double>(op, r, v3<double>(p.x, p.y, p.z), m, root, &chosen)) return -1;
+  x = mx::mk(r.x, r.y, r.z);
+  n = mx::mk(m.x, m.y, m.z);
+  return chosen;
+}
+
+// conic_hit for a ray as the trace meets it, by Newton steps from the one
+// crossing between the conic's ends (mx::conic_newton).  That crossing is
+// root 0, the intersection nearer to the plane x = 0, when the sum of both,
+// -beta / alpha, is more than twice as far from zero (in float, with room to
+// spare: beta / alpha is of the order of 1e5 mm).  A ray without such a
+// crossing certainly misses if it is not replayed and the screen says so;
+// all others, those that follow root 1 among them, take the double form.
+__device__ __forceinline__ int conic_root(const MxShellDev &h, int o, mx::D3 &x, const mx::D3 &p, mx::D3 &n, int root) {
+  if (root <= 0) {
+    mx::D3 r = x, m;
+    const int hit = mx::conic_newton(h, o, r, p, m);
+    if (hit > 0) {
+      const float inv = 1.0f / mx::d2f_trunc(p.x), my = mx::d2f_trunc(p.y) * inv, mz = mx::d2f_trunc(p.z) * inv;
+      const float xf = mx::d2f_trunc(r.x), m2 = fmaf(my, my, mz * mz), alpha = m2 - h.am1f[o];
+      const float beta = fmaf(2.0f, fmaf(mx::d2f_trunc(r.y), my, mx::d2f_trunc(r.z) * mz) - xf * m2, -h.bf[o]);
+      if (fabsf(beta) > fmaf(2.5f, fabsf(alpha * xf), 0.01f)) { x = r; n = m; return 0; }
+    } else if (hit < 0 && root < 0)
+      return -1;
+  }
+  return conic_root_double(h, o, x, p, n, root);
+}
+
+// p - 2 (p.n) n
+__device__ __forceinline__ mx::D3 reflected(const mx::D3 &p, const mx::D3 &n, double pdn) {
+  const double k = -2.0 * pdn;
+  return mx::mk(fma(k, n.x, p.x), fma(k, n.y, p.y), fma(k, n.z, p.z));
+}
+#endif
+
 // Everything a weighted ray needs besides the two optics of its shell.
 struct RayConst {
   double front;        // front_position of the shell (aperture plane)
