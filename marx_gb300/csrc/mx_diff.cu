@@ -12,17 +12,16 @@
 // splats its 32 rays together, one ray at a time, each lane adding four of
 // the 121 taps, so the lanes of one atomic instruction never collide.
 //
-// Adjoint: the ray is traced again with Dual6 scalars (FP64 value, FP32
-// derivatives with respect to the six parameters that move it), following
-// the decisions recorded by the forward pass; dL/dimage over the ray's
-// 11 x 11 window gives dL/d(u, v, w), and the ray's derivative of
-// (u, v, w) turns that into six parameter contributions.  Nothing per ray
-// is stored between the passes except the decision byte.  A block takes
-// the rays of a tile whose decision byte says they reached the focal plane
-// (a ballot and prefix sum into shared memory, in ascending order) and
-// traces only those, so that its lanes do not idle through the rays that
-// were lost.  Sums are deterministic: fixed tiles per block, fixed warp
-// order, fixed block order, one final reduction.
+// Adjoint: the recorded rays are traced again with mxd::Dual scalars (FP64
+// value, FP32 tangents of the four parameters that bend the ray's path: its
+// shell's two tilts and the source's two offsets; the decenters shift the
+// image); dL/dimage over the ray's 11 x 11 window gives dL/d(u, v, w), and the
+// tangents of (u, v, w) turn that into six parameter contributions.  Nothing
+// per ray is stored between the passes except the decision byte.  A block
+// takes the rays of a tile whose decision byte says they reached the focal
+// plane, in ascending order, and traces only those, so that its lanes do not
+// idle through the rays that were lost.  Sums are deterministic: fixed tiles
+// per block, fixed warp order, fixed block order, one final reduction.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -60,13 +59,6 @@ struct ImageGeom {
   long long top_u, top_v;        // mx::dkey of nx + HALF and ny + HALF
 };
 
-// What the aperture sampling needs of each shell (project_photon_to_hrma).
-struct Aperture {
-  double area[4], rmin[4], rmax[4];
-  uint32_t shutter[4];
-  int32_t ideal, area_uniform;
-};
-
 // One shell at theta: its geometry in the trace's own record (so that the
 // rays take the trace's conics, screens and struts), the source direction in
 // the paraboloid's frame, and the reflection's constants.
@@ -87,83 +79,24 @@ struct FwdArgs {
   ImageGeom g;
 };
 
+// One shell's geometry with its tangents.
+struct ShellTangents {
+  mxd::Turn front[3], fwd[9];    // of the paraboloid
+  mxd::Turn mid[9], off[3];
+  mxd::Turn bwd[9];              // of the hyperboloid
+  mxd::Dual p1[3];               // fwd p0, made on the device
+  double corr;                   // effective-area correction per reflection
+  double pad[2];                 // 624 bytes: lanes that load one field of different shells do not conflict
+};
+
 struct AdjArgs {
-  mxd::Optic<Dual6> opt[4][2];
-  mxd::Between<Dual6> mid[4];
-  mxd::RayConst rc[4];
-  Aperture ap;
-  Dual6 p0[3];
-  double vig;
-  ImageGeom g;
+  FwdArgs f;
+  ShellTangents d[4];
+  mxd::Dual p0[3];
+  mxd::Fresnel fr;
 };
 
 __host__ __device__ constexpr size_t align_up(size_t b) { return (b + 15) & ~(size_t) 15; }
-
-// Strut shadows (intersects_struts, hrma.c:928-968) at the three planes,
-// evaluated on the ray's values.
-struct StrutTest {
-  const MxTables *T;
-  template <class S>
-  __device__ bool operator()(int set, const mxd::V3<S> &x, const mxd::V3<S> &p) const {
-    if (!T->use_struts) return false;
-    return mx::struts_block(*T, set, mx::mk(mxd::val(x.x), mxd::val(x.y), mxd::val(x.z)),
-                            mx::mk(mxd::val(p.x), mxd::val(p.y), mxd::val(p.z)));
-  }
-  // The cap struts for a ray in the paraboloid's frame: screened on its
-  // MARX-frame coordinates formed in single precision (as the trace's
-  // cap_struts_block does), decided in double near a bar edge.
-  template <class S>
-  __device__ bool cap(const mxd::Optic<S> &P, const mxd::Between<S> &B, const mxd::V3<S> &x, const mxd::V3<S> &p) const {
-    if (!T->use_struts) return false;
-    const float xx = mx::d2f_trunc(mxd::val(x.x)), xy = mx::d2f_trunc(mxd::val(x.y)), xz = mx::d2f_trunc(mxd::val(x.z));
-    const float px = mx::d2f_trunc(mxd::val(p.x)), py = mx::d2f_trunc(mxd::val(p.y)), pz = mx::d2f_trunc(mxd::val(p.z));
-    const float *m = B.bwdf;
-    const int s = mx::struts_screen(*T, 1, fmaf(m[0], xx, fmaf(m[1], xy, m[2] * xz)) - B.tof[0],
-                                    fmaf(m[3], xx, fmaf(m[4], xy, m[5] * xz)) - B.tof[1],
-                                    fmaf(m[6], xx, fmaf(m[7], xy, m[8] * xz)) - B.tof[2],
-                                    fmaf(m[0], px, fmaf(m[1], py, m[2] * pz)), fmaf(m[3], px, fmaf(m[4], py, m[5] * pz)),
-                                    fmaf(m[6], px, fmaf(m[7], py, m[8] * pz)));
-    if (s >= 0) return s == 1;
-    mxd::V3<S> pm = mxd::matv(P.bwd, p), xm = mxd::matv(P.bwd, x) - mxd::v3<S>(P.to[0], P.to[1], P.to[2]);
-    return mx::struts_block_exact(*T, 1, mx::mk(mxd::val(xm.x), mxd::val(xm.y), mxd::val(xm.z)),
-                                  mx::mk(mxd::val(pm.x), mxd::val(pm.y), mxd::val(pm.z)));
-  }
-};
-
-// The aperture point of ray `tag`: the shell pick, radius and azimuth the
-// mirror stage draws for the photon of that tag (mirror_front), with the
-// vignetting draw consumed but turned into a weight.
-__device__ __forceinline__ bool aperture(const Aperture &ap, uint64_t seed, uint32_t tag, int &si, double &ry,
-                                         double &rz) {
-  mx::Rng rng;
-  rng.U = nullptr; rng.N = nullptr; rng.seed = seed; rng.n = 0; rng.i = 0; rng.tag = tag; rng.overrun = false;
-  rng.window(MX_U_MIRROR, 12, MX_N_MIRROR, 2);
-  if (!ap.ideal) (void) rng.uniform();
-  si = -1;
-  for (int guard = 0; guard < 64 && si < 0; guard++) {
-    const double r = rng.uniform();
-    if (rng.overrun) return false;
-    for (int i = 0; i < 4; i++)
-      if (mx::lt_pos(r, ap.area[i])) { si = i; break; }
-  }
-  if (si < 0) return false;
-  double radius;
-  const double r0 = ap.rmin[si], r1 = ap.rmax[si];
-  if (ap.area_uniform) radius = mx::sqrt_fast(r0 * r0 + (r1 * r1 - r0 * r0) * rng.uniform());
-  else radius = r0 + (r1 - r0) * rng.uniform();
-  double theta;
-  for (int guard = 0;; guard++) {
-    theta = rng.uniform();
-    const unsigned quad = mx::quarter_of(theta);
-    if (rng.overrun || guard >= 64) return false;
-    if (ap.shutter[si] & (1u << quad)) break;
-  }
-  double st, ct;
-  mx::sincospi_fast(fma(theta, 2.0, -0.25), &st, &ct);   // angle 2 pi (u - 1/8)
-  ry = radius * st;
-  rz = radius * ct;
-  return true;
-}
 
 // The pixel nearest to coordinate u, floor(u + 1/2), and the offset u - pixel
 // rounded to float; false unless -(HALF + 1) < u < n + HALF (the ray's 11 x 11
@@ -321,7 +254,7 @@ __device__ __forceinline__ void splat_warp(const ImageGeom &g, const SplatWindow
 // with the vignetting draw consumed but turned into a weight), and unless it
 // is replayed the pre-collimator struts and the float screen for rays that
 // certainly miss the paraboloid.  False for a ray that ends here.
-__device__ __forceinline__ bool ray_front(const FwdArgs &A, const MxTables &T, uint64_t seed, uint32_t tag, bool replay,
+__device__ __forceinline__ bool ray_front(const FwdArgs &A, const MxTables *T, uint64_t seed, uint32_t tag, bool replay,
                                           int &si, double &radius, mx::F2 &s, mx::F2 &c) {
   mx::Rng rng;
   rng.U = nullptr; rng.N = nullptr; rng.seed = seed; rng.n = 0; rng.i = 0; rng.tag = tag; rng.overrun = false;
@@ -350,11 +283,11 @@ __device__ __forceinline__ bool ray_front(const FwdArgs &A, const MxTables &T, u
   mx::df_turn_sincos(theta, true, s, c);   // of the angle 2 pi (u - 1/8)
   if (replay) return true;
   const float rf = mx::d2f_trunc(radius), yf = rf * s.h, zf = rf * c.h;
-  if (T.use_struts) {
+  if (T->use_struts) {
     const float pxf = mx::d2f_trunc(A.p0[0]), pyf = mx::d2f_trunc(A.p0[1]), pzf = mx::d2f_trunc(A.p0[2]);
-    int blocked = mx::struts_screen(T, 0, h.frontf, yf - h.osac0f[1], zf - h.osac0f[2], pxf, pyf, pzf);
+    int blocked = mx::struts_screen(*T, 0, h.frontf, yf - h.osac0f[1], zf - h.osac0f[2], pxf, pyf, pzf);
     if (blocked < 0)
-      blocked = mx::struts_block_exact(T, 0, mx::mk(h.front_position, radius * mx::df_join(s) - h.to_osac[0][1],
+      blocked = mx::struts_block_exact(*T, 0, mx::mk(h.front_position, radius * mx::df_join(s) - h.to_osac[0][1],
                                                     radius * mx::df_join(c) - h.to_osac[0][2]),
                                        mx::mk(A.p0[0], A.p0[1], A.p0[2])) ? 1 : 0;
     if (blocked) return false;
@@ -464,7 +397,7 @@ __global__ void __launch_bounds__(DBLOCK, FWD_BLOCKS) diff_forward_kernel(const 
       mx::F2 s{0.f, 0.f}, c{0.f, 0.f};
       bool on = i < n;
       if (on && replay) on = (codes[i] & mxd::RAY_HIT) != 0;
-      if (on) on = ray_front(A, T, seed, (uint32_t) i, replay, si, radius, s, c);
+      if (on) on = ray_front(A, &T, seed, (uint32_t) i, replay, si, radius, s, c);
       if (i < n && !on) {
         if (mode == MX_DIFF_RECORD) codes[i] = 0;
         if (!SPLAT) {
@@ -599,12 +532,70 @@ __device__ __forceinline__ float resid_at(const ImageGeom &g, const float *rw, c
   return 0.f;
 }
 
+// A recorded ray again, from the aperture to the focal plane x = 0, with
+// tangents.
+__device__ __forceinline__ bool ray_tangents(const AdjArgs &A, int si, double ry, double rz, int root, mxd::Dual &y,
+                                             mxd::Dual &z, float &w, float (&wd)[mxd::NT]) {
+  const ShellTangents &S = A.d[si];
+  const MxShellDev &h = A.f.sh[si].h;
+  mxd::V3 x = {mxd::turned(S.front[0], S.fwd[1], S.fwd[2], ry, rz), mxd::turned(S.front[1], S.fwd[4], S.fwd[5], ry, rz),
+               mxd::turned(S.front[2], S.fwd[7], S.fwd[8], ry, rz)};
+  mxd::V3 p = {S.p1[0], S.p1[1], S.p1[2]}, n;
+  if (!mxd::conic_tangents(h, 0, x, p, n, (root & mxd::RAY_ROOT_P) ? 1 : 0)) return false;
+  mxd::Dual pdn = mxd::dotp(p, n);
+  mx::F2 w1{1.0f, 0.0f}, w2{1.0f, 0.0f}, corr{1.0f, 0.0f};
+  float s1 = 0.0f, s2 = 0.0f;
+  if (A.f.weighted) {
+    corr = mx::split(S.corr);
+    mx::F2 r;
+    mxd::fresnel_slope(A.fr, mx::split(fabs(pdn.v)), r, s1);
+    w1 = mx::df_mul(r, corr);
+    s1 = mxd::tof(S.corr) * (mx::neg_bit(pdn.v) ? -s1 : s1);
+  }
+#pragma unroll
+  for (int k = 0; k < mxd::NT; k++) wd[k] = s1 * pdn.d[k];
+  {
+    const mxd::Dual q = 2.0 * pdn;
+    p = {p.x - q * n.x, p.y - q * n.y, p.z - q * n.z};
+  }
+  p = mxd::matv(S.mid, p);
+  x = mxd::matv(S.mid, x);
+  x = {x.x + S.off[0], x.y + S.off[1], x.z + S.off[2]};
+  if (!mxd::conic_tangents(h, 1, x, p, n, (root & mxd::RAY_ROOT_H) ? 1 : 0)) return false;
+  pdn = mxd::dotp(p, n);
+  if (A.f.weighted) {
+    mx::F2 r;
+    mxd::fresnel_slope(A.fr, mx::split(fabs(pdn.v)), r, s2);
+    w2 = mx::df_mul(r, corr);
+    s2 = mxd::tof(S.corr) * (mx::neg_bit(pdn.v) ? -s2 : s2);
+  }
+  const float w1f = mxd::tof(w1), w2f = mxd::tof(w2);
+#pragma unroll
+  for (int k = 0; k < mxd::NT; k++) wd[k] = w1f * (s2 * pdn.d[k]) + w2f * wd[k];
+  w = mx::df_mul(w1, w2).h;
+  {
+    const mxd::Dual q = 2.0 * pdn;
+    p = {p.x - q * n.x, p.y - q * n.y, p.z - q * n.z};
+  }
+  p = mxd::matv(S.bwd, p);
+  x = mxd::matv(S.bwd, x);
+  x = {x.x - h.to_osac[1][0], x.y - h.to_osac[1][1], x.z - h.to_osac[1][2]};
+  const mxd::Dual t = (0.0 - x.x) * mxd::drcp(p.x);
+  y = x.y + t * p.y;
+  z = x.z + t * p.z;
+  return true;
+}
+
 // part[block][NP] = sum over the block's rays of dl/dimage . d(image)/dtheta
-// (before the 1/n_rays factor).  Compiled for two resident blocks per SM
-// (128 registers): the tangents then spill about 600 bytes per thread to
-// local memory, but twice the warps hide the FP64 and load latencies that
-// left one block of 248 registers 43 % FP64-busy (2.45 -> 1.83 ms per 4e6
-// rays).
+// (before the 1/n_rays factor).
+//
+// Per 1e6 rays: 500 -> 305 us (FP64 pipe 57 % busy with 3.1 instead of 5.9
+// million instructions; the rest are the tangents' FP32 steps and the window
+// sums).  What went: the library's roots and divisions, the decenters'
+// tangents, which are constants, the Fresnel chain in six directions (one
+// slope, its values in double-float), the root that is not followed.  Two
+// blocks per SM (128 registers): three of 80 spill and take 2.40 instead of
+// 2.35 ms for a gradient step over 4e6 rays.
 __global__ void __launch_bounds__(DBLOCK, 2) diff_adjoint_kernel(const __grid_constant__ AdjArgs args, uint64_t n,
                                                                uint64_t seed, const uint8_t *codes,
                                                                const double *dl, double *part) {
@@ -613,97 +604,104 @@ __global__ void __launch_bounds__(DBLOCK, 2) diff_adjoint_kernel(const __grid_co
   float *rw = reinterpret_cast<float *>(smem + align_up(sizeof(AdjArgs)));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float *stage = rw + WIN * (WIN + 1) + warp * 32 * ADJ_STAGE;
+  uint32_t *wcnt = reinterpret_cast<uint32_t *>(rw + WIN * (WIN + 1) + DWARPS * 32 * ADJ_STAGE);   // DWARPS entries
+  uint16_t *list = reinterpret_cast<uint16_t *>(wcnt + DWARPS);                                    // ADJ_TILE entries
   {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(&args);
     uint32_t *dst = reinterpret_cast<uint32_t *>(smem);
     for (int k = threadIdx.x; k < (int) (sizeof(AdjArgs) / 4); k += DBLOCK) dst[k] = src[k];
-    for (int k = threadIdx.x; k < args.g.wnx * args.g.wny; k += DBLOCK) {
-      const int r = k / args.g.wnx, c = k - r * args.g.wnx;
-      rw[r * (WIN + 1) + c] = (float) dl[(size_t) (args.g.wy0 + r) * args.g.nx + args.g.wx0 + c];
+    const ImageGeom &q = args.f.g;
+    for (int k = threadIdx.x; k < q.wnx * q.wny; k += DBLOCK) {
+      const int r = k / q.wnx, c = k - r * q.wnx;
+      rw[r * (WIN + 1) + c] = (float) dl[(size_t) (q.wy0 + r) * q.nx + q.wx0 + c];
     }
   }
   __syncthreads();
-  const ImageGeom &g = A.g;
-  const mxd::V3<Dual6> p0 = mxd::v3<Dual6>(A.p0[0], A.p0[1], A.p0[2]);
-  const StrutTest none{nullptr};   // decisions are replayed: the strut test is never called
-  uint32_t *list = reinterpret_cast<uint32_t *>(rw + WIN * (WIN + 1) + DWARPS * 32 * ADJ_STAGE);   // ADJ_TILE entries
-  uint32_t *wcnt = list + ADJ_TILE;                                                 // DWARPS entries
+  if (threadIdx.x < 4) {
+    ShellTangents &S = A.d[threadIdx.x];
+    const mxd::V3 p = mxd::matv(S.fwd, {A.p0[0], A.p0[1], A.p0[2]});
+    S.p1[0] = p.x; S.p1[1] = p.y; S.p1[2] = p.z;
+  }
+  const ImageGeom &g = A.f.g;
   double pacc = 0.0;               // lane p < NP: this warp's sum for parameter p
   for (uint64_t tile = (uint64_t) blockIdx.x * ADJ_TILE; tile < n; tile += (uint64_t) gridDim.x * ADJ_TILE) {
     // The rays of the tile that reached the focal plane, in ascending order:
     // only they contribute, and lanes given the others would idle through
-    // the whole ray.
-    uint32_t nh = 0;
-    for (int j = 0; j < ADJ_TILE / DBLOCK; j++) {
-      const uint64_t i = tile + (uint64_t) j * DBLOCK + threadIdx.x;
-      const bool hit = i < n && (codes[i] & mxd::RAY_HIT);
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) wcnt[warp] = (uint32_t) __popc(m);
-      __syncthreads();
-      uint32_t off = nh, tot = nh;
-      for (int k = 0; k < DWARPS; k++) {
-        const uint32_t c = wcnt[k];
-        off += k < warp ? c : 0u;
-        tot += c;
-      }
-      if (hit) list[off + __popc(m & ((1u << lane) - 1u))] = (uint32_t) (i - tile);
-      __syncthreads();
-      nh = tot;
+    // the whole ray.  A thread takes eight decision bytes.
+    const uint64_t i0 = tile + 8 * threadIdx.x;
+    unsigned long long word = 0;
+    if (i0 + 8 <= n) word = *reinterpret_cast<const unsigned long long *>(codes + i0);
+    else
+      for (int b = 0; b < 8; b++)
+        if (i0 + b < n) word |= (unsigned long long) codes[i0 + b] << (8 * b);
+    word &= 0x0101010101010101ull * mxd::RAY_HIT;
+    const uint32_t mine = (uint32_t) __popcll(word);
+    uint32_t off = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, off, o);
+      if (lane >= o) off += v;
     }
-    for (uint32_t b0 = 0; b0 < nh; b0 += DBLOCK) {
-      const uint32_t kk = b0 + threadIdx.x;
-      const bool valid = kk < nh;
-      if (!__any_sync(0xffffffffu, valid)) continue;   // the warp has no ray in this round
-      const uint64_t i = valid ? tile + list[kk] : 0;
+    if (lane == 31) wcnt[warp] = off;
+    __syncthreads();
+    off -= mine;
+    uint32_t nh = 0;
+    for (int k = 0; k < DWARPS; k++) {
+      const uint32_t c = wcnt[k];
+      off += k < warp ? c : 0u;
+      nh += c;
+    }
+    for (int b = 0; b < 8; b++)
+      if ((word >> (8 * b)) & 1ull) list[off++] = (uint16_t) (8 * threadIdx.x + b);
+    __syncthreads();
+    for (uint32_t b0 = warp * 32; b0 < nh; b0 += DBLOCK) {
       float c6[mxd::ND];
 #pragma unroll
       for (int k = 0; k < mxd::ND; k++) c6[k] = 0.f;
       int si = -1;
-      uint8_t code = valid ? codes[i] : 0;
-      double ry, rz;
-      if (valid && aperture(A.ap, seed, (uint32_t) i, si, ry, rz)) {
-        Dual6 y, z, w;
+      double radius;
+      mx::F2 s2, c2;
+      const bool valid = b0 + lane < nh;
+      const uint32_t i = valid ? (uint32_t) (tile + list[b0 + lane]) : 0u;
+      if (valid && ray_front(A.f, nullptr, seed, i, true, si, radius, s2, c2)) {
+        mxd::Dual y, z;
+        float w, wd[mxd::NT];
         int ic, jc;
         float fu, fv;
-        if (mxd::weighted_ray<Dual6>(A.opt[si][0], A.opt[si][1], A.mid[si], A.rc[si], ry, rz, p0, true, code, none, y,
-                                     z, w) &&
-            w.v > 0.0 && splat_origin(g, y.v, z.v, ic, jc, fu, fv)) {
-          float ky[mxd::TAPS], kyd[mxd::TAPS], kz[mxd::TAPS], kzd[mxd::TAPS];
+        if (ray_tangents(A, si, radius * mx::df_join(s2), radius * mx::df_join(c2), codes[i], y, z, w, wd) && w > 0.0f &&
+            splat_origin(g, y.v, z.v, ic, jc, fu, fv)) {
+          float ky[mxd::TAPS], kyd[mxd::TAPS];
 #pragma unroll
           for (int k = 0; k < mxd::TAPS; k++) {
             ky[k] = tap(g, k, fu);
             kyd[k] = ((float) (k - mxd::HALF) - fu) * g.inv_s2 * ky[k];
-            kz[k] = tap(g, k, fv);
-            kzd[k] = ((float) (k - mxd::HALF) - fv) * g.inv_s2 * kz[k];
           }
           float sw = 0.f, su = 0.f, sv = 0.f;
           const bool inside = ic - mxd::HALF >= g.wx0 && ic + mxd::HALF < g.wx0 + g.wnx &&
                               jc - mxd::HALF >= g.wy0 && jc + mxd::HALF < g.wy0 + g.wny;
-          if (inside) {
-            const float *base_row = rw + (jc - mxd::HALF - g.wy0) * (WIN + 1) + (ic - mxd::HALF - g.wx0);
+          const float *base_row = rw + (jc - mxd::HALF - g.wy0) * (WIN + 1) + (ic - mxd::HALF - g.wx0);
 #pragma unroll
-            for (int a = 0; a < mxd::TAPS; a++) {
+          for (int a = 0; a < mxd::TAPS; a++) {
+            float t = 0.f, td = 0.f;
+            if (inside) {
               const float *q = base_row + a * (WIN + 1);
-              float t = 0.f, td = 0.f;
 #pragma unroll
               for (int b = 0; b < mxd::TAPS; b++) { t += q[b] * ky[b]; td += q[b] * kyd[b]; }
-              sw += kz[a] * t; su += kz[a] * td; sv += kzd[a] * t;
-            }
-          } else {
-#pragma unroll
-            for (int a = 0; a < mxd::TAPS; a++) {
-              float t = 0.f, td = 0.f;
+            } else {
 #pragma unroll
               for (int b = 0; b < mxd::TAPS; b++) {
                 const float r = resid_at(g, rw, dl, jc - mxd::HALF + a, ic - mxd::HALF + b);
                 t += r * ky[b]; td += r * kyd[b];
               }
-              sw += kz[a] * t; su += kz[a] * td; sv += kzd[a] * t;
             }
+            const float kz = tap(g, a, fv), kzd = ((float) (a - mxd::HALF) - fv) * g.inv_s2 * kz;
+            sw += kz * t; su += kz * td; sv += kzd * t;
           }
-          const float vig = (float) A.vig, wv = (float) w.v * vig, ip = (float) g.inv_pitch;
+          const float vig = (float) A.f.vig, wi = w * vig * (float) g.inv_pitch;
 #pragma unroll
-          for (int k = 0; k < mxd::ND; k++) c6[k] = vig * sw * w.d[k] + wv * ip * (su * y.d[k] + sv * z.d[k]);
+          for (int k = 0; k < mxd::NT; k++)
+            c6[k < 2 ? k : k + 2] = vig * sw * wd[k] + wi * (su * y.d[k] + sv * z.d[k]);
+          c6[2] = wi * (su * 1e-3f);    // the decenters shift the image, by a micrometre
+          c6[3] = wi * (sv * -1e-3f);   // each: x0 towards +y, y0 towards -z
         } else
           si = -1;
       }
@@ -745,8 +743,9 @@ struct mx_diff {
   mx_context *ctx = nullptr;
   mx_diff_config cfg;
   ImageGeom g;
-  Aperture ap;
-  mxd::RayConst rc[4];
+  int32_t weighted = 0;              // 0: unit weights (ideal mirrors)
+  float beta = 0.f, delta = 1.f;     // optical constants at the ray energy
+  double corr[4] = {1.0, 1.0, 1.0, 1.0};   // effective-area correction per reflection
   double vig = 1.0;
   DevBuf codes, acc, part, out;   // out: 4 moments, then NP gradient values
   double *h_out = nullptr;        // pinned: moments and gradient read back
@@ -766,8 +765,7 @@ int diff_fail(mx_diff *d, int code, const std::string &msg) { return mx_fail(d ?
 // and el_mis (degrees in the geometry file) and decenters x0 and y0 (mm),
 // as read_hrma_geometry_file (hrma.c:319-391) and init_hrma_shells take
 // them; the rotations are rebuilt as init_yaw_pitch does.
-int build_optics(mx_diff *d, const double *theta, mxd::Optic<Dual6> opt[4][2], mxd::Between<Dual6> mid[4],
-                 Dual6 p0[3]) {
+int build_optics(mx_diff *d, const double *theta, mxd::Optic opt[4][2], mxd::Between mid[4], Dual6 p0[3]) {
   mx_context *c = d->ctx;
   std::string err;
   size_t cnt = 0;
@@ -778,8 +776,7 @@ int build_optics(mx_diff *d, const double *theta, mxd::Optic<Dual6> opt[4][2], m
     const double cap_pos = c->cfg.hrma_cap_x + c->cfg.shell_xoffset[s];
     for (int o = 0; o < 2; o++) {
       const double *q = rdb + (4 * o + s) * 9;   // x0 y0 z0 p k rho0 az el l
-      mxd::Optic<Dual6> &op = opt[s][o];
-      op.a = h.a[o]; op.b = h.b[o]; op.c = h.c[o]; op.xmin = h.xmin[o]; op.xmax = h.xmax[o];
+      mxd::Optic &op = opt[s][o];
       Dual6 x0 = mxd::mkd(q[0] + theta[4 * s + 2] * 1e-3);
       x0.d[2] = 1e-3f;
       Dual6 y0 = mxd::mkd(q[1] + theta[4 * s + 3] * 1e-3);
@@ -791,23 +788,26 @@ int build_optics(mx_diff *d, const double *theta, mxd::Optic<Dual6> opt[4][2], m
       az.d[0] = (float) -ARCSEC;
       Dual6 el = mxd::mkd(-(q[7] + theta[4 * s + 1] / 3600.0) * (PI_D / 180.0));
       el.d[1] = (float) -ARCSEC;
-      mxd::yaw_pitch<Dual6>(op.fwd, op.bwd, az, el);
+      mxd::yaw_pitch(op.fwd, op.bwd, az, el);
       for (int r = 0; r < 3; r++) op.ff[r] = op.fwd[3 * r] * (h.front_position + op.to[0]);
     }
-    const mxd::Optic<Dual6> &P = opt[s][0], &H = opt[s][1];
-    mxd::Between<Dual6> &B = mid[s];
-    mxd::mat3_mul<Dual6>(B.m, H.fwd, P.bwd);
+    const mxd::Optic &P = opt[s][0], &H = opt[s][1];
+    mxd::Between &B = mid[s];
+    mxd::mat3_mul(B.m, H.fwd, P.bwd);
     const Dual6 dt[3] = {H.to[0] - P.to[0], H.to[1] - P.to[1], H.to[2] - P.to[2]};
     for (int r = 0; r < 3; r++) B.c[r] = H.fwd[3 * r] * dt[0] + H.fwd[3 * r + 1] * dt[1] + H.fwd[3 * r + 2] * dt[2];
-    for (int k = 0; k < 9; k++) B.bwdf[k] = (float) P.bwd[k].v;
-    for (int r = 0; r < 3; r++) B.tof[r] = (float) P.to[r].v;
   }
   Dual6 ay = mxd::mkd((d->cfg.src_y + theta[16]) * ARCSEC);
   ay.d[4] = (float) ARCSEC;
   Dual6 az = mxd::mkd((d->cfg.src_z + theta[17]) * ARCSEC);
   az.d[5] = (float) ARCSEC;
-  mxd::V3<Dual6> p = mxd::unit(mxd::v3<Dual6>(mxd::mkd(-1.0), 0.0 - mxd::dtan(ay), 0.0 - mxd::dtan(az)));
-  p0[0] = p.x; p0[1] = p.y; p0[2] = p.z;
+  const Dual6 ty = 0.0 - mxd::dtan(ay), tz = 0.0 - mxd::dtan(az), inv = mxd::drsqrt(1.0 + ty * ty + tz * tz);
+  p0[0] = 0.0 - inv; p0[1] = inv * ty; p0[2] = inv * tz;
+  for (int s = 0; s < 4; s++)
+    for (int r = 0; r < 3; r++) {
+      const Dual6 *m = opt[s][0].fwd + 3 * r;
+      mid[s].p1[r] = m[0] * p0[0] + m[1] * p0[1] + m[2] * p0[2];
+    }
   return MX_OK;
 }
 
@@ -819,13 +819,7 @@ int check_theta(mx_diff *d, const double *theta) {
   return MX_OK;
 }
 
-int fill_fwd(mx_diff *d, const double *theta, FwdArgs &F) {
-  mxd::Optic<Dual6> opt[4][2];
-  mxd::Between<Dual6> mid[4];
-  Dual6 p0[3];
-  int r = build_optics(d, theta, opt, mid, p0);
-  if (r) return r;
-  memset(&F, 0, sizeof(F));
+void fill_rays(mx_diff *d, const mxd::Optic opt[4][2], const mxd::Between mid[4], const Dual6 p0[3], FwdArgs &F) {
   for (int s = 0; s < 4; s++) {
     DiffShell &S = F.sh[s];
     MxShellDev &h = S.h;
@@ -834,35 +828,58 @@ int fill_fwd(mx_diff *d, const double *theta, FwdArgs &F) {
       for (int k = 0; k < 3; k++) h.to_osac[o][k] = opt[s][o].to[k].v;
       for (int k = 0; k < 9; k++) { h.fwd[o][k] = opt[s][o].fwd[k].v; h.bwd[o][k] = opt[s][o].bwd[k].v; }
     }
-    for (int k = 0; k < 3; k++) { h.front_fwd[k] = opt[s][0].ff[k].v; h.osac0f[k] = mid[s].tof[k]; }
+    for (int k = 0; k < 3; k++) { h.front_fwd[k] = opt[s][0].ff[k].v; h.osac0f[k] = (float) h.to_osac[0][k]; }
     h.front_fwdf = (float) h.front_fwd[0];
-    for (int k = 0; k < 9; k++) { h.mid[k] = mid[s].m[k].v; h.bwd0f[k] = mid[s].bwdf[k]; }
+    for (int k = 0; k < 9; k++) { h.mid[k] = mid[s].m[k].v; h.bwd0f[k] = (float) h.bwd[0][k]; }
     for (int k = 0; k < 3; k++) h.mid_off[k] = mid[s].c[k].v;
     for (int k = 0; k < 3; k++) {
-      S.p1[k] = h.fwd[0][3 * k] * p0[0].v + h.fwd[0][3 * k + 1] * p0[1].v + h.fwd[0][3 * k + 2] * p0[2].v;
+      S.p1[k] = mid[s].p1[k].v;
       S.p1f[k] = (float) S.p1[k];
     }
-    S.beta = (float) d->rc[s].beta;
-    S.delta = (float) d->rc[s].delta;
-    S.wscale = d->rc[s].corr * d->rc[s].corr * d->vig;
+    S.beta = d->beta;
+    S.delta = d->delta;
+    S.wscale = d->corr[s] * d->corr[s] * d->vig;
   }
   for (int k = 0; k < 3; k++) F.p0[k] = p0[k].v;
   F.vig = d->vig;
-  F.ideal = d->ap.ideal;
-  F.area_uniform = d->ap.area_uniform;
-  F.weighted = d->rc[0].weighted;
+  F.ideal = d->ctx->T.ideal;
+  F.area_uniform = d->ctx->T.area_uniform;
+  F.weighted = d->weighted;
   F.g = d->g;
+}
+
+int fill_fwd(mx_diff *d, const double *theta, FwdArgs &F) {
+  mxd::Optic opt[4][2];
+  mxd::Between mid[4];
+  Dual6 p0[3];
+  int r = build_optics(d, theta, opt, mid, p0);
+  if (r) return r;
+  memset(&F, 0, sizeof(F));
+  fill_rays(d, opt, mid, p0, F);
   return MX_OK;
 }
 
 int fill_adj(mx_diff *d, const double *theta, AdjArgs &A) {
-  memset(&A, 0, sizeof(A));
-  int r = build_optics(d, theta, A.opt, A.mid, A.p0);
+  mxd::Optic opt[4][2];
+  mxd::Between mid[4];
+  Dual6 p0[3];
+  int r = build_optics(d, theta, opt, mid, p0);
   if (r) return r;
-  for (int s = 0; s < 4; s++) A.rc[s] = d->rc[s];
-  A.ap = d->ap;
-  A.vig = d->vig;
-  A.g = d->g;
+  memset(&A, 0, sizeof(A));
+  fill_rays(d, opt, mid, p0, A.f);
+  const auto turn = [](const Dual6 &a) { return mxd::Turn{a.v, {a.d[0], a.d[1]}}; };
+  for (int s = 0; s < 4; s++) {
+    ShellTangents &D = A.d[s];
+    for (int j = 0; j < 3; j++) { D.front[j] = turn(opt[s][0].ff[j]); D.off[j] = turn(mid[s].c[j]); }
+    for (int j = 0; j < 9; j++) { D.fwd[j] = turn(opt[s][0].fwd[j]); D.mid[j] = turn(mid[s].m[j]); D.bwd[j] = turn(opt[s][1].bwd[j]); }
+    D.corr = d->corr[s];
+  }
+  for (int k = 0; k < 3; k++) A.p0[k] = mxd::Dual{p0[k].v, {0.f, 0.f, p0[k].d[4], p0[k].d[5]}};
+  const double nr = 1.0 - (double) d->delta, ni = d->beta;
+  const auto two = [](double v) { const float hi = (float) v; return mx::F2{hi, (float) (v - hi)}; };
+  A.fr.sr = two(nr * nr - ni * ni);
+  A.fr.si = two(2.0 * nr * ni);
+  A.fr.lost = two(1.0 - (nr * nr - ni * ni));
   return MX_OK;
 }
 
@@ -920,41 +937,29 @@ mx_diff *mx_diff_create(mx_context *c, const mx_diff_config *cfg) {
   g.shift = shift < 0 ? 0 : shift;
 
   const MxTables &T = c->T;
-  for (int s = 0; s < 4; s++) {
-    const MxShellDev &h = c->hm.shells[s];
-    d->ap.area[s] = h.area_fraction;
-    d->ap.rmin[s] = h.min_radius;
-    d->ap.rmax[s] = h.max_radius;
-    d->ap.shutter[s] = h.shutter;
-    mxd::RayConst &rc = d->rc[s];
-    rc.front = h.front_position;
-    rc.weighted = T.opt_n > 0;
-    rc.beta = 0.0; rc.delta = 1.0; rc.corr = 1.0;
-    if (rc.weighted) {
-      // the optical constants and correction at the ray energy, as the
-      // mirror stage interpolates them (float tables, float energy)
-      const float fe = (float) k.energy;
-      const float *optc = c->hm.optc.data();
-      const double *slope = c->hm.optc_slope.data();
-      const unsigned on = (unsigned) T.opt_n;
-      rc.beta = mx::interp_f(fe, optc, optc + on, slope, on);
-      rc.delta = mx::interp_f(fe, optc, optc + 2 * on, slope + (on - 1), on);
-      if (T.use_scale) {
-        const float *ce = optc + 3 * on + h.corr_off;
-        rc.corr = std::sqrt((double) mx::interp_f(fe, ce, ce + h.corr_n, slope + h.corr_slope_off, (unsigned) h.corr_n));
-      }
+  d->weighted = T.opt_n > 0;
+  if (d->weighted) {
+    // the optical constants and correction at the ray energy, as the
+    // mirror stage interpolates them (float tables, float energy)
+    const float fe = (float) k.energy;
+    const float *optc = c->hm.optc.data();
+    const double *slope = c->hm.optc_slope.data();
+    const unsigned on = (unsigned) T.opt_n;
+    d->beta = mx::interp_f(fe, optc, optc + on, slope, on);
+    d->delta = mx::interp_f(fe, optc, optc + 2 * on, slope + (on - 1), on);
+    for (int s = 0; s < 4 && T.use_scale; s++) {
+      const MxShellDev &h = c->hm.shells[s];
+      const float *ce = optc + 3 * on + h.corr_off;
+      d->corr[s] = std::sqrt((double) mx::interp_f(fe, ce, ce + h.corr_n, slope + h.corr_slope_off, (unsigned) h.corr_n));
     }
   }
-  d->ap.ideal = T.ideal;
-  d->ap.area_uniform = T.area_uniform;
   d->vig = T.ideal ? 1.0 : T.hrma_vig;
 
   cudaError_t e = cudaSetDevice(c->device);
   if (e == cudaSuccess) {
     d->rays_smem = align_up(sizeof(FwdArgs)) + DWARPS * sizeof(RayList);
     d->fwd_smem = d->rays_smem + 4 * (2 * WIN * WSTRIDE + DWARPS * 16 * STAGE_STRIDE);
-    d->adj_smem = align_up(sizeof(AdjArgs)) + 4 * WIN * (WIN + 1) + 4 * DWARPS * 32 * ADJ_STAGE + 4 * ADJ_TILE +
-                  4 * DWARPS;
+    d->adj_smem = align_up(sizeof(AdjArgs)) + 4 * WIN * (WIN + 1) + 4 * DWARPS * (32 * ADJ_STAGE + 1) + 2 * ADJ_TILE;
     e = occupancy(diff_forward_kernel<true, false>, d->fwd_smem, c->num_sms, &d->fwd_blocks);
   }
   if (e == cudaSuccess) e = occupancy(diff_forward_kernel<true, true>, d->fwd_smem, c->num_sms, &d->mom_blocks);

@@ -9,15 +9,14 @@
 // carries a weight: vignetting times, at each reflection, the Fresnel
 // reflectivity (reflect.c:39-77) times the effective-area correction.
 //
-// The trace is written once over a scalar type S.  S = double gives the
-// forward ray; S = Dual6 carries with each FP64 value its FP32 derivatives
-// with respect to the six parameters that can move this ray: its shell's
-// two tilts and two decenters and the source's two angular offsets.
+// The values are FP64; the derivatives with respect to the parameters that can
+// move a ray (its shell's two tilts and two decenters and the source's two
+// angular offsets) are FP32: Dual6 carries both through the geometry that the
+// host prepares, the adjoint kernel traces them ray by ray.
 #pragma once
 #include <stdint.h>
 
 #include <cmath>
-#include <type_traits>
 
 #include "mx_device.cuh"
 
@@ -31,196 +30,93 @@ namespace mxd {
 
 constexpr int ND = 6;   // tangent slots: tilt az, tilt el, decenter x, decenter y, source y, source z
 
+// A number with its derivatives, for the geometry that the host prepares.
 struct Dual6 {
   double v;
   float d[ND];
 };
 
-// A value rounded to single precision for the tangents, which are single
-// precision anyway: on the device by truncation on the integer pipe (a
-// conversion instruction would take an FP64-pipe slot).
-MXG float tof(double x) {
-#ifdef __CUDA_ARCH__
-  return mx::d2f_trunc(x);
-#else
-  return (float) x;
-#endif
-}
-
-MXG double val(double a) { return a; }
-MXG double val(const Dual6 &a) { return a.v; }
-
-MXG Dual6 mkd(double v) {
+inline Dual6 mkd(double v) {
   Dual6 r; r.v = v;
   for (int k = 0; k < ND; k++) r.d[k] = 0.f;
   return r;
 }
-MXG Dual6 operator+(const Dual6 &a, const Dual6 &b) {
+// f(a) with value v and slope s
+inline Dual6 chain(double v, float s, const Dual6 &a) {
+  Dual6 r; r.v = v;
+  for (int k = 0; k < ND; k++) r.d[k] = s * a.d[k];
+  return r;
+}
+inline Dual6 operator+(const Dual6 &a, const Dual6 &b) {
   Dual6 r; r.v = a.v + b.v;
   for (int k = 0; k < ND; k++) r.d[k] = a.d[k] + b.d[k];
   return r;
 }
-MXG Dual6 operator-(const Dual6 &a, const Dual6 &b) {
+inline Dual6 operator-(const Dual6 &a, const Dual6 &b) {
   Dual6 r; r.v = a.v - b.v;
   for (int k = 0; k < ND; k++) r.d[k] = a.d[k] - b.d[k];
   return r;
 }
-MXG Dual6 operator-(const Dual6 &a) {
-  Dual6 r; r.v = -a.v;
-  for (int k = 0; k < ND; k++) r.d[k] = -a.d[k];
-  return r;
-}
-MXG Dual6 operator*(const Dual6 &a, const Dual6 &b) {
+inline Dual6 operator*(const Dual6 &a, const Dual6 &b) {
   Dual6 r; r.v = a.v * b.v;
-  const float av = tof(a.v), bv = tof(b.v);
+  const float av = (float) a.v, bv = (float) b.v;
   for (int k = 0; k < ND; k++) r.d[k] = av * b.d[k] + bv * a.d[k];
   return r;
 }
-MXG Dual6 operator*(double s, const Dual6 &a) {
-  Dual6 r; r.v = s * a.v;
-  const float f = tof(s);
-  for (int k = 0; k < ND; k++) r.d[k] = f * a.d[k];
-  return r;
+inline Dual6 operator*(const Dual6 &a, double s) { return chain(s * a.v, (float) s, a); }
+inline Dual6 operator+(double s, const Dual6 &a) { return chain(s + a.v, 1.0f, a); }
+inline Dual6 operator-(double s, const Dual6 &a) { return chain(s - a.v, -1.0f, a); }
+inline Dual6 dsin(const Dual6 &a) { return chain(std::sin(a.v), cosf((float) a.v), a); }
+inline Dual6 dcos(const Dual6 &a) { return chain(std::cos(a.v), -sinf((float) a.v), a); }
+inline Dual6 dtan(const Dual6 &a) {
+  const float t = (float) std::tan(a.v);
+  return chain(std::tan(a.v), 1.0f + t * t, a);
 }
-MXG Dual6 operator*(const Dual6 &a, double s) { return s * a; }
-MXG Dual6 operator+(const Dual6 &a, double s) { Dual6 r = a; r.v = a.v + s; return r; }
-MXG Dual6 operator+(double s, const Dual6 &a) { Dual6 r = a; r.v = s + a.v; return r; }
-MXG Dual6 operator-(const Dual6 &a, double s) { Dual6 r = a; r.v = a.v - s; return r; }
-MXG Dual6 operator-(double s, const Dual6 &a) {
-  Dual6 r; r.v = s - a.v;
-  for (int k = 0; k < ND; k++) r.d[k] = -a.d[k];
-  return r;
-}
-MXG Dual6 operator/(const Dual6 &a, const Dual6 &b) {
-  Dual6 r; r.v = a.v / b.v;
-  const float ib = 1.0f / tof(b.v), q = tof(r.v);
-  for (int k = 0; k < ND; k++) r.d[k] = (a.d[k] - q * b.d[k]) * ib;
-  return r;
-}
-MXG Dual6 operator/(double s, const Dual6 &b) {
-  Dual6 r; r.v = s / b.v;
-  const float g = -tof(r.v) / tof(b.v);
-  for (int k = 0; k < ND; k++) r.d[k] = g * b.d[k];
-  return r;
-}
-MXG Dual6 operator/(const Dual6 &a, double s) {
-  Dual6 r; r.v = a.v / s;
-  const float f = 1.0f / tof(s);
-  for (int k = 0; k < ND; k++) r.d[k] = a.d[k] * f;
-  return r;
-}
-// 1 / a: for the double rays the Newton-Raphson reciprocal (within one ulp)
-MXG double drcp(double a) { return mx::rcp_fast(a); }
-MXG Dual6 drcp(const Dual6 &a) { return 1.0 / a; }
-// a < b and a == 0 on the values, on the integer pipe
-MXG bool vlt(double a, double b) { return mx::dkey(a) < mx::dkey(b); }
-MXG bool vzero(double a) { return mx::is_zero(a); }
-MXG double dsqrt(double a) { return sqrt(a); }
-MXG Dual6 dsqrt(const Dual6 &a) {
-  Dual6 r; r.v = sqrt(a.v);
-  const float h = 0.5f / tof(r.v);
-  for (int k = 0; k < ND; k++) r.d[k] = h * a.d[k];
-  return r;
-}
-// 1 / sqrt(a): one reciprocal square root instead of a square root and a
-// division (normalisations, the Fresnel root).
-MXG double drsqrt(double a) { return mx::mx_rsqrt(a); }
-MXG Dual6 drsqrt(const Dual6 &a) {
-  Dual6 r; r.v = mx::mx_rsqrt(a.v);
-  const float t = tof(r.v), h = -0.5f * t * t * t;
-  for (int k = 0; k < ND; k++) r.d[k] = h * a.d[k];
-  return r;
-}
-MXG double dcopysign(double a, double b) { return copysign(a, b); }
-MXG Dual6 dcopysign(const Dual6 &a, const Dual6 &b) { return (a.v < 0.0) != (b.v < 0.0) ? -a : a; }
-MXG double dabs(double a) { return fabs(a); }
-MXG Dual6 dabs(const Dual6 &a) { return a.v < 0.0 ? -a : a; }
-MXG double dsin(double a) { return sin(a); }
-MXG double dcos(double a) { return cos(a); }
-MXG Dual6 dsin(const Dual6 &a) {
-  Dual6 r; r.v = sin(a.v);
-  const float c = cosf(tof(a.v));
-  for (int k = 0; k < ND; k++) r.d[k] = c * a.d[k];
-  return r;
-}
-MXG Dual6 dcos(const Dual6 &a) {
-  Dual6 r; r.v = cos(a.v);
-  const float s = -sinf(tof(a.v));
-  for (int k = 0; k < ND; k++) r.d[k] = s * a.d[k];
-  return r;
-}
-MXG double dtan(double a) { return tan(a); }
-MXG Dual6 dtan(const Dual6 &a) {
-  Dual6 r; r.v = tan(a.v);
-  const float t = tof(r.v), s = 1.0f + t * t;
-  for (int k = 0; k < ND; k++) r.d[k] = s * a.d[k];
-  return r;
-}
-
-// A constant of type S (no derivatives).
-template <class S> MXG S cst(double v);
-template <> MXG double cst<double>(double v) { return v; }
-template <> MXG Dual6 cst<Dual6>(double v) { return mkd(v); }
-
-template <class S> struct V3 { S x, y, z; };
-template <class S> MXG V3<S> v3(S x, S y, S z) { V3<S> r; r.x = x; r.y = y; r.z = z; return r; }
-template <class S> MXG V3<S> operator+(const V3<S> &a, const V3<S> &b) { return v3<S>(a.x + b.x, a.y + b.y, a.z + b.z); }
-template <class S> MXG V3<S> operator-(const V3<S> &a, const V3<S> &b) { return v3<S>(a.x - b.x, a.y - b.y, a.z - b.z); }
-template <class S> MXG V3<S> scale(const S &s, const V3<S> &a) { return v3<S>(s * a.x, s * a.y, s * a.z); }
-template <class S> MXG S dotp(const V3<S> &a, const V3<S> &b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-template <class S> MXG V3<S> unit(const V3<S> &a) {
-  S inv = drsqrt(dotp(a, a));
-  return scale(inv, a);
-}
-template <class S> MXG V3<S> matv(const S *m, const V3<S> &v) {
-  return v3<S>(m[0] * v.x + m[1] * v.y + m[2] * v.z, m[3] * v.x + m[4] * v.y + m[5] * v.z,
-               m[6] * v.x + m[7] * v.y + m[8] * v.z);
+inline Dual6 drsqrt(const Dual6 &a) {
+  const float t = (float) mx::mx_rsqrt(a.v);
+  return chain(mx::mx_rsqrt(a.v), -0.5f * t * t * t, a);
 }
 
 // ------------------------------------------------ HRMA optic geometry --
-// One optic of one shell: conic x^2 + y^2 + z^2 = a x^2 + b x + c between
-// xmin and xmax in its own frame, the MARX -> optic translation `to` and the
+// One optic of one shell: the MARX -> optic translation `to` and the
 // pitch/yaw rotations fwd (into the optic's frame) and bwd (back).
-template <class S> struct Optic {
-  double a, b, c, xmin, xmax;
-  S to[3];
-  S fwd[9], bwd[9];
-  S ff[3];   // fwd (front + to[0], 0, 0): the aperture plane's part of fwd (x + to)
+struct Optic {
+  Dual6 to[3], fwd[9], bwd[9];
+  Dual6 ff[3];   // fwd (front + to[0], 0, 0): the aperture plane's part of fwd (x + to)
 };
 
 // A shell's way from the paraboloid's frame to the hyperboloid's: back to
 // the MARX frame (P.bwd, less P.to), then in (plus H.to, H.fwd) as one
 // matrix and offset, x' = m x + c, p' = m p, with m = H.fwd P.bwd and
-// c = H.fwd (H.to - P.to); and P.bwd, P.to in float for the cap struts'
-// screen in that frame.
-template <class S> struct Between {
-  S m[9], c[3];
-  float bwdf[9], tof[3];
+// c = H.fwd (H.to - P.to); and the source direction in the paraboloid's
+// frame, p1 = P.fwd p0.
+struct Between {
+  Dual6 m[9], c[3], p1[3];
 };
 
-// The rotation builders of init_yaw_pitch (hrma.c:842-880), over S.
-template <class S> MXG void rot_z(S m[9], const S &theta) {
-  S c = dcos(theta), s = 0.0 - dsin(theta);
-  m[0] = c; m[1] = s; m[2] = cst<S>(0.0);
+// The rotation builders of init_yaw_pitch (hrma.c:842-880).
+inline void rot_z(Dual6 m[9], const Dual6 &theta) {
+  Dual6 c = dcos(theta), s = 0.0 - dsin(theta);
+  m[0] = c; m[1] = s; m[2] = mkd(0.0);
   m[3] = 0.0 - s; m[4] = c; m[5] = m[2];
-  m[6] = m[2]; m[7] = m[2]; m[8] = cst<S>(1.0);
+  m[6] = m[2]; m[7] = m[2]; m[8] = mkd(1.0);
 }
-template <class S> MXG void rot_axis(S m[9], const S n[3], const S &theta) {
-  S c = dcos(theta), s = dsin(theta), c1 = 1.0 - c;
-  S n0 = n[0], n1 = n[1], n2 = n[2];
-  S n01 = n0 * n1 * c1, n02 = n0 * n2 * c1, n12 = n1 * n2 * c1;
+inline void rot_axis(Dual6 m[9], const Dual6 n[3], const Dual6 &theta) {
+  Dual6 c = dcos(theta), s = dsin(theta), c1 = 1.0 - c;
+  Dual6 n0 = n[0], n1 = n[1], n2 = n[2];
+  Dual6 n01 = n0 * n1 * c1, n02 = n0 * n2 * c1, n12 = n1 * n2 * c1;
   m[0] = n0 * n0 * c1 + c; m[1] = n01 - s * n2; m[2] = n02 + s * n1;
   m[3] = n01 + s * n2; m[4] = n1 * n1 * c1 + c; m[5] = n12 - s * n0;
   m[6] = n02 - s * n1; m[7] = n12 + s * n0; m[8] = n2 * n2 * c1 + c;
 }
-template <class S> MXG void mat3_mul(S c[9], const S a[9], const S b[9]) {
+inline void mat3_mul(Dual6 c[9], const Dual6 a[9], const Dual6 b[9]) {
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) c[3 * i + j] = a[3 * i] * b[j] + a[3 * i + 1] * b[3 + j] + a[3 * i + 2] * b[6 + j];
 }
 // fwd = R(ny, -el) Rz(-az) and bwd = Rz(az) R(ny, el), ny = Rz(-az) e_y, as
 // the reference builds them from the geometry file's az_mis and el_mis.
-template <class S> MXG void yaw_pitch(S fwd[9], S bwd[9], const S &az, const S &el) {
-  S rz[9], ry[9], ny[3];
+inline void yaw_pitch(Dual6 fwd[9], Dual6 bwd[9], const Dual6 &az, const Dual6 &el) {
+  Dual6 rz[9], ry[9], ny[3];
   rot_z(rz, 0.0 - az);
   ny[0] = rz[1]; ny[1] = rz[4]; ny[2] = rz[7];
   rot_axis(ry, ny, 0.0 - el);
@@ -230,99 +126,47 @@ template <class S> MXG void yaw_pitch(S fwd[9], S bwd[9], const S &az, const S &
   mat3_mul(bwd, rz, ry);
 }
 
-// Fresnel reflectivity averaged over polarisations (reflect.c:39-77) for a
-// grazing cosine cos_t and refractive index 1 - delta + i beta.
-template <class S> MXG S fresnel(const S &cos_t, double beta, double delta) {
-#ifdef __CUDA_ARCH__
-  if constexpr (std::is_same<S, double>::value) {
-    // the value alone: in double-float on the FP32 pipe (mx::reflectivity_df,
-    // beta and delta are floats), within about 2^-40 of the expression below
-    mx::F2 num, den;
-    mx::reflectivity_df(mx::split(cos_t), mx::d2f_trunc(beta), mx::d2f_trunc(delta), num, den);
-    return mx::df_to(mx::df_div(num, den));
-  }
-#endif
-  const double nr = 1.0 - delta, ni = beta;
-  const double sr = nr * nr - ni * ni, si = 2.0 * nr * ni;
-  S sin2 = 1.0 - cos_t * cos_t;
-  S wr = sr - sin2;
-  const double wi = si;
-  // the principal square root of wr + i wi: with q^2 = h = (r + |wr|) / 2,
-  // q = h / sqrt(h) and wi / (2 q) = (wi / 2) / sqrt(h), one reciprocal
-  // square root for both
-  S r = dsqrt(wr * wr + wi * wi);
-  S rr, ri;
-  if (val(wr) >= 0.0) {
-    S h = 0.5 * (r + wr), inv = drsqrt(h);
-    rr = h * inv; ri = (0.5 * wi) * inv;
-  } else {
-    S h = 0.5 * (r - wr), inv = drsqrt(h);
-    rr = (0.5 * wi) * inv; ri = h * inv;
-    if (val(rr) < 0.0) { rr = 0.0 - rr; ri = 0.0 - ri; }
-  }
-  S a1 = (cos_t - rr) * (cos_t - rr) + ri * ri, b1 = (cos_t + rr) * (cos_t + rr) + ri * ri;
-  S pr = cos_t * sr, pi_ = cos_t * si;
-  S a2 = (pr - rr) * (pr - rr) + (pi_ - ri) * (pi_ - ri);
-  S b2 = (pr + rr) * (pr + rr) + (pi_ + ri) * (pi_ + ri);
-  return 0.5 * (a1 * b2 + a2 * b1) / (b1 * b2);
-}
-
-// compute_conic_intersection (hrma.c:411-478) with the roots of
-// JDMquadratic_root (qroot.c:36-70).  root < 0: choose as the reference does
-// (a root inside [xmin, xmax), the larger x when both are) and report the
-// choice in *chosen (0 = the -2c/(b f) root, 1 = the -b f/(2a) root).
-// root 0 or 1: take that root without the x-limit test, so that the ray
-// stays on the same branch while the optic moves.  Returns false on a miss.
-template <class S>
-MXG bool conic_hit(const Optic<S> &o, V3<S> &x0, const V3<S> &p, V3<S> &n, int root, int *chosen) {
-  S t_plus = (0.0 - x0.x) * drcp(p.x);
-  S x_y = x0.y + t_plus * p.y, x_z = x0.z + t_plus * p.z;
-  S alpha = o.a * (p.x * p.x) - 1.0;
-  S beta = o.b * p.x - 2.0 * (p.y * x_y + p.z * x_z);
-  S gamma = o.c - x_z * x_z - x_y * x_y;
-  if (vzero(val(alpha))) return false;
-  S bsqr = beta * beta, ac4 = alpha * gamma * 4.0;
-  if (!vlt(val(ac4), val(bsqr))) return false;
-  // the roots -2 gamma / (beta f) and -beta f / (2 alpha) of the reference,
-  // f = 1 + sqrt(1 - 4 alpha gamma / beta^2), from b f = beta + sign(beta)
-  // sqrt(beta^2 - 4 alpha gamma) and one reciprocal of alpha b f
-  S bf = beta + dcopysign(dsqrt(bsqr - ac4), beta), inv = drcp(alpha * bf);
-  S tp = (-2.0 * gamma) * alpha * inv, tm = (-0.5 * bf) * bf * inv;
-  int pick = root;
-  if (root < 0) {
-    const double xp = val(p.x) * val(tp), xm = val(p.x) * val(tm);
-    const bool okp = !vlt(xp, o.xmin) && vlt(xp, o.xmax), okm = !vlt(xm, o.xmin) && vlt(xm, o.xmax);
-    if (okp) pick = (okm && vlt(xp, xm)) ? 1 : 0;
-    else if (okm) pick = 1;
-    else return false;
-    *chosen = pick;
-  }
-  S t = pick ? tm : tp;
-  x0 = v3<S>(p.x * t, x_y + p.y * t, x_z + p.z * t);
-  n = unit(v3<S>((o.a - 1.0) * x0.x + 0.5 * o.b, 0.0 - x0.y, 0.0 - x0.z));
-  return true;
-}
-
 // Per-ray decision byte: what the ray did the last time it was traced
 // afresh.  Replaying it keeps the traced function smooth in the parameters.
 enum : uint8_t { RAY_HIT = 1, RAY_ROOT_P = 2, RAY_ROOT_H = 4 };
 
 #ifdef __CUDACC__
-// conic_hit in double for the few rays conic_root leaves to it: the root
-// taken (0 or 1), -1 for a miss.
+// compute_conic_intersection (hrma.c:411-478) with the roots of
+// JDMquadratic_root (qroot.c:36-70), in double, for the few rays conic_root
+// leaves to it.  root < 0: choose as the reference does (a root inside
+// [xmin, xmax), the larger x when both are); 0 = the -2c/(b f) root, 1 = the
+// -b f/(2a) root: take that root without the x-limit test, so that the ray
+// stays on the same branch while the optic moves.  The root taken, -1 for a
+// miss.
 static __device__ __noinline__ int conic_root_double(const MxShellDev &h, int o, mx::D3 &x, const mx::D3 &p, mx::D3 &n,
                                                      int root) {
-  Optic<double> op;
-  op.a = h.a[o]; op.b = h.b[o]; op.c = h.c[o]; op.xmin = h.xmin[o]; op.xmax = h.xmax[o];
-  V3<double> r = v3<double>(x.x, x.y, x.z), m;
-  int chosen = root;
-  if (!conic_hit<double>(op, r, v3<double>(p.x, p.y, p.z), m, root, &chosen)) return -1;
-  x = mx::mk(r.x, r.y, r.z);
-  n = mx::mk(m.x, m.y, m.z);
-  return chosen;
+  const double t_plus = -x.x * mx::rcp_fast(p.x);
+  const double x_y = x.y + t_plus * p.y, x_z = x.z + t_plus * p.z;
+  const double alpha = h.a[o] * (p.x * p.x) - 1.0;
+  const double beta = h.b[o] * p.x - 2.0 * (p.y * x_y + p.z * x_z);
+  const double gamma = h.c[o] - x_z * x_z - x_y * x_y;
+  if (mx::is_zero(alpha)) return -1;
+  const double bsqr = beta * beta, ac4 = alpha * gamma * 4.0;
+  if (!(mx::dkey(ac4) < mx::dkey(bsqr))) return -1;
+  // the roots -2 gamma / (beta f) and -beta f / (2 alpha) of the reference,
+  // f = 1 + sqrt(1 - 4 alpha gamma / beta^2), from b f = beta + sign(beta)
+  // sqrt(beta^2 - 4 alpha gamma) and one reciprocal of alpha b f
+  const double bf = beta + copysign(sqrt(bsqr - ac4), beta), inv = mx::rcp_fast(alpha * bf);
+  const double tp = (-2.0 * gamma) * alpha * inv, tm = (-0.5 * bf) * bf * inv;
+  if (root < 0) {
+    const double xp = p.x * tp, xm = p.x * tm;
+    const bool okp = xp >= h.xmin[o] && xp < h.xmax[o], okm = xm >= h.xmin[o] && xm < h.xmax[o];
+    if (!okp && !okm) return -1;
+    root = okp && !(okm && xp < xm) ? 0 : 1;
+  }
+  const double t = root ? tm : tp;
+  x = mx::mk(p.x * t, x_y + p.y * t, x_z + p.z * t);
+  n = mx::mk((h.a[o] - 1.0) * x.x + 0.5 * h.b[o], -x.y, -x.z);
+  n = mx::mx_rsqrt(mx::dot(n, n)) * n;
+  return root;
 }
 
-// conic_hit for a ray as the trace meets it, by Newton steps from the one
+// The same for a ray as the trace meets it, by Newton steps from the one
 // crossing between the conic's ends (mx::conic_newton).  That crossing is
 // root 0, the intersection nearer to the plane x = 0, when the sum of both,
 // -beta / alpha, is more than twice as far from zero (in float, with room to
@@ -349,69 +193,174 @@ __device__ __forceinline__ mx::D3 reflected(const mx::D3 &p, const mx::D3 &n, do
   const double k = -2.0 * pdn;
   return mx::mk(fma(k, n.x, p.x), fma(k, n.y, p.y), fma(k, n.z, p.z));
 }
-#endif
+// ------------------------------------------- the adjoint's arithmetic --
+// A value of a recorded ray with its single-precision tangents in the four
+// directions that bend its path: the shell's tilts (0, 1) and the source's
+// offsets (2, 3); the decenters move both optics alike and shift the image
+// alone.  Turn: an entry of the geometry, which only the tilts move.
+constexpr int NT = 4;
+struct Dual { double v; float d[NT]; };
+struct Turn { double v; float d[2]; };
 
-// Everything a weighted ray needs besides the two optics of its shell.
-struct RayConst {
-  double front;        // front_position of the shell (aperture plane)
-  double beta, delta;  // optical constants at the ray energy
-  double corr;         // effective-area correction per reflection
-  bool weighted;       // false: unit weights (ideal mirrors)
-};
+// A value rounded to single precision for the tangents: by truncation on the
+// integer pipe (a conversion instruction would take an FP64-pipe slot).
+__device__ __forceinline__ float tof(double x) { return mx::d2f_trunc(x); }
+// The truncation of a double-float.
+__device__ __forceinline__ float tof(mx::F2 a) {
+  a = mx::quick_sum(a.h, a.l);
+  const uint32_t u = __float_as_uint(a.h);
+  return __uint_as_float(u - ((a.l != 0.0f && ((u ^ __float_as_uint(a.l)) >> 31)) ? 1u : 0u));
+}
 
-// One weighted ray from the aperture point (front, ry, rz) -- ry, rz as
-// r sin(phi), r cos(phi) -- along the source direction p0, through the
-// paraboloid P and hyperboloid H of its shell, to the focal plane.
-// replay: code holds the decisions to follow; otherwise they are made here
-// and written to code (0 when the ray is lost).  blocked(set, x, p) is the
-// strut test at the pre-collimator (0) and post-collimator (2), and
-// blocked.cap(P, B, x, p) at the cap for a ray given in the paraboloid's
-// frame.  B takes the ray from the paraboloid's frame to the hyperboloid's.
-template <class S, class Struts>
-MXG bool weighted_ray(const Optic<S> &P, const Optic<S> &H, const Between<S> &B, const RayConst &rc, double ry,
-                      double rz, const V3<S> &p0, bool replay, uint8_t &code, const Struts &blocked, S &y, S &z,
-                      S &w) {
-  int rootP = replay ? ((code & RAY_ROOT_P) ? 1 : 0) : -1;
-  int rootH = replay ? ((code & RAY_ROOT_H) ? 1 : 0) : -1;
-  if (replay && !(code & RAY_HIT)) return false;
-  if (!replay) code = 0;
-  V3<S> p = p0;
-  if (!replay && blocked(0, v3<S>(cst<S>(rc.front), ry - P.to[1], rz - P.to[2]), p)) return false;
-  // fwd (x + to) with x + to = (front + to[0], ry, rz): (ry - to[1]) + to[1]
-  // is ry to within an ulp of to[1]
-  V3<S> x = v3<S>(P.ff[0] + P.fwd[1] * ry + P.fwd[2] * rz, P.ff[1] + P.fwd[4] * ry + P.fwd[5] * rz,
-                  P.ff[2] + P.fwd[7] * ry + P.fwd[8] * rz);
-  p = matv(P.fwd, p);
-  V3<S> n;
-  int ch = 0;
-  if (!conic_hit(P, x, p, n, rootP, &ch)) return false;
-  if (!replay) rootP = ch;
-  S pdn = dotp(p, n);
-  S wt = rc.weighted ? fresnel(dabs(pdn), rc.beta, rc.delta) * rc.corr : cst<S>(1.0);
-  p = p - scale(2.0 * pdn, n);
-  if (!replay && blocked.cap(P, B, x, p)) return false;
-  p = matv(B.m, p);
-  x = matv(B.m, x) + v3<S>(B.c[0], B.c[1], B.c[2]);
-  if (!conic_hit(H, x, p, n, rootH, &ch)) return false;
-  if (!replay) rootH = ch;
-  pdn = dotp(p, n);
-  if (rc.weighted) wt = wt * (fresnel(dabs(pdn), rc.beta, rc.delta) * rc.corr);
-  p = p - scale(2.0 * pdn, n);
-  p = matv(H.bwd, p);
-  x = matv(H.bwd, x);
-  x = x - v3<S>(H.to[0], H.to[1], H.to[2]);
-  if (!replay && blocked(2, x, p)) return false;
-  S t = (0.0 - x.x) * drcp(p.x);
-  y = x.y + t * p.y;
-  z = x.z + t * p.z;
-  w = wt;
-  if (!replay) code = (uint8_t) (RAY_HIT | (rootP ? RAY_ROOT_P : 0) | (rootH ? RAY_ROOT_H : 0));
+__device__ __forceinline__ Dual operator+(const Dual &a, const Dual &b) {
+  Dual r; r.v = a.v + b.v;
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = a.d[k] + b.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual operator-(const Dual &a, const Dual &b) {
+  Dual r; r.v = a.v - b.v;
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = a.d[k] - b.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual operator-(const Dual &a) {
+  Dual r; r.v = -a.v;
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = -a.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual operator*(const Dual &a, const Dual &b) {
+  Dual r; r.v = a.v * b.v;
+  const float av = tof(a.v), bv = tof(b.v);
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = av * b.d[k] + bv * a.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual operator*(double s, const Dual &a) {
+  Dual r; r.v = s * a.v;
+  const float f = tof(s);
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = f * a.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual operator+(const Dual &a, double s) { Dual r = a; r.v = a.v + s; return r; }
+__device__ __forceinline__ Dual operator-(const Dual &a, double s) { Dual r = a; r.v = a.v - s; return r; }
+__device__ __forceinline__ Dual operator-(double s, const Dual &a) { Dual r = -a; r.v = s - a.v; return r; }
+__device__ __forceinline__ Dual operator*(const Turn &a, const Dual &b) {
+  Dual r; r.v = a.v * b.v;
+  const float av = tof(a.v), bv = tof(b.v);
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = k < 2 ? av * b.d[k] + bv * a.d[k & 1] : __fmul_rn(av, b.d[k]);   // as with a zero a.d
+  return r;
+}
+// a + b y + c z, the aperture point (0, y, z) in a turned frame
+__device__ __forceinline__ Dual turned(const Turn &a, const Turn &b, const Turn &c, double y, double z) {
+  Dual r; r.v = a.v + b.v * y + c.v * z;
+  const float yf = tof(y), zf = tof(z);
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = k < 2 ? a.d[k & 1] + yf * b.d[k & 1] + zf * c.d[k & 1] : 0.0f;
+  return r;
+}
+__device__ __forceinline__ Dual operator+(const Dual &a, const Turn &b) {
+  Dual r = a; r.v = a.v + b.v;
+  r.d[0] += b.d[0]; r.d[1] += b.d[1];
+  return r;
+}
+// 1 / a, sqrt(a) and 1 / sqrt(a): Newton steps from a float seed (within one
+// ulp); sizes outside 2^-39 .. 2^39, which no ray of a mirror meets, take the
+// library's.
+__device__ __forceinline__ bool usual(double a) { return (unsigned) (mx::dbits(a) >> 52) - (1023u - 39u) < 78u; }
+static __device__ __noinline__ double rsqrt_library(double a) { return rsqrt(a); }
+static __device__ __noinline__ double sqrt_library(double a) { return sqrt(a); }
+__device__ __forceinline__ Dual drcp(const Dual &a) {
+  Dual r; r.v = mx::rcp_fast(a.v);
+  const float g = -tof(r.v) / tof(a.v);
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = g * a.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual dsqrt(const Dual &a) {
+  Dual r; r.v = usual(a.v) ? a.v * mx::rsqrt_seeded(a.v) : sqrt_library(a.v);
+  const float h = 0.5f / tof(r.v);
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = h * a.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual drsqrt(const Dual &a) {
+  Dual r; r.v = usual(a.v) ? mx::rsqrt_seeded(a.v) : rsqrt_library(a.v);
+  const float t = tof(r.v), h = -0.5f * t * t * t;
+#pragma unroll
+  for (int k = 0; k < NT; k++) r.d[k] = h * a.d[k];
+  return r;
+}
+
+struct V3 { Dual x, y, z; };
+__device__ __forceinline__ Dual dotp(const V3 &a, const V3 &b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ V3 matv(const Turn *m, const V3 &v) {
+  return {m[0] * v.x + m[1] * v.y + m[2] * v.z, m[3] * v.x + m[4] * v.y + m[5] * v.z, m[6] * v.x + m[7] * v.y + m[8] * v.z};
+}
+
+// conic_root_double with tangents for a ray that follows a recorded root.
+// False when the ray misses the conic.
+__device__ __forceinline__ bool conic_tangents(const MxShellDev &h, int o, V3 &x0, const V3 &p, V3 &n, int root) {
+  const Dual t_plus = (0.0 - x0.x) * drcp(p.x);
+  const Dual x_y = x0.y + t_plus * p.y, x_z = x0.z + t_plus * p.z;
+  const Dual alpha = h.a[o] * (p.x * p.x) - 1.0;
+  const Dual beta = h.b[o] * p.x - 2.0 * (p.y * x_y + p.z * x_z);
+  const Dual gamma = h.c[o] - x_z * x_z - x_y * x_y;
+  if (mx::is_zero(alpha.v)) return false;
+  const Dual bsqr = beta * beta, ac4 = 4.0 * (alpha * gamma);
+  if (!(mx::dkey(ac4.v) < mx::dkey(bsqr.v))) return false;
+  const Dual sq = dsqrt(bsqr - ac4), bf = mx::neg_bit(beta.v) ? beta - sq : beta + sq, inv = drcp(alpha * bf);
+  Dual t;
+  if (root == 0) t = (-2.0 * gamma) * alpha * inv;
+  else t = (-0.5 * bf) * bf * inv;
+  x0 = {p.x * t, x_y + p.y * t, x_z + p.z * t};
+  n = {(h.a[o] - 1.0) * x0.x + 0.5 * h.b[o], -x0.y, -x0.z};
+  const Dual len = drsqrt(dotp(n, n));
+  n = {len * n.x, len * n.y, len * n.z};
   return true;
 }
 
-}  // namespace mxd
-
-namespace mxd {
+// The Fresnel reflectivity of mx::reflectivity_df for refractive index
+// n, sr + i si = n^2 and lost = 1 - sr, with its derivative by the grazing
+// cosine: one chain of single-precision tangents beside the double-float
+// values instead of one for every direction beside double values.
+struct Fresnel { mx::F2 sr, si, lost; };
+__device__ __forceinline__ void fresnel_slope(const Fresnel &f, mx::F2 c, mx::F2 &value, float &slope) {
+  using mx::F2;
+  const float cf = tof(c);
+  const F2 wr = mx::df_sub(mx::df_prod(c, c), f.lost), wi = f.si;
+  const float wrd = 2.0f * cf;
+  const F2 r = mx::df_sqrt(mx::df_sum(mx::df_prod(wr, wr), mx::df_prod(wi, wi)));
+  const float rd = 0.5f / tof(r) * (2.0f * tof(wr) * wrd);
+  const bool right = wr.h >= 0.0f;
+  const F2 h2 = mx::df_sum(r, right ? wr : mx::df_neg(wr));
+  const F2 h = mx::quick_sum(0.5f * h2.h, 0.5f * h2.l), inv = mx::df_rsqrt(h), hw = {0.5f * wi.h, 0.5f * wi.l};
+  const float hd = 0.5f * (right ? rd + wrd : rd - wrd), invf = tof(inv), invd = -0.5f * invf * invf * invf * hd;
+  const F2 big = mx::df_prod(h, inv), small = mx::df_prod(hw, inv);
+  const float bigd = tof(h) * invd + invf * hd, smalld = tof(hw) * invd;
+  F2 rr = right ? big : small, ri = right ? small : big;
+  float rrd = right ? bigd : smalld, rid = right ? smalld : bigd;
+  if (!right && rr.h < 0.0f) { rr = mx::df_neg(rr); ri = mx::df_neg(ri); rrd = -rrd; rid = -rid; }
+  const F2 ri2 = mx::df_prod(ri, ri), cm = mx::df_sub(c, rr), cp = mx::df_sum(c, rr);
+  const float ri2d = 2.0f * tof(ri) * rid;
+  const F2 a1 = mx::df_sum(mx::df_prod(cm, cm), ri2), b1 = mx::df_sum(mx::df_prod(cp, cp), ri2);
+  const float a1d = 2.0f * tof(cm) * (1.0f - rrd) + ri2d, b1d = 2.0f * tof(cp) * (1.0f + rrd) + ri2d;
+  const F2 pr = mx::df_prod(c, f.sr), pi = mx::df_prod(c, f.si);
+  const float srf = tof(f.sr), sif = tof(f.si);
+  const F2 pm = mx::df_sub(pr, rr), pp = mx::df_sum(pr, rr), im = mx::df_sub(pi, ri), ip = mx::df_sum(pi, ri);
+  const F2 a2 = mx::df_sum(mx::df_prod(pm, pm), mx::df_prod(im, im)), b2 = mx::df_sum(mx::df_prod(pp, pp), mx::df_prod(ip, ip));
+  const float a2d = 2.0f * tof(pm) * (srf - rrd) + 2.0f * tof(im) * (sif - rid);
+  const float b2d = 2.0f * tof(pp) * (srf + rrd) + 2.0f * tof(ip) * (sif + rid);
+  const F2 t = mx::df_sum(mx::df_prod(a1, b2), mx::df_prod(a2, b1)), den = mx::df_mul(b1, b2);
+  const float numd = 0.5f * ((tof(a1) * b2d + tof(b2) * a1d) + (tof(a2) * b1d + tof(b1) * a2d));
+  const float dend = tof(b1) * b2d + tof(b2) * b1d;
+  value = mx::df_div(mx::quick_sum(0.5f * t.h, 0.5f * t.l), den);
+  slope = (numd - tof(value) * dend) * (1.0f / tof(den));
+}
+#endif
 
 // exp(-x) for x >= 0 in single precision with every operation explicitly
 // rounded (Cody-Waite reduction x = n ln2 + r with ln2 in two parts, then

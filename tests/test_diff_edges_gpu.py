@@ -85,3 +85,41 @@ def test_mse(engine, nx, ny):
     assert float(loss) == pytest.approx(float((r * r).mean()), rel=1e-13)
     np.testing.assert_allclose(dl.cpu().numpy().reshape(ny, nx), 2.0 * r / (nx * ny), rtol=4e-16, atol=0)
     d.close()
+
+
+@pytest.mark.parametrize("ideal", [False, True])
+@pytest.mark.parametrize("n,scale", [(1, 0.5), (33, 0.5), (130, 30.0), (20_011, 0.5), (20_011, 30.0)])
+def test_adjoint_matches_central_differences(cuda, n, scale, ideal):
+    """The adjoint of a linear function of the image, sum dl image, whose
+    gradient keeps one sign over rays and taps (dl rises along both axes).
+    Tolerance: the derivatives are sums of single-precision terms (1e-5 of
+    their size at worst); the taps' rounding (2^-24) over the 4e-3 pixels of
+    a step of 2e-3 arcsec gives the differences 3e-5, and the third order
+    they leave out 1e-5: 1e-3 of the gradient's norm leaves room for the
+    tilts' smaller steps."""
+    import torch
+    from marx_gb300._native import Engine
+    theta = _theta(scale)
+    eng = Engine(diff_mirror_config(ideal=ideal))
+    centred = DiffImage.centred(eng, diff_workload(n_rays=20_011).cfg, theta)   # one ray alone may miss
+    cfg = centred.cfg.copy()
+    cfg.n_rays = n
+    cfg.nx, cfg.ny = 40, 80
+    cfg.center_z += 25 * cfg.pitch   # rays across the window's edge
+    d = DiffImage(eng, cfg)
+    row, col = np.mgrid[0:cfg.ny, 0:cfg.nx]
+    dl = torch.from_numpy(0.3 + 0.01 * col + 0.007 * row + 2e-4 * col * row).cuda()
+    d.forward(theta, RECORD)
+    g = d.adjoint(theta, dl)
+    h, fd = 2e-3, np.empty(NPARAM)
+    for k in range(NPARAM):
+        v = []
+        for sign in (1.0, -1.0):
+            t = theta.copy()
+            t[k] += sign * h
+            v.append(float((d.forward(t, REPLAY) * dl).sum()))
+        fd[k] = (v[0] - v[1]) / (2 * h)
+    assert np.linalg.norm(g - fd) <= 1e-3 * np.linalg.norm(fd), (g, fd)
+    assert np.array_equal(g, d.adjoint(theta, dl))
+    d.close()
+    centred.close()
