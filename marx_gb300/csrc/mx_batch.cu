@@ -532,7 +532,7 @@ static int build_graph(mx_batch *b) {
     e = cudaLaunchKernelEx(&lc, mx_batch_kernel, T, io);
   }
   // with an FEF: the pulse heights and streaks of the photons on a chip
-  if (e == cudaSuccess && (T.acis_fef || T.acis_qe)) e = launch_acis_fef(T, io.io, c->num_sms * 8, st, io.seed);
+  if (e == cudaSuccess && (T.acis_fef || T.acis_qe)) e = launch_acis_fef(T, io.io, c->num_sms * MX_FEF_BLOCKS, st, io.seed);
   cudaGraph_t g = nullptr;
   cudaError_t e2 = cudaStreamEndCapture(st, &g);
   cudaStreamDestroy(st);

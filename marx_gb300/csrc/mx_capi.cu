@@ -413,7 +413,7 @@ int mx_trace_queues(mx_context *c, const MxTables &T, const mx_photons *ph, uint
     c->launches++;
   }
   if (e == cudaSuccess && (stages & MX_STAGE_DETECT) && (T.acis_fef || T.acis_qe)) {
-    e = launch_acis_fef(T, io, c->num_sms * 8, st);
+    e = launch_acis_fef(T, io, c->num_sms * MX_FEF_BLOCKS, st);
     c->launches++;
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "launching the trace kernels");

@@ -2224,8 +2224,18 @@ MXD bool acis_qe_accept(const MxTables &T, int ccd, const Ph &ph, Rng &rng) {
 constexpr int MX_FEF_MAX_GAUSS = MX_FEF_GAUSSIANS;
 
 // gaussian_integral (acis_fef.c:380-392) over [0, inf) and (-inf, 0]: the
-// erf of the upper (lower) infinite bound is 1 (-1).
+// erf of the upper (lower) infinite bound is 1 (-1).  erf is exactly -1 in
+// double from -6 on, so that a gaussian whose centre lies further than that
+// above zero, as nearly all do, has all its area there: two multiplications
+// instead of an error function and a division.
 MXD void fef_areas(float amp, float center, float sigma, double &above, double &below) {
+#ifdef __CUDA_ARCH__
+  if (sigma > 0.0f && center > 8.5f * sigma) {   // 6 sqrt(2) = 8.486
+    above = f2d(amp) * (2.5066282746310002 * f2d(sigma));
+    below = flip_sign(0.0, amp < 0.0f);
+    return;
+  }
+#endif
   const double s = (double) sigma * 1.4142135623730951;
   if (s == 0.0) { above = below = 0.0; return; }
   const double e0 = erf((0 - (double) center) / s), w = 2.5066282746310002 * (double) sigma;
@@ -2258,7 +2268,7 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
   unsigned k = bsearch_f((float) energy, E, n);
   if (k == 0) k++;
   if (k == n) k--;
-  const double t = (energy - (double) E[k - 1]) / (double) (E[k] - E[k - 1]);
+  const double t = (energy - f2d(E[k - 1])) / f2d(E[k] - E[k - 1]);
   const float *g0 = G + 3 * (size_t) (k - 1) * ng, *g1 = g0 + 3 * ng;
   float amp[MX_FEF_MAX_GAUSS], cen[MX_FEF_MAX_GAUSS], sig[MX_FEF_MAX_GAUSS], cum[MX_FEF_MAX_GAUSS];
   bool tail[MX_FEF_MAX_GAUSS];
@@ -2270,25 +2280,31 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
     if (g >= ng) continue;
     const float a0 = g0[3 * g], c0 = g0[3 * g + 1], s0 = g0[3 * g + 2];
     const float a1 = g1[3 * g], c1 = g1[3 * g + 1], s1 = g1[3 * g + 2];
-    cen[g] = (float) ((double) c0 + t * (double) (c1 - c0));
-    double v = (double) s0 + t * (double) (s1 - s0);
-    if (v > 0.0) {
-      sig[g] = (float) v;
-      v = (double) a0 + t * (double) (a1 - a0);
-      if ((v < 0.0) && ((a1 > 0.0f) || (a0 > 0.0f))) v = 0.0;
-      amp[g] = (float) v;
+    cen[g] = d2f_rn(f2d(c0) + t * f2d(c1 - c0));
+    double v = f2d(s0) + t * f2d(s1 - s0);
+    if (dkey(v) > 0) {
+      sig[g] = d2f_rn(v);
+      v = f2d(a0) + t * f2d(a1 - a0);
+      if (dkey(v) < 0 && ((a1 > 0.0f) || (a0 > 0.0f))) v = 0.0;
+      amp[g] = d2f_rn(v);
     }
     double above, below;
     fef_areas(amp[g], cen[g], sig[g], above, below);
     if (below > above) tail[g] = above / below < 0.1;
     if (above >= 0) pos += above;
     else neg -= above;
-    cum[g] = (float) pos;
+    cum[g] = d2f_rn(pos);
   }
   if (pos <= neg) return false;               // HAS_TOTAL_NEG_AREA
   if (pos > 0) {
+    const double rpos = 1.0 / pos;
 #pragma unroll
-    for (int g = 0; g < MX_FEF_MAX_GAUSS; g++) cum[g] = (float) ((double) cum[g] / pos);
+    for (int g = 0; g < MX_FEF_MAX_GAUSS; g++) {
+      if (g >= ng) continue;
+      // the correctly rounded quotient, as the division's, for areas of usual size
+      const double c = f2d(cum[g]);
+      cum[g] = d2f_rn(cum[g] > 1e-30f && cum[g] < 1e30f ? div_by(c, pos, rpos) : c / pos);
+    }
   }
   double pha = -1.0;
   for (int tries = 0; tries < 100; tries++) {   // compute_pha_with_neg_amps (one pass when no amplitude is negative)
@@ -2300,14 +2316,14 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
       bool drawn = false;
 #pragma unroll
       for (int g = 0; g < MX_FEF_MAX_GAUSS; g++) {
-        if (drawn || g >= ng || (double) cum[g] <= r) continue;
+        if (drawn || g >= ng || dkey(f2d(cum[g])) <= dkey(r)) continue;
         drawn = true;
         if (!tail[g]) {
           int count = 0;
           do {
-            pha = (double) cen[g] + (double) sig[g] * rng.normal();
+            pha = f2d(cen[g]) + f2d(sig[g]) * rng.normal();
             count++;
-          } while ((pha < 0) && (count < 100) && !rng.overrun);
+          } while (dkey(pha) < 0 && (count < 100) && !rng.overrun);
         } else {
           const double s = (double) ((0.0f - cen[g]) / sig[g]);
           double u, xx;
@@ -2321,7 +2337,7 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
         }
       }
       if (rng.overrun) return false;
-      if (drawn && !(pha < 0)) break;           // else: a new choice of gaussian
+      if (drawn && dkey(pha) >= 0) break;       // else: a new choice of gaussian
     }
     if (neg == 0.0) break;
     double psum = 0.0, sum = 0.0;
@@ -2338,10 +2354,10 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
     if (u * psum < sum) break;
     if (tries == 99) return false;
   }
-  const int16_t ipha = (int16_t) pha;
-  const double ph2 = (double) ipha - rng.uniform();
+  const int16_t ipha = dkey(pha) < dkey(32768.0) ? (int16_t) trunc_to_unsigned(pha) : (int16_t) pha;
+  const double ph2 = (ipha >= 0 ? u2d((unsigned) ipha) : (double) ipha) - rng.uniform();
   if (rng.overrun) return false;
-  const float pi = interp_f((float) ph2, CH, E, T.fef_slope + f.s_off, n);
+  const float pi = interp_f(d2f_rn(ph2), CH, E, T.fef_slope + f.s_off, n);
   if (pi < 0) return false;
   pha_out = ipha;
   pi_out = pi;

@@ -12,6 +12,7 @@
 #define MX_TRACE_BLOCK 64
 // Threads per block of the wavefront kernels, and the resident blocks per SM
 // each is compiled for.
+#define MX_FEF_BLOCKS 3   // resident blocks per SM of the ACIS response pass
 #define MX_WAVE_BLOCK 256
 #define MX_WAVE_A_BLOCKS 3
 #define MX_WAVE_T_BLOCKS 3

@@ -76,7 +76,7 @@ extern "C" int mx_trace_static(mx_context *c, const mx_photons *ph, uint32_t sta
   e = launch_wavefront(c->T, io, w, c->num_sms, c->wave_blocks, (int) c->shared_bytes, (cudaStream_t) stream);
   c->launches += wave_kernels(c->T, stages);
   if (e == cudaSuccess && (stages & MX_STAGE_DETECT) && (c->T.acis_fef || c->T.acis_qe)) {
-    e = launch_acis_fef(c->T, io, c->num_sms * 8, (cudaStream_t) stream);
+    e = launch_acis_fef(c->T, io, c->num_sms * MX_FEF_BLOCKS, (cudaStream_t) stream);
     c->launches++;
   }
   return e == cudaSuccess ? MX_OK : mx_cuda_fail(c, e, "mx_trace_static: launching the trace kernels");
