@@ -47,6 +47,8 @@ static int upload_model(mx_context *c) {
   size_t o_ht = put(blob, M.hrc_tab), o_hs = put(blob, M.hrc_slope);
   size_t o_fm = put(blob, M.fef_map), o_fr = put(blob, M.fef), o_ff = put(blob, M.fef_f), o_fs = put(blob, M.fef_slope);
   size_t o_co = put(blob, M.contam);
+  if (M.find_first.empty()) M.find_first.push_back(0);
+  size_t o_fn = put(blob, M.find_first);
   cudaError_t e = c->tables.ensure(blob.size());
   if (e != cudaSuccess) return cuda_fail(c, e, "allocating device tables");
   e = cudaMemcpy(c->tables.ptr, blob.data(), blob.size(), cudaMemcpyHostToDevice);
@@ -78,6 +80,7 @@ static int upload_model(mx_context *c) {
   c->T.fef_f = (const float *) (b + o_ff);
   c->T.fef_slope = (const double *) (b + o_fs);
   c->T.contam = (const MxContamDev *) (b + o_co);
+  c->T.find_first = (const uint16_t *) (b + o_fn);
   c->T.asp_t = (const double *) c->asp.ptr;
   c->T.asp_v = c->asp.ptr ? (const double *) c->asp.ptr + ((c->asp_n + 1 + 7) & ~7u) : nullptr;
   c->T.asp_n = c->asp_n;
@@ -680,7 +683,7 @@ int mx_probe_fp64(double *tflops, double *ms) {
 }
 
 int mx_math_check(int fn, const double *x, double *y, size_t n) {
-  if (fn < 0 || fn > 10 || (n && (!x || !y))) return MX_EINVAL;
+  if (fn < 0 || fn > 11 || (n && (!x || !y))) return MX_EINVAL;
   if (n > ((size_t) 1 << 32)) return MX_ERANGE;
   return math_check(fn, x, y, n) == cudaSuccess ? MX_OK : MX_ECUDA;
 }

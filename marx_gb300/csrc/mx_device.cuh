@@ -709,15 +709,36 @@ MXD unsigned bsearch_d(double x, const double *xp, unsigned n) {  // JDMbinary_s
   }
   return (x >= MX_LDG(xp + n0)) ? n1 : n0;
 }
+// The first of a table's abscissae that is not below x, from its index table;
+// 0 where that does not apply (x not inside the table, no index table).
+// Three dependent loads or so where the bisection takes 8 (an effective-area
+// correction) to 16 (a detector's efficiency).
+MXD unsigned find_first(const MxFindDev &f, const uint16_t *first, float x, const float *xp) {
+#ifdef __CUDA_ARCH__
+  if (f.shift && x > f.lo && x < f.hi) {
+    unsigned k = MX_LDG(first + f.off + ((__float_as_uint(x) >> f.shift) - (__float_as_uint(f.lo) >> f.shift)));
+    while (MX_LDG(xp + k) < x) k++;   // hi is not below x
+    return k;
+  }
+#else
+  (void) f; (void) first; (void) x; (void) xp;
+#endif
+  return 0;
+}
+// bsearch_f by the index table: the same index for every x, an abscissa that
+// x equals among several equal ones being the bisection's to choose.
+MXD unsigned locate_f(const MxFindDev &f, const uint16_t *first, float x, const float *xp, unsigned n) {
+  const unsigned k = find_first(f, first, x, xp);
+  return k && !(f.repeats && xp[k] == x) ? k : bsearch_f(x, xp, n);
+}
 // JDMinterpolate_f (finterpo.c:59-86).  The result is rounded to float, so
 // the double expression is evaluated without contraction exactly as the
 // reference writes it.
 // The interval slopes (float dy over double dx, as the reference divides)
 // are precomputed on the host, so the kernel only multiplies; the slope of
 // the interval between n0 and n1 is slope[min(n0, n1)] in either order.
-MXD float interp_f(float x, const float *xp, const float *yp, const double *slope, unsigned n) {
-  if (n == 1) return yp[0];
-  unsigned n1 = bsearch_f(x, xp, n), n0 = n1 - 1;
+MXD float interp_at(unsigned n1, float x, const float *xp, const float *yp, const double *slope, unsigned n) {
+  unsigned n0 = n1 - 1;
   if (n1 < n && x == xp[n1]) return yp[n1];
   if (n1 == n) { n1--; n0--; }
   if (n1 == 0) n0 = 1;
@@ -726,12 +747,21 @@ MXD float interp_f(float x, const float *xp, const float *yp, const double *slop
   double q = slope[n0 < n1 ? n0 : n1];
   return d2f_rn(MX_DADD(f2d(yp[n0]), MX_DMUL(q, MX_DADD(f2d(x), -f2d(xf0)))));
 }
+MXD float interp_f(float x, const float *xp, const float *yp, const double *slope, unsigned n) {
+  if (n == 1) return yp[0];
+  return interp_at(bsearch_f(x, xp, n), x, xp, yp, slope, n);
+}
+MXD float interp_f(const MxFindDev &f, const uint16_t *first, float x, const float *xp, const float *yp,
+                   const double *slope, unsigned n) {
+  if (n == 1) return yp[0];
+  return interp_at(locate_f(f, first, x, xp, n), x, xp, yp, slope, n);
+}
 // Two tables over the same abscissae (the optical constants beta and
-// delta): interp_f of each with one binary search.
-MXD void interp2_f(float x, const float *xp, const float *ya, const float *yb, const double *sa, const double *sb,
+// delta): interp_f of each with one search.
+MXD void interp2_f(const MxFindDev &f, const uint16_t *first, float x, const float *xp, const float *ya, const float *yb, const double *sa, const double *sb,
                    unsigned n, float &a, float &b) {
   if (n == 1) { a = ya[0]; b = yb[0]; return; }
-  unsigned n1 = bsearch_f(x, xp, n), n0 = n1 - 1;
+  unsigned n1 = locate_f(f, first, x, xp, n), n0 = n1 - 1;
   if (n1 < n && x == xp[n1]) { a = ya[n1]; b = yb[n1]; return; }
   if (n1 == n) { n1--; n0--; }
   if (n1 == 0) n0 = 1;
@@ -1503,10 +1533,10 @@ MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *
   m.beta = 0.0f; m.delta = 1.0f; m.corr = F2{1.0f, 0.0f};
   if (T.opt_n) {
     float fe = d2f_rn(ph.e);
-    interp2_f(fe, optc, optc + T.opt_n, optc + 2 * T.opt_n, slope, slope + (T.opt_n - 1), T.opt_n, m.beta, m.delta);
+    interp2_f(T.opt_find, T.find_first, fe, optc, optc + T.opt_n, optc + 2 * T.opt_n, slope, slope + (T.opt_n - 1), T.opt_n, m.beta, m.delta);
     if (T.use_scale) {
       const float *ce = optc + 3 * T.opt_n + h.corr_off;
-      m.corr = sqrt_of_float(interp_f(fe, ce, ce + h.corr_n, slope + h.corr_slope_off, h.corr_n));
+      m.corr = sqrt_of_float(interp_f(h.corr_find, T.find_first, fe, ce, ce + h.corr_n, slope + h.corr_slope_off, h.corr_n));
     }
   }
   if (-1 == conic_intersection(h, 0, m.x, m.p, m.n) ||
@@ -1947,13 +1977,17 @@ MXD_COLD int choose_order_double(const float *ge, unsigned idx, const float *cum
 // more than 1e-6 from every probe falls on the same side of each in double.
 // Other draws (one in 10^5 or so) take the double form, 10 FP64 operations
 // and 6 for each of 3 to 7 probes.
-MXD int choose_order(const float *ge, unsigned n, const float *cum, int norders, bool monotone, float fe, double r) {
+// idx is order_bin's.
+MXD unsigned order_bin(const MxFindDev &f, const uint16_t *first, const float *ge, unsigned n, float fe) {
+  if (const unsigned k = find_first(f, first, fe, ge)) return k;
   unsigned lo = 1, hi = n - 1;
   while (lo < hi) {
     unsigned mid = (lo + hi) >> 1;
     if (fe > MX_LDG(ge + mid)) lo = mid + 1; else hi = mid;   // floats compare as their doubles do
   }
-  const unsigned idx = lo;
+  return lo;
+}
+MXD int choose_order(const float *ge, unsigned idx, const float *cum, int norders, bool monotone, float fe, double r) {
 #ifdef __CUDA_ARCH__
   const float x0 = MX_LDG(ge + idx - 1), x1 = MX_LDG(ge + idx);
   if (monotone && fe >= x0 && fe <= x1 && x1 > x0) {
@@ -2012,8 +2046,9 @@ MXD int grating_front(const MxTables &T, const MxGratingDev *grs, int kind, Ph &
   x = rot_x(ph.x, g.cos_m, g.sin_m);
   p = rot_x(ph.p, g.cos_m, g.sin_m);
   if (-1 == rowland_intersect(x, p, g.rowland)) ph.flags |= MX_PHOTON_UNDIFFRACTED;
-  const int chosen = choose_order(T.geff_energy + g.geff_off, (unsigned) g.nenergy, T.geff_cum + g.cum_off, g.norders,
-                                  g.monotone != 0, d2f_rn(ph.e), rng.uniform());
+  const float fe = d2f_rn(ph.e), *ge = T.geff_energy + g.geff_off;
+  const int chosen = choose_order(ge, order_bin(g.find, T.find_first, ge, (unsigned) g.nenergy, fe), T.geff_cum + g.cum_off,
+                                  g.norders, g.monotone != 0, fe, rng.uniform());
   if (chosen < 0) {
     // no order: the LETG's supports are skipped (the photon is flagged)
     ph.flags |= MX_PHOTON_UNDIFFRACTED;
@@ -2041,11 +2076,12 @@ MXD void grating_back(const MxTables &T, const MxGratingDev *grs, int kind, Ph &
   else {
     if (letg) {
       const float fe = d2f_rn(ph.e);
+      const unsigned bin = order_bin(T.support_find, T.find_first, T.support_energy, (unsigned) T.support_nenergy, fe);
       for (int s = 0; s < 4; s++) {
         const MxSupportDev &sg = T.supports[s];
         if (!sg.norders) continue;
         if (ph.flags & MX_BAD_PHOTON_MASK) continue;
-        int k = choose_order(T.support_energy, (unsigned) T.support_nenergy, T.support_cum + sg.cum_off, sg.norders,
+        int k = choose_order(T.support_energy, bin, T.support_cum + sg.cum_off, sg.norders,
                              sg.monotone != 0, fe, rng.uniform());
         if (k < 0) { ph.flags |= MX_PHOTON_UNDIFFRACTED; continue; }
         // order list 0, +1, -1, +2, -2, ... (init_one_grating, diffract.c:392-405)
@@ -2190,7 +2226,7 @@ MXD double acis_contam(const MxTables &T, const MxContamDev &c, double en, doubl
     }
     for (int i = 0; i < c.nl; i++) {
       const MxTabDev &t = c.mu[i];
-      const double mu = f2d(interp_f(fe, T.fef_f + t.x_off, T.fef_f + t.y_off, T.fef_slope + t.s_off, (unsigned) t.n));
+      const double mu = f2d(interp_f(t.find, T.find_first, fe, T.fef_f + t.x_off, T.fef_f + t.y_off, T.fef_slope + t.s_off, (unsigned) t.n));
       v += mu * (c.tau0[i] + c.tau1[i] * fxy);
     }
   } else {
@@ -2200,7 +2236,7 @@ MXD double acis_contam(const MxTables &T, const MxContamDev &c, double en, doubl
     const unsigned ofs = (1024u / (unsigned) c.blk) * (unsigned) cy + (unsigned) cx;
     for (int i = 0; i < c.nl; i++) {
       const MxTabDev &t = c.mu[i];
-      const double mu = f2d(interp_f(fe, T.fef_f + t.x_off, T.fef_f + t.y_off, T.fef_slope + t.s_off, (unsigned) t.n));
+      const double mu = f2d(interp_f(t.find, T.find_first, fe, T.fef_f + t.x_off, T.fef_f + t.y_off, T.fef_slope + t.s_off, (unsigned) t.n));
       fxy = f2d(T.fef_f[c.fxy_off[i] + ofs]);
       v += mu * (c.tau0[i] + c.tau1[i] * fxy);
     }
@@ -2214,7 +2250,7 @@ MXD double acis_contam(const MxTables &T, const MxContamDev &c, double en, doubl
 MXD bool acis_qe_accept(const MxTables &T, int ccd, const Ph &ph, Rng &rng) {
   const double r = rng.uniform();
   const MxContamDev &c = T.contam[ccd];
-  const double qe = f2d(interp_f((float) ph.e, T.fef_f + c.qe.x_off, T.fef_f + c.qe.y_off, T.fef_slope + c.qe.s_off,
+  const double qe = f2d(interp_f(c.qe.find, T.find_first, (float) ph.e, T.fef_f + c.qe.x_off, T.fef_f + c.qe.y_off, T.fef_slope + c.qe.s_off,
                                  (unsigned) c.qe.n));
   const double qe_filter = 1.0;
   const double qe_contam = acis_contam(T, c, ph.e, (double) ph.ypix, (double) ph.zpix);
@@ -2411,7 +2447,7 @@ MXD void detect_stage(const MxTables &T, const MxChipDev *chips, int nchips, Ph 
 
 // ---------------------------------------------------------------- HRC --
 MXD float hrc_interp(const MxTables &T, const MxTabDev &t, float x) {   // JDMinterpolate_f
-  return interp_f(x, T.hrc_tab + t.x_off, T.hrc_tab + t.y_off, T.hrc_slope + t.s_off, (unsigned) t.n);
+  return interp_f(t.find, T.find_first, x, T.hrc_tab + t.x_off, T.hrc_tab + t.y_off, T.hrc_slope + t.s_off, (unsigned) t.n);
 }
 
 // _marx_hrc_compute_pha (hrc-i.c:71-91): delta E / E = 1 (FWHM).

@@ -39,7 +39,11 @@ struct HostModel {
   std::vector<float> fef_f;
   std::vector<double> fef_slope;
   std::vector<MxContamDev> contam;
+  std::vector<uint16_t> find_first;
 };
+
+// The index table of n abscissae (MxFindDev), appended to first.
+MxFindDev find_table(std::vector<uint16_t> &first, const float *x, size_t n);
 
 bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string &err);
 

@@ -2,8 +2,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "mx_device.cuh"
+#include "mx_host.h"
 #include "mx_kernels.cuh"
 #include "mx_wave.cuh"
 
@@ -662,8 +664,42 @@ __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, d
   }
 }
 
+// fn 11: how many of xp[i], the floats next to it and the points a quarter and
+// a half on the way to xp[i + 1] the index table places otherwise than the
+// bisection does.
+__global__ void mx_find_check(MxFindDev f, const uint16_t *first, const float *xp, unsigned n, double *y) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float a = xp[i], b = i + 1 < n ? xp[i + 1] : 2.0f * a;
+  const float v[6] = {a, nextafterf(a, 3e38f), nextafterf(a, -3e38f), a + 0.25f * (b - a), a + 0.5f * (b - a), -a};
+  int bad = 0;
+  for (int k = 0; k < 6; k++) bad += mx::locate_f(f, first, v[k], xp, n) != mx::bsearch_f(v[k], xp, n);
+  y[i] = (double) bad;
+}
+static cudaError_t find_check(const double *x, double *y, size_t n) {
+  std::vector<double> v(n);
+  cudaError_t e = cudaMemcpy(v.data(), x, n * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return e;
+  std::vector<float> t(v.begin(), v.end());
+  std::vector<uint16_t> first;
+  const MxFindDev f = mx::find_table(first, t.data(), n);
+  const size_t at = n * sizeof(float), bytes = at + first.size() * sizeof(uint16_t);
+  char *d = nullptr;
+  if ((e = cudaMalloc(&d, bytes)) != cudaSuccess) return e;
+  e = cudaMemcpy(d, t.data(), at, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !first.empty()) e = cudaMemcpy(d + at, first.data(), bytes - at, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    mx_find_check<<<(unsigned) ((n + 255) / 256), 256>>>(f, (const uint16_t *) (d + at), (const float *) d, (unsigned) n, y);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  }
+  const cudaError_t e2 = cudaFree(d);
+  return e != cudaSuccess ? e : e2;
+}
+
 cudaError_t math_check(int fn, const double *x, double *y, size_t n) {
   if (n == 0) return cudaSuccess;
+  if (fn == 11) return find_check(x, y, n);
   const unsigned blocks = (unsigned) ((n + 255) / 256);
   mx_math_kernel<<<blocks, 256>>>(fn, x, y, n);
   cudaError_t e = cudaGetLastError();

@@ -115,6 +115,32 @@ static void hi_lo(double d, float f[2]) {
   f[1] = (float) (d - (double) f[0]);
 }
 
+// The index table of abscissae x (MxFindDev), one to two entries for each;
+// none for abscissae that are not positive, finite and in order, or that do
+// not fit 16-bit indices.
+MxFindDev find_table(std::vector<uint16_t> &first, const float *x, size_t n) {
+  MxFindDev f;
+  memset(&f, 0, sizeof(f));
+  if (n < 8 || n > 65535 || !(x[0] > 0.0f) || !std::isfinite(x[n - 1])) return f;
+  for (size_t k = 1; k < n; k++) {
+    if (!(x[k] >= x[k - 1])) return f;
+    if (x[k] == x[k - 1]) f.repeats = 1;
+  }
+  auto bits = [](float v) { uint32_t u; memcpy(&u, &v, 4); return u; };
+  const uint32_t b0 = bits(x[0]), b1 = bits(x[n - 1]);
+  unsigned s = 1;
+  while ((b1 >> s) - (b0 >> s) + 1 > 2 * n) s++;
+  f.lo = x[0]; f.hi = x[n - 1];
+  f.off = (int32_t) first.size();
+  f.shift = (uint16_t) s;
+  size_t k = 0;
+  for (uint32_t b = b0 >> s; b <= b1 >> s; b++) {
+    while (k < n && (bits(x[k]) >> s) < b) k++;
+    first.push_back((uint16_t) k);
+  }
+  return f;
+}
+
 // True if every energy row of a cumulative table [energy][order] is
 // non-decreasing in the order index (the trace may then bisect it).
 static bool rows_monotone(const float *cum, size_t nenergy, int norders) {
@@ -276,6 +302,7 @@ static bool build_letg(const Pack &pk, const mx_config &cfg, HostModel &M, std::
     }
     g.geff_off = (int32_t) M.geff_energy.size();
     M.geff_energy.insert(M.geff_energy.end(), e, e + ne);
+    g.find = find_table(M.find_first, e, ne);
     g.cum_off = (int32_t) M.geff_cum.size();
     for (unsigned j = 0; j < ne; j++)
       for (unsigned k = 0; k < no; k++) M.geff_cum.push_back(cum[k * ne + j]);   // [energy][order]
@@ -326,6 +353,7 @@ static bool build_letg(const Pack &pk, const mx_config &cfg, HostModel &M, std::
     d.cos_t = cos(angle[s]); d.sin_t = sin(angle[s]);
   }
   T.support_nenergy = (int32_t) NE;
+  T.support_find = find_table(M.find_first, E.data(), NE);
   return true;
 }
 
@@ -387,6 +415,7 @@ static bool hrc_table(const Pack &pk, const std::string &name, int col, HostMode
   append_slopes(M.hrc_slope, a, a + (size_t) col * n, n);
   M.hrc_slope.push_back(0.0);
   t.n = (int32_t) n;
+  t.find = find_table(M.find_first, a, n);
   return true;
 }
 
@@ -521,6 +550,7 @@ static MxTabDev response_table(HostModel &M, const float *x, const float *y, uns
   M.fef_f.insert(M.fef_f.end(), y, y + n);
   t.s_off = (int32_t) M.fef_slope.size();
   append_slopes(M.fef_slope, x, y, n);
+  t.find = find_table(M.find_first, x, n);
   return t;
 }
 
@@ -802,6 +832,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
   M.optc.assign(opt, opt + 3 * optn);
   append_slopes(M.optc_slope, opt, opt + optn, optn);          // beta
   append_slopes(M.optc_slope, opt, opt + 2 * optn, optn);      // delta
+  T.opt_find = find_table(M.find_first, opt, optn);
   double total_area = 0.0;
   T.p_unturned = 1;
   M.shells.resize(4);
@@ -878,6 +909,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
     M.optc.insert(M.optc.end(), corr, corr + cnt);
     h.corr_slope_off = (int32_t) M.optc_slope.size();
     append_slopes(M.optc_slope, corr, corr + h.corr_n, (unsigned) h.corr_n);
+    h.corr_find = find_table(M.find_first, corr, (size_t) h.corr_n);
   }
   if (total_area <= 0.0) { err = "The mirror geometric area is 0.  Check shutters."; return false; }
   M.geom_area_cm2 = (total_area * PI_) / 100.0;
@@ -977,6 +1009,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
       }
       g.geff_off = (int32_t) M.geff_energy.size();
       M.geff_energy.insert(M.geff_energy.end(), e, e + ne);
+    g.find = find_table(M.find_first, e, ne);
       g.cum_off = (int32_t) M.geff_cum.size();
       for (unsigned j = 0; j < ne; j++)
         for (unsigned k = 0; k < no; k++) M.geff_cum.push_back(cum[k * ne + j]);   // [energy][order]

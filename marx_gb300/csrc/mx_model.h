@@ -10,6 +10,18 @@
 #define MX_MAX_SECTORS 64
 #define MX_MAX_GRATINGS 8     // HETG shells 1,3,4,6 then LETG shells 1,3,4,6
 
+// Where a value lies among a table's increasing positive abscissae, without a
+// search: floats of one sign order as their bits, so first[off + b] is the
+// index of the first abscissa whose top bits (bits >> shift) are those of
+// abscissa 0 plus b, or more; the few that share the value's top bits are
+// looked through.  For lo < value < hi, the first and last abscissa;
+// shift 0: the table has none.
+struct MxFindDev {
+  float lo, hi;
+  int32_t off;
+  uint16_t shift, repeats;                     // repeats: some abscissae are equal
+};
+
 // One HRMA shell: both optics (index 0 = paraboloid P, 1 = hyperboloid H).
 struct MxShellDev {
   double a[2], b[2], c[2], xmin[2], xmax[2];   // conic x^2+r^2 = a x^2 + b x + c, x-limits (hrma.c:555-575)
@@ -38,7 +50,8 @@ struct MxShellDev {
   // as hi + lo
   float xlimf[2][2], r2limf[2][2], am1f[2], bf[2], quarter_l2f, frontf, front_fwdf;
   float blurf[2][2], scatf[2][2];
-  float bank_pad[17];
+  MxFindDev corr_find;                         // of the correction-factor table
+  float bank_pad[13];
 };
 static_assert(sizeof(MxShellDev) % 128 == 96, "shell records of 736 + 128 k bytes: four distinct bank offsets");
 
@@ -49,6 +62,7 @@ struct MxGratingDev {
   int32_t geff_off, cum_off, nenergy, norders; // cumulative efficiencies [energy][order]
   int32_t max_order, order_off, sec_off, nsec; // order_k offset; sectors [6][nsec]
   int32_t monotone, pad;                       // every energy row non-decreasing in the order index
+  MxFindDev find;                              // of the energies
 };
 
 // One LETG support grating as the trace meets it (diffract.c:1097-1114):
@@ -65,6 +79,7 @@ struct MxSupportDev {
 // hrc_slope + s_off; n = 0 means a perfect efficiency (no table).
 struct MxTabDev {
   int32_t x_off, y_off, s_off, n;
+  MxFindDev find;
 };
 
 // One Drake-flat plate section (drake.c:48-58, 188-230).
@@ -160,6 +175,8 @@ struct MxTables {
   const float *support_cum;     // [energy][order] per support grating
   const double *support_k;      // order * (2 pi hbar c) / period per support grating and order
   int32_t support_nenergy, pad_support;
+  MxFindDev support_find, opt_find;   // of support_energy and of the optical constants' energies
+  const uint16_t *find_first;         // the index tables of every MxFindDev
   // mirror
   int32_t ideal, use_blur, use_wfold, use_struts, use_scale, area_uniform;
   double hrma_vig, source_distance, cap, cos30, sin30;
