@@ -298,7 +298,7 @@ int mx_trace(mx_context *ctx, const mx_photons *ph, uint32_t stages,
  * intersections into three kernels with survivor queues between them (the
  * photons lost on the way then stop occupying SIMT lanes) and needs
  * 2 x 128 bytes of device scratch per photon; AUTO picks the wavefront from
- * MX_WAVEFRONT_MIN_PHOTONS photons up, without a grating only from more than
+ * MX_WAVEFRONT_MIN_PHOTONS photons up, but not before a list is longer than
  * the fused kernel holds at once.  Both give the same per-photon results. */
 #define MX_MODE_AUTO 0
 #define MX_MODE_FUSED 1

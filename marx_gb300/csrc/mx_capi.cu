@@ -318,19 +318,18 @@ static int pipe_streams(mx_context *c) {
 }
 
 // Whether a list of n photons takes the wavefront kernels.  In AUTO mode those
-// of MX_WAVEFRONT_MIN_PHOTONS or more do, but without a grating only where
-// the fused kernel could not hold them all at once, a photon to a thread
-// (97 280 on 152 SMs): its single round then saves four launches and the
-// queues (66 000 plain_scatter photons 78 against 116 us, on axis 56 against
-// 75; 100 000 120 against 122; with the HETG 66 000 109 against 145 us but
-// 100 000 173 against 153, with the LETG 66 000 198 against 209 and 100 000
-// 338 against 217).  Both give the same results bit for bit.
+// of MX_WAVEFRONT_MIN_PHOTONS or more do that the fused kernel could not hold
+// all at once, a photon to a thread (97 280 on 152 SMs): its single round
+// saves four or five launches and the queues.  97 000 photons fused / in
+// queues: on axis 60 / 75 us, plain_scatter 80 / 106, HETG 107 / 125, LETG 120
+// / 137, HRC-I 105 / 117, LETG with HRC-S 160 / 160; 120 000: 71 / 79, 116 /
+// 113, 165 / 138, 184 / 148, 171 / 137, 263 / 169.  Both give the same results
+// bit for bit.
 static bool takes_wavefront(const mx_context *c, const MxTables &T, uint32_t n, uint32_t stages) {
   if (!(stages & MX_STAGE_MIRROR) || c->mode == MX_MODE_FUSED) return false;
   if (c->mode == MX_MODE_WAVEFRONT) return true;
   const uint32_t resident = (uint32_t) (c->num_sms * c->trace_blocks[1]) * MX_TRACE_BLOCK;
-  const bool grating = (stages & MX_STAGE_GRATING) && T.grating;
-  return n >= (grating ? MX_WAVEFRONT_MIN_PHOTONS : std::max((uint32_t) MX_WAVEFRONT_MIN_PHOTONS, resident + 1));
+  return n >= std::max((uint32_t) MX_WAVEFRONT_MIN_PHOTONS, resident + 1);
 }
 
 // A device trace that takes the wavefront kernels with Philox draws, from
