@@ -216,10 +216,18 @@ __global__ void __launch_bounds__(256) mx_generate_kernel(const __grid_constant_
   }
 }
 
+// A phase's work tile: at most the batch's parameter, and small enough that a
+// warp claims four or more (a queue of 400,000 records in tiles of 256 leaves
+// a third of the warps without one).
+__device__ __forceinline__ uint32_t phase_tile(uint32_t count, int tile) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5), t = (count / (4u * warps)) & ~31u;
+  return min((uint32_t) tile, max(t, 32u));
+}
+
 // A warp's claim of `tile` consecutive work items from a global counter.
-__device__ __forceinline__ uint32_t claim(unsigned int *ctr, int tile) {
+__device__ __forceinline__ uint32_t claim(unsigned int *ctr, uint32_t tile) {
   unsigned base = 0;
-  if ((threadIdx.x & 31) == 0) base = atomicAdd(ctr, (unsigned) tile);
+  if ((threadIdx.x & 31) == 0) base = atomicAdd(ctr, tile);
   return __shfl_sync(0xffffffffu, base, 0);
 }
 
@@ -250,17 +258,69 @@ __device__ __forceinline__ void batch_finish(const MxTables &T, const MxChipDev 
   }
 }
 
+// The groups of 32 records a warp works on in one phase: from the tiles it
+// claims, and of those it left for later (photons scattered into the far tail,
+// one in a hundred: mirror_middle's `late`) as soon as it has 32 of them, the
+// rest at its end.  In line, a quarter of the groups would run the tail's 135
+// FP64 operations for a lane or two.  A short queue, of fewer than
+// MX_BATCH_LATE groups per warp, keeps them in line: the warp's last group of
+// late photons would cost it more.
+#define MX_BATCH_LATE 3
+struct TileRounds {
+  unsigned int *ctr;
+  uint32_t count, tile, j, end, n_late;
+  uint32_t *late;               // this warp's list, 64 entries
+  bool use, done;
+  __device__ __forceinline__ TileRounds(unsigned int *c, uint32_t n, int t, uint32_t *list)
+      : ctr(c), count(n), tile(phase_tile(n, t)), j(0), end(0), n_late(0), late(list), done(false) {
+    use = count / MX_BATCH_LATE >= gridDim.x * blockDim.x;
+  }
+  // The next group: this lane's record k in it, if any (have), and whether
+  // the record may be left for later.
+  __device__ __forceinline__ bool next(uint32_t &k, bool &have, bool &may_defer) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (j >= end && !done && n_late < 32) {
+      j = claim(ctr, tile);
+      end = min(j + tile, count);
+      done = j >= count;
+    }
+    if (n_late >= 32 || (done && n_late > 0)) {
+      const uint32_t take = min(n_late, 32u);
+      n_late -= take;
+      have = lane < take;
+      k = have ? late[n_late + lane] : 0u;
+      may_defer = false;
+      __syncwarp();   // read before the list grows again
+      return true;
+    }
+    if (done) return false;
+    k = j + lane;
+    have = k < end;
+    may_defer = use;
+    j += 32;
+    return true;
+  }
+  __device__ __forceinline__ void defer(bool later, uint32_t k) {
+    const unsigned m = __ballot_sync(0xffffffffu, later);
+    if (later) late[n_late + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = k;
+    n_late += (uint32_t) __popc(m);
+    __syncwarp();
+  }
+};
+
 // The whole batch in one persistent cooperative launch.  The five phases
 // of the wavefront trace (A, T, B, C and the gratings' D) are separated by
 // grid-wide barriers; inside a
 // phase warps claim tiles of work from a counter, so uneven sources and
 // uneven survivor counts spread over every SM.  Every thread reaches every
 // barrier: the claim loops end for a whole warp at once and nothing
-// returns early.  Compiled for three resident blocks of 256 threads per SM
-// (80 registers; about 250 bytes per thread spill to local memory): the
-// autotuner picks three blocks per SM then, 2 % faster than two blocks of
-// 128 registers on the 256-source batch.
-__global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b) {
+// returns early.  Two resident blocks of 256 threads per SM (114 registers);
+// three (80 registers, 900 bytes of spilled loads) are as fast over the
+// sizes below.  The far-scattered photons kept for
+// later and tiles that follow the queue's length: 256 sources with 3.7e7
+// photons 10.1 -> 9.2 ms, with 2.2e6 1240 -> 777 us, with 1e6 688 -> 423 us.
+__global__ void __launch_bounds__(256, 2) mx_batch_kernel(const __grid_constant__ MxTables T, const __grid_constant__ BatchIO b) {
+  __shared__ uint32_t late_lists[8][64];
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   extern __shared__ __align__(16) unsigned char smem[];
@@ -278,10 +338,10 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
   const uint32_t lane = threadIdx.x & 31;
 
   // Phase A: generation, dither, aperture.
-  for (;;) {
-    const uint32_t base = claim(&b.ctr[2], b.tile);
+  for (const uint32_t tile = phase_tile(io.n, b.tile);;) {
+    const uint32_t base = claim(&b.ctr[2], tile);
     if (base >= io.n) break;
-    const uint32_t end = min(base + (uint32_t) b.tile, io.n);
+    const uint32_t end = min(base + tile, io.n);
     for (uint32_t j = base; j < end; j += 32) {
       const uint32_t i = j + lane;
       bool keep = false;
@@ -318,10 +378,10 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
 
   // Phase T: the paraboloid's intersection, normal blur and reflectivity test.
   const uint32_t nt = __ldcg(&b.ctr[0]);
-  for (;;) {
-    const uint32_t base = claim(&b.ctr[6], b.tile);
+  for (const uint32_t tile = phase_tile(nt, b.tile);;) {
+    const uint32_t base = claim(&b.ctr[6], tile);
     if (base >= nt) break;
-    const uint32_t end = min(base + (uint32_t) b.tile, nt);
+    const uint32_t end = min(base + tile, nt);
     for (uint32_t j = base; j < end; j += 32) {
       const uint32_t k = j + lane;
       bool keep = false;
@@ -343,73 +403,67 @@ __global__ void __launch_bounds__(256, 3) mx_batch_kernel(MxTables T, BatchIO b)
 
   // Phase B: the rest of the paraboloid reflection, hyperboloid
   // intersection and reflectivity test (q1 is free again).
-  const uint32_t nb = __ldcg(&b.ctr[1]);
-  for (;;) {
-    const uint32_t base = claim(&b.ctr[3], b.tile);
-    if (base >= nb) break;
-    const uint32_t end = min(base + (uint32_t) b.tile, nb);
-    for (uint32_t j = base; j < end; j += 32) {
-      const uint32_t k = j + lane;
-      bool keep = false;
-      MxRec rec;
-      if (k < end) {
-        rec = b.q2[k];
-        Ph q; MirrorState m; Rng r;
-        from_rec(rec, q, m, r, io);
-        if (mirror_middle(T, sh, q, r, m)) {
-          keep = true;
-          to_rec(rec, q, m, r, rec.i);
-        } else
-          store_core(io, rec.i, q, r.overrun);
-      }
-      append(keep, rec, b.q1, &b.ctr[5]);
+  uint32_t *late = late_lists[threadIdx.x >> 5];
+  uint32_t k;
+  bool have, may_defer;
+  for (TileRounds rounds(&b.ctr[3], __ldcg(&b.ctr[1]), b.tile, late); rounds.next(k, have, may_defer);) {
+    bool keep = false, later = false;
+    MxRec rec;
+    if (have) {
+      rec = b.q2[k];
+      Ph q; MirrorState m; Rng r;
+      from_rec(rec, q, m, r, io);
+      const int next = mirror_middle(T, sh, q, r, m, may_defer);
+      if (next == 1) {
+        keep = true;
+        to_rec(rec, q, m, r, rec.i);
+      } else if (next == 2)
+        later = true;
+      else
+        store_core(io, rec.i, q, r.overrun);
     }
+    append(keep, rec, b.q1, &b.ctr[5]);
+    rounds.defer(later, k);
   }
   grid.sync();
 
   // Phase C: hyperboloid reflection, the source's grating up to its order
   // choice; the photons given an order go on to phase D (q2 is free again),
   // the others run the detector (without a grating) and are stored.
-  const uint32_t nc = __ldcg(&b.ctr[5]);
-  for (;;) {
-    const uint32_t base = claim(&b.ctr[4], b.tile);
-    if (base >= nc) break;
-    const uint32_t end = min(base + (uint32_t) b.tile, nc);
-    for (uint32_t j = base; j < end; j += 32) {
-      const uint32_t k = j + lane;
-      bool to_d = false;
-      MxRec rec;
-      if (k < end) {
-        rec = b.q1[k];
-        const MxSourceDev &S = ssrc[source_of(rec.i, sstart, b.nsrc)];
-        const uint32_t i = rec.i;
-        Ph q; MirrorState m; Rng r;
-        from_rec(rec, q, m, r, io);
-        const int unset = 0x7fff;
-        q.order = unset; q.ccd = unset;
-        mirror_back(T, sh, q, r, m);
-        if (!r.overrun && S.grating && !(q.flags & MX_BAD_PHOTON_MASK)) {
-          D3 gx, gp;
-          const int chosen = grating_front(T, gr, S.grating, q, r, gx, gp);
-          if (chosen >= 0) {
-            to_d = true;
-            to_rec_d(rec, gx, gp, q, r, i, chosen);
-          }
+  for (TileRounds rounds(&b.ctr[4], __ldcg(&b.ctr[5]), b.tile, late); rounds.next(k, have, may_defer);) {
+    bool to_d = false, later = false;
+    MxRec rec;
+    if (have) {
+      rec = b.q1[k];
+      const MxSourceDev &S = ssrc[source_of(rec.i, sstart, b.nsrc)];
+      const uint32_t i = rec.i;
+      Ph q; MirrorState m; Rng r;
+      from_rec(rec, q, m, r, io);
+      const int unset = 0x7fff;
+      q.order = unset; q.ccd = unset;
+      later = !mirror_back(T, sh, q, r, m, may_defer);
+      if (!later && !r.overrun && S.grating && !(q.flags & MX_BAD_PHOTON_MASK)) {
+        D3 gx, gp;
+        const int chosen = grating_front(T, gr, S.grating, q, r, gx, gp);
+        if (chosen >= 0) {
+          to_d = true;
+          to_rec_d(rec, gx, gp, q, r, i, chosen);
         }
-        if (!to_d) batch_finish(T, ch, S, io, i, q, r);
       }
-      append(to_d, rec, b.q2, &b.ctr[7]);
+      if (!later && !to_d) batch_finish(T, ch, S, io, i, q, r);
     }
+    append(to_d, rec, b.q2, &b.ctr[7]);
+    rounds.defer(later, k);
   }
   grid.sync();
 
   // Phase D: the diffraction into the chosen order, the detector, the
   // output columns.
   const uint32_t nd = __ldcg(&b.ctr[7]);
-  for (;;) {
-    const uint32_t base = claim(&b.ctr[8], b.tile);
+  for (const uint32_t tile = phase_tile(nd, b.tile);;) {
+    const uint32_t base = claim(&b.ctr[8], tile);
     if (base >= nd) break;
-    const uint32_t end = min(base + (uint32_t) b.tile, nd);
+    const uint32_t end = min(base + tile, nd);
     for (uint32_t k = base + lane; k < end; k += 32) {
       const MxRec rec = b.q2[k];
       const uint32_t i = rec.i;
