@@ -494,6 +494,30 @@ __device__ __forceinline__ F2 df_neg_log(unsigned long long f) {
   return df_add(df_mul_f(F2{0x1.62e430p-1f, -0x1.05c610p-29f}, e), F2{-2.0f * h.h, -2.0f * h.l});
 }
 
+// exp(y) - 1, 0 <= y < 80, within 2^-42: y = k ln 2 + r, |r| <= ln(2) / 2, and
+// the Taylor series of exp(r) - 1 nested, r (1 + r/2 (1 + r/3 (...))), its
+// terms from r^8/8! to r^13/13! in single precision.
+__device__ __forceinline__ F2 df_expm1(F2 y) {
+  const float k = rintf(y.h * 1.44269504f);
+  const F2 r = df_add(y, df_mul_f(F2{-0x1.62e430p-1f, 0x1.05c610p-29f}, k));
+  float g = fmaf(r.h, 1.0f / 13.0f, 1.0f);
+  g = fmaf(r.h * (1.0f / 12.0f), g, 1.0f);
+  g = fmaf(r.h * (1.0f / 11.0f), g, 1.0f);
+  g = fmaf(r.h * (1.0f / 10.0f), g, 1.0f);
+  g = fmaf(r.h * (1.0f / 9.0f), g, 1.0f);
+  F2 q = df_add_less(F2{1.0f, 0.0f}, df_prod(r, df_mul_f(F2{0x1p-3f, 0.0f}, g)));
+  q = df_add_less(F2{1.0f, 0.0f}, df_mul(r, df_prod(q, F2{0x1.24924ap-3f, -0x1.b6db6ep-28f})));   // 1/7
+  q = df_add_less(F2{1.0f, 0.0f}, df_mul(r, df_prod(q, F2{0x1.555556p-3f, -0x1.555556p-28f})));   // 1/6
+  q = df_add_less(F2{1.0f, 0.0f}, df_mul(r, df_prod(q, F2{0x1.99999ap-3f, -0x1.99999ap-29f})));   // 1/5
+  q = df_add_less(F2{1.0f, 0.0f}, df_mul(r, df_prod(q, F2{0.25f, 0.0f})));
+  q = df_add_less(F2{1.0f, 0.0f}, df_mul(r, df_prod(q, F2{0x1.555556p-2f, -0x1.555556p-27f})));   // 1/3
+  q = df_add_less(F2{1.0f, 0.0f}, df_mul(r, df_prod(q, F2{0.5f, 0.0f})));
+  const F2 e = df_mul(r, q);
+  if (k == 0.0f) return e;
+  const float p = __int_as_float(((int) k + 127) << 23);
+  return df_add(df_add(F2{p, 0.0f}, F2{-1.0f, 0.0f}), F2{e.h * p, e.l * p});
+}
+
 // The Fresnel numerator and denominator of reflectivity_parts in
 // double-float arithmetic on the FP32 pipe (beta, delta are floats), with
 // the same branches.  n^2 - sin^2 is formed without cancelling two numbers
@@ -2022,7 +2046,12 @@ MXD int diffract_support(const MxTables &T, const MxSupportDev &g, int order_idx
   const double p_l = fma(cs, c.x, MX_DMUL(sn, c.y)), p_d = nlod + fma(cs, c.y, -MX_DMUL(sn, c.x));
   const double pn2 = fma(-p_d, p_d, fma(-p_l, p_l, 1.0));
   if (neg_bit(pn2) && !is_zero(pn2)) return -1;
-  c = mk(fma(p_l, cs, -MX_DMUL(p_d, sn)), fma(p_l, sn, MX_DMUL(p_d, cs)), sqrt_fast(pn2));
+#ifdef __CUDA_ARCH__
+  const double root = lt_pos(0x1p-20, pn2) ? pn2 * rsqrt_seeded(pn2) : sqrt_fast(pn2);
+#else
+  const double root = sqrt_fast(pn2);
+#endif
+  c = mk(fma(p_l, cs, -MX_DMUL(p_d, sn)), fma(p_l, sn, MX_DMUL(p_d, cs)), root);
   return 0;
 }
 
@@ -2451,18 +2480,44 @@ MXD float hrc_interp(const MxTables &T, const MxTabDev &t, float x) {   // JDMin
 }
 
 // _marx_hrc_compute_pha (hrc-i.c:71-91): delta E / E = 1 (FWHM).
-MXD int16_t hrc_pha(double energy, Rng &rng) {
+MXD_COLD int16_t hrc_pha_double(double energy, double normal) {
   if (energy <= 0.5) energy = 141.582 * sqrt(energy);
   else if (energy < 2.0) energy = 107.299 * pow(energy, 0.1);
   else energy = 115.0;
-  energy = energy * (1.0 + 0.424661 * rng.normal());
+  energy = energy * (1.0 + 0.424661 * normal);
   if (energy < 0.0) energy = 0.0;
   return (int16_t) energy;
+}
+// The same whole number in double-float, the tenth root by one Newton step
+// on y^10 = E from its single-precision value; a pulse height within 1e-5 of
+// a whole number, of 32000 or more, or of an energy below 1e-9 keV is left to
+// the double form (a square root or a power, 20 to 80 FP64 operations).
+MXD int16_t hrc_pha(double energy, Rng &rng) {
+#ifdef __CUDA_ARCH__
+  const F2 z = rng.normal_df(), e = split(energy);
+  F2 v = {115.0f, 0.0f};
+  if (dkey(energy) <= dkey(0.5)) v = df_mul(df_sqrt(e), F2{0x1.1b29fcp+7f, -0x1.89374cp-21f});
+  else if (dkey(energy) < dkey(2.0)) {
+    const float y = exp2f(0.1f * log2f(e.h));
+    const F2 y2 = df_mul(F2{y, 0.0f}, F2{y, 0.0f}), y5 = df_mul_f(df_mul(y2, y2), y);
+    const F2 gap = df_sub(e, df_mul(y5, y5));
+    v = df_mul(quick_sum(y, y * (gap.h / (10.0f * e.h))), F2{0x1.ad322ep+6f, -0x1.e353f8p-19f});
+  }
+  const F2 s = df_add(F2{1.0f, 0.0f}, df_mul(F2{0x1.b2da56p-2f, -0x1.68e820p-27f}, z)), w = df_mul(v, s);
+  if (e.h > 1e-9f && w.h < 32000.0f) {
+    if (w.h < 0.99f) return 0;
+    const float fl = floorf(w.h), frac = (w.h - fl) + w.l;
+    if (frac > 1e-5f && frac < 0.99999f) return (int16_t) (int) fl;
+  }
+  return hrc_pha_double(energy, f2d(z.h) + f2d(z.l));
+#else
+  return hrc_pha_double(energy, rng.normal());
+#endif
 }
 
 // get_filter_region (hrc-s.c:119-185): UV/ion shield region 0..3 at (y, z)
 // in the MARX frame, or -1 in a gap.
-MXD int hrc_filter_region(const MxHrcDev &h, double y, double z) {
+MXD_COLD int hrc_filter_region(const MxHrcDev &h, double y, double z) {
   y -= h.shield_yc;
   z -= h.shield_zc;
   if (y < 0) {
@@ -2478,6 +2533,23 @@ MXD int hrc_filter_region(const MxHrcDev &h, double y, double z) {
   return -1;
 }
 
+// The region for a photon at x going along p, in single precision unless it
+// passes within 0.02 mm of an edge (positions there are good to 1e-3 mm).
+MXD int hrc_region(const MxHrcDev &h, D3 x, D3 p) {
+#ifdef __CUDA_ARCH__
+  const float t = (d2f_trunc(h.shield_x) - d2f_trunc(x.x)) / d2f_trunc(p.x);
+  const float y = fmaf(t, d2f_trunc(p.y), d2f_trunc(x.y)) - d2f_trunc(h.shield_yc);
+  const float z = fmaf(t, d2f_trunc(p.z), d2f_trunc(x.z)) - d2f_trunc(h.shield_zc), a = fabsf(y);
+  const bool left = y < 0.0f;
+  const float e0 = d2f_trunc(left ? h.shield_l : h.shield_r), e1 = d2f_trunc(left ? h.shield_sl : h.shield_sr);
+  const float e2 = d2f_trunc(left ? h.shield_sl_gap : h.shield_sr_gap), e3 = d2f_trunc(h.shield_t), m = 0.02f;
+  if (a > m && fabsf(a - e0) > m && fabsf(a - e1) > m && fabsf(a - e2) > m && fabsf(z - e3) > m && a < 1e3f)
+    return a < e0 ? 0 : a < e1 ? (z > e3 ? 0 : 1) : a > e2 ? (z > e3 ? 2 : 3) : -1;
+#endif
+  const double s = (h.shield_x - x.x) / p.x;
+  return hrc_filter_region(h, x.y + s * p.y, x.z + s * p.z);
+}
+
 // rand_gauss2d_radius (hrcblur.c:233-245): a draw of exactly 0 is redrawn.
 MXD double gauss2d_radius(double sigma, Rng &rng) {
   double c;
@@ -2486,9 +2558,11 @@ MXD double gauss2d_radius(double sigma, Rng &rng) {
   return sigma * sqrt(-2 * log(c));
 }
 
-// _marx_hrc_blur_position (hrcblur.c:258-298).
-MXD void hrc_blur(const MxHrcDev &h, bool extend, double &dx, double &dy, Rng &rng) {
-  double r = rng.uniform(), x0, y0;
+// _marx_hrc_blur_position (hrcblur.c:258-298).  On the device the radius (a
+// logarithm or an exponential and a root) and the angle's sine and cosine are
+// double-floats: four FP64 operations instead of about 150.
+MXD_COLD void hrc_blur_double(const MxHrcDev &h, double r, double &dx, double &dy, Rng &rng) {
+  double x0, y0;
   if (r < h.g1_w) { r = gauss2d_radius(h.g1_sigma, rng); x0 = 0.0; y0 = 0.0; }
   else if (r < h.g1_w + h.g2_w) { r = gauss2d_radius(h.g2_sigma, rng); x0 = h.g2_x; y0 = h.g2_y; }
   else {
@@ -2499,18 +2573,64 @@ MXD void hrc_blur(const MxHrcDev &h, bool extend, double &dx, double &dy, Rng &r
   double theta = (2.0 * PI) * rng.uniform();
   dx += x0 + r * cos(theta);
   dy += y0 + r * sin(theta);
-  if (!extend) {
-    if (dx < 0.0) dx = 0.0;
-    if (dy < 0.0) dy = 0.0;
+}
+MXD void hrc_blur(const MxHrcDev &h, bool extend, double &dx, double &dy, Rng &rng) {
+  const double r = rng.uniform();
+#ifdef __CUDA_ARCH__
+  const int upos = rng.upos;
+  const bool g1 = lt_pos(r, h.g1_w), g2 = !g1 && lt_pos(r, h.g1_w + h.g2_w);
+  const unsigned long long u = rng.uniform_fixed();
+  F2 rad;
+  if (g1 || g2) {
+    const F2 l = df_neg_log(u | 1ull);
+    rad = df_mul(df_sqrt(F2{2.0f * l.h, 2.0f * l.l}), split(g1 ? h.g1_sigma : h.g2_sigma));
+  } else
+    rad = df_mul(df_sqrt(df_expm1(df_mul(split(unit_from_bits(u >> 11)), F2{h.l1_log[0], h.l1_log[1]}))), split(h.l1_hwhm));
+  F2 sn, cs;
+  df_turn_sincos(rng.uniform_fixed(), false, sn, cs);
+  // draws below 2^-40 or next to 1 (where a radius is near 0) keep the double form
+  if (!rng.overrun && u >> 24 && ~u >> 24) {
+    const F2 c = df_mul(rad, cs), s = df_mul(rad, sn);
+    dx += df_join(c) + (g1 ? 0.0 : g2 ? h.g2_x : h.l1_x);
+    dy += df_join(s) + (g1 ? 0.0 : g2 ? h.g2_y : h.l1_y);
+  } else {
+    rng.upos = upos;
+    hrc_blur_double(h, r, dx, dy, rng);
   }
+#else
+  hrc_blur_double(h, r, dx, dy, rng);
+#endif
+  if (!extend) {
+    if (dkey(dx) < 0) dx = 0.0;
+    if (dkey(dy) < 0) dy = 0.0;
+  }
+}
+
+// Whether a ray certainly misses a Drake plate's rectangle, in single
+// precision: its coordinates there are good to 6e-3 mm / |p.n| (positions of
+// up to 1e4 mm); the margin is fifteen times that.
+MXD bool plate_missed(const MxPlateDev &r, float x0, float x1, float x2, float p0, float p1, float p2) {
+  const float d0 = x0 - r.f_a[0], d1 = x1 - r.f_a[1], d2 = x2 - r.f_a[2];
+  const float inv = 1.0f / (p0 * r.f_normal[0] + p1 * r.f_normal[1] + p2 * r.f_normal[2]);
+  const float t = -(d0 * r.f_normal[0] + d1 * r.f_normal[1] + d2 * r.f_normal[2]) * inv;
+  const float q0 = d0 + t * p0, q1 = d1 + t * p1, q2 = d2 + t * p2, m = 0.1f + 0.1f * fabsf(inv);
+  const float xx = q0 * r.f_e1[0] + q1 * r.f_e1[1] + q2 * r.f_e1[2], yy = q0 * r.f_e2[0] + q1 * r.f_e2[1] + q2 * r.f_e2[2];
+  return xx < -m || xx > r.f_len1 + m || yy < -m || yy > r.f_len2 + m;
 }
 
 // drake_intersection + the reflection of _marx_drake_reflect (drake.c:250-351)
 // for one photon, in the MARX frame.
 MXD void drake_reflect(const MxTables &T, const MxHrcDev &h, Ph &ph, Rng &rng) {
   const D3 x0 = ph.x, p = ph.p;
+#ifdef __CUDA_ARCH__
+  const float fx0 = d2f_trunc(x0.x), fx1 = d2f_trunc(x0.y), fx2 = d2f_trunc(x0.z);
+  const float fp0 = d2f_trunc(p.x), fp1 = d2f_trunc(p.y), fp2 = d2f_trunc(p.z);
+#endif
   for (int i = 0; i < h.drake_n; i++) {
     const MxPlateDev &r = h.plates[i];
+#ifdef __CUDA_ARCH__
+    if (plate_missed(r, fx0, fx1, fx2, fp0, fp1, fp2)) continue;
+#endif
     const D3 nrm = mk(r.normal[0], r.normal[1], r.normal[2]), a = mk(r.a[0], r.a[1], r.a[2]);
     double pdn = dot(p, nrm);
     if (pdn == 0.0) continue;
@@ -2595,16 +2715,15 @@ MXD void hrc_detect_stage(const MxTables &T, const MxChipDev *chips, int nchips,
   bool ok = true;
   const int m = hrcs ? d.id - 1 : 0;                     // facet index 0..2
   const MxTabDev &mcp = h.mcp[hrcs ? 2 - m : 0];         // HRC-S MCP ids 1, 2, 3 use QE files 2, 1, 0
-  if (mcp.n && rng.uniform() >= (double) hrc_interp(T, mcp, fe)) ok = false;
+  if (mcp.n && dkey(rng.uniform()) >= dkey(f2d(hrc_interp(T, mcp, fe)))) ok = false;
   int region = 0;
   if (ok && hrcs) {
-    double t = (h.shield_x - x.x) / p.x;
-    region = hrc_filter_region(h, x.y + t * p.y, x.z + t * p.z);
+    region = hrc_region(h, x, p);
     if (region < 0) ok = false;
   }
   if (ok) {
     const MxTabDev &f = h.filt[region];
-    if (f.n && rng.uniform() >= (double) hrc_interp(T, f, fe)) ok = false;
+    if (f.n && dkey(rng.uniform()) >= dkey(f2d(hrc_interp(T, f, fe)))) ok = false;
   }
   if (!ok) {
     ph.flags |= MX_PHOTON_UNDETECTED;
@@ -2618,13 +2737,13 @@ MXD void hrc_detect_stage(const MxTables &T, const MxChipDev *chips, int nchips,
     if (hrcs) {   // _marx_hrc_s_compute_pixel (hrc_s_geom.c:289-340)
       double u = h.u_active0 + div_by(dx, h.pix[0], h.inv_pix[0]);
       double v = h.v_active0[m] + div_by(dy, h.pix[1], h.inv_pix[1]);
-      ph.upix = (float) u; ph.vpix = (float) v;
+      ph.upix = d2f_rn(u); ph.vpix = d2f_rn(v);
       ph.set |= MX_SET_UV;
-      ph.ypix = (float) (h.cxcy0[m][0] + (u - h.uv0[m][0]));
-      ph.zpix = (float) (h.cxcy0[m][1] + (v - h.uv0[m][1]));
+      ph.ypix = d2f_rn(h.cxcy0[m][0] + (u - h.uv0[m][0]));
+      ph.zpix = d2f_rn(h.cxcy0[m][1] + (v - h.uv0[m][1]));
     } else {      // _marx_hrc_i_compute_pixel (hrc_i_geom.c:134-143)
-      ph.ypix = (float) (h.ll_cxcy[0] + div_by(dx, h.pix[0], h.inv_pix[0]));
-      ph.zpix = (float) (h.ll_cxcy[1] + div_by(dy, h.pix[1], h.inv_pix[1]));
+      ph.ypix = d2f_rn(h.ll_cxcy[0] + div_by(dx, h.pix[0], h.inv_pix[0]));
+      ph.zpix = d2f_rn(h.ll_cxcy[1] + div_by(dy, h.pix[1], h.inv_pix[1]));
     }
   }
   det_leave(T, fr, x, p);

@@ -33,6 +33,7 @@ struct HostModel {
   std::vector<float> support_energy, support_cum;
   std::vector<double> support_k;
   std::vector<float> hrc_tab;
+  std::vector<MxTabDev> hrc_seen;   // the tables in hrc_tab so far
   std::vector<double> hrc_slope;
   std::vector<int32_t> fef_map;
   std::vector<MxFefDev> fef;

@@ -667,6 +667,7 @@ __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, d
   else if (fn == 6) y[i] = mx::u2d(mx::trunc_to_unsigned(v));
   else if (fn == 7) y[i] = mx::sqrt_fast(v);
   else if (fn == 8) y[i] = mx::quarter_of(v);
+  else if (fn == 12) y[i] = mx::f2_double(mx::df_expm1(mx::split(v)));
   else if (fn == 9) y[i] = mx::df_join(mx::split(v));
   else if (fn == 10) {
     mx::F2 sn, cs;

@@ -133,11 +133,11 @@ MxFindDev find_table(std::vector<uint16_t> &first, const float *x, size_t n) {
   f.lo = x[0]; f.hi = x[n - 1];
   f.off = (int32_t) first.size();
   f.shift = (uint16_t) s;
-  size_t k = 0;
-  for (uint32_t b = b0 >> s; b <= b1 >> s; b++) {
-    while (k < n && (bits(x[k]) >> s) < b) k++;
-    first.push_back((uint16_t) k);
-  }
+  first.resize(first.size() + (b1 >> s) - (b0 >> s) + 1);
+  uint16_t *at = first.data() + f.off;
+  uint32_t b = b0 >> s;
+  for (size_t k = 0; k < n; k++)
+    for (const uint32_t e = bits(x[k]) >> s; b <= e; b++) *at++ = (uint16_t) k;
   return f;
 }
 
@@ -407,15 +407,23 @@ static bool hrc_table(const Pack &pk, const std::string &name, int col, HostMode
   int ncol = name.find("optconst") != std::string::npos ? 3 : 2;
   unsigned n = (unsigned) (cnt / ncol);
   if (n < 1) { err = name + ": empty table"; return false; }
-  t.x_off = (int32_t) M.hrc_tab.size();
-  M.hrc_tab.insert(M.hrc_tab.end(), a, a + n);
+  // tables over the same energies (the shield's regions, a layer's beta and
+  // delta) share them and their index
+  t.x_off = -1;
+  for (const MxTabDev &o : M.hrc_seen)
+    if (o.n == (int32_t) n && !memcmp(&M.hrc_tab[o.x_off], a, n * sizeof(float))) { t.x_off = o.x_off; t.find = o.find; }
+  if (t.x_off < 0) {
+    t.x_off = (int32_t) M.hrc_tab.size();
+    M.hrc_tab.insert(M.hrc_tab.end(), a, a + n);
+    t.find = find_table(M.find_first, a, n);
+  }
   t.y_off = (int32_t) M.hrc_tab.size();
   M.hrc_tab.insert(M.hrc_tab.end(), a + (size_t) col * n, a + (size_t) (col + 1) * n);
   t.s_off = (int32_t) M.hrc_slope.size();
   append_slopes(M.hrc_slope, a, a + (size_t) col * n, n);
   M.hrc_slope.push_back(0.0);
   t.n = (int32_t) n;
-  t.find = find_table(M.find_first, a, n);
+  M.hrc_seen.push_back(t);
   return true;
 }
 
@@ -443,6 +451,7 @@ static bool hrc_blur(const double *b, double pixelsize, MxHrcDev &h, std::string
   if (norm > 0) { g1w /= norm; g2w /= norm; l1w /= norm; }
   h.g1_sigma = g1s; h.g1_w = g1w; h.g2_sigma = g2s; h.g2_x = g2x; h.g2_y = g2y; h.g2_w = g2w;
   h.l1_hwhm = l1h; h.l1_x = l1x; h.l1_y = l1y; h.l1_rmax = l1r; h.l1_w = l1w;
+  hi_lo(log1p((l1r / l1h) * (l1r / l1h)), h.l1_log);
   return true;
 }
 
@@ -636,7 +645,7 @@ static bool build_hrc(const Pack &pk, const mx_config &cfg, HostModel &M, std::s
   memset(&h, 0, sizeof(h));
   h.kind = cfg.detector;
   h.blur = !cfg.det_ideal;
-  M.hrc_tab.clear(); M.hrc_slope.clear();
+  M.hrc_tab.clear(); M.hrc_slope.clear(); M.hrc_seen.clear();
   auto table = [&](const char *name, int col, MxTabDev &t) {
     if (cfg.det_ideal) { memset(&t, 0, sizeof(t)); return true; }   // _marx_hrc_read_efficiencies: perfect
     return hrc_table(pk, name, col, M, t, err);
@@ -772,6 +781,11 @@ static bool build_hrc(const Pack &pk, const mx_config &cfg, HostModel &M, std::s
           v3_sum(a, gc, corner);
           for (int k = 0; k < 3; k++) { r.a[k] = a[k]; r.e1[k] = e1[k]; r.e2[k] = e2[k]; r.normal[k] = nrm[k]; }
           r.len1 = cfg.hesf_length; r.len2 = l2;
+          for (int k = 0; k < 3; k++) {
+            r.f_a[k] = (float) r.a[k]; r.f_e1[k] = (float) r.e1[k];
+            r.f_e2[k] = (float) r.e2[k]; r.f_normal[k] = (float) r.normal[k];
+          }
+          r.f_len1 = (float) r.len1; r.f_len2 = (float) r.len2;
         }
         cz -= htt;
         cx += hh;
@@ -1113,7 +1127,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
     T.nchips = cfg.detector == MX_DETECTOR_NONE ? 0 : (cfg.detector == MX_DETECTOR_ACIS_I ? 4 : 6);
     T.det_kind = cfg.detector;
     T.det_ideal = cfg.det_ideal != 0;
-    M.hrc_tab.clear(); M.hrc_slope.clear();
+    M.hrc_tab.clear(); M.hrc_slope.clear(); M.hrc_seen.clear();
     memset(&T.hrc, 0, sizeof(T.hrc));
     if (!acis && cfg.detector != MX_DETECTOR_NONE && !build_hrc(pk, cfg, M, err)) return false;
     if (M.hrc_tab.empty()) { M.hrc_tab.push_back(0.f); M.hrc_slope.push_back(0.0); }

@@ -86,6 +86,7 @@ struct MxTabDev {
 struct MxPlateDev {
   double a[3], e1[3], e2[3], normal[3];
   double len1, len2;
+  float f_a[3], f_e1[3], f_e2[3], f_normal[3], f_len1, f_len2;   // in float (the miss screen)
 };
 
 // The configured HRC (hrc-i.c, hrc-s.c, hrc_i_geom.c, hrc_s_geom.c,
@@ -103,6 +104,7 @@ struct MxHrcDev {
       shield_x;
   // position blur (hrcblur.c:105-188), mm, centred on the first gaussian
   double g1_sigma, g1_w, g2_sigma, g2_x, g2_y, g2_w, l1_hwhm, l1_x, l1_y, l1_rmax, l1_w;
+  float l1_log[2], pad_l1[2];   // log1p((l1_rmax / l1_hwhm)^2) as hi + lo
   // Drake flat (HRC-S): 2 x plates sections, carbon and chromium constants
   int32_t drake_n, pad;
   double drake_cr_width;
