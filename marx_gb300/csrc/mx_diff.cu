@@ -178,39 +178,41 @@ struct SplatWindow {
   unsigned last_x, last_y, shift;
 };
 
-// Splat the warp's rays: lane L's ray is valid when valid is set, with its
-// window origin and taps computed by that lane into its stage row; then
-// the warp adds the 121 taps of each valid ray together.  The window's 64-bit
+// Splat the warp's rays: lane L's ray is valid when valid is set; its window
+// origin and taps go to a row of the stage, then the warp adds the 121 taps
+// of each valid ray together.  The window's 64-bit
 // sums are kept as two planes of 32-bit words, the carry added to the upper
 // one: 9.5 cycles of the SM for a warp's update where a 64-bit shared atomic
 // takes 13.6.
-// A lane writes its taps for half a warp's rays at a time (16 rows of the
-// stage).
+// Half the rays at a time (16 rows of the stage), a lane making the eleven
+// taps of one ray along one axis.
 __device__ __forceinline__ void splat_warp(const ImageGeom &g, const SplatWindow &W, bool valid, double y, double z, double w, uint32_t *stage,
                                            uint32_t *lo, uint32_t *hi, unsigned long long *acc, const TapLane &tl,
                                            int lane) {
   int ic = 0, jc = 0;
   float fu = 0.f, fv = 0.f;
   if (valid) valid = mx::dkey(w) > 0 && splat_origin(g, y, z, ic, jc, fu, fv);
-  uint32_t ty[mxd::TAPS], tz[mxd::TAPS];
-  if (valid) {
-    const uint32_t wq = weight_fixed(w);
-#pragma unroll
-    for (int k = 0; k < mxd::TAPS; k++) {
-      const uint32_t gy = __float2uint_rn(FMUL(tap(g, k, fu), 2147483648.0f));   // K 2^31
-      ty[k] = __umulhi(wq, gy);                                                  // w K 2^30
-      tz[k] = __float2uint_rn(FMUL(tap(g, k, fv), 2147483648.0f));
-    }
-  }
+  const uint32_t wq = valid ? weight_fixed(w) : 0u;
   const unsigned vm = __ballot_sync(0xffffffffu, valid);
 #pragma unroll 1
   for (int half = 0; half < 32; half += 16) {
-  if (valid && (lane & 16) == half) {
-    uint32_t *row = stage + (lane & 15) * STAGE_STRIDE;
-    row[0] = (uint32_t) ic;
-    row[1] = (uint32_t) jc;
-#pragma unroll
-    for (int k = 0; k < mxd::TAPS; k++) { row[2 + k] = ty[k]; row[2 + mxd::TAPS + k] = tz[k]; }
+  {
+    const int src = half + (lane & 15);
+    const float f0 = __shfl_sync(0xffffffffu, fu, src), f1 = __shfl_sync(0xffffffffu, fv, src);
+    const int c = __shfl_sync(0xffffffffu, ic, src), r = __shfl_sync(0xffffffffu, jc, src);
+    const uint32_t ww = __shfl_sync(0xffffffffu, wq, src);
+    if ((vm >> src) & 1u) {
+      uint32_t *row = stage + (lane & 15) * STAGE_STRIDE;
+      const bool second = lane >= 16;
+      const float f = second ? f1 : f0;
+      row[second] = (uint32_t) (second ? r : c);
+      row += second ? 2 + mxd::TAPS : 2;
+#pragma unroll 1
+      for (int k = 0; k < mxd::TAPS; k++) {
+        const uint32_t t = __float2uint_rn(FMUL(tap(g, k, f), 2147483648.0f));   // K 2^31
+        row[k] = second ? t : __umulhi(ww, t);                                   // w K 2^30
+      }
+    }
   }
   __syncwarp();
   for (unsigned hm = (vm >> half) & 0xffffu; hm; hm &= hm - 1) {
@@ -301,6 +303,7 @@ __device__ __forceinline__ bool ray_front(const FwdArgs &A, const MxTables *T, u
                                 A.sh[si].p1f[2]);
 }
 
+static_assert(mxd::RAY_ROOT_P == 2 && mxd::RAY_ROOT_H == 4, "optic o's root is bit o + 1 of the decision byte");
 // Part 2: through both mirrors to the focal plane x = 0.  root holds the
 // recorded conic roots (RAY_ROOT_* bits) of a replayed ray, and receives
 // those taken otherwise.
@@ -313,30 +316,32 @@ __device__ __forceinline__ bool ray_image(const FwdArgs &A, const MxTables &T, i
   const double *f = h.fwd[0];
   mx::D3 x = mx::mk(fma(f[2], rz, fma(f[1], ry, h.front_fwd[0])), fma(f[5], rz, fma(f[4], ry, h.front_fwd[1])),
                     fma(f[8], rz, fma(f[7], ry, h.front_fwd[2])));
-  mx::D3 p = mx::mk(S.p1[0], S.p1[1], S.p1[2]), n;
-  const int rp = mxd::conic_root(h, 0, x, p, n, replay ? ((root & mxd::RAY_ROOT_P) ? 1 : 0) : -1);
-  if (rp < 0) return false;
+  mx::D3 p = mx::mk(S.p1[0], S.p1[1], S.p1[2]);
   mx::F2 num{1.0f, 0.0f}, den{1.0f, 0.0f};
-  double pdn = mx::dot(p, n);
-  if (A.weighted) mx::reflectivity_df(mx::split(fabs(pdn)), S.beta, S.delta, num, den);
-  p = mxd::reflected(p, n, pdn);
-  if (!replay && T.use_struts && mx::cap_struts_block(T, h, x, p)) return false;
-  {
-    const double *M = h.mid, *c = h.mid_off;
-    p = mx::mat_mul(M, p);
-    x = mx::mk(fma(M[0], x.x, fma(M[1], x.y, fma(M[2], x.z, c[0]))), fma(M[3], x.x, fma(M[4], x.y, fma(M[5], x.z, c[1]))),
-               fma(M[6], x.x, fma(M[7], x.y, fma(M[8], x.z, c[2]))));
+  int taken = 0;
+#pragma unroll 1
+  for (int o = 0; o < 2; o++) {   // one copy of the code: the warps of a block are at different places in it
+    mx::D3 n;
+    const int r = mxd::conic_root(h, o, x, p, n, replay ? (root >> (o + 1)) & 1 : -1);
+    if (r < 0) return false;
+    taken |= r << (o + 1);
+    const double pdn = mx::dot(p, n);
+    if (A.weighted) {
+      mx::F2 a, b;
+      mx::reflectivity_df(mx::split(fabs(pdn)), S.beta, S.delta, a, b);
+      num = mx::df_mul(num, a);
+      den = mx::df_mul(den, b);
+    }
+    p = mxd::reflected(p, n, pdn);
+    if (o == 0) {
+      if (!replay && T.use_struts && mx::cap_struts_block(T, h, x, p)) return false;
+      const double *M = h.mid, *c = h.mid_off;
+      p = mx::mat_mul(M, p);
+      x = mx::mk(fma(M[0], x.x, fma(M[1], x.y, fma(M[2], x.z, c[0]))), fma(M[3], x.x, fma(M[4], x.y, fma(M[5], x.z, c[1]))),
+                 fma(M[6], x.x, fma(M[7], x.y, fma(M[8], x.z, c[2]))));
+    }
   }
-  const int rh = mxd::conic_root(h, 1, x, p, n, replay ? ((root & mxd::RAY_ROOT_H) ? 1 : 0) : -1);
-  if (rh < 0) return false;
-  pdn = mx::dot(p, n);
-  if (A.weighted) {
-    mx::F2 n2, d2;
-    mx::reflectivity_df(mx::split(fabs(pdn)), S.beta, S.delta, n2, d2);
-    w = mx::df_join(mx::df_div(mx::df_mul(num, n2), mx::df_mul(den, d2))) * S.wscale;
-  } else
-    w = A.vig;
-  p = mxd::reflected(p, n, pdn);
+  w = A.weighted ? mx::df_join(mx::df_div(num, den)) * S.wscale : A.vig;
   p = mx::mat_mul(h.bwd[1], p);
   x = mx::mat_mul(h.bwd[1], x);
   x = x - mx::mk(h.to_osac[1][0], h.to_osac[1][1], h.to_osac[1][2]);
@@ -344,7 +349,7 @@ __device__ __forceinline__ bool ray_image(const FwdArgs &A, const MxTables &T, i
   const double t = -x.x * mx::rcp_fast(p.x);
   y = fma(t, p.y, x.y);
   z = fma(t, p.z, x.z);
-  root = (rp ? mxd::RAY_ROOT_P : 0) | (rh ? mxd::RAY_ROOT_H : 0);
+  root = taken;
   return true;
 }
 
@@ -356,10 +361,12 @@ __device__ __forceinline__ bool ray_image(const FwdArgs &A, const MxTables &T, i
 // the paraboloid, and traced where they stood they left 24 lanes of a warp
 // busy on average and the FP64 work of a whole ray to every warp.  With the
 // Newton intersections the FP64 instructions fall from 8.3 to 2.6 million per
-// 1e6 rays (48 % of the pipe; the splat's atomics and the aperture's and
-// weights' FP32 steps are the rest): 697 -> 315 us per 1e6 rays.  Three
-// blocks per SM (80 registers, 190 bytes spilled) rather than two of 110
-// without spills: a gradient step over 4e6 rays takes 3.05 instead of 3.38 ms.
+// 1e6 rays: 697 -> 315 us.  The warps of a block are at different places of the
+// kernel, so its length counts: with one copy of the code for both optics and
+// for all taps (a third of the issue slots waited for instructions before)
+// 255 us, FP64 pipe 58 % and issue 50 % busy.  Three blocks per SM (72
+// registers); two took 3.38 ms for a gradient step over 4e6 rays where three
+// took 3.05.
 template <bool SPLAT, bool MOMENTS>
 __global__ void __launch_bounds__(DBLOCK, FWD_BLOCKS) diff_forward_kernel(const __grid_constant__ FwdArgs args, const __grid_constant__ MxTables T,
                                                                uint64_t n, uint64_t seed, uint8_t *codes, int mode,
