@@ -2293,6 +2293,8 @@ constexpr int MX_FEF_MAX_GAUSS = MX_FEF_GAUSSIANS;
 // double from -6 on, so that a gaussian whose centre lies further than that
 // above zero, as nearly all do, has all its area there: two multiplications
 // instead of an error function and a division.
+// The error function of the others, out of line: the gaussians' loop is unrolled.
+MXD_COLD double fef_erf(float center, double s) { return erf((0 - (double) center) / s); }
 MXD void fef_areas(float amp, float center, float sigma, double &above, double &below) {
 #ifdef __CUDA_ARCH__
   if (sigma > 0.0f && center > 8.5f * sigma) {   // 6 sqrt(2) = 8.486
@@ -2303,9 +2305,24 @@ MXD void fef_areas(float amp, float center, float sigma, double &above, double &
 #endif
   const double s = (double) sigma * 1.4142135623730951;
   if (s == 0.0) { above = below = 0.0; return; }
-  const double e0 = erf((0 - (double) center) / s), w = 2.5066282746310002 * (double) sigma;
+  const double e0 = fef_erf(center, s), w = 2.5066282746310002 * (double) sigma;
   above = 0.5 * amp * (1.0 - e0) * w;
   below = 0.5 * amp * (e0 - -1.0) * w;
+}
+
+// sqrt(s^2 - 2 ln v): in double-float (within 2^-43) for v in 2^-40 .. 1 - 2^-40
+// and s below 2^10, an addition's worth of FP64 where the library's logarithm
+// and root take forty.
+MXD double fef_tail(float sf, double v) {
+#ifdef __CUDA_ARCH__
+  const unsigned long long f = unit_to_fixed(v);
+  if (f >> 24 && ~f >> 24 && fabsf(sf) < 1024.0f && lt_pos(v, 1.0)) {
+    const F2 l = df_neg_log(f), s2 = {__fmul_rn(sf, sf), __fmaf_rn(sf, sf, -__fmul_rn(sf, sf))};
+    return df_join(df_sqrt(df_add(s2, F2{2.0f * l.h, 2.0f * l.l})));
+  }
+#endif
+  const double s = (double) sf;
+  return sqrt(s * s - 2 * log(v));
 }
 
 // marx_apply_acis_rmf (acis_fef.c:910-1079) for a photon at chip pixel
@@ -2355,7 +2372,10 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
     }
     double above, below;
     fef_areas(amp[g], cen[g], sig[g], above, below);
-    if (below > above) tail[g] = above / below < 0.1;
+    if (dkey(below) > dkey(above)) {   // above / below < 0.1, by the float quotient where it is clear
+      const float ratio = d2f_trunc(above) / d2f_trunc(below);
+      tail[g] = fabsf(ratio - 0.1f) > 1e-4f ? ratio < 0.1f : above / below < 0.1;
+    }
     if (above >= 0) pos += above;
     else neg -= above;
     cum[g] = d2f_rn(pos);
@@ -2378,33 +2398,38 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
       const double r = rng.uniform();
       if (rng.overrun) return false;
       pha = -1.0;
-      bool drawn = false;
+      // the first gaussian whose cumulative area exceeds r, then one draw for
+      // whichever it is (lanes with different gaussians draw together)
+      bool drawn = false, from_tail = false;
+      float c = 0.0f, w = 0.0f;
 #pragma unroll
       for (int g = 0; g < MX_FEF_MAX_GAUSS; g++) {
         if (drawn || g >= ng || dkey(f2d(cum[g])) <= dkey(r)) continue;
         drawn = true;
-        if (!tail[g]) {
-          int count = 0;
-          do {
-            pha = f2d(cen[g]) + f2d(sig[g]) * rng.normal();
-            count++;
-          } while (dkey(pha) < 0 && (count < 100) && !rng.overrun);
-        } else {
-          const double s = (double) ((0.0f - cen[g]) / sig[g]);
-          double u, xx;
-          do {
-            u = rng.uniform();
-            double vv;
-            do { vv = rng.uniform(); } while (vv == 0.0 && !rng.overrun);
-            xx = sqrt(s * s - 2 * log(vv));
-          } while ((xx * u > s) && !rng.overrun);
-          pha = (double) cen[g] + xx * (double) sig[g];
-        }
+        from_tail = tail[g];
+        c = cen[g]; w = sig[g];
+      }
+      if (drawn && !from_tail) {
+        int count = 0;
+        do {
+          pha = f2d(c) + f2d(w) * rng.normal();
+          count++;
+        } while (dkey(pha) < 0 && (count < 100) && !rng.overrun);
+      } else if (drawn) {
+        const float sf = (0.0f - c) / w;
+        double u, xx;
+        do {
+          u = rng.uniform();
+          double vv;
+          do { vv = rng.uniform(); } while (is_zero(vv) && !rng.overrun);
+          xx = fef_tail(sf, vv);
+        } while (dkey(xx * u) > dkey(f2d(sf)) && !rng.overrun);
+        pha = f2d(c) + xx * f2d(w);
       }
       if (rng.overrun) return false;
       if (drawn && dkey(pha) >= 0) break;       // else: a new choice of gaussian
     }
-    if (neg == 0.0) break;
+    if (is_zero(neg)) break;
     double psum = 0.0, sum = 0.0;
 #pragma unroll
     for (int g = 0; g < MX_FEF_MAX_GAUSS; g++) {

@@ -157,11 +157,12 @@ __device__ void acis_response(const MxTables &T, const TraceIO &io, uint32_t i, 
 // A fifth or less of the photons reach a chip, and each costs several
 // hundred operations here, so each warp gathers the indices of pending
 // photons, 128 photons at a time, into a list of its own and works on 32 of
-// them together.  2e6 plain_scatter photons: 251 -> 177 us, with 3.4 -> 2.2
+// them together.  2e6 plain_scatter photons: 251 -> 150 us, with 3.4 -> 1.9
 // million FP64 instructions (75 % of the pipe: one error function per photon
 // is left, for a gaussian that reaches below zero, and the divisions by the
-// energy step and the area).  Three blocks of 80 registers per SM; two of 128
-// take 180 us, four of 64 186.
+// energy step and the area).  Three blocks of 80 registers per SM; with the
+// draws still inside the gaussians' loop two of 128 took 180 us, three 177,
+// four of 64 186.
 __global__ void __launch_bounds__(256, MX_FEF_BLOCKS) mx_acis_fef_kernel(MxTables T, TraceIO io, const uint64_t *seedp) {
   __shared__ uint32_t lists[8][160];   // up to 31 left over and 128 new
   const uint64_t seed = seedp ? *seedp : io.seed;
