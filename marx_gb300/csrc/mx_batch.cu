@@ -217,10 +217,12 @@ __global__ void __launch_bounds__(256) mx_generate_kernel(const __grid_constant_
 }
 
 // A phase's work tile: at most the batch's parameter, and small enough that a
-// warp claims four or more (a queue of 400,000 records in tiles of 256 leaves
-// a third of the warps without one).
+// warp claims 64 or more: tiles of 256 leave a third of the warps without one
+// in a queue of 400,000 records, and in a long one each warp far from its
+// neighbours' records.  With at least 4, 64, 256 claims a warp 3.7e7 photons
+// take 9.24, 8.96, 9.04 ms, 5.5e6 1.71, 1.57, 1.57.
 __device__ __forceinline__ uint32_t phase_tile(uint32_t count, int tile) {
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5), t = (count / (4u * warps)) & ~31u;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5), t = (count / (64u * warps)) & ~31u;
   return min((uint32_t) tile, max(t, 32u));
 }
 
@@ -314,11 +316,11 @@ struct TileRounds {
 // phase warps claim tiles of work from a counter, so uneven sources and
 // uneven survivor counts spread over every SM.  Every thread reaches every
 // barrier: the claim loops end for a whole warp at once and nothing
-// returns early.  Two resident blocks of 256 threads per SM (114 registers);
+// returns early.  Two resident blocks of 256 threads per SM (122 registers);
 // three (80 registers, 900 bytes of spilled loads) are as fast over the
 // sizes below.  The far-scattered photons kept for
 // later and tiles that follow the queue's length: 256 sources with 3.7e7
-// photons 10.1 -> 9.2 ms, with 2.2e6 1240 -> 777 us, with 1e6 688 -> 423 us.
+// photons 10.1 -> 9.0 ms, with 2.2e6 1240 -> 748 us, with 1e6 688 -> 429 us.
 __global__ void __launch_bounds__(256, 2) mx_batch_kernel(const __grid_constant__ MxTables T, const __grid_constant__ BatchIO b) {
   __shared__ uint32_t late_lists[8][64];
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
