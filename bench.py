@@ -9,7 +9,8 @@ axis, 8 arcsec Lissajous dither, mirror blur and WFold scattering, ACIS-I).
 
 value     photons/s with the batch resident in HBM (inputs > L2, so no flush);
           each step restores the batch's input directions and flags, then
-          traces it (from 65536 photons: the four wavefront kernels).
+          traces it (in the four wavefront kernels, from more photons than
+          the fused kernel holds at once).
 e2e       the same metric through mx_trace_host: pinned host buffers in,
           host buffers out, copies inside the timed region.
 roofline  the trace kernel against the measured FP64 FMA peak (it is FP64
@@ -49,7 +50,7 @@ METRIC = "photons/s HRMA+grating+ACIS trace"
 # DRAM bytes the four wavefront kernels move per photon of plain_scatter
 # (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of 2e6
 # photons); the traffic of a step grows with its photon count.
-TRAFFIC_BYTES_PER_PHOTON = 557.0
+TRAFFIC_BYTES_PER_PHOTON = 519.0
 
 
 def parse():
@@ -477,8 +478,8 @@ def bench_events(a):
     eng.close()
     return {"workload": "1e7 ACIS-I events, EDSER, INTERNAL dither, frames of ~30 events, device-resident",
             "events": n, "ms": ms, "events_per_s": n / (ms * 1e-3), "gpu_launches_per_step": launches,
-            "roofline": {"bound": "fp64", "note": "sin, cos, acos, asin, atan and about 26 divisions per event; "
-                                                  "ncu: FP64 pipe 87% busy",
+            "roofline": {"bound": "fp64", "note": "the chain DETX/DETY round through; the sky angles in "
+                                                  "double-float; ncu: FP64 pipe 77% busy",
                          "hbm": {"achieved": gbs, "peak": hbm_peak, "unit": "GB/s", "frac": gbs / hbm_peak,
                                  "bytes_per_event": EVENT_BYTES}},
             "cpu_baseline": {"value": cpu_rate, "unit": "events/s", "cores": 1, "kind": "port",
@@ -739,6 +740,8 @@ def main():
                      "traffic_note": "bytes per step of the four wavefront kernels, scaled from an ncu capture "
                                      "of 2e6 photons",
                      "algorithmic_flops_per_photon": fpp,
+                     "note": "operations the restatement does in FP64; a part of them runs in double-float on the "
+                             "FP32 pipe here, so frac may exceed 1 (ncu: FP64 pipe 28-59% busy per kernel)",
                      "peak_source": "measured live: mx_probe_fp64 DFMA kernel (MEASURED_PEAKS.json has no FP64 figure)",
                      "hbm": {"achieved_gbs": hbm_achieved, "peak_gbs": hbm_peak, "frac": hbm_achieved / hbm_peak,
                              "bytes_per_photon": bytes_per_photon}},

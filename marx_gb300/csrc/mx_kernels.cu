@@ -233,19 +233,22 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 //   T  52 128 128  57      66 165 167 108
 //   B 222 222 222 113     180 188 181 147
 //   C 116 116 116  81      89  89  88  79
-// 1e7 photons 5.76 5.37 4.70 3.83 ms; 1e6 on axis 416 368 340 284 us.  A is
-// bound by the issue of FP32 and integer instructions now (61 %), C by the
-// FP64 pipe (60 %), T and B by latency (FP64 46 and 51 %, issue 43 and 31 %;
-// B also waits for instructions), which is why A, T and B are compiled for
-// three resident blocks (80 registers, 100 bytes of spills in B) and gain
-// 8-11 % over two, while C loses 6 % and D is not bound by either.
+// 1e7 photons 5.76 5.37 4.70 3.83 ms; 1e6 on axis 416 368 340 284 us.  With
+// the far-scattered photons gathered, leaner double-float steps and index
+// tables for the lookups: A 87, T 79, B 110, C 66 us, 1e7 photons 3.16 ms, 1e6
+// on axis 263 us.  A is bound by the issue of FP32 and integer instructions
+// (61 %), C by the FP64 pipe (59 %), T and B by latency (FP64 55 and 57 %,
+// issue 41 and 32 %; B also waits for instructions), which is why A, T and B
+// are compiled for three resident blocks (80 registers, 100 bytes of spills in
+// B) and gain 8-11 % over two, while C loses 6 % and D is not bound by either;
+// a fourth block changes none of them by more than 1.5 %.
 // With a grating: the Rowland torus from a float iteration and two steps on
 // the quartic's double value, the order choice decided in float away from
 // its thresholds, and one facet basis for the LETG's primary and four
 // supports, whose direction stays in its components: per 1e6 photons C
 // 114 -> 95 us (HETG) and D 219 -> 190 us (LETG and HRC-S, 3.4e6 -> 2.0e6
-// FP64 instructions); HETG 2e7 7.73 -> 7.08 ms, LETG + HRC-S 4e6 2.35 ->
-// 1.88 ms.
+// FP64 instructions), and 84 us with the HRC's plates, pulse height and blur
+// off the FP64 pipe; HETG 2e7 7.73 -> 6.92 ms, LETG + HRC-S 4e6 2.35 -> 1.62.
 
 // A phase's blocks start as those of the phase before it end, stage their
 // tables meanwhile and read its queues when all of it has completed
@@ -651,7 +654,7 @@ cudaError_t launch_compact(const uint32_t *flags, uint32_t n, uint32_t *idx_out,
 // 5 the Fresnel numerator and denominator in double-float and in double,
 // 6 (double) (unsigned) x on the integer pipe, 7 sqrt_fast, 8 quarter_of,
 // 9 df_join of split, 10 df_turn_sincos less an eighth (y[2i], y[2i+1] = sin,
-// cos of 2 pi x - pi/4, 0 <= x < 1).
+// cos of 2 pi x - pi/4, 0 <= x < 1), 12 df_expm1 (11: mx_find_check).
 __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, double *y, size_t n) {
   const size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
   if (i >= n) return;
