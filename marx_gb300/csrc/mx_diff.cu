@@ -83,11 +83,12 @@ struct FwdArgs {
 struct ShellTangents {
   mxd::Turn front[3], fwd[9];    // of the paraboloid
   mxd::Turn mid[9], off[3];
-  mxd::Turn bwd[9];              // of the hyperboloid
+  mxd::Turn bwd[9], back[3];     // of the hyperboloid: bwd[1] and -to_osac[1] (its decenters taken apart)
   mxd::Dual p1[3];               // fwd p0, made on the device
   double corr;                   // effective-area correction per reflection
-  double pad[2];                 // 624 bytes: lanes that load one field of different shells do not conflict
+  double pad[4];                 // 688 bytes: lanes that load one field of different shells do not conflict
 };
+static_assert(sizeof(ShellTangents) == 688, "four shells on distinct bank offsets");
 
 struct AdjArgs {
   FwdArgs f;
@@ -547,46 +548,40 @@ __device__ __forceinline__ bool ray_tangents(const AdjArgs &A, int si, double ry
   const MxShellDev &h = A.f.sh[si].h;
   mxd::V3 x = {mxd::turned(S.front[0], S.fwd[1], S.fwd[2], ry, rz), mxd::turned(S.front[1], S.fwd[4], S.fwd[5], ry, rz),
                mxd::turned(S.front[2], S.fwd[7], S.fwd[8], ry, rz)};
-  mxd::V3 p = {S.p1[0], S.p1[1], S.p1[2]}, n;
-  if (!mxd::conic_tangents(h, 0, x, p, n, (root & mxd::RAY_ROOT_P) ? 1 : 0)) return false;
-  mxd::Dual pdn = mxd::dotp(p, n);
-  mx::F2 w1{1.0f, 0.0f}, w2{1.0f, 0.0f}, corr{1.0f, 0.0f};
-  float s1 = 0.0f, s2 = 0.0f;
-  if (A.f.weighted) {
-    corr = mx::split(S.corr);
-    mx::F2 r;
-    mxd::fresnel_slope(A.fr, mx::split(fabs(pdn.v)), r, s1);
-    w1 = mx::df_mul(r, corr);
-    s1 = mxd::tof(S.corr) * (mx::neg_bit(pdn.v) ? -s1 : s1);
-  }
+  mxd::V3 p = {S.p1[0], S.p1[1], S.p1[2]};
+  mx::F2 w1{1.0f, 0.0f}, corr{1.0f, 0.0f};
+  if (A.f.weighted) corr = mx::split(S.corr);
+#pragma unroll 1
+  for (int o = 0; o < 2; o++) {   // one copy of the code, as in ray_image
+    mxd::V3 n;
+    if (!mxd::conic_tangents(h, o, x, p, n, (root >> (o + 1)) & 1)) return false;
+    const mxd::Dual pdn = mxd::dotp(p, n);
+    mx::F2 wo{1.0f, 0.0f};
+    float slope = 0.0f;
+    if (A.f.weighted) {
+      mx::F2 r;
+      mxd::fresnel_slope(A.fr, mx::split(fabs(pdn.v)), r, slope);
+      wo = mx::df_mul(r, corr);
+      slope = mxd::tof(S.corr) * (mx::neg_bit(pdn.v) ? -slope : slope);
+    }
+    if (o == 0) {
+      w1 = wo;
 #pragma unroll
-  for (int k = 0; k < mxd::NT; k++) wd[k] = s1 * pdn.d[k];
-  {
+      for (int k = 0; k < mxd::NT; k++) wd[k] = slope * pdn.d[k];
+    } else {
+      const float w1f = mxd::tof(w1), w2f = mxd::tof(wo);
+#pragma unroll
+      for (int k = 0; k < mxd::NT; k++) wd[k] = w1f * (slope * pdn.d[k]) + w2f * wd[k];
+      w = mx::df_mul(w1, wo).h;
+    }
     const mxd::Dual q = 2.0 * pdn;
     p = {p.x - q * n.x, p.y - q * n.y, p.z - q * n.z};
+    // into the hyperboloid's frame, then back to the MARX frame
+    const mxd::Turn *m = o ? S.bwd : S.mid, *c = o ? S.back : S.off;
+    p = mxd::matv(m, p);
+    x = mxd::matv(m, x);
+    x = {x.x + c[0], x.y + c[1], x.z + c[2]};
   }
-  p = mxd::matv(S.mid, p);
-  x = mxd::matv(S.mid, x);
-  x = {x.x + S.off[0], x.y + S.off[1], x.z + S.off[2]};
-  if (!mxd::conic_tangents(h, 1, x, p, n, (root & mxd::RAY_ROOT_H) ? 1 : 0)) return false;
-  pdn = mxd::dotp(p, n);
-  if (A.f.weighted) {
-    mx::F2 r;
-    mxd::fresnel_slope(A.fr, mx::split(fabs(pdn.v)), r, s2);
-    w2 = mx::df_mul(r, corr);
-    s2 = mxd::tof(S.corr) * (mx::neg_bit(pdn.v) ? -s2 : s2);
-  }
-  const float w1f = mxd::tof(w1), w2f = mxd::tof(w2);
-#pragma unroll
-  for (int k = 0; k < mxd::NT; k++) wd[k] = w1f * (s2 * pdn.d[k]) + w2f * wd[k];
-  w = mx::df_mul(w1, w2).h;
-  {
-    const mxd::Dual q = 2.0 * pdn;
-    p = {p.x - q * n.x, p.y - q * n.y, p.z - q * n.z};
-  }
-  p = mxd::matv(S.bwd, p);
-  x = mxd::matv(S.bwd, x);
-  x = {x.x - h.to_osac[1][0], x.y - h.to_osac[1][1], x.z - h.to_osac[1][2]};
   const mxd::Dual t = (0.0 - x.x) * mxd::drcp(p.x);
   y = x.y + t * p.y;
   z = x.z + t * p.z;
@@ -596,13 +591,15 @@ __device__ __forceinline__ bool ray_tangents(const AdjArgs &A, int si, double ry
 // part[block][NP] = sum over the block's rays of dl/dimage . d(image)/dtheta
 // (before the 1/n_rays factor).
 //
-// Per 1e6 rays: 500 -> 305 us (FP64 pipe 57 % busy with 3.1 instead of 5.9
-// million instructions; the rest are the tangents' FP32 steps and the window
-// sums).  What went: the library's roots and divisions, the decenters'
-// tangents, which are constants, the Fresnel chain in six directions (one
-// slope, its values in double-float), the root that is not followed.  Two
-// blocks per SM (128 registers): three of 80 spill and take 2.40 instead of
-// 2.35 ms for a gradient step over 4e6 rays.
+// Per 1e6 rays: 500 -> 305 us with 3.1 instead of 5.9 million FP64 instructions
+// (the rest are the tangents' FP32 steps and the window sums).  What went: the
+// library's roots and divisions, the decenters' tangents, which are constants,
+// the Fresnel chain in six directions (one slope, its values in double-float),
+// the root that is not followed.  305 -> 279 us with one copy of the code for
+// both optics and for the window's rows (a tenth of the issue slots waited for
+// instructions): FP64 pipe 68 %, issue 42 %.  Two blocks per SM (128
+// registers): three of 80 spill and took 2.40 instead of 2.35 ms for a gradient
+// step over 4e6 rays.
 __global__ void __launch_bounds__(DBLOCK, 2) diff_adjoint_kernel(const __grid_constant__ AdjArgs args, uint64_t n,
                                                                uint64_t seed, const uint8_t *codes,
                                                                const double *dl, double *part) {
@@ -686,7 +683,7 @@ __global__ void __launch_bounds__(DBLOCK, 2) diff_adjoint_kernel(const __grid_co
           const bool inside = ic - mxd::HALF >= g.wx0 && ic + mxd::HALF < g.wx0 + g.wnx &&
                               jc - mxd::HALF >= g.wy0 && jc + mxd::HALF < g.wy0 + g.wny;
           const float *base_row = rw + (jc - mxd::HALF - g.wy0) * (WIN + 1) + (ic - mxd::HALF - g.wx0);
-#pragma unroll
+#pragma unroll 1
           for (int a = 0; a < mxd::TAPS; a++) {
             float t = 0.f, td = 0.f;
             if (inside) {
@@ -879,6 +876,7 @@ int fill_adj(mx_diff *d, const double *theta, AdjArgs &A) {
     ShellTangents &D = A.d[s];
     for (int j = 0; j < 3; j++) { D.front[j] = turn(opt[s][0].ff[j]); D.off[j] = turn(mid[s].c[j]); }
     for (int j = 0; j < 9; j++) { D.fwd[j] = turn(opt[s][0].fwd[j]); D.mid[j] = turn(mid[s].m[j]); D.bwd[j] = turn(opt[s][1].bwd[j]); }
+    for (int j = 0; j < 3; j++) D.back[j] = mxd::Turn{-opt[s][1].to[j].v, {0.f, 0.f}};
     D.corr = d->corr[s];
   }
   for (int k = 0; k < 3; k++) A.p0[k] = mxd::Dual{p0[k].v, {0.f, 0.f, p0[k].d[4], p0[k].d[5]}};
