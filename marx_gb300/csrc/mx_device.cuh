@@ -71,6 +71,7 @@ MXD long long dkey(double x) {
   return (long long) ((long long) b < 0 ? 0x8000000000000000ull - b : b);
 }
 MXD bool is_zero(double x) { return (dbits(x) << 1) == 0; }   // x = +0 or -0
+MXD bool is_pos(double x) { return dbits(x) - 1ull < 0x7ff0000000000000ull; }   // x > 0 (false for NaN, of either sign)
 // -x when neg, else x: a sign-bit flip on the integer pipe (a negation that
 // is not folded into the next operation issues as a DADD)
 MXD double flip_sign(double x, bool neg) {
@@ -2364,7 +2365,7 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
     const float a1 = g1[3 * g], c1 = g1[3 * g + 1], s1 = g1[3 * g + 2];
     cen[g] = d2f_rn(f2d(c0) + t * f2d(c1 - c0));
     double v = f2d(s0) + t * f2d(s1 - s0);
-    if (dkey(v) > 0) {
+    if (is_pos(v)) {   // a NaN width leaves the gaussian out, as zero does
       sig[g] = d2f_rn(v);
       v = f2d(a0) + t * f2d(a1 - a0);
       if (dkey(v) < 0 && ((a1 > 0.0f) || (a0 > 0.0f))) v = 0.0;
@@ -2373,8 +2374,9 @@ MXD bool acis_fef(const MxTables &T, int ccd, float x, float y, double energy, R
     double above, below;
     fef_areas(amp[g], cen[g], sig[g], above, below);
     if (dkey(below) > dkey(above)) {   // above / below < 0.1, by the float quotient where it is clear
+      // (areas outside a float's range make it 0, infinite or NaN)
       const float ratio = d2f_trunc(above) / d2f_trunc(below);
-      tail[g] = fabsf(ratio - 0.1f) > 1e-4f ? ratio < 0.1f : above / below < 0.1;
+      tail[g] = ratio != 0.0f && fabsf(ratio - 0.1f) > 1e-4f ? ratio < 0.1f : above / below < 0.1;
     }
     if (above >= 0) pos += above;
     else neg -= above;
