@@ -192,7 +192,7 @@ __device__ __forceinline__ void splat_warp(const ImageGeom &g, const SplatWindow
                                            int lane) {
   int ic = 0, jc = 0;
   float fu = 0.f, fv = 0.f;
-  if (valid) valid = mx::dkey(w) > 0 && splat_origin(g, y, z, ic, jc, fu, fv);
+  if (valid) valid = mx::is_pos(w) && splat_origin(g, y, z, ic, jc, fu, fv);
   const uint32_t wq = valid ? weight_fixed(w) : 0u;
   const unsigned vm = __ballot_sync(0xffffffffu, valid);
 #pragma unroll 1
@@ -342,7 +342,7 @@ __device__ __forceinline__ bool ray_image(const FwdArgs &A, const MxTables &T, i
                  fma(M[6], x.x, fma(M[7], x.y, fma(M[8], x.z, c[2]))));
     }
   }
-  w = A.weighted ? mx::df_join(mx::df_div(num, den)) * S.wscale : A.vig;
+  w = A.weighted ? mx::f2_double(mx::df_div(num, den)) * S.wscale : A.vig;   // NaN stays NaN, which df_join does not keep
   p = mx::mat_mul(h.bwd[1], p);
   x = mx::mat_mul(h.bwd[1], x);
   x = x - mx::mk(h.to_osac[1][0], h.to_osac[1][1], h.to_osac[1][2]);
