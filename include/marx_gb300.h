@@ -443,7 +443,8 @@ typedef struct mx_batch mx_batch;
 typedef struct mx_batch_params {
   int32_t block;            /* threads per block: 32 to 256 in whole warps */
   int32_t tile;             /* photons a warp claims per visit of the work counter (multiple of 32) */
-  int32_t blocks_per_sm;    /* resident blocks per SM (<= the occupancy limit) */
+  int32_t blocks_per_sm;    /* resident blocks per SM: up to 24 warps' worth and what shared memory holds
+                               of the sources; a launch takes as many of them as fit */
   int32_t reserved;
 } mx_batch_params;
 

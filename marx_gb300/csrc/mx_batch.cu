@@ -47,6 +47,7 @@ struct BatchIO {
   const MxSourceFine *fine;
   const uint32_t *start;        // nsrc + 1 offsets
   int32_t nsrc, tile;
+  int32_t stage_starts, pad;    // whether the offsets are copied to shared memory
   MxRec *q1, *q2;
   unsigned int *ctr;            // [0] q1 entries [1] q2 entries [2..4] work counters of phases A, B, C
                                 // [5] q1 entries of phase B (q1 reused) [6] work counter of phase T
@@ -268,10 +269,11 @@ __device__ __forceinline__ void batch_finish(const MxTables &T, const MxChipDev 
 // MX_BATCH_LATE groups per warp, keeps them in line: the warp's last group of
 // late photons would cost it more.
 #define MX_BATCH_LATE 3
+constexpr int LATE_LIST = 64;
 struct TileRounds {
   unsigned int *ctr;
   uint32_t count, tile, j, end, n_late;
-  uint32_t *late;               // this warp's list, 64 entries
+  uint32_t *late;               // this warp's list, LATE_LIST entries
   bool use, done;
   __device__ __forceinline__ TileRounds(unsigned int *c, uint32_t n, int t, uint32_t *list)
       : ctr(c), count(n), tile(phase_tile(n, t)), j(0), end(0), n_late(0), late(list), done(false) {
@@ -316,20 +318,21 @@ struct TileRounds {
 // phase warps claim tiles of work from a counter, so uneven sources and
 // uneven survivor counts spread over every SM.  Every thread reaches every
 // barrier: the claim loops end for a whole warp at once and nothing
-// returns early.  Two resident blocks of 256 threads per SM (122 registers);
-// three (80 registers, 900 bytes of spilled loads) are as fast over the
-// sizes below.  The far-scattered photons kept for
-// later and tiles that follow the queue's length: 256 sources with 3.7e7
-// photons 10.1 -> 9.0 ms, with 2.2e6 1240 -> 748 us, with 1e6 688 -> 429 us.
+// returns early.  Two resident blocks of 256 threads per SM (122 registers):
+// three (80 registers, 900 bytes of spilled loads) take 8.81 ms instead of
+// 8.91 for 3.7e7 photons, but 183 us instead of 162 for 2e5.  The far-scattered
+// photons kept for later and tiles that follow the queue's length: 256 sources
+// with 3.7e7 photons 10.1 -> 9.0 ms, with 2.2e6 1240 -> 748 us, with 1e6 688 -> 429 us.
 __global__ void __launch_bounds__(256, 2) mx_batch_kernel(const __grid_constant__ MxTables T, const __grid_constant__ BatchIO b) {
-  __shared__ uint32_t late_lists[8][64];
   MxShellDev *sh; MxGratingDev *gr; MxChipDev *ch; float *optc; double *slope;
   stage_tables(T, sh, gr, ch, optc, slope);
   extern __shared__ __align__(16) unsigned char smem[];
   MxSourceDev *ssrc = (MxSourceDev *) (smem + tables_shared_bytes(T));
-  uint32_t *sstart = (uint32_t *) (ssrc + b.nsrc);
+  uint32_t *late = (uint32_t *) (ssrc + b.nsrc) + (threadIdx.x >> 5) * LATE_LIST;   // this warp's list
+  uint32_t *staged = (uint32_t *) (ssrc + b.nsrc) + (blockDim.x >> 5) * LATE_LIST;
+  const uint32_t *sstart = b.stage_starts ? staged : b.start;
   copy_words((uint32_t *) ssrc, (const uint32_t *) b.src, (size_t) b.nsrc * sizeof(MxSourceDev) / 4);
-  copy_words(sstart, b.start, (size_t) b.nsrc + 1);
+  if (b.stage_starts) copy_words(staged, b.start, (size_t) b.nsrc + 1);
   __syncthreads();
 
   cg::grid_group grid = cg::this_grid();
@@ -405,7 +408,6 @@ __global__ void __launch_bounds__(256, 2) mx_batch_kernel(const __grid_constant_
 
   // Phase B: the rest of the paraboloid reflection, hyperboloid
   // intersection and reflectivity test (q1 is free again).
-  uint32_t *late = late_lists[threadIdx.x >> 5];
   uint32_t k;
   bool have, may_defer;
   for (TileRounds rounds(&b.ctr[3], __ldcg(&b.ctr[1]), b.tile, late); rounds.next(k, have, may_defer);) {
@@ -506,9 +508,33 @@ struct mx_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t done = nullptr;
-  size_t shared_bytes = 0;
+  bool stage_starts = true;
   std::string key;
 };
+
+// Dynamic shared memory of a launch: the tables, the sources, a list for
+// each warp and, where they fit, the sources' offsets (1238 sources and more
+// would not; the kernel then reads them from global memory).
+static size_t starts_bytes(const mx_batch *b) { return align16((b->dsrc.size() + 1) * sizeof(uint32_t)); }
+static size_t batch_shared_bytes(const mx_batch *b, int block) {
+  return tables_shared_bytes(b->ctx->T) + align16(b->dsrc.size() * sizeof(MxSourceDev)) +
+         (size_t) (block / 32) * LATE_LIST * sizeof(uint32_t) + (b->stage_starts ? starts_bytes(b) : 0);
+}
+// The most blocks per SM that a launch shape may ask for: 24 warps, and what
+// shared memory holds with 7024 bytes of tables, the sources and their
+// offsets; 0 if not one block fits.  The limit stays there whatever registers
+// the kernel is compiled for and however its tables and lists grow, so that a
+// program's saved shapes stay valid; a launch takes as many of the blocks as
+// fit (16 warps: see the kernel).
+static int shape_limit(const mx_batch *b, int block) {
+  int sm = 0, optin = 0, reserved = 0;
+  cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->ctx->device);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->ctx->device);
+  cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, b->ctx->device);
+  const size_t bytes = 7024 + align16(b->dsrc.size() * sizeof(MxSourceDev)) + starts_bytes(b);
+  if (bytes > (size_t) optin) return 0;
+  return std::min(24 / (block / 32), (int) ((size_t) sm / ((bytes + reserved + 127) & ~(size_t) 127)));
+}
 
 static mx_photons batch_view(mx_batch *b) {
   mx_photons d;
@@ -522,9 +548,13 @@ static mx_photons batch_view(mx_batch *b) {
 }
 
 static int batch_max_blocks(mx_batch *b, int block, int *blocks) {
-  cudaError_t e = cudaFuncSetAttribute(mx_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b->shared_bytes);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, mx_batch_kernel, block, b->shared_bytes);
-  if (e != cudaSuccess) return mx_cuda_fail(b->ctx, e, "batch occupancy");
+  const size_t shared = batch_shared_bytes(b, block);
+  cudaError_t e = cudaFuncSetAttribute(mx_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shared);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, mx_batch_kernel, block, shared);
+  if (e != cudaSuccess) {
+    (void) cudaGetLastError();   // not the next launch's error
+    return mx_cuda_fail(b->ctx, e, "batch occupancy");
+  }
   return MX_OK;
 }
 
@@ -559,6 +589,7 @@ static int build_graph(mx_batch *b) {
   io.start = (const uint32_t *) (io.fine + b->dsrc.size());
   io.nsrc = (int32_t) b->dsrc.size();
   io.tile = b->params.tile;
+  io.stage_starts = b->stage_starts;
   size_t qbytes = (size_t) b->total * sizeof(MxRec);
   io.q1 = (MxRec *) b->queues.ptr;
   io.q2 = (MxRec *) ((char *) b->queues.ptr + qbytes);
@@ -578,7 +609,7 @@ static int build_graph(mx_batch *b) {
     memset(&lc, 0, sizeof(lc));
     lc.gridDim = dim3(c->num_sms * per_sm);
     lc.blockDim = dim3(b->params.block);
-    lc.dynamicSmemBytes = b->shared_bytes;
+    lc.dynamicSmemBytes = batch_shared_bytes(b, b->params.block);
     lc.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -811,7 +842,6 @@ mx_batch *mx_batch_create(mx_context *c, const mx_source *sources, int nsrc) {
   if (tot >= (1ull << 31)) { g_create_err = "mx_batch_create: more than 2^31 photons"; delete b; return nullptr; }
   if (c->cfg.acis_exposure_time <= 0) { g_create_err = "mx_batch_create: ACIS_Exposure_Time must be > 0"; delete b; return nullptr; }
   b->total = tot;
-  b->shared_bytes = tables_shared_bytes(c->T) + align16((size_t) nsrc * sizeof(MxSourceDev)) + align16((size_t) (nsrc + 1) * 4);
   const size_t elem[12] = {8, 24, 24, 8, 4, 4, 1, 1, 1, 4, 4, 12};
   cudaError_t e = b->d_src.ensure(b->dsrc.size() * (sizeof(MxSourceDev) + sizeof(MxSourceFine)) + b->start.size() * 4);
   for (int k = 0; k < 12 && e == cudaSuccess; k++) e = b->cols[k].ensure(std::max<size_t>(16, tot * elem[k]));
@@ -835,8 +865,10 @@ mx_batch *mx_batch_create(mx_context *c, const mx_source *sources, int nsrc) {
   }
   *b->h_seed = 0;
   b->key = batch_key(b);
-  int maxb = 0;
-  if (batch_max_blocks(b, 256, &maxb) != MX_OK || maxb < 1) {
+  int maxb = 0, optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  b->stage_starts = batch_shared_bytes(b, 256) <= (size_t) optin;
+  if (shape_limit(b, 256) < 1 || batch_max_blocks(b, 256, &maxb) != MX_OK || maxb < 1) {
     g_create_err = "mx_batch_create: the batch kernel cannot be resident (" + c->err + ")";
     mx_batch_destroy(b);
     return nullptr;
@@ -872,10 +904,7 @@ int mx_batch_set_params(mx_batch *b, const mx_batch_params *p) {
       p->blocks_per_sm < 1)
     return mx_fail(b->ctx, MX_EINVAL, "mx_batch_set_params: block must be 32 to 256 threads in whole warps, "
                                       "tile a positive multiple of 32");
-  int maxb = 0;
-  int r = batch_max_blocks(b, p->block, &maxb);
-  if (r) return r;
-  if (p->blocks_per_sm > maxb) return mx_fail(b->ctx, MX_ERANGE, "mx_batch_set_params: more blocks per SM than fit");
+  if (p->blocks_per_sm > shape_limit(b, p->block)) return mx_fail(b->ctx, MX_ERANGE, "mx_batch_set_params: more blocks per SM than fit");
   b->params = *p;
   drop_graph(b);
   return MX_OK;
