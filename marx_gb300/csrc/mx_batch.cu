@@ -676,6 +676,11 @@ static bool source_dev(const mx_source &q, MxSourceDev &S, std::vector<double> &
   if (l != 0.0) { pn[0] = pn[0] / l; pn[1] = pn[1] / l; pn[2] = pn[2] / l; }
   for (int k = 0; k < 3; k++) S.pn[k] = pn[k];
   S.kind = q.kind;
+  // the photons of an extended source are p and a change perpendicular to it:
+  // unit vectors if p is one (a p off by rounding alone stays as it is)
+  const double len = src_len(q.p);
+  if ((q.kind == MX_SOURCE_GAUSS || q.kind == MX_SOURCE_BETA || q.kind == MX_SOURCE_DISK) && fabs(len - 1.0) > 1e-15)
+    for (int k = 0; k < 3; k++) S.p[k] = q.p[k] / len;
   if (q.spectrum_n > 0) {
     if (!q.spectrum_energy || !q.spectrum_flux) { err = "FILE spectrum arrays missing"; return false; }
     const unsigned n = q.spectrum_n;
