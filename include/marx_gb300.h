@@ -284,7 +284,13 @@ const char *mx_last_error(const mx_context *ctx);  /* ctx may be NULL */
  * more traced with Philox draws by the wavefront kernels runs as two halves
  * at once on two streams of the context, forked from stream and joined back
  * into it, so that work queued on stream after the call starts after the
- * whole trace. */
+ * whole trace.
+ *
+ * The calls of one context (made from one thread at a time) may come on
+ * different streams: those that use the same buffers of the context, the
+ * survivor queues here and the frame scan of mx_event_coords, take turns on the
+ * GPU.  A call captured into a CUDA graph is not part of that order: let its
+ * replays overlap no other work of the context. */
 int mx_trace(mx_context *ctx, const mx_photons *ph, uint32_t stages,
              const mx_variates *var, uint64_t seed, void *stream);
 
@@ -294,9 +300,9 @@ int mx_trace(mx_context *ctx, const mx_photons *ph, uint32_t stages,
  * acceptance, FEF pulse height and PI, frame-transfer streak). */
 
 /* Kernel organisation for mx_trace / mx_trace_host.  FUSED runs every stage
- * of a photon in one kernel; WAVEFRONT splits the mirror at its two conic
- * intersections into three kernels with survivor queues between them (the
- * photons lost on the way then stop occupying SIMT lanes) and needs
+ * of a photon in one kernel; WAVEFRONT splits the trace where photons are
+ * lost into four kernels, five with a grating, with survivor queues between
+ * them (the photons lost on the way then stop occupying SIMT lanes) and needs
  * 2 x 128 bytes of device scratch per photon; AUTO picks the wavefront from
  * MX_WAVEFRONT_MIN_PHOTONS photons up, but not before a list is longer than
  * the fused kernel holds at once.  Both give the same per-photon results. */

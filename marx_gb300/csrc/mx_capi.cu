@@ -228,6 +228,8 @@ void mx_destroy(mx_context *c) {
   c->ev_tab.release();
   c->ev_scan.release();
   c->ev_io.release();
+  c->wave_turn.release();
+  c->ev_turn.release();
   for (int k = 0; k < MX_PIPE_STREAMS; k++) {
     c->pipe_wave[k].release();
     if (c->pipe[k]) cudaStreamDestroy(c->pipe[k]);
@@ -408,7 +410,10 @@ int mx_trace_queues(mx_context *c, const MxTables &T, const mx_photons *ph, uint
     w.q1 = (MxRec *) queues.ptr;
     w.q2 = (MxRec *) ((char *) queues.ptr + qbytes);
     w.counts = (unsigned int *) ((char *) queues.ptr + 2 * qbytes);
-    e = launch_wavefront(T, io, w, c->num_sms, c->wave_blocks, (int) c->shared_bytes, st);
+    const bool shared = &queues == &c->wave;   // a pipeline stream's queues serve that stream alone
+    e = shared ? c->wave_turn.before(st) : cudaSuccess;
+    if (e == cudaSuccess) e = launch_wavefront(T, io, w, c->num_sms, c->wave_blocks, (int) c->shared_bytes, st);
+    if (e == cudaSuccess && shared) e = c->wave_turn.after(st);
     c->launches += wave_kernels(T, stages);
   } else {
     e = launch_trace(T, io, c->num_sms * c->trace_blocks[slots ? 0 : 1], (int) c->shared_bytes, slots != 0, st);

@@ -23,6 +23,28 @@ struct DevBuf {
   void release() { if (ptr) cudaFree(ptr); ptr = nullptr; bytes = 0; }
 };
 
+// Orders the calls that share a buffer of the context, whatever streams they
+// come on: between before and after, work on st uses the buffer alone.  A
+// captured call is not part of the order (its work runs at the replays).
+struct BufTurn {
+  cudaEvent_t last = nullptr;   // the latest use
+  static bool captured(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) (void) cudaGetLastError();
+    return s != cudaStreamCaptureStatusNone;
+  }
+  cudaError_t before(cudaStream_t st) {
+    return last && !captured(st) ? cudaStreamWaitEvent(st, last, 0) : cudaSuccess;
+  }
+  cudaError_t after(cudaStream_t st) {
+    if (captured(st)) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (!last) e = cudaEventCreateWithFlags(&last, cudaEventDisableTiming);
+    return e == cudaSuccess ? cudaEventRecord(last, st) : e;
+  }
+  void release() { if (last) cudaEventDestroy(last); last = nullptr; }
+};
+
 #define MX_PIPE_STREAMS 2
 #define MX_PIPE_CHUNKS 16           // nominal chunks: about 2^19 photons each, 4 to 16
 #define MX_PIPE_MAX_CHUNKS (MX_PIPE_CHUNKS + 4)   // with the shorter chunks at both ends
@@ -44,6 +66,7 @@ struct mx_context {
   DevBuf io[22];           // staging for mx_trace_host: 19 columns, U, N
   DevBuf scan;             // compaction block counts
   DevBuf wave;             // wavefront record queues
+  BufTurn wave_turn;
   DevBuf spec;             // FILE spectrum of the last mx_generate_source call
   int wave_blocks[5] = {};     // resident blocks per SM of the wavefront kernels a, t, b, c, d
   int mode = MX_MODE_AUTO;
@@ -53,6 +76,7 @@ struct mx_context {
   bool events_ready = false;
   alignas(16) char ev_geom[2048];   // the launch copy of the facet geometry
   DevBuf ev_tab, ev_scan, ev_io;
+  BufTurn ev_turn;         // of ev_scan
   unsigned long long *d_event_bad = nullptr;
   // mx_trace_host on large lists: chunks traced on MX_PIPE_STREAMS streams,
   // copied in on pipe_in and out on pipe_out; pipe_ev[0][j] marks chunk j

@@ -850,6 +850,7 @@ static int launch_events(mx_context *c, const mx_event_params *params, const mx_
   uint32_t *tiles = nullptr;
   if (a.frames) {
     cudaError_t e = c->ev_scan.ensure((size_t) ntiles * sizeof(uint32_t));
+    if (e == cudaSuccess) e = c->ev_turn.before(st);
     if (e != cudaSuccess) return mx_cuda_fail(c, e, "allocating the frame scan");
     tiles = (uint32_t *) c->ev_scan.ptr;
     mx_event_frame_tiles<<<grid, EV_BLOCK, 0, st>>>(a, ntiles, tiles);
@@ -859,6 +860,7 @@ static int launch_events(mx_context *c, const mx_event_params *params, const mx_
   mx_event_kernel<<<grid, EV_BLOCK, 0, st>>>(a, G, ntiles, tiles);
   c->launches += 1;
   cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && a.frames) e = c->ev_turn.after(st);
   if (e != cudaSuccess) return mx_cuda_fail(c, e, "launching the event pass");
   return MX_OK;
 }
