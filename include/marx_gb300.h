@@ -288,9 +288,11 @@ const char *mx_last_error(const mx_context *ctx);  /* ctx may be NULL */
  *
  * The calls of one context (made from one thread at a time) may come on
  * different streams: those that use the same buffers of the context, the
- * survivor queues here and the frame scan of mx_event_coords, take turns on the
- * GPU.  A call captured into a CUDA graph is not part of that order: let its
- * replays overlap no other work of the context. */
+ * survivor queues here, the frame scan of mx_event_coords and the spectrum or
+ * image table of mx_generate_source, take turns on the GPU (a source with such
+ * a table also waits, on the host, for the one before it).  A call captured
+ * into a CUDA graph is not part of that order: let its replays overlap no
+ * other work of the context. */
 int mx_trace(mx_context *ctx, const mx_photons *ph, uint32_t stages,
              const mx_variates *var, uint64_t seed, void *stream);
 

@@ -801,20 +801,35 @@ int mx_generate_source(mx_context *c, const mx_source *s, uint32_t first_tag, ui
   std::vector<double> spec;
   std::string err;
   if (!source_dev(*s, S, spec, err)) return mx_fail(c, MX_EINVAL, "mx_generate_source: " + err);
-  const double *dspec = nullptr;
-  if (!spec.empty()) {
-    cudaError_t e = c->spec.ensure(spec.size() * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemcpy(c->spec.ptr, spec.data(), spec.size() * sizeof(double), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return mx_cuda_fail(c, e, "mx_generate_source: uploading the spectrum");
-    dspec = (const double *) c->spec.ptr;
-  }
   int grid = std::max(1, std::min((int) ((d->n + 255) / 256), c->num_sms * 8));
   uint32_t stride = d->stride ? d->stride : d->n;
   if (stride < d->n) return mx_fail(c, MX_EINVAL, "mx_generate_source: stride below n");
-  mx_generate_kernel<<<grid, 256, 0, (cudaStream_t) stream>>>(S, source_fine(S), dspec, first_tag, seed, d->energy, d->p,
-                                                              d->arrival_time, d->flags, d->tag, d->n, stride);
+  cudaStream_t st = (cudaStream_t) stream;
+  const double *dspec = nullptr;
+  if (!spec.empty()) {
+    // one table for all of the context's sources: the upload follows the last
+    // source's photons, on whatever stream they were drawn, and is ordered on
+    // this one; its host copy stays until it has been read.  While the stream
+    // is captured the upload happens at once, where the capture allows it.
+    const bool captured = BufTurn::captured(st);
+    cudaError_t e = cudaSuccess;
+    if (!captured && c->spec_turn.last) e = cudaEventSynchronize(c->spec_turn.last);
+    const size_t bytes = spec.size() * sizeof(double);
+    if (e == cudaSuccess) e = c->spec.ensure(bytes);
+    if (e == cudaSuccess && captured) e = cudaMemcpy(c->spec.ptr, spec.data(), bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !captured) {
+      c->spec_host.swap(spec);
+      e = cudaMemcpyAsync(c->spec.ptr, c->spec_host.data(), bytes, cudaMemcpyHostToDevice, st);
+    }
+    if (e != cudaSuccess) return mx_cuda_fail(c, e, "mx_generate_source: uploading the spectrum");
+    dspec = (const double *) c->spec.ptr;
+  }
+  mx_generate_kernel<<<grid, 256, 0, st>>>(S, source_fine(S), dspec, first_tag, seed, d->energy, d->p,
+                                           d->arrival_time, d->flags, d->tag, d->n, stride);
   c->launches++;
   cudaError_t e = cudaGetLastError();
+  const cudaError_t turn = dspec ? c->spec_turn.after(st) : cudaSuccess;
+  if (e == cudaSuccess) e = turn;
   return e == cudaSuccess ? MX_OK : mx_cuda_fail(c, e, "launching photon generation");
 }
 

@@ -228,6 +228,8 @@ void mx_destroy(mx_context *c) {
   c->ev_tab.release();
   c->ev_scan.release();
   c->ev_io.release();
+  if (c->spec_turn.last) cudaEventSynchronize(c->spec_turn.last);   // the upload reads spec_host
+  c->spec_turn.release();
   c->wave_turn.release();
   c->ev_turn.release();
   for (int k = 0; k < MX_PIPE_STREAMS; k++) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/marx_gb300.h"
 #include "mx_host.h"
@@ -67,7 +68,9 @@ struct mx_context {
   DevBuf scan;             // compaction block counts
   DevBuf wave;             // wavefront record queues
   BufTurn wave_turn;
-  DevBuf spec;             // FILE spectrum of the last mx_generate_source call
+  DevBuf spec;             // FILE spectrum or IMAGE table of the last mx_generate_source call,
+  std::vector<double> spec_host;   // the copy it is uploaded from
+  BufTurn spec_turn;
   int wave_blocks[5] = {};     // resident blocks per SM of the wavefront kernels a, t, b, c, d
   int mode = MX_MODE_AUTO;
   unsigned long long *d_overrun = nullptr;

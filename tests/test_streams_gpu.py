@@ -1,6 +1,6 @@
 """Calls of one context on several streams: they share the context's survivor
-queues and its frame scan, and give what the same calls give with a wait after
-each.  No tolerance: every column is
+queues, its frame scan and its table of the source's spectrum, and give what
+the same calls give with a wait after each.  No tolerance: every column is
 equal."""
 import numpy as np
 import pytest
@@ -35,6 +35,40 @@ def test_traces_take_turns_at_the_queues(cuda, streams):
         out.append(d)
     for a, b in zip(*out):
         for c in COLUMNS:
+            assert torch.equal(getattr(a, c), getattr(b, c)), c
+
+
+@pytest.mark.parametrize("streams", [1, 2])
+@pytest.mark.parametrize("kind", ["spectrum", "image"])
+def test_sources_take_turns_at_the_table(cuda, kind, streams):
+    """Tables of one length, then a longer one: each source draws from its own."""
+    import torch
+    from marx_gb300 import batched as B
+    from marx_gb300._native import DevicePhotons, Engine
+    eng = Engine(B.batched_config())
+    n, p, r = 3_000_000, np.array([-1.0, 0.0, 0.0]), np.random.default_rng(4)
+    sources = []
+    for k in range(5):
+        m = 300 if k < 4 else 3000
+        if kind == "spectrum":
+            spec = (np.linspace(0.3 + 0.1 * k, 2.0 + k, m), r.random(m))
+            sources.append(B.make_source(p, "POINT", (), spectrum=spec, num_photons=n))
+        else:
+            sources.append(B.make_source(p, "IMAGE", (1e-4, 1e-4), image=r.random((10, m // 10)).astype(np.float32),
+                                         num_photons=n))
+    side = [torch.cuda.Stream() for _ in range(streams)]
+    out = []
+    for apart in (True, False):
+        d = [DevicePhotons(n) for _ in sources]
+        _wait()
+        for k, (s, q) in enumerate(zip(sources, d)):
+            B.generate_source(eng, s, 0, k, q, stream=side[k % streams])
+            if apart:
+                _wait()
+        _wait()
+        out.append(d)
+    for a, b in zip(*out):
+        for c in ("energy", "p"):
             assert torch.equal(getattr(a, c), getattr(b, c)), c
 
 
