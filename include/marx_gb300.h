@@ -768,7 +768,8 @@ int mx_probe_fp64(double *tflops, double *ms);
  *   fn 9  y = x split into two floats and joined again (within 2^-46)
  *   fn 10 y[2i], y[2i+1] = sin, cos(2 pi x - pi/4), 0 <= x < 1 (within 2^-45)
  *   fn 11 x is a table's abscissae (floats); y: how many of six values at and
- *         after x the table's index places otherwise than a bisection (0)
+ *         after x the table's index places otherwise than a bisection, or
+ *         after more loads (0)
  *   fn 12 y = exp(x) - 1, 0 <= x < 80, in double-float (within 2^-42)
  * Synchronises the device.  MX_EINVAL for an unknown fn or null pointers. */
 int mx_math_check(int fn, const double *x, double *y, size_t n);

@@ -736,7 +736,8 @@ MXD unsigned bsearch_d(double x, const double *xp, unsigned n) {  // JDMbinary_s
 }
 // The first of a table's abscissae that is not below x, from its index table;
 // 0 where that does not apply (x not inside the table, no index table).
-// Three dependent loads or so where the bisection takes 8 (an effective-area
+// Three or four dependent loads on average over the calibration's tables, and
+// never more than a bisection's (find_table), which are 8 (an effective-area
 // correction) to 16 (a detector's efficiency).
 MXD unsigned find_first(const MxFindDev &f, const uint16_t *first, float x, const float *xp) {
 #ifdef __CUDA_ARCH__

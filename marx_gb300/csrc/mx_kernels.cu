@@ -696,14 +696,20 @@ __global__ void __launch_bounds__(256) mx_math_kernel(int fn, const double *x, d
 
 // fn 11: how many of xp[i], the floats next to it and the points a quarter and
 // a half on the way to xp[i + 1] the index table places otherwise than the
-// bisection does.
+// bisection does, or after more loads than its log2(n).
 __global__ void mx_find_check(MxFindDev f, const uint16_t *first, const float *xp, unsigned n, double *y) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float a = xp[i], b = i + 1 < n ? xp[i + 1] : 2.0f * a;
   const float v[6] = {a, nextafterf(a, 3e38f), nextafterf(a, -3e38f), a + 0.25f * (b - a), a + 0.5f * (b - a), -a};
   int bad = 0;
-  for (int k = 0; k < 6; k++) bad += mx::locate_f(f, first, v[k], xp, n) != mx::bsearch_f(v[k], xp, n);
+  for (int k = 0; k < 6; k++) {
+    bad += mx::locate_f(f, first, v[k], xp, n) != mx::bsearch_f(v[k], xp, n);
+    if (f.shift && v[k] > f.lo && v[k] < f.hi) {
+      const unsigned from = first[f.off + ((__float_as_uint(v[k]) >> f.shift) - (__float_as_uint(f.lo) >> f.shift))];
+      bad += (mx::find_first(f, first, v[k], xp) - from) + 2u > 32u - (unsigned) __clz((int) (n - 1));
+    }
+  }
   y[i] = (double) bad;
 }
 static cudaError_t find_check(const double *x, double *y, size_t n) {

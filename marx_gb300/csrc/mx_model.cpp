@@ -115,9 +115,13 @@ static void hi_lo(double d, float f[2]) {
   f[1] = (float) (d - (double) f[0]);
 }
 
-// The index table of abscissae x (MxFindDev), one to two entries for each;
-// none for abscissae that are not positive, finite and in order, or that do
-// not fit 16-bit indices.
+// The index table of abscissae x (MxFindDev): the coarsest from two entries
+// per abscissa down that a lookup never loads more of than a bisection would,
+// that is an entry and the abscissae of the fullest cell and the one past
+// them, within log2(n).  A table crowded somewhere (the LETG's 324 energies
+// put 22 in one cell at two entries each) takes a finer one, up to eight
+// entries per abscissa; none for one that would need more, for abscissae that
+// are not positive, finite and in order, or that do not fit 16-bit indices.
 MxFindDev find_table(std::vector<uint16_t> &first, const float *x, size_t n) {
   MxFindDev f;
   memset(&f, 0, sizeof(f));
@@ -128,12 +132,24 @@ MxFindDev find_table(std::vector<uint16_t> &first, const float *x, size_t n) {
   }
   auto bits = [](float v) { uint32_t u; memcpy(&u, &v, 4); return u; };
   const uint32_t b0 = bits(x[0]), b1 = bits(x[n - 1]);
-  unsigned s = 1;
-  while ((b1 >> s) - (b0 >> s) + 1 > 2 * n) s++;
+  auto entries = [&](unsigned s) { return (size_t) ((b1 >> s) - (b0 >> s) + 1); };
+  auto fullest = [&](unsigned s) {
+    size_t most = 0, here = 0;
+    for (size_t k = 0; k < n; k++) {
+      here = k && bits(x[k]) >> s == bits(x[k - 1]) >> s ? here + 1 : 1;
+      most = std::max(most, here);
+    }
+    return most;
+  };
+  unsigned s = 1, steps = 0;
+  while (entries(s) > 2 * n) s++;
+  while ((n - 1) >> steps) steps++;
+  while (s && fullest(s) + 2 > steps) s = s > 1 && entries(s - 1) <= 8 * n ? s - 1 : 0;
+  if (!s) return f;
   f.lo = x[0]; f.hi = x[n - 1];
   f.off = (int32_t) first.size();
   f.shift = (uint16_t) s;
-  first.resize(first.size() + (b1 >> s) - (b0 >> s) + 1);
+  first.resize(first.size() + entries(s));
   uint16_t *at = first.data() + f.off;
   uint32_t b = b0 >> s;
   for (size_t k = 0; k < n; k++)
