@@ -514,6 +514,9 @@ static bool build_fef(const Pack &pk, int min_ccd, int max_ccd, HostModel &M, st
         M.fef_f.push_back(g[1]);                                   // center
         M.fef_f.push_back((float) (FWHM_TO_SIGMA * g[0]));         // sigma
       }
+    // the response interpolates between two energies (one alone makes the
+    // reference read ahead of its table)
+    if (f.n_e < 2) { err = "Expecting an FEF region to have more than one energy"; return false; }
     // check_fef_validity: energies and channels increasing
     const float *e = M.fef_f.data() + f.e_off, *ch = e + f.n_e;
     for (int k = 0; k + 1 < f.n_e; k++)
