@@ -333,7 +333,7 @@ def bench_diff(a, fp64_peak):
                          "algorithmic_flops_per_ray": flops_per_ray,
                          "forward": {"achieved": fwd_tf, "frac": fwd_tf / fp64_peak},
                          "adjoint": {"achieved": adj_tf, "frac": adj_tf / fp64_peak,
-                                     "note": "FP64 values only; the six FP32 tangents per value are not counted"}},
+                                     "note": "FP64 values only; the four FP32 tangents per value are not counted"}},
             }
 
 

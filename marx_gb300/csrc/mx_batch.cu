@@ -318,7 +318,7 @@ struct TileRounds {
 // phase warps claim tiles of work from a counter, so uneven sources and
 // uneven survivor counts spread over every SM.  Every thread reaches every
 // barrier: the claim loops end for a whole warp at once and nothing
-// returns early.  Two resident blocks of 256 threads per SM (122 registers):
+// returns early.  Two resident blocks of 256 threads per SM (119 registers):
 // three (80 registers, 900 bytes of spilled loads) take 8.81 ms instead of
 // 8.91 for 3.7e7 photons, but 183 us instead of 162 for 2e5.  The far-scattered
 // photons kept for later and tiles that follow the queue's length: 256 sources

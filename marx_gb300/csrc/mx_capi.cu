@@ -327,9 +327,10 @@ static int pipe_streams(mx_context *c) {
 // saves four or five launches and the queues.  97 000 photons fused / in
 // queues: on axis 60 / 75 us, plain_scatter 80 / 106, HETG 107 / 125, LETG 120
 // / 137, HRC-I 105 / 117, LETG with HRC-S 160 / 160; 120 000: 71 / 79, 116 /
-// 113, 165 / 138, 184 / 148, 171 / 137, 263 / 169.  Both give the same results
-// bit for bit.
-static bool takes_wavefront(const mx_context *c, const MxTables &T, uint32_t n, uint32_t stages) {
+// 113, 165 / 138, 184 / 148, 171 / 137, 263 / 169 (on axis the line could lie
+// higher).  Both give the same results bit for bit.  The chunks of a pipelined
+// host list take the queues at any length.
+static bool takes_wavefront(const mx_context *c, uint32_t n, uint32_t stages) {
   if (!(stages & MX_STAGE_MIRROR) || c->mode == MX_MODE_FUSED) return false;
   if (c->mode == MX_MODE_WAVEFRONT) return true;
   const uint32_t resident = (uint32_t) (c->num_sms * c->trace_blocks[1]) * MX_TRACE_BLOCK;
@@ -345,7 +346,7 @@ static bool takes_wavefront(const mx_context *c, const MxTables &T, uint32_t n, 
 // its first photon's index), so the results equal the one-pass trace's.
 int mx_trace_tables(mx_context *c, const MxTables &T, const mx_photons *ph, uint32_t stages, const double *U,
                     const double *N, uint64_t seed, cudaStream_t st, bool fresh) {
-  if (!ph || !takes_wavefront(c, T, ph->n, stages) || U || N || ph->n < MX_SPLIT_MIN_PHOTONS)
+  if (!ph || !takes_wavefront(c, ph->n, stages) || U || N || ph->n < MX_SPLIT_MIN_PHOTONS)
     return mx_trace_queues(c, T, ph, stages, U, N, seed, st, fresh, c->wave);
   TraceIO io;   // the argument checks, before anything is queued
   int r = mx_trace_io(c, T, ph, stages, U, N, seed, fresh, io, "mx_trace");
@@ -404,7 +405,7 @@ int mx_trace_queues(mx_context *c, const MxTables &T, const mx_photons *ph, uint
   io.tag0 = tag0;
   int slots = U != nullptr;
   cudaError_t e;
-  if ((stages & MX_STAGE_MIRROR) && c->mode != MX_MODE_FUSED && (force_wave || takes_wavefront(c, T, ph->n, stages))) {
+  if ((stages & MX_STAGE_MIRROR) && c->mode != MX_MODE_FUSED && (force_wave || takes_wavefront(c, ph->n, stages))) {
     size_t qbytes = (size_t) ph->n * sizeof(MxRec);
     e = queues.ensure(2 * qbytes + 256);
     if (e != cudaSuccess) return cuda_fail(c, e, "allocating wavefront queues");

@@ -1,14 +1,17 @@
 // Per-photon trace stages for the GB300 kernels.
 //
 // Each stage follows the reference function it replaces (paths inside MARX
-// 5.5.3, cited per function) in FP64 for geometry and FP32 where the
-// reference keeps float tables.  Unlike the oracle it is written for the
-// GPU's scarce FP64 pipe: one reciprocal square root instead of a scaled
-// hypot plus three divisions per normalisation, sincos pairs, precomputed
-// per-shell sines and cosines, and |a/b|^2 = |a|^2/|b|^2 in the Fresnel
-// reflectivity.  These change results only at the last-bit level; every
-// comparison that decides a photon's fate (shell, reflectivity, order,
-// chip) uses the same quantities and order as the reference.
+// 5.5.3, cited per function): positions, directions and their sums in FP64,
+// FP32 where the reference keeps float tables.  Unlike the oracle it is
+// written for the GPU's scarce FP64 pipe: what changes a direction by little
+// (blur, scattering, dither, a small source's extent) and the Fresnel
+// reflectivity are double-floats, two floats of 44 to 48 bits together;
+// angles are reduced on the integer pipe; roots and intersections start from
+// floats; float screens pass the certain cases of a test.  Positions stay
+// within 1e-9 mm and directions within 1e-12 of the reference's, and a
+// comparison that decides a photon's fate (shell, reflectivity, order, chip)
+// goes to the double form wherever the cheaper value is not clear of the
+// threshold.
 #pragma once
 #include <stdint.h>
 #include "mx_model.h"
@@ -180,24 +183,6 @@ MXD void sincos_small(double x, double *s, double *c) {
     *c = 1.0 + x2 * (-0.5 + x2 * (1.0 / 24.0 + x2 * (-1.0 / 720.0 + x2 * (1.0 / 40320.0))));
   } else
     mx_sincos(x, s, c);
-}
-// sin(pi y), cos(pi y): the argument needs no reduction by pi.
-MXD void mx_sincospi(double y, double *s, double *c) {
-#ifdef __CUDA_ARCH__
-  sincospi(y, s, c);
-#else
-  *s = std::sin(PI * y); *c = std::cos(PI * y);
-#endif
-}
-MXD D3 rotate_unit_angle(D3 p, D3 n, double theta) {
-  double s, c;
-  mx_sincos(theta, &s, &c);
-  return rotate_unit(p, n, c, s);
-}
-MXD D3 rotate_unit_small(D3 p, D3 n, double theta) {
-  double s, c;
-  sincos_small(theta, &s, &c);
-  return rotate_unit(p, n, c, s);
 }
 MXD D3 mat_mul(const double *m, D3 v) {  // JDM3m_vector_mul (rotate.c:121), row-major 3x3
   return mk(m[0] * v.x + m[1] * v.y + m[2] * v.z, m[3] * v.x + m[4] * v.y + m[5] * v.z,
@@ -1804,13 +1789,9 @@ MXD void dither_stage(const MxTables &T, Ph &ph, Rng &rng) {
 // ------------------------------------------------------------ grating --
 MXD D3 rot_x(D3 a, double c, double s) { return mk(a.x, c * a.y - s * a.z, s * a.y + c * a.z); }
 
-// a l + b d + c n with a fixed order of fused multiply-adds, so that every
-// kernel that inlines it rounds it alike (left to the compiler, the
-// contraction of a sum of products may differ from one kernel to another).
-MXD D3 comb3(double a, D3 l, double b, D3 d, double c, D3 n) {
-  return mk(fma(a, l.x, fma(b, d.x, MX_DMUL(c, n.x))), fma(a, l.y, fma(b, d.y, MX_DMUL(c, n.y))),
-            fma(a, l.z, fma(b, d.z, MX_DMUL(c, n.z))));
-}
+// The grating's sums of products are written with a fixed order of fused
+// multiply-adds, so that every kernel that inlines them rounds them alike
+// (left to the compiler, the contraction may differ from one to another).
 // intersect + newtons_quartic (diffract.c:622-687): Rowland torus, the root
 // of t^4 + a t^3 + b t^2 + c t + d near -R sqrt(px^2 + pz^2).
 MXD_COLD int newtons_quartic(double a, double b, double c, double d, double t0, double &root) {
@@ -1827,8 +1808,9 @@ MXD_COLD int newtons_quartic(double a, double b, double c, double d, double t0, 
 }
 // The Newton iteration runs in single precision until its step falls below
 // 0.1 mm (a root to about 0.01 mm); two more steps with the quartic's value
-// in double and its derivative in float leave 1e-13 mm: ten FP64 operations
-// where two or three iterations in double take 20 each.
+// in double and its derivative in float, which is off by 6e-5 (5 / R times the
+// last float step), leave 4e-11 mm at worst: ten FP64 operations where two or
+// three iterations in double take 20 each.
 MXD int rowland_intersect(D3 &x0, D3 p, double rowland) {
   double t = -x0.x * rcp_fast(p.x);
   x0 = mk(0.0, fma(p.y, t, x0.y), fma(p.z, t, x0.z));

@@ -365,9 +365,9 @@ __device__ __forceinline__ bool ray_image(const FwdArgs &A, const MxTables &T, i
 // 1e6 rays: 697 -> 315 us.  The warps of a block are at different places of the
 // kernel, so its length counts: with one copy of the code for both optics and
 // for all taps (a third of the issue slots waited for instructions before)
-// 255 us, FP64 pipe 58 % and issue 50 % busy.  Three blocks per SM (72
-// registers); two took 3.38 ms for a gradient step over 4e6 rays where three
-// took 3.05.
+// 255 us, FP64 pipe 58 % and issue 50 % busy.  Three blocks per SM (68
+// registers, 72 with the moments); two took 3.38 ms for a gradient step over
+// 4e6 rays where three took 3.05.
 template <bool SPLAT, bool MOMENTS>
 __global__ void __launch_bounds__(DBLOCK, FWD_BLOCKS) diff_forward_kernel(const __grid_constant__ FwdArgs args, const __grid_constant__ MxTables T,
                                                                uint64_t n, uint64_t seed, uint8_t *codes, int mode,
@@ -933,10 +933,10 @@ mx_diff *mx_diff_create(mx_context *c, const mx_diff_config *cfg) {
   g.half_inv_s2 = (float) (0.5 / (k.sigma * k.sigma));
   g.inv_s2 = (float) (1.0 / (k.sigma * k.sigma));
   g.knorm = (float) (1.0 / (std::sqrt(2.0 * PI_D) * k.sigma));
-  // Each tap product is below w K^2 2^61 with w < 2; a pixel sums at most
-  // n_rays of them, so shifting by log2(n K^2 / 4) + 1 keeps it in 64 bits.
   g.top_u = mx::dkey(g.nx + (double) mxd::HALF);
   g.top_v = mx::dkey(g.ny + (double) mxd::HALF);
+  // Each tap product is below w K^2 2^61 with w < 2; a pixel sums at most
+  // n_rays of them, so shifting by log2(n K^2 / 4) + 1 keeps it in 64 bits.
   const double kmax = g.knorm;
   int shift = (int) std::ceil(std::log2((double) k.n_rays * kmax * kmax / 4.0)) + 1;
   g.shift = shift < 0 ? 0 : shift;

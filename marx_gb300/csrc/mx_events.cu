@@ -134,19 +134,22 @@ __device__ __forceinline__ double rcp_seeded(double d) {
   const double y = df_to(y2);
   return fma(fma(-d, y, 1.0), y, y);
 }
-// sqrt(v), 1 <= v < 4, rounded as sqrt rounds it: the reciprocal root to
-// 2^-44 on the FP32 pipe, then the root g = v y corrected by its exact
-// remainder (v - g^2) y / 2, whose error of 2^-88 leaves nothing but the
-// last rounding.  Four FP64 operations instead of nine.
+// sqrt(v), 1 <= v < 4: the reciprocal root to 2^-44 on the FP32 pipe, then the
+// root g = v y corrected by its exact remainder (v - g^2) y / 2, which is
+// within 2^-88 of the true root before its one rounding: rounded as sqrt
+// rounds it unless the root lies that close to a midpoint of two doubles.
+// Four FP64 operations instead of nine.
 __device__ __forceinline__ double sqrt_seeded(double v) {
   const F2 y2 = df_rsqrt(split(v));
   const double y = df_to(y2), g = v * y;
   return fma(fma(-g, g, v), 0.5 * y, g);
 }
-// JDMv_normalize's value bit for bit: the five quotients by two divisors
-// are Markstein divisions (div_by) from two reciprocals, and the
-// comparisons run on the integer pipe; 36 FP64 operations instead of about
-// 60.  Components far outside the geometry's range take the divisions.
+// JDMv_normalize's value, the bits too but where a reciprocal (within 2^-37 of
+// an ulp) or the root falls on the other side of a midpoint: the five
+// quotients by two divisors are Markstein divisions (div_by) from two
+// reciprocals, and the comparisons run on the integer pipe; 36 FP64
+// operations instead of about 60.  Components far outside the geometry's
+// range take the divisions.
 __device__ __forceinline__ D3 chip_direction(D3 a) {
   double x = fabs(a.x), y = fabs(a.y), z = fabs(a.z), t;
   if (lt_pos(z, x)) { t = z; z = x; x = t; }

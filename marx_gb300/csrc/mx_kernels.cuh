@@ -10,9 +10,9 @@
 // spread them evenly over the SMs (48611 HETG photons 107 us at 256 threads,
 // 97 at 128, 94 at 64, 95 at 32; a thousand photons 58, 55, 56, 56 us).
 #define MX_TRACE_BLOCK 64
+#define MX_FEF_BLOCKS 3   // resident blocks per SM of the ACIS response pass
 // Threads per block of the wavefront kernels, and the resident blocks per SM
 // each is compiled for.
-#define MX_FEF_BLOCKS 3   // resident blocks per SM of the ACIS response pass
 #define MX_WAVE_BLOCK 256
 #define MX_WAVE_A_BLOCKS 3
 #define MX_WAVE_T_BLOCKS 3

@@ -1042,7 +1042,7 @@ bool build_model(const Pack &pk, const mx_config &cfg, HostModel &M, std::string
       }
       g.geff_off = (int32_t) M.geff_energy.size();
       M.geff_energy.insert(M.geff_energy.end(), e, e + ne);
-    g.find = find_table(M.find_first, e, ne);
+      g.find = find_table(M.find_first, e, ne);
       g.cum_off = (int32_t) M.geff_cum.size();
       for (unsigned j = 0; j < ne; j++)
         for (unsigned k = 0; k < no; k++) M.geff_cum.push_back(cum[k * ne + j]);   // [energy][order]
