@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(256, 2) mx_batch_kernel(const __grid_constant_
         Ph q; MirrorState m; Rng r;
         const MxRecA rec_in = ((const MxRecA *) b.q1)[k];
         from_rec_a(rec_in, q, m, r, io);
-        if (mirror_ptest(T, sh, optc, slope, q, r, m)) {
+        if (mirror_ptest(T, sh, optc, slope, q, r, m, T.dither != 0)) {
           keep = true;
           to_rec(rec, q, m, r, r.i);
         } else

@@ -1021,9 +1021,10 @@ __device__ __forceinline__ double rsqrt_seeded(double d) {
 // equation's own terms, as in the closed form.  27 FP64 operations with the
 // normal instead of 56.  1: hit; -1: a certain miss (end values of one sign
 // further from zero than the quadratic can bow between them, see
-// paraboloid_missed); 0, for other rays: not known.  Nothing is written but
-// for a hit.
-__device__ __forceinline__ int conic_newton(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal) {
+// paraboloid_missed); 0, for other rays, and for odd ones, whose p is not of the
+// unit length that the closed form takes it to be (off_unit): not known.
+// Nothing is written but for a hit.
+__device__ __forceinline__ int conic_newton(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal, bool odd = false) {
   const float fx = d2f_trunc(x0.x), fy = d2f_trunc(x0.y), fz = d2f_trunc(x0.z);
   const float px = d2f_trunc(p.x), py = d2f_trunc(p.y), pz = d2f_trunc(p.z);
   const float inv = 1.0f / px, my = py * inv, mz = pz * inv;
@@ -1032,7 +1033,7 @@ __device__ __forceinline__ int conic_newton(const MxShellDev &h, int o, D3 &x0, 
   const float yb = fmaf(len, my, ya), zb = fmaf(len, mz, za);
   const float ra = fmaf(ya, ya, za * za), rb = fmaf(yb, yb, zb * zb);
   const float ga = ra - h.r2limf[o][0], gb = rb - h.r2limf[o][1], rise = gb - ga;
-  const float margin = fmaf(1e-5f, ra + rb, 2.0f);
+  const float margin = odd ? 1e30f : fmaf(1e-5f, ra + rb, 2.0f);
   const float A = fmaf(my, my, fmaf(mz, mz, -am1)) * len * len, B = rise - A;
   if (!(fabsf(ga) > margin && fabsf(gb) > margin && (ga < 0.0f) != (gb < 0.0f) && fabsf(rise) > 1000.0f &&
         fabsf(A) < 0.25f * fabsf(rise))) {
@@ -1060,9 +1061,11 @@ __device__ __forceinline__ int conic_newton(const MxShellDev &h, int o, D3 &x0, 
   return 1;
 }
 #endif
-MXD int conic_intersection(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal) {
+MXD int conic_intersection(const MxShellDev &h, int o, D3 &x0, D3 p, D3 &normal, bool odd) {
 #ifdef __CUDA_ARCH__
-  if (const int r = conic_newton(h, o, x0, p, normal)) return r < 0 ? -1 : 0;
+  if (const int r = conic_newton(h, o, x0, p, normal, odd)) return r < 0 ? -1 : 0;
+#else
+  (void) odd;
 #endif
   return conic_intersection_double(h, o, x0, p, normal);
 }
@@ -1225,12 +1228,13 @@ MXD_COLD double wfold_angle(const MxTables &T, int table, double energy, double 
   return wfold_interp(T, table, energy, sin_alpha, r);
 }
 // JDMv_rotate_unit_vector(p, p x n, dg): with a = p x n, p.a = 0 and
-// a x p = n - (p.n) p for unit p, p becomes cos(dg) p + sin(dg) (n - (p.n) p).
+// a x p = (p.p) n - (p.n) p, p becomes cos(dg) p + sin(dg) ((p.p) n - (p.n) p),
+// made a unit vector.
 MXD_COLD D3 scatter_double(D3 p, D3 n, double dg) {
   double sg, cg;
   sincos_small(dg, &sg, &cg);
-  const double pn = dot(p, n);
-  return normalized_unit(cg * p + sg * (n + (-pn) * p));
+  const double pn = dot(p, n), pp = dot(p, p);
+  return normalized_unit(cg * p + sg * (pp * n + (-pn) * p));
 }
 #ifdef __CUDACC__
 // fold_theta in double-float for a probability p 2^-64 inside the table; tail
@@ -1284,9 +1288,10 @@ __device__ __forceinline__ void df_small_turn(F2 a, F2 &s, F2 &v) {
 #endif
 // late: whether a photon scattered into the far tail may be left for later
 // (2 is returned then, with p and the draws as they were): the wavefront
-// gathers these few and turns them on full warps.
+// gathers these few and turns them on full warps.  odd: p is not of unit
+// length; the double form makes it so.
 MXD int reflect_finish(const MxTables &T, const MxShellDev &h, int o, int table, D3 &p, D3 n, double pdn,
-                       double energy, Rng &rng, bool late = false) {
+                       double energy, Rng &rng, bool odd, bool late) {
   const D3 q = p + (-2.0 * pdn) * n;
   if (!T.use_wfold) { p = q; return 0; }
   const int upos = rng.upos;
@@ -1295,7 +1300,7 @@ MXD int reflect_finish(const MxTables &T, const MxShellDev &h, int o, int table,
   // makes to p, -(1 - cos dg) p + sin dg (n - (p.n) p) with p.n = -pdn, in
   // double-float, and added to p: three FP64 operations instead of 25, and
   // none in the tables instead of 20.
-  bool tail = false;
+  bool tail = odd;
   const F2 pd = split(pdn);
   const F2 a = df_mul(wfold_df(T, table, split(energy), df_neg(pd), rng.uniform_fixed(), tail),
                       F2{h.scatf[o][0], h.scatf[o][1]});
@@ -1321,7 +1326,7 @@ MXD int reflect_finish(const MxTables &T, const MxShellDev &h, int o, int table,
   rng.upos = upos;
   if (late) return 2;
 #else
-  (void) upos; (void) late;
+  (void) upos; (void) odd; (void) late;
 #endif
   p = q;
   double dg = wfold_angle(T, table, energy, -pdn, rng.uniform()) * h.scat[o];
@@ -1415,6 +1420,8 @@ MXD bool cap_struts_block(const MxTables &T, const MxShellDev &h, D3 x, D3 p) {
 // the photon at a conic intersection (OSAC frame of that optic) that passed
 // that optic's reflectivity test, its incoming direction, the blurred
 // normal there and p.n, and the optical constants at the photon's energy.
+// After part 2 the correction factor's sign is turned for a photon whose p is
+// not of unit length (off_unit).
 struct MirrorState {
   D3 x, p, n;
   double pdn;
@@ -1429,7 +1436,9 @@ struct MirrorState {
 // within |curvature| L^2 / 4 of the chord between its end values, so that
 // end values of one sign further than that from zero leave no root inside.
 // The float evaluation of G is good to about 0.2 mm^2 (positions of 700 mm)
-// or 1e-6 of the squares; the margin is ten times that.  Rays it does not
+// or 1e-6 of the squares; the margin is ten times that, and 8 mm^2 for what a
+// direction widened from single precision moves the closed form's squares
+// (off_unit; 6e-8 of the squared distance to the plane x = 0).  Rays it does not
 // rule out, NaN among them, take the double-precision intersection, which
 // alone decides a hit.
 MXD bool paraboloid_missed(const MxShellDev &h, float x0, float y0, float z0, float px, float py, float pz) {
@@ -1440,9 +1449,34 @@ MXD bool paraboloid_missed(const MxShellDev &h, float x0, float y0, float z0, fl
   const float ra = ya * ya + za * za, rb = yb * yb + zb * zb;
   const float ga = ra - h.r2limf[0][0], gb = rb - h.r2limf[0][1];
   const float bow = fabsf(my * my + mz * mz - h.am1f[0]) * h.quarter_l2f;
-  const float margin = 2.0f + 1e-5f * (ra + rb) + bow;
+  const float margin = 10.0f + 1e-5f * (ra + rb) + bow;
   return (ga > margin && gb > margin) || (ga < -margin && gb < -margin);
 }
+
+// Directions that are not of unit length.  The reference's closed form of an
+// intersection takes them for it, the Newton form does not: for a direction
+// widened from single precision, 3e-8 off, it would put the photon 4e-5 mm
+// elsewhere on the detector.  Such photons keep to the closed form until the
+// reference makes the direction a unit vector: with the dither, or with the
+// scattering at the paraboloid.
+//
+// Whether p's length is off 1 by more than the square of it is known to here:
+// 2^-22 of y^2 + z^2 from their truncation to floats, 2^-23 from the
+// roundings; x enters with its low part.  Directions off by less (1e-12, and
+// 5e-7 of the squared off-axis angle) move a photon by less than 1e-8 mm up to
+// 15 arcmin off axis.  The test and its consequences cost 0.7 % of
+// plain_scatter (1e7 photons 3158 -> 3180 us); in double, in phase A or with
+// the photon marked in a record's flags they cost 1 to 2 %.
+MXD bool off_unit(D3 p) {
+#ifdef __CUDA_ARCH__
+  const float x = d2f_trunc(p.x), y = d2f_trunc(p.y), z = d2f_trunc(p.z), t = fmaf(y, y, z * z);
+  const float e = fmaf(2.0f * x, split(p.x).l, fmaf(x, x, -1.0f)) + t;
+  return !(fabsf(e) <= fmaf(t, 0x1p-21f, 1e-12f));
+#else
+  return !(fabs(dot(p, p) - 1.0) <= 1e-12);
+#endif
+}
+MXD_COLD D3 normalized_cold(D3 p) { return normalized(p); }
 
 // _marx_hrma_mirror_reflect per photon (hrma.c:1183-1339), part 1:
 // vignetting, project_photon_to_hrma (hrma.c:984-1050), transform into the
@@ -1537,9 +1571,9 @@ MXD bool mirror_front(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &
 
 // Part 2: optical constants, paraboloid intersection, normal blur and
 // reflectivity test there.  Returns false if the photon misses the
-// paraboloid or is absorbed.
+// paraboloid or is absorbed.  dithered: the dither turned the direction.
 MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
-                      Rng &rng, MirrorState &m) {
+                      Rng &rng, MirrorState &m, bool dithered) {
   const MxShellDev &h = shells[ph.shell];
   m.beta = 0.0f; m.delta = 1.0f; m.corr = F2{1.0f, 0.0f};
   if (T.opt_n) {
@@ -1550,10 +1584,16 @@ MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *
       m.corr = sqrt_of_float(interp_f(h.corr_find, T.find_first, fe, ce, ce + h.corr_n, slope + h.corr_slope_off, h.corr_n));
     }
   }
-  if (-1 == conic_intersection(h, 0, m.x, m.p, m.n) ||
+  bool odd = off_unit(m.p);
+  if (odd && dithered) {
+    m.p = normalized_cold(m.p);
+    odd = false;
+  }
+  if (-1 == conic_intersection(h, 0, m.x, m.p, m.n, odd) ||
       !reflect_test(T, h, 0, m.p, m.n, m.pdn, m.beta, m.delta, m.corr, rng)) {
     ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = m.x; ph.p = m.p; return false;
   }
+  if (odd) m.corr = F2{-m.corr.h, -m.corr.l};
   return true;
 }
 
@@ -1564,7 +1604,7 @@ MXD bool mirror_ptest(const MxTables &T, const MxShellDev *shells, const float *
 MXD int mirror_middle(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m, bool late = false) {
   const MxShellDev &h = shells[ph.shell];
   D3 x = m.x, p = m.p;
-  if (const int r = reflect_finish(T, h, 0, 2 * ph.shell, p, m.n, m.pdn, ph.e, rng, late)) {
+  if (const int r = reflect_finish(T, h, 0, 2 * ph.shell, p, m.n, m.pdn, ph.e, rng, m.corr.h < 0.0f, late)) {
     if (r == 2) return 2;
     ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0;
   }
@@ -1583,7 +1623,10 @@ MXD int mirror_middle(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &
            fma(M[6], x.x, fma(M[7], x.y, fma(M[8], x.z, c[2]))));
   }
   D3 n;
-  if (-1 == conic_intersection(h, 1, x, p, n)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0; }
+  const bool odd = m.corr.h < 0.0f;
+  if (odd) m.corr = F2{-m.corr.h, -m.corr.l};
+  // (the scattering, if there is any, has made p a unit vector)
+  if (-1 == conic_intersection(h, 1, x, p, n, odd && !T.use_wfold)) { ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0; }
   if (!reflect_test(T, h, 1, p, n, m.pdn, m.beta, m.delta, m.corr, rng)) {
     ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return 0;
   }
@@ -1597,7 +1640,7 @@ MXD int mirror_middle(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &
 MXD bool mirror_back(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &rng, MirrorState &m, bool late = false) {
   const MxShellDev &h = shells[ph.shell];
   D3 x = m.x, p = m.p;
-  if (const int r = reflect_finish(T, h, 1, 2 * ph.shell + 1, p, m.n, m.pdn, ph.e, rng, late)) {
+  if (const int r = reflect_finish(T, h, 1, 2 * ph.shell + 1, p, m.n, m.pdn, ph.e, rng, false, late)) {
     if (r == 2) return false;
     ph.flags |= MX_PHOTON_UNREFLECTED; ph.x = x; ph.p = p; return true;
   }
@@ -1610,9 +1653,9 @@ MXD bool mirror_back(const MxTables &T, const MxShellDev *shells, Ph &ph, Rng &r
 }
 
 MXD void mirror_stage(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope, Ph &ph,
-                      Rng &rng) {
+                      Rng &rng, bool dithered) {
   MirrorState m;
-  if (mirror_front(T, shells, ph, rng, m) && mirror_ptest(T, shells, optc, slope, ph, rng, m) &&
+  if (mirror_front(T, shells, ph, rng, m) && mirror_ptest(T, shells, optc, slope, ph, rng, m, dithered) &&
       mirror_middle(T, shells, ph, rng, m))
     mirror_back(T, shells, ph, rng, m);
 }
@@ -2772,8 +2815,10 @@ MXD void any_detect_stage(const MxTables &T, const MxChipDev *chips, int nchips,
 // whose stage ran out of pre-drawn variates is not traced further.
 MXD void trace_photon(const MxTables &T, const MxShellDev *shells, const float *optc, const double *slope,
                       const MxGratingDev *grs, const MxChipDev *chips, uint32_t stages, Ph &ph, Rng &rng) {
-  if ((stages & MX_STAGE_DITHER) && T.dither) dither_stage(T, ph, rng);
-  if ((stages & MX_STAGE_MIRROR) && !(ph.flags & MX_BAD_PHOTON_MASK)) mirror_stage(T, shells, optc, slope, ph, rng);
+  const bool dithered = (stages & MX_STAGE_DITHER) && T.dither;
+  if (dithered) dither_stage(T, ph, rng);
+  if ((stages & MX_STAGE_MIRROR) && !(ph.flags & MX_BAD_PHOTON_MASK))
+    mirror_stage(T, shells, optc, slope, ph, rng, dithered);
   if (rng.overrun) return;
   if ((stages & MX_STAGE_GRATING) && T.grating && !(ph.flags & MX_BAD_PHOTON_MASK))
     grating_stage(T, grs, T.grating, ph, rng);

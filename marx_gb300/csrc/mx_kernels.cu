@@ -403,7 +403,7 @@ mx_wave_t(const __grid_constant__ MxTables T, const __grid_constant__ TraceIO io
   Rounds rounds(late, *(volatile const unsigned int *) &w.counts[0]);
   rounds.late = false;
   wave_pass(io, (const MxRecA *) w.q1, rounds, w.q2, &w.counts[1],
-            [&](Ph &q, Rng &r, MirrorState &m, bool) { return (int) mirror_ptest(T, sh, optc, slope, q, r, m); });
+            [&](Ph &q, Rng &r, MirrorState &m, bool) { return (int) mirror_ptest(T, sh, optc, slope, q, r, m, (io.stages & MX_STAGE_DITHER) && T.dither); });
 }
 
 __global__ void __launch_bounds__(MX_WAVE_BLOCK, MX_WAVE_B_BLOCKS)
