@@ -267,9 +267,10 @@ __device__ __forceinline__ void roll_sincos(float roll, F2 &s, F2 &c) {
 // rolled unit vector.  They are formed in double-float on the FP32 pipe
 // (relative error of an offset below 2^-43, within 1e-10 pixel), 4 FP64
 // operations in place of about 480.  The acos form's own rounding moves an
-// event at angle t by up to 2e-16 / t: 1e-9 of the coordinate at SKY_NEAR,
-// so that from there out the two agree; nearer the axes of the pointing (1 %
-// of a field's events) sky_reference keeps the reference's rounding.
+// event at angle t by up to 3e-16 / t, 2.5e-9 of the coordinate (1e-5 pixel) at
+// SKY_NEAR and less from there out, which these values are free of; nearer the
+// axes of the pointing (1 % of a field's events) sky_reference keeps the
+// reference's rounding.
 // False, with nothing written, also when the event is not within 0.03 rad
 // of the pointing or its dither not below 1e-4 rad.
 constexpr float SKY_NEAR = 1.2e-5f;

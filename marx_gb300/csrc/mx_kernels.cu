@@ -235,11 +235,11 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 //   C 116 116 116  81      89  89  88  79
 // 1e7 photons 5.76 5.37 4.70 3.83 ms; 1e6 on axis 416 368 340 284 us.  With
 // the far-scattered photons gathered, leaner double-float steps and index
-// tables for the lookups: A 87, T 79, B 110, C 66 us, 1e7 photons 3.16 ms, 1e6
+// tables for the lookups: A 90, T 78, B 113, C 66 us, 1e7 photons 3.18 ms, 1e6
 // on axis 263 us.  A is bound by the issue of FP32 and integer instructions
-// (61 %), C by the FP64 pipe (59 %), T and B by latency (FP64 55 and 57 %,
-// issue 41 and 32 %; B also waits for instructions), which is why A, T and B
-// are compiled for three resident blocks (80 registers, 100 bytes of spills in
+// (61 %), C by the FP64 pipe (59 %), T and B by latency (FP64 55 and 56 %,
+// issue 42 and 32 %; B also waits for instructions), which is why A, T and B
+// are compiled for three resident blocks (80 registers, 130 bytes of spills in
 // B) and gain 8-11 % over two, while C loses 6 % and D is not bound by either;
 // a fourth block changes none of them by more than 1.5 %.
 // With a grating: the Rowland torus from a float iteration and two steps on
@@ -248,7 +248,7 @@ cudaError_t launch_acis_fef(const MxTables &T, const TraceIO &io, int grid, cuda
 // supports, whose direction stays in its components: per 1e6 photons C
 // 114 -> 95 us (HETG) and D 219 -> 190 us (LETG and HRC-S, 3.4e6 -> 2.0e6
 // FP64 instructions), and 84 us with the HRC's plates, pulse height and blur
-// off the FP64 pipe; HETG 2e7 7.73 -> 6.92 ms, LETG + HRC-S 4e6 2.35 -> 1.62.
+// off the FP64 pipe; HETG 2e7 7.73 -> 6.98 ms, LETG + HRC-S 4e6 2.35 -> 1.63.
 
 // A phase's blocks start as those of the phase before it end, stage their
 // tables meanwhile and read its queues when all of it has completed
